@@ -145,6 +145,8 @@ struct Workspace {
 };
 struct MixedOperator;  // tensor-core form (kinship_mixed.cu)
 void destroy_mixed(MixedOperator* m);
+struct SliceOperator;  // FP64 on the tensor cores (kinship_slices.cu)
+void destroy_slices(SliceOperator* s);
 }  // namespace cs
 
 // Kinship operator over a (keep, variants) selection of a cs_genotypes matrix.
@@ -169,13 +171,18 @@ struct cs_kinship {
     cs::Workspace ws;
     cs::DeviceBuffer<double> buf_x, buf_u, buf_y;
     cs::MixedOperator* mixed = nullptr;
+    cs::SliceOperator* slices = nullptr;
+    bool slices_unavailable = false;  // no device memory for them: FP64-pipe kernels only
     bool autotune = true;  // the tensor-core passes may tune their plan on new shapes
     // the samples pass may keep a sample-major copy of the packed view (one more packed matrix
     // in HBM) and read its A operand from tensor memory (six operand sets at the widths where
     // that is the default); otherwise A stays in shared memory and every samples pass runs the
     // five-set form, so a column's result does not depend on how many columns share its apply
     bool sample_major_copy = true;
-    ~cs_kinship() { cs::destroy_mixed(mixed); }
+    ~cs_kinship() {
+        cs::destroy_slices(slices);
+        cs::destroy_mixed(mixed);
+    }
 };
 
 namespace cs {
@@ -195,6 +202,10 @@ void mixed_multiply_zt(cs_kinship* op, const double* X, int64_t ldx, int64_t k, 
                        int64_t ldu, cudaStream_t s);
 void mixed_multiply_z(cs_kinship* op, const double* Wcol, int64_t k, double* Y, int64_t ldy,
                       cudaStream_t s);
+
+// Waits for the stream and fails if the operator's last FP64 tensor-core pass gave up waiting (its
+// results are NaN; kinship_slices.cu).
+void check_slices(cs_kinship* op, cudaStream_t s);
 
 // The reference's Gaussian test matrix (std::normal_distribution over std::mt19937_64) on the
 // device, written row-major n x ld (omega.cu).

@@ -15,6 +15,7 @@
 #include <cmath>
 
 #include "cs_internal.h"
+#include "slices_internal.h"
 
 namespace cs {
 
@@ -162,6 +163,7 @@ static void kinship_apply_fp64(cs_kinship* op, const double* X, int64_t ldx, int
         CS_CUDA(cudaMemset2DAsync(Y, ldy * 8, 0, k * 8, op->rows, s));
         return;
     }
+    if (kinship_apply_slices(op, StridedIn{X, ldx, 1}, k, StridedOut{Y, ldy, 1}, s)) return;
     op->buf_u.resize(R * k);
     decode_gemm_rows_fp64(op->view, op->d_lut.get(), X, ldx, k, op->buf_u.get(), k, op->ws, s);
     decode_gemm_samples_fp64(op->view, op->d_lut.get(), op->buf_u.get(), k, k, Y, ldy, scale,
@@ -225,6 +227,12 @@ void kinship_apply_f32(cs_kinship* op, const float* X, int64_t ldx, int64_t k, f
     }
 }
 
+// Whether two column-major blocks (ld, rows x k) share memory.
+static bool overlap(const double* a, int64_t lda, int64_t rows_a, const double* b, int64_t ldb,
+                    int64_t rows_b, int64_t k) {
+    return a < b + (k - 1) * ldb + rows_b && b < a + (k - 1) * lda + rows_a;
+}
+
 // Public column-major apply (device pointers): transposes in and out around the kernels.
 void kinship_apply_colmajor(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* Y,
                             int64_t ldy, int precision, cudaStream_t s) {
@@ -233,6 +241,12 @@ void kinship_apply_colmajor(cs_kinship* op, const double* X, int64_t ldx, int64_
     if (ldx < op->rows || ldy < op->rows)
         fail(CS_ERR_INVALID_ARGUMENT, "PlinkKinshipOperator::apply: dimension mismatch");
     const int64_t n = op->rows;
+    // the slice kernels read and write column-major as it is (Y in X's place included; blocks that
+    // overlap in another way go through the copies below)
+    if (precision == CS_PRECISION_FP64 &&
+        ((X == Y && ldx == ldy) || !overlap(X, ldx, n, Y, ldy, n, k)) &&
+        kinship_apply_slices(op, StridedIn{X, 1, ldx}, k, StridedOut{Y, 1, ldy}, s))
+        return;
     op->buf_x.resize(n * k);
     op->buf_y.resize(n * k);
     colmajor_to_rowmajor(X, ldx, n, k, op->buf_x.get(), k, s);
@@ -334,6 +348,11 @@ void genotype_multiply_zt(cs_kinship* op, const double* X, int64_t ldx, int64_t 
         fail(CS_ERR_INVALID_ARGUMENT, "Dimension mismatch in multiply_Zt_v");
     if (k == 0) return;
     const int64_t n = op->rows, nv = op->num_variants;
+    if (precision == CS_PRECISION_FP64 && !overlap(X, ldx, n, U, ldu, nv, k)) {
+        // rows of variants the view dropped (1/sd == 0) stay zero
+        if (op->n_active < nv) CS_CUDA(cudaMemset2DAsync(U, ldu * 8, 0, nv * 8, k, s));
+        if (multiply_zt_slices(op, StridedIn{X, 1, ldx}, k, StridedOut{U, 1, ldu}, s)) return;
+    }
     op->buf_x.resize(n * k);
     op->buf_y.resize(nv * k);
     colmajor_to_rowmajor(X, ldx, n, k, op->buf_x.get(), k, s);
@@ -348,6 +367,9 @@ void genotype_multiply_z(cs_kinship* op, const double* V, int64_t ldv, int64_t k
         fail(CS_ERR_INVALID_ARGUMENT, "Dimension mismatch in multiply_Z_v");
     if (k == 0) return;
     const int64_t n = op->rows, nv = op->num_variants;
+    if (precision == CS_PRECISION_FP64 && !overlap(V, ldv, nv, Y, ldy, n, k) &&
+        multiply_z_slices(op, StridedIn{V, 1, ldv}, k, StridedOut{Y, 1, ldy}, s))
+        return;
     op->buf_x.resize(nv * k);
     op->buf_y.resize(n * k);
     colmajor_to_rowmajor(V, ldv, nv, k, op->buf_x.get(), k, s);

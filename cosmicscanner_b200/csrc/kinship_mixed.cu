@@ -60,6 +60,7 @@
 #include <vector>
 
 #include "cs_internal.h"
+#include "mixed_internal.h"
 #include "sm100.cuh"
 
 namespace cs {
@@ -68,7 +69,7 @@ namespace {
 
 using namespace sm100;
 
-constexpr int kTile = 128;        // MMA M, and SNP rows / samples per decoded tile
+constexpr int kTile = kTcTile;
 constexpr int kKBlock = 128;      // K elements (int8) per stage: one 128-byte swizzle row
 constexpr int kMaxKc = 80;        // column-tile width cap (MMA N = 3 kc <= 256)
 constexpr int kWarps = 15;
@@ -78,7 +79,7 @@ constexpr int kEpiWarp0 = 10;
 constexpr int kPackedWarp = 14;
 constexpr uint32_t kTmemCols = 512;
 constexpr double kBase = 254.0;
-constexpr int kImputeQ = 63;          // dosage scale of the imputed-code tile
+constexpr int kImputeQ = kTcQ;
 constexpr int kMaxKbPerAccum = 1024;  // K-blocks one int32 accumulation may hold:
                                       // 1024 * 128 * (126 * 127 + 127) < 2^31
 
@@ -226,23 +227,7 @@ struct PassArgs {
     int decode_alt;              // TMEMA: two groups of four decoder warps take alternate K-blocks
 };
 
-// 16 codes (one 32-bit word, code j in bits 2j..2j+1) -> 16 int8 imputed codes (byte c of
-// the row's table `lut` for code c) and 16 missing indicators in the interleaved sample order
-// 0 2 4 .. 14 1 3 .. 15 within the group: the even codes, masked in place, are already
-// byte-permute selectors (one nibble each), and so are the odd codes after one shift.
-// sample_at(p) / position_of(s) convert.
-__device__ __forceinline__ void decode_word_interleaved(uint32_t w, uint32_t lut, uint4& dos, uint4& mis) {
-    const uint32_t se = w & 0x33333333u, so = (w >> 2) & 0x33333333u;
-    dos.x = __byte_perm(lut, 0u, se);
-    dos.y = __byte_perm(lut, 0u, se >> 16);
-    dos.z = __byte_perm(lut, 0u, so);
-    dos.w = __byte_perm(lut, 0u, so >> 16);
-    mis.x = __byte_perm(0x00000100u, 0u, se);
-    mis.y = __byte_perm(0x00000100u, 0u, se >> 16);
-    mis.z = __byte_perm(0x00000100u, 0u, so);
-    mis.w = __byte_perm(0x00000100u, 0u, so >> 16);
-}
-// The same for 16 codes of 16 different SNPs (a word of the sample-major copy): the observed
+// decode_word_interleaved for 16 codes of 16 different SNPs (a word of the sample-major copy): the observed
 // calls through the fixed table 2Q / 0 / Q / 0, a 0xFF byte per missing call, and the SNPs'
 // imputed codes q (four per word, in the interleaved order) put in under that mask.  The mask
 // itself is the missing-indicator tile, as int8 -1: the samples operand of this form carries
@@ -259,10 +244,6 @@ __device__ __forceinline__ void decode_word_imputed(uint32_t w, const uint4& q, 
     dos.z = __byte_perm(kObservedCodes, 0u, so) | (mis.z & q.z);
     dos.w = __byte_perm(kObservedCodes, 0u, so >> 16) | (mis.w & q.w);
 }
-// position p (0..15) of the interleaved order -> sample offset in the group, and back
-__host__ __device__ __forceinline__ int sample_at(int p) { return p < 8 ? 2 * p : 2 * (p - 8) + 1; }
-__host__ __device__ __forceinline__ int position_of(int s) { return (s & 1) ? 8 + (s >> 1) : s >> 1; }
-
 template <bool ROWS, bool PAIR, bool NARROW, int TMEMA>
 __global__ void __launch_bounds__(kThreads, 1)
 k_mixed_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
@@ -1111,7 +1092,8 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
-// 2D uint8 tensor map: inner extent `inner` bytes, `outer` rows of `row_bytes`.
+}  // namespace
+
 CUtensorMap make_map_u8(const void* base, uint64_t inner, uint64_t outer, uint64_t row_bytes,
                         uint32_t box_inner, uint32_t box_outer, bool swizzle) {
     CUtensorMap m;
@@ -1128,6 +1110,8 @@ CUtensorMap make_map_u8(const void* base, uint64_t inner, uint64_t outer, uint64
         fail(CS_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
     return m;
 }
+
+namespace {
 
 // Both passes run on CTA pairs (cta_group::2) for more than 32 right-hand sides unless
 // CS_B200_CTA_PAIRS=0 selects the single-CTA kernels (=1: pairs for every width).  Measured
@@ -1240,22 +1224,6 @@ int choose_splits(int64_t units_per_split, int kb_total, int64_t target) {
 }
 
 }  // namespace
-
-struct MixedRows {
-    // a packed view with per-row centring statistics, ready for the rows pass
-    int64_t R = 0, n = 0, r_pad = 0, n_pad = 0;
-    DeviceBuffer<double> mu, exc, s, resid;
-    DeviceBuffer<uint32_t> lut;  // imputed code of each 2-bit code, one byte per code
-    // q_t (byte 1 of lut[t]) at K position (t & ~15) + position_of(t & 15): the samples pass
-    // over the sample-major copy reads the imputed codes of 16 SNPs per uint4
-    DeviceBuffer<uint4> qperm;
-    CUtensorMap tm{};
-    const uint8_t* rows = nullptr;  // the view's packed rows (owned by the operator)
-    int64_t stride = 0;
-    // sample-major copy for the narrow samples pass with A in TMEM (made on first use)
-    DeviceBuffer<uint8_t> packed_t;
-    CUtensorMap tm_t{};
-};
 
 struct MixedWorkspace {
     DeviceBuffer<int8_t> b1, b2;
@@ -1407,6 +1375,8 @@ void init_rows(MixedRows& r, const cs_packed_view& v, const double* mean, const 
     r.stride = v.stride;
 }
 
+}  // namespace
+
 // The sample-major copy of the view (once per context): n_pad rows of r_pad / 4 bytes.
 void ensure_transposed(MixedRows& r, cudaStream_t s) {
     if (r.packed_t.get()) return;
@@ -1420,6 +1390,8 @@ void ensure_transposed(MixedRows& r, cudaStream_t s) {
     }
     r.tm_t = make_map_u8(r.packed_t.get(), stride_t, r.n_pad, stride_t, 32, kTile, false);
 }
+
+namespace {
 
 struct Tiling {
     int n_ctiles, kc, kc_last;
@@ -1893,6 +1865,8 @@ static MixedOperator* mixed_for(cs_kinship* op) {
     op->mixed = m;
     return m;
 }
+
+MixedRows& mixed_rows_for(cs_kinship* op) { return mixed_for(op)->rows; }
 
 void kinship_apply_mixed(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* Y,
                          int64_t ldy, cudaStream_t s) {

@@ -1,0 +1,1399 @@
+// The FP64 form of the kinship products on the int8 tensor cores.
+//
+// Arithmetic.  Each right-hand side column becomes a 55-bit fixed-point column (one power of two
+// per column, the largest element just below 2^55), split into seven int8 digits of base 256
+// (balanced, -128..127): x = 2^-e sum_p d_p 256^(6-p) with an error of at most 2^-55 of the
+// column's maximum.  Genotype codes are small integers, so every product and every sum of the
+// int8 MMAs is exact in int32, the seven sums of an output are put together in 64-bit
+// integers, and the centring by the SNP means is done on those before the single conversion
+// to FP64.  (Splitting a floating-point operand into slices whose products accumulate exactly:
+// Ozaki, Ogita, Oishi, Rump 2012; on integer matrix units: Ootomo, Ozaki, Yokota 2024.)  An
+// FP64 sum of K products carries a rounding error of the order of 2^-53 sqrt(K) of the result
+// at best; here only the operand's own rounding remains.
+//
+//   rows pass     63 u_t / s_t = sum_obs 63 G x + sum_miss q_t x + (63 mu_t - q_t) sum_miss x
+//                                - 63 mu_t sum x
+//     with the imputed-code tile (63 G, or q_t = rint(63 mu_t) for a missing call) against the
+//     seven digits and the missing-indicator tile against the first six (|63 mu_t - q_t| <= 1/2
+//     takes the place of the last); 63 mu_t and the sums are carried in two doubles each, so the
+//     difference of the large terms does not round.
+//   samples pass  M y_i = sum_t G w + sum_miss (mu w) - sum_t (mu w),  w = s o U
+//     with w and mu o w split at one scale (seven digits each) into the same accumulators; the
+//     last sum is taken over the same digits, so that a missing call cancels exactly.
+//
+// Kernel.  The passes keep the genotype tiles in tensor memory (A, K-major: the packed rows in
+// the rows pass, the operator's sample-major copy in the samples pass) and stream the digits (B)
+// through shared memory; kinship_mixed.cu has the same structure at three digits.  Warp 0 loads
+// B, warp 2 the packed tiles (both TMA), warps 8.. decode in groups of four that take K-blocks
+// in turn (a warp may touch only its own quarter of the TMEM lanes), warp 1 issues the MMAs from
+// one thread, warps 4-7 drain the accumulators.  The MMA thread's own instructions set the pace of
+// narrow blocks, so a K-block's B rows and its decoded tile share one ring stage (one wait, one commit),
+// and a packed tile spans four K-blocks.  What bounds them now is the decode: 13 integer
+// operations per 16 genotypes at half rate are 208 of the 400 clocks a K-block takes, the ring and
+// wait instructions of all warps about 120 more (ncu: ALU pipe 70 % busy, tensor pipe 14 %, DRAM a
+// third of its rate).  Wide blocks are bound by the MMAs: 448 clocks a K-block of a 16-column
+// rows tile, 896 of a 32-column samples tile.  Wide blocks run on CTA pairs (cta_group::2):
+// each CTA holds half of the B rows, which halves the L2 reads of B that would otherwise bound
+// a wide block (64 bytes per clock and SM at the full MMA rate).
+//
+// Column tiles.  Up to 4 columns a column's digits sit in eight adjacent B rows (N = 8 w);
+// wider tiles are digit-major in widths of 8 per CTA.  TMEM (512 columns) holds the
+// accumulators (rows: main and missing-call sums apart, 13 per column; samples: 7) and the
+// A stages (64 columns each).
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <string>
+
+#include "cs_internal.h"
+#include "mixed_internal.h"
+#include "slices_internal.h"
+#include "sm100.cuh"
+
+namespace cs {
+
+namespace {
+
+using namespace sm100;
+
+constexpr int kTile = kTcTile;
+constexpr int kKBlock = 128;
+constexpr int kDigits = 7;
+constexpr int kEpiWarp0 = 4, kDecWarp0 = 8;
+// decoder groups of four warps: G, by kernel
+constexpr int threads_for(int groups) { return (kDecWarp0 + 4 * groups) * 32; }
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kAStage = 64;              // TMEM columns of a decoded K-block
+constexpr int kMaxStages = 16;
+constexpr int kPackedKb = 4;                  // K-blocks of a packed tile: one 128-byte row each
+constexpr int kPackedBytes = kTile * 32 * kPackedKb;
+constexpr int kMaxKbPerAccum = 1024;          // 1024 * 128 * 126 * 128 < 2^31
+constexpr int kBarBytes = (4 * kMaxStages + 2 * 2 + 1) * 8 + 8;
+constexpr int kSmemMax = 227 * 1024;
+constexpr int kPassStatusOk = kOk;
+
+struct SliceArgs {
+    int n_tiles, n_ctiles, n_splits;
+    int kb_total, kb_per_split;
+    int k, w, hw;           // columns, columns per tile, per CTA
+    int cmajor;             // digits of a column adjacent (eight B rows per column)
+    int nm, nx;             // MMA N: main (and samples' second) product, rows' missing product
+    int set_rows;           // B rows of one set in this CTA's shared memory
+    int sd, sp, nb;         // ring depths: stages (B rows + decoded tile), packed tiles, accumulators
+    uint32_t acc_stride, a0;
+    const uint32_t* lut;    // rows pass: imputed code of each 2-bit code, per SNP row
+    const double* mu;       // rows pass: per SNP row
+    const longlong2* ksum;  // [n_splits][k]: sum of the fixed-point values (hi, lo) per slice
+    double* part;           // [n_splits][k][ld]
+    int64_t ld;
+    int* status;
+    uint32_t poll_ns, poll_dec_ns;
+};
+
+// hi 2^32 + lo of the seven digit sums of one output
+__device__ __forceinline__ void join_digits(const int32_t (&m)[8], int64_t& hi, int64_t& lo) {
+    hi = ((int64_t)m[0] << 16) + ((int64_t)m[1] << 8) + (int64_t)m[2];
+    lo = ((int64_t)m[3] << 24) + ((int64_t)m[4] << 16) + ((int64_t)m[5] << 8) + (int64_t)m[6];
+}
+
+// Per SNP row: 63 mu in two doubles and 63 mu - q.
+struct RowCentre {
+    double ah, al, b;
+};
+
+// 63 u 2^e of one rows-pass output: M and X the joined main and missing-call sums, S the sum
+// of the slice's fixed-point values.
+__device__ __forceinline__ double rows_value(const RowCentre& c, int64_t mh, int64_t ml, int64_t xh,
+                                             int64_t xl, double sh, double sl) {
+    const double two32 = 4294967296.0;
+    const double m1 = (double)mh * two32, m0 = (double)ml;
+    const double x = fma((double)xh, two32, (double)xl);
+    const double p = c.ah * sh, pe = fma(c.ah, sh, -p);
+    const double d = m1 - p;
+    return d + (((m0 - c.ah * sl) - pe) + fma(c.b, x, c.al * (x - (sh + sl))));
+}
+
+template <bool ROWS, bool PAIR, int G>
+__global__ void __launch_bounds__(threads_for(G), 1)
+k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
+             const SliceArgs P) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    constexpr int kSets = ROWS ? 1 : 2;
+    const int b_bytes = kSets * P.set_rows * 128;  // a multiple of 1024
+    unsigned char* smem_b = smem;
+    unsigned char* smem_p = smem + P.sd * b_bytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_p + P.sp * kPackedBytes);
+    uint64_t* full = bars;                    // stage ready: B rows landed (1 arrival + tx bytes) and
+                                              // tile decoded (one arrival per warp of a group); pair:
+                                              // the leader's also counts the other CTA's decoders and
+                                              // its landed B rows, the other CTA's only its B rows
+    uint64_t* empty = full + kMaxStages;      // MMAs reading the stage done (commit)
+    uint64_t* full_p = empty + kMaxStages;    // packed tile landed
+    uint64_t* empty_p = full_p + kMaxStages;  // packed tile read (one arrival per decoder warp)
+    uint64_t* acc_full = empty_p + kMaxStages;
+    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* drained = acc_empty + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+    const int SD = P.sd, SP = P.sp, NB = P.nb;
+    if (threadIdx.x == 0) {
+        for (int d = 0; d < SD; ++d) {
+            mbar_init(&full[d], PAIR ? (rank == 0 ? 10 : 1) : 5);
+            mbar_init(&empty[d], 1);
+        }
+        for (int s = 0; s < SP; ++s) {
+            mbar_init(&full_p[s], 1);
+            mbar_init(&empty_p[s], 4 * G);
+        }
+        for (int b = 0; b < NB; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], PAIR ? 8 : 4);
+        }
+        mbar_init(drained, 1);
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        if (PAIR)
+            tmem_alloc_pair(tmem_slot, kTmemCols);
+        else
+            tmem_alloc(tmem_slot, kTmemCols);
+    }
+    tc_fence_before();
+    if (PAIR)
+        cluster_sync_all();
+    else
+        __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    // A unit is one M tile (pair: two) x one column tile x one K slice, column tiles fastest so
+    // that the CTAs running at one time share packed tiles through L2.
+    const int groups = PAIR ? P.n_tiles / 2 : P.n_tiles;
+    const int units = groups * P.n_ctiles * P.n_splits;
+    const int u0 = PAIR ? (int)cluster_id_x() : (int)blockIdx.x;
+    const int ustep = PAIR ? (int)cluster_count_x() : (int)gridDim.x;
+    auto unit_coords = [&](int u, int& tile, int& ct, int& split, int& kb0, int& kb1) {
+        ct = u % P.n_ctiles;
+        const int rest = u / P.n_ctiles;
+        const int g = rest % groups;
+        tile = PAIR ? 2 * g + (int)rank : g;
+        split = rest / groups;
+        kb0 = split * P.kb_per_split;
+        kb1 = min(P.kb_total, kb0 + P.kb_per_split);
+    };
+    // barriers that MMA commits or the other CTA arrive on: pairs poll (a suspended try_wait can
+    // sleep through a remote arrival); long waits off the critical path pause between polls
+    auto wait_peer = [&](uint64_t* bar, uint32_t parity, int code) {
+        return PAIR ? mbar_poll_cluster_look(bar, parity, P.status, code)
+                    : mbar_wait_look(bar, parity, P.status, code);
+    };
+    auto wait_idle = [&](uint64_t* bar, uint32_t parity, int code, uint32_t ns) {
+        return PAIR ? mbar_poll_sleep_look(bar, parity, P.status, code, ns)
+                    : mbar_wait_look(bar, parity, P.status, code);
+    };
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ TMA producer (B)
+        if (elect_one()) {
+            prefetch_tensormap(&tm_b);
+            // a third of a deep ring at a time: stages come free in order, so the last one's
+            // barrier stands for all
+            const int batch = SD >= 6 ? SD / 3 : 1;
+            int d = 0, loaded = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int u = u0; u < units && ok; u += ustep) {
+                int tile, ct, split, kb0, kb1;
+                unit_coords(u, tile, ct, split, kb0, kb1);
+                const int row0 = (ct * (PAIR ? 2 : 1) + (int)rank) * kSets * P.set_rows;
+                for (int kb = kb0; kb < kb1;) {
+                    const int n = min(batch, kb1 - kb);
+                    const int last = d + n - 1;
+                    ok = wait_idle(&empty[last >= SD ? last - SD : last], last >= SD ? ph : ph ^ 1,
+                                   kTimeoutTma, P.poll_ns);
+                    if (!ok) break;
+                    for (int i = 0; i < n; ++i, ++kb) {
+                        mbar_arrive_expect_tx(&full[d], (uint32_t)b_bytes);
+#pragma unroll
+                        for (int q = 0; q < kSets; ++q)
+                            tma_load_2d(smem_b + d * b_bytes + q * P.set_rows * 128, &tm_b, kb * kKBlock,
+                                        row0 + q * P.set_rows, &full[d]);
+                        ++loaded;
+                        if (++d == SD) { d = 0; ph ^= 1; }
+                    }
+                }
+            }
+            // leave no copy in flight (in a pass that ran through, the MMAs have waited for them all)
+            for (int q = min(loaded, SD); q > 0; --q) {
+                if (--d < 0) { d = SD - 1; ph ^= 1; }
+                mbar_wait_look(&full[d], ph, P.status, kTimeoutTma, 1u << 20);
+            }
+        }
+    } else if (warp == 2) {
+        // ------------------------------------------------------------ TMA producer (packed)
+        if (elect_one()) {
+            prefetch_tensormap(&tm_a);
+            int s = 0, loaded = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int u = u0; u < units && ok; u += ustep) {
+                int tile, ct, split, kb0, kb1;
+                unit_coords(u, tile, ct, split, kb0, kb1);
+                for (int kb = kb0; kb < kb1; kb += kPackedKb) {
+                    if (!(ok = mbar_wait_look(&empty_p[s], ph ^ 1, P.status, kTimeoutTma))) break;
+                    mbar_arrive_expect_tx(&full_p[s], (uint32_t)kPackedBytes);
+                    // 128 rows x 128 bytes (zeros past the row's end)
+                    tma_load_2d(smem_p + s * kPackedBytes, &tm_a, kb * 32, tile * kTile, &full_p[s]);
+                    ++loaded;
+                    if (++s == SP) { s = 0; ph ^= 1; }
+                }
+            }
+            for (int q = min(loaded, SP); q > 0; --q) {
+                if (--s < 0) { s = SP - 1; ph ^= 1; }
+                mbar_wait_look(&full_p[s], ph, P.status, kTimeoutTma, 1u << 20);
+            }
+        }
+    } else if (warp == 1 && (!PAIR || rank == 0)) {
+        // ------------------------------------------------------------ MMA issuer (pair: leader)
+        // The whole role under elect: tcgen05 operands are uniform registers, and where the compiler
+        // cannot see that one lane runs, it issues lane by lane (700 clocks a K-block, not 100).
+        if (elect_one()) {
+            // s8 x s8 -> s32, both operands K-major, M = 128 (pair: 256)
+            const uint32_t idesc0 = (2u << 4) | (1u << 7) | (1u << 10) |
+                                    ((uint32_t)((PAIR ? 2 : 1) * kTile >> 4) << 24);
+            const uint32_t idesc = idesc0 | ((uint32_t)(P.nm >> 3) << 17);
+            const uint32_t idesc_x = idesc0 | ((uint32_t)((ROWS ? P.nx : P.nm) >> 3) << 17);
+            int d = 0, buf = 0;
+            uint32_t ph = 0, ph_a = 0;
+            bool ok = true;
+            for (int u = u0; u < units && ok; u += ustep) {
+                int tile, ct, split, kb0, kb1;
+                unit_coords(u, tile, ct, split, kb0, kb1);
+                if (!(ok = wait_peer(&acc_empty[buf], ph_a ^ 1, kTimeoutMma))) break;
+                tc_fence_after();
+                const uint32_t acc = tmem_base + buf * P.acc_stride;
+                // rows: the missing-call sums beside the main ones; samples: the same columns
+                const uint32_t acc_x = ROWS ? acc + P.nm : acc;
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    if (!(ok = wait_peer(&full[d], ph, kTimeoutMma))) break;
+                    tc_fence_after();
+                    const uint32_t ta = tmem_base + P.a0 + d * kAStage;
+                    const uint64_t db = smem_desc_sw128(smem_addr(smem_b + d * b_bytes), 16, 1024);
+                    const uint64_t dbx = ROWS ? db : db + (uint64_t)(P.set_rows * 128 >> 4);
+#pragma unroll
+                    for (int ks = 0; ks < kKBlock / 32; ++ks) {
+                        const uint32_t first = (kb == kb0 && ks == 0) ? 0u : 1u;
+                        if constexpr (PAIR) {
+                            mma_i8_pair_tmem_a(acc, ta + ks * 8, db + 2 * ks, idesc, first);
+                            mma_i8_pair_tmem_a(acc_x, ta + kAStage / 2 + ks * 8, dbx + 2 * ks, idesc_x,
+                                               ROWS ? first : 1u);
+                        } else {
+                            mma_i8_tmem_a(acc, ta + ks * 8, db + 2 * ks, idesc, first);
+                            mma_i8_tmem_a(acc_x, ta + kAStage / 2 + ks * 8, dbx + 2 * ks, idesc_x,
+                                          ROWS ? first : 1u);
+                        }
+                    }
+                    if (PAIR)
+                        mma_commit_pair(&empty[d], 3);
+                    else
+                        mma_commit(&empty[d]);
+                    if (++d == SD) { d = 0; ph ^= 1; }
+                }
+                if (ok) {
+                    if (PAIR)
+                        mma_commit_pair(&acc_full[buf], 3);
+                    else
+                        mma_commit(&acc_full[buf]);
+                }
+                if (++buf == NB) { buf = 0; ph_a ^= 1; }
+            }
+            if (PAIR)
+                mma_commit_pair(drained, 1);
+            else
+                mma_commit(drained);
+            mbar_wait_look(drained, 0, P.status, kTimeoutMma, 1u << 20);
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
+            // the leader's MMA also reads this CTA's half of each stage's B rows: tell it (one
+            // arrival on its full) once they have landed here
+            int d = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int u = u0; u < units && ok; u += ustep) {
+                int tile, ct, split, kb0, kb1;
+                unit_coords(u, tile, ct, split, kb0, kb1);
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    if (!(ok = mbar_wait_look(&full[d], ph, P.status, kTimeoutDecode))) break;
+                    mbar_arrive_remote(mapa_shared(&full[d], 0));
+                    if (++d == SD) { d = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else if (warp >= kDecWarp0) {
+        // ------------------------------------------------------------ decoders
+        // lane = TMEM lane (row of A) 32 (warp % 4) + lane; group g = (warp - 8) / 4 takes K-blocks
+        // g, g + G, .. of every packed tile whole: 128 codes per lane, 32 TMEM columns of each tile
+        static_assert(kPackedKb % G == 0, "a packed tile holds the same number of K-blocks per group");
+        constexpr int kOwn = kPackedKb / G;
+        const int q = warp & 3, grp = (warp - kDecWarp0) >> 2;
+        const int r = 32 * q + lane;
+        // Stage of this group's next K-block.  Every unit holds a multiple of four K-blocks and the
+        // ring has at least four stages, so that a group is never more than a lap ahead of the
+        // MMAs on the stage that it waits for (a parity tells one lap from the next, no more).
+        int sp = 0, d = grp;
+        uint32_t ph_p = 0, ph_d = 0;
+        bool ok = true;
+        for (int u = u0; u < units && ok; u += ustep) {
+            int tile, ct, split, kb0, kb1;
+            unit_coords(u, tile, ct, split, kb0, kb1);
+            const uint32_t lut = ROWS ? __ldg(P.lut + (int64_t)tile * kTile + r) : 0x00010002u;
+            for (int kb = kb0; kb < kb1 && ok; kb += kPackedKb) {
+                // (votes keep the warp together when a wait gives up)
+                ok = __all_sync(0xffffffffu, mbar_wait_look(&full_p[sp], ph_p, P.status, kTimeoutDecode));
+                if (!ok) break;
+                const unsigned char* src = smem_p + sp * kPackedBytes + r * 128;
+                uint32_t words[kOwn][8];
+#pragma unroll
+                for (int o = 0; o < kOwn; ++o) {
+                    const int c = 2 * (grp + o * G);  // 16-byte chunk of the row, 128-byte swizzle
+                    const uint4 p0 = *reinterpret_cast<const uint4*>(src + ((c ^ (r & 7)) << 4));
+                    const uint4 p1 = *reinterpret_cast<const uint4*>(src + (((c + 1) ^ (r & 7)) << 4));
+                    words[o][0] = p0.x; words[o][1] = p0.y; words[o][2] = p0.z; words[o][3] = p0.w;
+                    words[o][4] = p1.x; words[o][5] = p1.y; words[o][6] = p1.z; words[o][7] = p1.w;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty_p[sp]);  // the packed tile has been read
+                if (++sp == SP) { sp = 0; ph_p ^= 1; }
+#pragma unroll
+                for (int o = 0; o < kOwn; ++o) {
+                    // half a K-block (64 codes of this lane) at a time: 16 TMEM columns of each tile;
+                    // the first half is decoded before the wait for a free stage
+                    uint32_t ev[16], mv[16];
+                    auto decode_half = [&](int h) {
+#pragma unroll
+                        for (int cj = 0; cj < 4; ++cj) {
+                            uint4 dos, mis;
+                            decode_word_interleaved(words[o][4 * h + cj], lut, dos, mis);
+                            ev[4 * cj] = dos.x; ev[4 * cj + 1] = dos.y; ev[4 * cj + 2] = dos.z; ev[4 * cj + 3] = dos.w;
+                            mv[4 * cj] = mis.x; mv[4 * cj + 1] = mis.y; mv[4 * cj + 2] = mis.z; mv[4 * cj + 3] = mis.w;
+                        }
+                    };
+                    decode_half(0);
+                    ok = __all_sync(0xffffffffu, wait_idle(&empty[d], ph_d ^ 1, kTimeoutDecode, P.poll_dec_ns));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t ta = tmem_base + ((uint32_t)(32 * q) << 16) + P.a0 + d * kAStage;
+                    tmem_st16(ta, ev);
+                    tmem_st16(ta + kAStage / 2, mv);
+                    decode_half(1);
+                    tmem_st16(ta + 16, ev);
+                    tmem_st16(ta + kAStage / 2 + 16, mv);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (PAIR)
+                            mbar_arrive_remote(mapa_shared(&full[d], 0));
+                        else
+                            mbar_arrive(&full[d]);
+                    }
+                    d += G;
+                    if (d >= SD) { d -= SD; ph_d ^= 1; }
+                }
+            }
+        }
+    } else if (warp >= kEpiWarp0) {
+        // ------------------------------------------------------------ epilogue
+        const int q = warp & 3;  // TMEM lane quarter this warp may access
+        int buf = 0;
+        uint32_t ph_a = 0;
+        bool ok = true;
+        for (int u = u0; u < units && ok; u += ustep) {
+            int tile, ct, split, kb0, kb1;
+            unit_coords(u, tile, ct, split, kb0, kb1);
+            const int64_t row = (int64_t)tile * kTile + 32 * q + lane;
+            RowCentre rc{0.0, 0.0, 0.0};
+            if (ROWS) {
+                const double m = P.mu[row];
+                rc.ah = (double)kTcQ * m;
+                rc.al = fma((double)kTcQ, m, -rc.ah);
+                rc.b = rc.ah - (double)((P.lut[row] >> 8) & 0xFFu);
+            }
+            ok = __all_sync(0xffffffffu, wait_idle(&acc_full[buf], ph_a, kTimeoutEpilogue, P.poll_ns));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t tb = tmem_base + buf * P.acc_stride + ((uint32_t)(32 * q) << 16);
+            const int c_base = ct * P.w;
+            const int cols = min(P.w, P.k - c_base);
+            double* dst = P.part + ((int64_t)split * P.k + c_base) * P.ld + row;
+            const longlong2* ks = P.ksum + (int64_t)split * P.k + c_base;
+            auto emit = [&](int c, int64_t mh, int64_t ml, int64_t xh, int64_t xl) {
+                const longlong2 sum = ks[c];
+                double v;
+                if (ROWS)
+                    v = rows_value(rc, mh, ml, xh, xl, (double)sum.x * 4294967296.0, (double)sum.y);
+                else
+                    v = fma((double)(mh - sum.x), 4294967296.0, (double)(ml - sum.y));
+                dst[(int64_t)c * P.ld] = v;
+            };
+            if (P.cmajor) {
+                for (int c = 0; c < cols; ++c) {
+                    int32_t m[8];
+                    int64_t mh, ml, xh = 0, xl = 0;
+                    tmem_ld8i(tb + 8 * c, m);
+                    join_digits(m, mh, ml);
+                    if (ROWS) {
+                        tmem_ld8i(tb + P.nm + 8 * c, m);
+                        m[6] = 0;
+                        join_digits(m, xh, xl);
+                    }
+                    emit(c, mh, ml, xh, xl);
+                }
+            } else {
+                // D columns: half h of the tile's columns (pair: from CTA h's B rows), then digit,
+                // then column; eight columns at a time
+                for (int c0 = 0; c0 < cols; c0 += 8) {
+                    const int h = c0 >= P.hw ? 1 : 0;  // single CTA: hw = w
+                    const int cl = c0 - h * P.hw;
+                    const uint32_t cm = tb + h * (P.nm / 2) + cl;
+                    int64_t mh[8], ml[8], xh[8], xl[8];
+                    int32_t m[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) mh[i] = ml[i] = xh[i] = xl[i] = 0;
+#pragma unroll
+                    for (int p = 0; p < kDigits; ++p) {
+                        tmem_ld8i(cm + p * P.hw, m);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            if (p < 3) mh[i] = mh[i] * 256 + m[i];
+                            else ml[i] = ml[i] * 256 + m[i];
+                        }
+                    }
+                    if (ROWS) {
+                        const uint32_t cx = tb + P.nm + h * (P.nx / 2) + cl;
+#pragma unroll
+                        for (int p = 0; p < kDigits - 1; ++p) {
+                            tmem_ld8i(cx + p * P.hw, m);
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                if (p < 3) xh[i] = xh[i] * 256 + m[i];
+                                else xl[i] = xl[i] * 256 + m[i];
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (c0 + i < cols) emit(c0 + i, mh[i], ml[i], xh[i], xl[i] * 256);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                if (PAIR)
+                    mbar_arrive_remote(mapa_shared(&acc_empty[buf], 0));
+                else
+                    mbar_arrive(&acc_empty[buf]);
+            }
+            if (++buf == NB) { buf = 0; ph_a ^= 1; }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    if (PAIR)
+        cluster_sync_all();
+    else
+        __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        if (PAIR)
+            tmem_dealloc_pair(tmem_base, kTmemCols);
+        else
+            tmem_dealloc(tmem_base, kTmemCols);
+    }
+}
+
+// ---------------------------------------------------------------- operand preparation
+
+// Exponent e of the column's scale: |x| 2^e <= 127 2^48 for every element, 2^54 <= max 2^e or the
+// half of it.
+__device__ __forceinline__ int slice_exponent(unsigned long long max_bits) {
+    if (max_bits == 0) return 0;
+    const int ex = (int)(max_bits >> 52) - 1023;
+    // mantissa above 127/64 would round up to 128 2^48
+    const bool top = (max_bits & 0xFFFFFFFFFFFFFull) > 0xFC00000000000ull;
+    return max(-kSliceMaxExp, min(kSliceMaxExp + 60, (top ? 53 : 54) - ex));
+}
+__device__ __forceinline__ double pow2(int e) {
+    return __longlong_as_double((long long)(e + 1023) << 52);
+}
+
+__device__ __forceinline__ void range_of(double v, unsigned long long& mx, long long& es, unsigned& n) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+    mx = b > mx ? b : mx;
+    if (b) {
+        es += (int)(b >> 52) - 1023;
+        ++n;
+    }
+}
+
+__device__ __forceinline__ unsigned long long shfl_max(unsigned long long v, int width) {
+    for (int off = width / 2; off; off >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, off);
+        v = o > v ? o : v;
+    }
+    return v;
+}
+__device__ __forceinline__ long long shfl_sum(long long v, int width) {
+    for (int off = width / 2; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+
+__device__ __forceinline__ void add_range(ColumnRange* out, unsigned long long mx, long long es,
+                                          unsigned long long n) {
+    atomicMax(&out->max_bits, mx);
+    atomicAdd(reinterpret_cast<unsigned long long*>(&out->exp_sum), (unsigned long long)es);
+    atomicAdd(&out->count, n);
+}
+
+// Ranges of X's columns: a block covers kc columns x rows_per_block rows, kc a power of two: one for
+// column-major input, otherwise up to 32, so that a warp reads adjacent elements either way.
+__global__ void __launch_bounds__(256)
+k_slice_ranges(const StridedIn X, int64_t n, int64_t k, int kc, int64_t rows_per_block,
+               ColumnRange* __restrict__ out) {
+    __shared__ unsigned long long s_mx[256];
+    __shared__ long long s_es[256];
+    __shared__ unsigned s_n[256];
+    const int tc = threadIdx.x % kc, tr = threadIdx.x / kc, nr = 256 / kc;
+    const int64_t c = (int64_t)blockIdx.y * kc + tc;
+    const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;
+    const int64_t r1 = min(n, r0 + rows_per_block);
+    unsigned long long mx = 0;
+    long long es = 0;
+    unsigned cnt = 0;
+    if (c < k) {
+#pragma unroll 4
+        for (int64_t r = r0 + tr; r < r1; r += nr) range_of(X.p[r * X.rs + c * X.cs], mx, es, cnt);
+    }
+    s_mx[threadIdx.x] = mx;
+    s_es[threadIdx.x] = es;
+    s_n[threadIdx.x] = cnt;
+    __syncthreads();
+    for (int off = nr / 2; off > 0; off >>= 1) {
+        if (tr < off) {
+            const int o = threadIdx.x + off * kc;
+            s_mx[threadIdx.x] = max(s_mx[threadIdx.x], s_mx[o]);
+            s_es[threadIdx.x] += s_es[o];
+            s_n[threadIdx.x] += s_n[o];
+        }
+        __syncthreads();
+    }
+    if (tr == 0 && c < k) add_range(&out[c], s_mx[threadIdx.x], s_es[threadIdx.x], s_n[threadIdx.x]);
+}
+
+// Transposes 4 x 4 bytes: out[j] = byte j of in[0..3].
+__device__ __forceinline__ void transpose4(const uint32_t (&in)[4], uint32_t (&out)[4]) {
+    const uint32_t a = __byte_perm(in[0], in[1], 0x5140), b = __byte_perm(in[2], in[3], 0x5140);
+    const uint32_t c = __byte_perm(in[0], in[1], 0x7362), d = __byte_perm(in[2], in[3], 0x7362);
+    out[0] = __byte_perm(a, b, 0x5410);
+    out[1] = __byte_perm(a, b, 0x7632);
+    out[2] = __byte_perm(c, d, 0x5410);
+    out[3] = __byte_perm(c, d, 0x7632);
+}
+
+// The seven digits of 16 fixed-point values, each digit's 16 bytes in the interleaved order of
+// the decoded tiles: dig[p] for digit p (0 the most significant).
+__device__ __forceinline__ void digits16(const int64_t (&v)[16], uint4 (&dig)[kDigits]) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        // positions 4g .. 4g + 3 hold samples sample_at(4g) ..
+        uint32_t lo[4], hi[4], tl[4], th[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            // adding 128 to each of the lower six digits makes the plain bytes the balanced
+            // digits plus 128
+            const uint64_t u = (uint64_t)v[sample_at(4 * g + j)] + 0x0000808080808080ull;
+            lo[j] = (uint32_t)u ^ 0x80808080u;
+            hi[j] = (uint32_t)(u >> 32) ^ 0x00008080u;
+        }
+        transpose4(lo, tl);
+        transpose4(hi, th);
+        uint32_t* w = reinterpret_cast<uint32_t*>(dig);
+        w[0 * 4 + g] = th[2];
+        w[1 * 4 + g] = th[1];
+        w[2 * 4 + g] = th[0];
+        w[3 * 4 + g] = tl[3];
+        w[4 * 4 + g] = tl[2];
+        w[5 * 4 + g] = tl[1];
+        w[6 * 4 + g] = tl[0];
+    }
+}
+
+// (hi, lo) of v = hi 2^32 + lo with lo the value of the four lower digits
+__device__ __forceinline__ void split_value(int64_t v, int64_t& hi, int64_t& lo) {
+    hi = (v + 0x80808080ll) >> 32;
+    lo = v - (hi << 32);
+}
+
+struct BLayout {
+    int w, hw, cmajor, halves, sets, set_rows;
+    // row of B that holds digit p of column c (set q)
+    __device__ __forceinline__ int64_t row(int64_t c, int q, int p) const {
+        const int64_t ct = c / w;
+        const int cw = (int)(c - ct * w);
+        const int h = cw / hw, cl = cw - h * hw;
+        const int in = cmajor ? 8 * cl + p : p * hw + cl;
+        return ((ct * halves + h) * sets + q) * set_rows + in;
+    }
+};
+
+// The words a call clears before its kernels add to them (see SliceCall).
+struct SliceSums {
+    int* status;
+    ColumnRange* range;        // of X, per column
+    ColumnRange* range_w;      // of the samples operand
+    unsigned long long* sum;   // [slices][k][2]: (hi, lo) sums of the fixed-point values, rows pass
+    unsigned long long* sum_w; // the same of mu o w, samples pass
+    int splits, splits_w;
+};
+
+__device__ __forceinline__ void add_sums(unsigned long long* dst, int64_t hi, int64_t lo) {
+    atomicAdd(dst, (unsigned long long)hi);
+    atomicAdd(dst + 1, (unsigned long long)lo);
+}
+
+// 16 fixed-point values of column c -> their digits' bytes at rows B.row(c, set, p), from K
+// position i0 on; their sums are added to (hi, lo).
+__device__ __forceinline__ void emit_digits(const int64_t (&v)[16], const BLayout& B, int64_t c, int set,
+                                            int64_t i0, int64_t pitch, int8_t* out) {
+    uint4 dig[kDigits];
+    digits16(v, dig);
+#pragma unroll
+    for (int p = 0; p < kDigits; ++p)
+        *reinterpret_cast<uint4*>(out + B.row(c, set, p) * pitch + i0) = dig[p];
+}
+
+// Rows-pass operand: B rows of X's columns (columns k .. k_pad with zeros), and the sums of the
+// fixed-point values per K slice.  A block takes COLS columns x ROWS rows through shared memory; a
+// thread takes 16 rows of a column.
+template <int COLS, int ROWS>
+__global__ void __launch_bounds__(ROWS / 16 * COLS)
+k_slice_rows_operand(const StridedIn X, int64_t n, int64_t k, int64_t k_pad, int64_t n_pad,
+                     int slice_rows, const SliceSums S, BLayout B, int8_t* __restrict__ out) {
+    constexpr int T = ROWS / 16 * COLS;
+    static_assert(ROWS % 256 == 0 && (ROWS / 16) % 16 == 0, "a half warp covers 256 rows of a column");
+    // one pad every 16 rows and one per column: conflict-free both ways
+    __shared__ double tile[COLS][ROWS + ROWS / 16 + 1];
+    const int64_t r0 = (int64_t)blockIdx.x * ROWS, c0 = (int64_t)blockIdx.y * COLS;
+    for (int e = threadIdx.x; e < ROWS * COLS; e += T) {
+        const int rr = X.rs == 1 ? e % ROWS : e / COLS, cc = X.rs == 1 ? e / ROWS : e % COLS;
+        const int64_t r = r0 + rr, c = c0 + cc;
+        tile[cc][rr + (rr >> 4)] = (r < n && c < k) ? X.p[r * X.rs + c * X.cs] : 0.0;
+    }
+    __syncthreads();
+    const int grp = threadIdx.x % (ROWS / 16), cc = threadIdx.x / (ROWS / 16);
+    const int64_t c = c0 + cc, i0 = r0 + 16 * grp;
+    const bool live = c < k_pad && i0 < n_pad;
+    int64_t sh = 0, sl = 0;
+    if (live) {
+        const double f = c < k ? pow2(slice_exponent(S.range[c].max_bits)) : 0.0;
+        int64_t v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            v[j] = __double2ll_rn(tile[cc][17 * grp + j] * f);
+            int64_t h, l;
+            split_value(v[j], h, l);
+            sh += h;
+            sl += l;
+        }
+        emit_digits(v, B, c, 0, i0, n_pad, out);
+    }
+    // 16 threads hold 256 rows, which lie in one slice
+    sh = shfl_sum(sh, 16);
+    sl = shfl_sum(sl, 16);
+    if ((threadIdx.x & 15) == 0 && live && c < k) add_sums(S.sum + 2 * ((i0 / slice_rows) * k + c), sh, sl);
+}
+
+// The same for a short X, one block per column and 16 rows a thread, held in registers from the range
+// to the digits; the call's other words are cleared here, so that a small call needs neither the
+// memset nor the range kernel (a launch costs such a call more than the work in it).
+constexpr int64_t kWholeRows = 8192;
+__global__ void __launch_bounds__(kWholeRows / 16)
+k_slice_rows_operand_whole(const StridedIn X, int64_t n, int64_t k, int64_t n_pad, int slice_rows,
+                           const SliceSums S, BLayout B, int8_t* __restrict__ out) {
+    __shared__ unsigned long long s_mx[16], s_sum[64][2];
+    __shared__ long long s_es[16];
+    __shared__ unsigned s_n[16];
+    const int64_t c = blockIdx.x, i0 = 16 * (int64_t)threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
+    double x[16];
+    unsigned long long mx = 0;
+    long long es = 0;
+    unsigned cnt = 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = (c < k && i0 + j < n) ? X.p[(i0 + j) * X.rs + c * X.cs] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) range_of(x[j], mx, es, cnt);
+    mx = shfl_max(mx, 32);
+    es = shfl_sum(es, 32);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) {
+        s_mx[warp] = mx;
+        s_es[warp] = es;
+        s_n[warp] = cnt;
+    }
+    for (int z = threadIdx.x; z < 2 * S.splits; z += blockDim.x) s_sum[z >> 1][z & 1] = 0;
+    if (c == 0 && threadIdx.x == 0) *S.status = kPassStatusOk;
+    if (c < k) {
+        if (threadIdx.x == 0) S.range_w[c] = ColumnRange{0, 0, 0, 0};
+        for (int z = threadIdx.x; z < 2 * S.splits_w; z += blockDim.x)
+            S.sum_w[2 * ((z >> 1) * k + c) + (z & 1)] = 0;
+    }
+    __syncthreads();
+    unsigned long long n_all = 0;
+    mx = 0;
+    es = 0;
+    for (int w = 0; w < warps; ++w) {
+        mx = max(mx, s_mx[w]);
+        es += s_es[w];
+        n_all += s_n[w];
+    }
+    if (threadIdx.x == 0 && c < k) S.range[c] = ColumnRange{mx, es, n_all, 0};
+    const double f = pow2(slice_exponent(mx));
+    int64_t v[16], sh = 0, sl = 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        v[j] = __double2ll_rn(x[j] * f);
+        int64_t h, l;
+        split_value(v[j], h, l);
+        sh += h;
+        sl += l;
+    }
+    if (i0 < n_pad) emit_digits(v, B, c, 0, i0, n_pad, out);
+    sh = shfl_sum(sh, 16);
+    sl = shfl_sum(sl, 16);
+    if ((threadIdx.x & 15) == 0 && i0 < n_pad) {
+        atomicAdd(&s_sum[i0 / slice_rows][0], (unsigned long long)sh);
+        atomicAdd(&s_sum[i0 / slice_rows][1], (unsigned long long)sl);
+    }
+    __syncthreads();
+    if (c < k)
+        for (int z = threadIdx.x; z < 2 * S.splits; z += blockDim.x)
+            S.sum[2 * ((z >> 1) * k + c) + (z & 1)] = s_sum[z >> 1][z & 1];
+}
+
+// Samples-pass operand from W^T (column-major, R per column): the digits of w and of mu o w at
+// one scale per column, and the sums of mu o w per K slice.  One column per blockIdx.y, 2048 SNPs
+// per block.
+__global__ void __launch_bounds__(128)
+k_slice_samples_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int64_t r_pad,
+                        int slice_rows, const double* __restrict__ mu, const SliceSums S, BLayout B,
+                        int8_t* __restrict__ out) {
+    const int64_t c = blockIdx.y;
+    const int64_t t0 = ((int64_t)blockIdx.x * 128 + threadIdx.x) * 16;
+    const bool live = t0 < r_pad;
+    int64_t sh = 0, sl = 0;
+    if (live) {
+        const double f = c < k ? pow2(slice_exponent(S.range_w[c].max_bits)) : 0.0;
+        int64_t v[16], m[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const double w = (c < k && t0 + j < R) ? Wt[c * R + t0 + j] : 0.0;
+            v[j] = __double2ll_rn(w * f);
+            m[j] = __double2ll_rn((mu[t0 + j] * w) * f);
+            int64_t h, l;
+            split_value(m[j], h, l);
+            sh += h;
+            sl += l;
+        }
+        emit_digits(v, B, c, 0, t0, r_pad, out);
+        emit_digits(m, B, c, 1, t0, r_pad, out);
+    }
+    // 16 threads hold 256 SNPs, which lie in one slice
+    sh = shfl_sum(sh, 16);
+    sl = shfl_sum(sl, 16);
+    if ((threadIdx.x & 15) == 0 && live && c < k) add_sums(S.sum_w + 2 * ((t0 / slice_rows) * k + c), sh, sl);
+}
+
+// A pass that gave up waiting leaves NaN, so that the failure shows wherever the caller looks.
+__device__ __forceinline__ double checked(double v, const int* status) {
+    return *status == kPassStatusOk ? v : __longlong_as_double(0x7FF8000000000000ll);
+}
+
+// (G - mu) of a 2-bit code, 0 for a missing call
+__device__ __forceinline__ double centred(uint32_t code, double mu) {
+    return code == 0u ? 2.0 - mu : code == 1u ? 0.0 : code == 2u ? 1.0 - mu : -mu;
+}
+
+struct PackedRows {
+    const uint8_t* rows;
+    int64_t stride;
+};
+
+// u_t / s_t of a column outside the fixed-point range: the plain FP64 sum over a packed row by one
+// warp, 64 samples per lane at a time.  Missing calls multiply by zero, so a non-finite value
+// reaches every row, as it does in the FP64-pipe kernels.
+__device__ double direct_row(const PackedRows& G, int64_t t, double mu, const StridedIn& X, int64_t c,
+                             int64_t n, int lane) {
+    double acc = 0.0;
+    for (int64_t i0 = 64 * lane; i0 < n; i0 += 64 * 32) {
+        const uint4 w = *reinterpret_cast<const uint4*>(G.rows + t * G.stride + (i0 >> 2));
+        const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            for (int j = 0; j < 16; ++j) {
+                const int64_t i = i0 + 16 * q + j;
+                if (i < n) acc = fma(centred((words[q] >> (2 * j)) & 3u, mu), X.p[i * X.rs + c * X.cs], acc);
+            }
+    }
+    for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    return acc;
+}
+
+// Rows-pass result u / s = 2^-e / 63 sum_z part (or the direct sum).  1024 SNPs per block, one column
+// per blockIdx.y.  With Wt: W^T (column-major, R per column) = s^2 (u / s) and the ranges of
+// max(|W|, |mu W|) for the samples operand; with out: s (u / s) at row pos[t].
+__global__ void __launch_bounds__(256)
+k_slice_reduce_rows(const double* __restrict__ part, int64_t ld, int64_t R, int64_t k,
+                    const double* __restrict__ s_row, const double* __restrict__ mu,
+                    const PackedRows G, const StridedIn X, int64_t n, const SliceSums S,
+                    double* __restrict__ Wt, const int32_t* __restrict__ pos, StridedOut out) {
+    const int64_t c = blockIdx.y;
+    const ColumnRange rg = S.range[c];
+    const double f = pow2(-slice_exponent(rg.max_bits)) / (double)kTcQ;
+    const bool direct = range_excluded(rg);
+    unsigned long long mx = 0;
+    long long es = 0;
+    unsigned cnt = 0;
+    const int64_t t0 = (int64_t)blockIdx.x * 1024, t1 = min(R, t0 + 1024);
+    auto finish = [&](int64_t t, double v) {
+        const double s = s_row[t];
+        if (Wt) {
+            const double w = v * s * s;
+            Wt[c * R + t] = w;
+            range_of(mu[t] > 1.0 ? mu[t] * w : w, mx, es, cnt);
+        } else {
+            out.p[(int64_t)pos[t] * out.rs + c * out.cs] = v * s;
+        }
+    };
+    if (direct) {
+        const int lane = threadIdx.x & 31;
+        for (int64_t t = t0 + (threadIdx.x >> 5); t < t1; t += 8) {
+            const double v = direct_row(G, t, mu[t], X, c, n, lane);
+            if (lane == 0) finish(t, v);
+        }
+    } else {
+        for (int64_t t = t0 + threadIdx.x; t < t1; t += 256) {
+            double acc = 0.0;
+            for (int z = 0; z < S.splits; ++z) acc += part[((int64_t)z * k + c) * ld + t];
+            finish(t, checked(acc * f, S.status));
+        }
+    }
+    if (!Wt) return;
+    mx = shfl_max(mx, 32);
+    es = shfl_sum(es, 32);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if ((threadIdx.x & 31) == 0) add_range(&S.range_w[c], mx, es, cnt);
+}
+
+// The samples operand of a half-pass: W^T[c][t] = s_t V[pos[t]][c] and its ranges (1024 SNPs per
+// block, one column per blockIdx.y).
+__global__ void __launch_bounds__(256)
+k_slice_gather(const StridedIn V, int64_t R, const int32_t* __restrict__ pos,
+               const double* __restrict__ s_row, const double* __restrict__ mu, const SliceSums S,
+               double* __restrict__ Wt) {
+    const int64_t c = blockIdx.y;
+    unsigned long long mx = 0;
+    long long es = 0;
+    unsigned cnt = 0;
+    const int64_t t0 = (int64_t)blockIdx.x * 1024;
+    for (int64_t t = t0 + threadIdx.x; t < min(R, t0 + 1024); t += 256) {
+        const double w = s_row[t] * V.p[(int64_t)pos[t] * V.rs + c * V.cs];
+        Wt[c * R + t] = w;
+        range_of(mu[t] > 1.0 ? mu[t] * w : w, mx, es, cnt);
+    }
+    mx = shfl_max(mx, 32);
+    es = shfl_sum(es, 32);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if ((threadIdx.x & 31) == 0) add_range(&S.range_w[c], mx, es, cnt);
+}
+
+// Samples-pass result: Y[i][c] = scale 2^-e sum_z part[z][c][i] (or the direct sum over the column's
+// W).  Column-major output: a warp's lanes are samples; row-major: tiles of 32 samples x 32 columns
+// through shared memory, so that both sides are coalesced.
+__global__ void __launch_bounds__(256)
+k_slice_reduce_samples(const double* __restrict__ part, int64_t ld, int64_t n, int64_t k,
+                       const double* __restrict__ Wt, int64_t R, const double* __restrict__ mu,
+                       const PackedRows G, const SliceSums S, double scale, StridedOut Y) {
+    __shared__ double tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t i0 = (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
+    const int64_t i = i0 + tx;
+    for (int cc = ty; cc < 32; cc += 8) {
+        const int64_t c = c0 + cc;
+        if (c >= k || i >= n) continue;
+        const ColumnRange rg = S.range_w[c];
+        double acc = 0.0;
+        if (range_excluded(rg)) {
+            const uint8_t* g = G.rows + (i >> 2);
+            const int sh = 2 * (int)(i & 3);
+            for (int64_t t = 0; t < R; ++t)
+                acc = fma(centred((g[t * G.stride] >> sh) & 3u, mu[t]), Wt[c * R + t], acc);
+            acc *= scale;
+        } else {
+            for (int z = 0; z < S.splits_w; ++z) acc += part[((int64_t)z * k + c) * ld + i];
+            acc = checked(acc * (pow2(-slice_exponent(rg.max_bits)) * scale), S.status);
+        }
+        if (Y.rs == 1) Y.p[i + c * Y.cs] = acc;
+        else tile[cc][tx] = acc;
+    }
+    if (Y.rs == 1) return;
+    __syncthreads();
+    for (int ii = ty; ii < 32; ii += 8) {
+        const int64_t r = i0 + ii, c = c0 + tx;
+        if (r < n && c < k) Y.p[r * Y.rs + c * Y.cs] = tile[tx][ii];
+    }
+}
+
+// ---------------------------------------------------------------- plans
+
+struct SlicePlan {
+    bool pair = false;
+    int w = 0, hw = 0, cmajor = 0, n_ctiles = 0;
+    int nm = 0, nx = 0, set_rows = 0;
+    int sd = 0, sp = 0, nb = 0;
+    uint32_t acc_stride = 0, a0 = 0;
+    int splits = 1, kbs = 0;
+    size_t smem = 0;
+    double cost = 0.0;
+    BLayout blayout(bool rows) const {
+        return BLayout{w, hw, cmajor, pair ? 2 : 1, rows ? 1 : 2, set_rows};
+    }
+    int64_t b_rows(bool rows) const {
+        return (int64_t)n_ctiles * (pair ? 2 : 1) * (rows ? 1 : 2) * set_rows;
+    }
+};
+
+// Layout of column tiles of w columns; false when it does not fit.
+bool lay_out(bool rows, bool pair, int w, int64_t k, SlicePlan& p) {
+    const int halves = pair ? 2 : 1;
+    p.pair = pair;
+    p.w = w;
+    p.hw = w / halves;
+    p.cmajor = w <= 4 ? 1 : 0;
+    p.n_ctiles = (int)((k + w - 1) / w);
+    auto up16 = [](int x) { return (x + 15) / 16 * 16; };
+    const int half_m = p.cmajor ? up16(8 * w) : up16(kDigits * p.hw);
+    const int half_x = p.cmajor ? half_m : up16((kDigits - 1) * p.hw);
+    p.nm = halves * half_m;
+    p.nx = halves * half_x;
+    p.set_rows = half_m;
+    if (p.nm > 256) return false;
+    p.acc_stride = (uint32_t)(rows ? p.nm + p.nx : p.nm);
+    p.nb = 2 * p.acc_stride + 4 * kAStage <= kTmemCols ? 2 : 1;
+    p.a0 = (p.nb * p.acc_stride + 31) / 32 * 32;
+    p.sp = 4;
+    const int b_bytes = (rows ? 1 : 2) * p.set_rows * 128;
+    const int room = (kSmemMax - 1024 - kBarBytes - p.sp * kPackedBytes) / b_bytes;
+    p.sd = std::min(std::min(8, room), ((int)kTmemCols - (int)p.a0) / (int)kAStage);
+    if (p.sd < 4) return false;
+    p.smem = (size_t)p.sd * b_bytes + (size_t)p.sp * kPackedBytes + kBarBytes + 1024;
+    return true;
+}
+
+// K slices: the count (at most 1024 K-blocks and a multiple of four in each) with the shortest
+// last finisher, a unit costing its K-blocks plus the fill and drain of its pipeline.
+void choose_slices(SlicePlan& p, int64_t units, int kb, int ctas) {
+    double best = 1e300;
+    for (int s = 1; s <= 64; ++s) {
+        int kbs = (kb + s - 1) / s;
+        kbs = (kbs + kPackedKb - 1) / kPackedKb * kPackedKb;
+        if (kbs > kMaxKbPerAccum) continue;
+        const int real = (kb + kbs - 1) / kbs;
+        if (real != s) continue;
+        const double waves = std::ceil((double)units * real / ctas);
+        const double cost = waves * (kbs + 6.0) + 0.25 * real;
+        if (cost < best) {
+            best = cost;
+            p.splits = real;
+            p.kbs = kbs;
+        }
+    }
+    if (best >= 1e300) {  // more than 64 slices of 1024
+        p.kbs = kMaxKbPerAccum;
+        p.splits = (kb + p.kbs - 1) / p.kbs;
+        best = std::ceil((double)units * p.splits / ctas) * (p.kbs + 6.0);
+    }
+    p.cost = best;
+}
+
+// The plan with the least estimated time.  A K-block costs its MMAs (N / 2 clocks for each of
+// 4 + 4 instructions on a CTA) or its decode, whichever is longer.
+SlicePlan choose_slice_plan(bool rows, int64_t tiles, int kb, int64_t k) {
+    SlicePlan best;
+    best.cost = 1e300;
+    auto consider = [&](bool pair, int w) {
+        SlicePlan p;
+        if (!lay_out(rows, pair, w, k, p)) return;
+        const int ctas = pair ? num_sms() / 2 : num_sms();
+        choose_slices(p, (pair ? tiles / 2 : tiles) * p.n_ctiles, kb, ctas);
+        const double mma = 2.0 * (rows ? p.nm + p.nx : 2 * p.nm);
+        // a single CTA streams all B rows from L2 itself
+        const double l2 = (pair ? 0.5 : 1.0) * (rows ? 1 : 2) * p.nm * 128.0 / 28.0;
+        p.cost *= std::max(std::max(mma, l2), pair ? 420.0 : 380.0);
+        if (p.cost < best.cost) best = p;
+    };
+    if (k <= 4) {
+        consider(false, (int)k);
+    } else {
+        for (int w = 8; w <= 32; w += 8) consider(false, w);
+        if (num_sms() >= 2)
+            for (int w = 16; w <= 32; w += 16) consider(true, w);
+    }
+    return best;
+}
+
+// Decoder groups: single CTAs are bound by the decode, pairs by the MMAs.
+constexpr int kSingleGroups = 4, kPairGroups = 2;
+template <bool PAIR>
+constexpr int groups_of() { return PAIR ? kPairGroups : kSingleGroups; }
+
+template <bool ROWS, bool PAIR>
+cudaError_t allow_smem() {
+    return cudaFuncSetAttribute(k_slice_pass<ROWS, PAIR, groups_of<PAIR>()>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kSmemMax);
+}
+
+void configure_slices() {
+    static PerDeviceOnce configured;
+    once_per_device(configured, [] {
+        cudaError_t e = allow_smem<true, false>();
+        if (e == cudaSuccess) e = allow_smem<false, false>();
+        if (e == cudaSuccess) e = allow_smem<true, true>();
+        if (e == cudaSuccess) e = allow_smem<false, true>();
+        return e;
+    }, "configure slice kernels");
+}
+
+template <bool ROWS, bool PAIR>
+void launch_slice_pass(const SlicePlan& p, const CUtensorMap& ta, const CUtensorMap& tb,
+                       const SliceArgs& A, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(threads_for(groups_of<PAIR>()));
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    if constexpr (PAIR) {
+        cfg.gridDim = dim3((unsigned)(num_sms() & ~1));
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        // as many pairs as are resident together (an SM without a partner in its GPC stays idle)
+        static int resident[PerDeviceOnce::kMaxDevices] = {};
+        int dev = 0;
+        CS_CUDA(cudaGetDevice(&dev));
+        int& pairs = resident[dev];
+        if (pairs == 0) {
+            cudaLaunchConfig_t probe = cfg;
+            probe.dynamicSmemBytes = kSmemMax;
+            int c = 0;
+            CS_CUDA(cudaOccupancyMaxActiveClusters(&c, k_slice_pass<ROWS, true, kPairGroups>, &probe));
+            pairs = std::max(1, std::min(c, num_sms() / 2));
+        }
+        cfg.gridDim = dim3((unsigned)(2 * pairs));
+    } else {
+        cfg.gridDim = dim3((unsigned)std::min<int64_t>(
+            num_sms(), std::max<int64_t>(1, (int64_t)A.n_tiles * A.n_ctiles * A.n_splits)));
+    }
+    CS_CUDA(cudaLaunchKernelEx(&cfg, k_slice_pass<ROWS, PAIR, groups_of<PAIR>()>, ta, tb, A));
+}
+
+}  // namespace
+
+struct SliceOperator {
+    DeviceBuffer<int8_t> b;
+    DeviceBuffer<double> part, W;
+    DeviceBuffer<unsigned long long> words;  // SliceCall's
+    // packed rows and their sample-major copy, 128 rows x 128 bytes at a time (both belong to the
+    // operator and keep their place for its lifetime)
+    CUtensorMap tm_packed{}, tm_packed_t{};
+    bool map_rows = false, map_samples = false;
+};
+
+void destroy_slices(SliceOperator* s) { delete s; }
+
+namespace {
+
+// Columns per call of the passes: bounds the operand buffers (14 bytes per row and column) and
+// keeps a K slice's digits in L2.
+constexpr int64_t kChunkColumns = 288;
+
+// One chunk of columns: the plans of the passes it runs and its cleared words (status: 8 words;
+// ranges of X and W: 4 a column; slice sums of both passes: 2 a column and slice).
+struct SliceCall {
+    SlicePlan rows, samples;
+    int64_t k = 0, range = 0, range_w = 0, sum = 0, sum_w = 0, words = 0;
+};
+
+SliceCall plan_call(const MixedRows& r, int64_t k) {
+    SliceCall c;
+    c.k = k;
+    c.rows = choose_slice_plan(true, r.r_pad / kTile, (int)(r.n_pad / kKBlock), k);
+    c.samples = choose_slice_plan(false, r.n_pad / kTile, (int)(r.r_pad / kKBlock), k);
+    c.range = 8;
+    c.range_w = c.range + 4 * k;
+    c.sum = c.range_w + 4 * k;
+    c.sum_w = c.sum + 2 * k * c.rows.splits;
+    c.words = c.sum_w + 2 * k * c.samples.splits;
+    return c;
+}
+
+SliceSums sums_of(SliceOperator& so, const SliceCall& c) {
+    unsigned long long* z = so.words.get();
+    SliceSums S;
+    S.status = reinterpret_cast<int*>(z);
+    S.range = reinterpret_cast<ColumnRange*>(z + c.range);
+    S.range_w = reinterpret_cast<ColumnRange*>(z + c.range_w);
+    S.sum = z + c.sum;
+    S.sum_w = z + c.sum_w;
+    S.splits = c.rows.splits;
+    S.splits_w = c.samples.splits;
+    return S;
+}
+
+void reserve(SliceOperator& so, const MixedRows& r, const SliceCall& c) {
+    so.b.resize(std::max(c.rows.b_rows(true) * r.n_pad, c.samples.b_rows(false) * r.r_pad));
+    so.part.resize(c.k * std::max(c.rows.splits * r.r_pad, c.samples.splits * r.n_pad));
+    so.W.resize(r.R * c.k);
+    so.words.resize(c.words);
+}
+
+SliceArgs slice_args(const SlicePlan& p, bool rows, int64_t tiles, int kb, int64_t k) {
+    SliceArgs A{};
+    A.n_tiles = (int)tiles;
+    A.n_ctiles = p.n_ctiles;
+    A.n_splits = p.splits;
+    A.kb_total = (kb + kPackedKb - 1) / kPackedKb * kPackedKb;  // past the operand's end: zeros
+    A.kb_per_split = p.kbs;
+    A.k = (int)k;
+    A.w = p.w;
+    A.hw = p.hw;
+    A.cmajor = p.cmajor;
+    A.nm = p.nm;
+    A.nx = rows ? p.nx : p.nm;
+    A.set_rows = p.set_rows;
+    A.sp = p.sp;
+    A.sd = p.sd;
+    A.nb = p.nb;
+    A.acc_stride = p.acc_stride;
+    A.a0 = p.a0;
+    A.poll_ns = 128;
+    A.poll_dec_ns = 32;
+    return A;
+}
+
+// The sums of the rows pass of one chunk (X's digits, then the pass) into so.part.
+void run_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSums& S, StridedIn X,
+              cudaStream_t s) {
+    const int64_t n = r.n, R = r.R, k = c.k;
+    const SlicePlan& p = c.rows;
+    const int64_t k_pad = (int64_t)p.n_ctiles * p.w;
+    const BLayout B = p.blayout(true);
+    const int slice_rows = p.kbs * kKBlock;
+    if (n <= kWholeRows && p.splits <= 64) {
+        prof::Scope ps("slice_prep_rows_operand", s, 0.0, 16.0 * n * k + 7.0 * k_pad * r.n_pad);
+        const unsigned threads = (unsigned)round_up(r.n_pad / 16, 32);
+        k_slice_rows_operand_whole<<<(unsigned)k_pad, threads, 0, s>>>(X, n, k, r.n_pad, slice_rows, S, B,
+                                                                   so.b.get());
+        CS_LAUNCH("slice rows operand");
+    } else {
+        CS_CUDA(cudaMemsetAsync(so.words.get(), 0, 8 * c.words, s));
+        prof::Scope ps("slice_prep_rows_operand", s, 0.0, 16.0 * n * k + 7.0 * k_pad * r.n_pad);
+        int kc = 1;
+        while (X.rs != 1 && kc < k && kc < 32) kc *= 2;
+        const int64_t rpb = std::max<int64_t>(256, 4096 / kc);
+        k_slice_ranges<<<dim3((unsigned)((n + rpb - 1) / rpb), (unsigned)((k + kc - 1) / kc)), 256, 0, s>>>(
+            X, n, k, kc, rpb, S.range);
+        if (k_pad <= 1)
+            k_slice_rows_operand<1, 1024><<<dim3((unsigned)((r.n_pad + 1023) / 1024), 1), 64, 0, s>>>(
+                X, n, k, k_pad, r.n_pad, slice_rows, S, B, so.b.get());
+        else if (k_pad <= 4)
+            k_slice_rows_operand<4, 512><<<dim3((unsigned)((r.n_pad + 511) / 512), 1), 128, 0, s>>>(
+                X, n, k, k_pad, r.n_pad, slice_rows, S, B, so.b.get());
+        else
+            k_slice_rows_operand<16, 256><<<dim3((unsigned)(r.n_pad / 256), (unsigned)((k_pad + 15) / 16)),
+                                            256, 0, s>>>(X, n, k, k_pad, r.n_pad, slice_rows, S, B,
+                                                         so.b.get());
+        CS_LAUNCH("slice rows operand");
+    }
+    const CUtensorMap tb = make_map_u8(so.b.get(), (uint64_t)r.n_pad, (uint64_t)p.b_rows(true),
+                                       (uint64_t)r.n_pad, kKBlock, (uint32_t)p.set_rows, true);
+    SliceArgs A = slice_args(p, true, r.r_pad / kTile, (int)(r.n_pad / kKBlock), k);
+    A.lut = r.lut.get();
+    A.mu = r.mu.get();
+    A.ksum = reinterpret_cast<const longlong2*>(S.sum);
+    A.part = so.part.get();
+    A.ld = r.r_pad;
+    A.status = S.status;
+    prof::Scope ps("kinship_rows_slices", s, 2.0 * (double)n * (double)R * (double)k,
+                   (double)R * (double)((n + 3) / 4));
+    if (p.pair)
+        launch_slice_pass<true, true>(p, so.tm_packed, tb, A, s);
+    else
+        launch_slice_pass<true, false>(p, so.tm_packed, tb, A, s);
+    CS_LAUNCH("kinship_rows_slices");
+}
+
+// Y (n x k) = scale Z_c W of one chunk, from so.W and its ranges.
+void run_samples(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSums& S, double scale,
+                 StridedOut Y, cudaStream_t s) {
+    const int64_t n = r.n, R = r.R, k = c.k;
+    const SlicePlan& p = c.samples;
+    const int64_t k_pad = (int64_t)p.n_ctiles * p.w;
+    {
+        prof::Scope ps("slice_prep_samples_operand", s, 0.0, 8.0 * R * k + 14.0 * k_pad * r.r_pad);
+        k_slice_samples_operand<<<dim3((unsigned)((r.r_pad + 2047) / 2048), (unsigned)k_pad), 128, 0, s>>>(
+            so.W.get(), R, k, r.r_pad, p.kbs * kKBlock, r.mu.get(), S, p.blayout(false), so.b.get());
+        CS_LAUNCH("slice samples operand");
+    }
+    const CUtensorMap tb = make_map_u8(so.b.get(), (uint64_t)r.r_pad, (uint64_t)p.b_rows(false),
+                                       (uint64_t)r.r_pad, kKBlock, (uint32_t)p.set_rows, true);
+    SliceArgs A = slice_args(p, false, r.n_pad / kTile, (int)(r.r_pad / kKBlock), k);
+    A.ksum = reinterpret_cast<const longlong2*>(S.sum_w);
+    A.part = so.part.get();
+    A.ld = r.n_pad;
+    A.status = S.status;
+    {
+        prof::Scope ps("kinship_samples_slices", s, 2.0 * (double)n * (double)R * (double)k,
+                       (double)R * (double)((n + 3) / 4));
+        if (p.pair)
+            launch_slice_pass<false, true>(p, so.tm_packed_t, tb, A, s);
+        else
+            launch_slice_pass<false, false>(p, so.tm_packed_t, tb, A, s);
+        CS_LAUNCH("kinship_samples_slices");
+    }
+    prof::Scope ps("slice_reduce_samples", s, 0.0, 8.0 * (p.splits + 1) * (double)k * n);
+    k_slice_reduce_samples<<<dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)), 256, 0, s>>>(
+        so.part.get(), r.n_pad, n, k, so.W.get(), R, r.mu.get(), PackedRows{r.rows, r.stride}, S, scale, Y);
+    CS_LAUNCH("slice_reduce_samples");
+}
+
+// W (Wt) or s o u at the rows' positions (out) from the sums of run_rows.
+void finish_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSums& S, StridedIn X,
+                 double* Wt, const int32_t* pos, StridedOut out, cudaStream_t s) {
+    prof::Scope ps("slice_reduce_rows", s, 0.0, 8.0 * (c.rows.splits + 1) * (double)c.k * r.R);
+    k_slice_reduce_rows<<<dim3((unsigned)((r.R + 1023) / 1024), (unsigned)c.k), 256, 0, s>>>(
+        so.part.get(), r.r_pad, r.R, c.k, r.s.get(), r.mu.get(), PackedRows{r.rows, r.stride}, X, r.n, S,
+        Wt, pos, out);
+    CS_LAUNCH("slice_reduce_rows");
+}
+
+// The operator's slice state with room for k columns, or null (no sample-major copy allowed, or no
+// device memory for it or for the operands).  The slices are taken at every shape: against the
+// FP64-pipe kernels an apply took (us) 36 / 99 at n=40, M=1000 and one column, 52 / 152 at n=2000,
+// M=10000, 950 / 7210 at n=50000, M=100000; 56 / 187, 110 / 470 and 212 / 954 at n=2000, M=10000 and
+// 8, 80 and 200 columns; 2570 / 23480 at n=18009, M=27006 and 266.
+SliceOperator* slices_for(cs_kinship* op, int64_t k, bool samples, cudaStream_t s) {
+    const int64_t R = op->n_active;
+    if (!op->sample_major_copy || op->slices_unavailable || R == 0 || k <= 0) return nullptr;
+    try {
+        MixedRows& r = mixed_rows_for(op);
+        configure_slices();
+        if (!op->slices) op->slices = new SliceOperator();
+        SliceOperator& so = *op->slices;
+        if (!so.map_rows) {
+            so.tm_packed = make_map_u8(r.rows, r.stride, R, r.stride, 128, kTile, true);
+            so.map_rows = true;
+        }
+        if (samples) ensure_transposed(r, s);
+        if (samples && !so.map_samples) {
+            so.tm_packed_t = make_map_u8(r.packed_t.get(), r.r_pad / 4, r.n_pad, r.r_pad / 4, 128, kTile, true);
+            so.map_samples = true;
+        }
+        if (k >= kChunkColumns) reserve(so, r, plan_call(r, kChunkColumns));
+        if (k % kChunkColumns) reserve(so, r, plan_call(r, k % kChunkColumns));
+        return &so;
+    } catch (const Error&) {
+        // the FP64-pipe kernels need neither the copy nor the operands
+        destroy_slices(op->slices);
+        op->slices = nullptr;
+        op->slices_unavailable = true;
+        return nullptr;
+    }
+}
+
+template <class Chunk>
+void for_chunks(const MixedRows& r, int64_t k, Chunk&& chunk) {
+    for (int64_t c0 = 0; c0 < k; c0 += kChunkColumns)
+        chunk(c0, plan_call(r, std::min(kChunkColumns, k - c0)));
+}
+
+StridedIn from_column(StridedIn m, int64_t c) { return StridedIn{m.p + c * m.cs, m.rs, m.cs}; }
+StridedOut from_column(StridedOut m, int64_t c) { return StridedOut{m.p + c * m.cs, m.rs, m.cs}; }
+
+}  // namespace
+
+bool kinship_apply_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut Y, cudaStream_t s) {
+    SliceOperator* so = slices_for(op, k, true, s);
+    if (!so) return false;
+    MixedRows& r = mixed_rows_for(op);
+    for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
+        const SliceSums S = sums_of(*so, c);
+        const StridedIn x = from_column(X, c0);
+        run_rows(*so, r, c, S, x, s);
+        finish_rows(*so, r, c, S, x, so->W.get(), nullptr, StridedOut{}, s);
+        run_samples(*so, r, c, S, 1.0 / (double)op->num_variants, from_column(Y, c0), s);
+    });
+    return true;
+}
+
+bool multiply_zt_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut U, cudaStream_t s) {
+    SliceOperator* so = slices_for(op, k, false, s);
+    if (!so) return false;
+    MixedRows& r = mixed_rows_for(op);
+    for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
+        const SliceSums S = sums_of(*so, c);
+        const StridedIn x = from_column(X, c0);
+        run_rows(*so, r, c, S, x, s);
+        finish_rows(*so, r, c, S, x, nullptr, op->d_view_pos.get(), from_column(U, c0), s);
+    });
+    return true;
+}
+
+bool multiply_z_slices(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cudaStream_t s) {
+    SliceOperator* so = slices_for(op, k, true, s);
+    if (!so) return false;
+    MixedRows& r = mixed_rows_for(op);
+    for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
+        const SliceSums S = sums_of(*so, c);
+        CS_CUDA(cudaMemsetAsync(so->words.get(), 0, 8 * c.words, s));
+        {
+            prof::Scope ps("slice_gather", s, 0.0, 16.0 * r.R * c.k);
+            k_slice_gather<<<dim3((unsigned)((r.R + 1023) / 1024), (unsigned)c.k), 256, 0, s>>>(
+                from_column(V, c0), r.R, op->d_view_pos.get(), r.s.get(), r.mu.get(), S, so->W.get());
+            CS_LAUNCH("slice_gather");
+        }
+        run_samples(*so, r, c, S, 1.0, from_column(Y, c0), s);
+    });
+    return true;
+}
+
+void check_slices(cs_kinship* op, cudaStream_t s) {
+    if (!op->slices || !op->slices->words.get()) return;
+    int status = 0;
+    CS_CUDA(cudaMemcpyAsync(&status, op->slices->words.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    CS_CUDA(cudaStreamSynchronize(s));
+    if (status != kPassStatusOk)
+        fail(CS_ERR_CUDA, "tensor-core kinship kernel gave up waiting (status " + std::to_string(status) + ")");
+}
+
+}  // namespace cs

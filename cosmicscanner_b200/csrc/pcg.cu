@@ -486,6 +486,8 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
         }
         CS_CUDA(cudaMemcpyAsync(rr_h.data(), ws.rr.get(), 8 * ka, cudaMemcpyDeviceToHost, s));
         CS_CUDA(cudaStreamSynchronize(s));
+        for (int64_t c = 0; c < ka; ++c)
+            if (std::isnan(rr_h[c])) check_slices(A.op, s);  // an apply that gave up leaves NaN
         std::vector<int32_t> keep_pos;
         for (int64_t c = 0; c < ka; ++c) {
             st.iterations[map[c]] = it + 1;

@@ -1,0 +1,62 @@
+// The FP64 kinship products on the int8 tensor cores (kinship_slices.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "cs_internal.h"
+
+namespace cs {
+
+// Range of a column's values: the bits of max |x| (NaN and infinity compare above every finite
+// value) and the exponents of the nonzero |x|, summed and counted.  All integers, so the
+// atomics that gather them are order independent.
+struct ColumnRange {
+    unsigned long long max_bits;
+    long long exp_sum;
+    unsigned long long count;
+    unsigned long long pad;
+};
+
+// A fixed-point column of 55 bits below its maximum holds every element to 2^-55 of that
+// maximum.  Normwise that is always finer than FP64 sums are (max <= sqrt(n) rms), but a row
+// whose large elements all meet missing calls depends on the small ones alone, so a column
+// whose elements lie on average more than 2^kSliceRange below its maximum is computed on the FP64
+// pipe, like one with a non-finite value or a maximum near the ends of the exponent range.  A
+// normal sample of 50,000 lies 2^3 below its maximum; W = s^2 o Z^T X down to a minor allele
+// frequency of 0.01 at most 2^4 more.
+constexpr int kSliceRange = 10;
+constexpr int kSliceMaxExp = 960;
+
+__device__ __forceinline__ bool range_excluded(const ColumnRange& r) {
+    const int ex = (int)(r.max_bits >> 52) - 1023;
+    if (ex > kSliceMaxExp) return true;                       // NaN, infinity, huge
+    if (r.count == 0) return false;                           // all zero
+    if (ex < -kSliceMaxExp) return true;
+    return (long long)ex * (long long)r.count - r.exp_sum > (long long)kSliceRange * (long long)r.count;
+}
+
+struct SliceOperator;
+void destroy_slices(SliceOperator* s);
+
+// A matrix operand with element (i, c) at p[i * rs + c * cs]: row-major (cs = 1) or column-major
+// (rs = 1).
+struct StridedIn {
+    const double* p;
+    int64_t rs, cs;
+};
+struct StridedOut {
+    double* p;
+    int64_t rs, cs;
+};
+
+// FP64 products through the slices where the operator has (or may have) a sample-major copy and
+// the shape is large enough; false when the FP64-pipe kernels are to be used.  Results may
+// overwrite the input.
+// Y (rows x k) = K X.
+bool kinship_apply_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut Y, cudaStream_t s);
+// U (selected variants x k; rows of inactive variants are left alone) = Z^T X.
+bool multiply_zt_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut U, cudaStream_t s);
+// Y (rows x k) = Z V, V (selected variants x k).
+bool multiply_z_slices(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cudaStream_t s);
+
+}  // namespace cs

@@ -343,6 +343,33 @@ __device__ __forceinline__ bool mbar_poll_cluster(uint64_t* bar, uint32_t parity
     atomicCAS(status, kOk, code);
     return false;
 }
+// The bounded waits with one look at the barrier ahead of the loop, which stands out of line: a wait
+// on a phase that is complete costs 70 clocks so, 115 to 195 with the loop in its place (one warp
+// timed alone).
+static __device__ __noinline__ bool mbar_wait_loop(uint64_t* bar, uint32_t parity, int* status,
+                                                   int code, uint32_t limit) {
+    return mbar_wait(bar, parity, status, code, limit);
+}
+static __device__ __noinline__ bool mbar_poll_sleep_loop(uint64_t* bar, uint32_t parity, int* status,
+                                                         int code, uint32_t ns, uint32_t limit) {
+    return mbar_poll_sleep(bar, parity, status, code, ns, limit);
+}
+static __device__ __noinline__ bool mbar_poll_cluster_loop(uint64_t* bar, uint32_t parity, int* status,
+                                                           int code, uint32_t limit) {
+    return mbar_poll_cluster(bar, parity, status, code, limit);
+}
+__device__ __forceinline__ bool mbar_wait_look(uint64_t* bar, uint32_t parity, int* status, int code,
+                                               uint32_t limit = (1u << 24)) {
+    return mbar_try_wait(bar, parity) || mbar_wait_loop(bar, parity, status, code, limit);
+}
+__device__ __forceinline__ bool mbar_poll_sleep_look(uint64_t* bar, uint32_t parity, int* status,
+                                                     int code, uint32_t ns, uint32_t limit = (1u << 26)) {
+    return mbar_test_wait(bar, parity) || mbar_poll_sleep_loop(bar, parity, status, code, ns, limit);
+}
+__device__ __forceinline__ bool mbar_poll_cluster_look(uint64_t* bar, uint32_t parity, int* status,
+                                                       int code, uint32_t limit = (1u << 26)) {
+    return mbar_test_wait_cluster(bar, parity) || mbar_poll_cluster_loop(bar, parity, status, code, limit);
+}
 // Every thread of both CTAs.
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
