@@ -187,21 +187,31 @@ struct cs_kinship {
 
 namespace cs {
 
+// A matrix operand with element (i, c) at p[i * rs + c * cs]: row-major (cs = 1) or column-major
+// (rs = 1).
+template <class T>
+struct Strided {
+    T* p;
+    int64_t rs, cs;
+};
+using StridedIn = Strided<const double>;
+using StridedOut = Strided<double>;
+
 // Y_rm (rows x ldy) = K X_rm (rows x ldx), both row-major device buffers, k columns.
 // Y may equal X.  precision: CS_PRECISION_*.
 void kinship_apply_rowmajor(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* Y,
                             int64_t ldy, int precision, cudaStream_t s);
-void kinship_apply_mixed(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* Y,
-                         int64_t ldy, cudaStream_t s);
+// The tensor-core form on operands of either layout; T is double, or float for callers that keep
+// their vectors in single precision (FP64 inside, one rounding of the result).  Y may be X.
+template <class T>
+void kinship_apply_mixed(cs_kinship* op, Strided<const T> X, int64_t k, Strided<T> Y, cudaStream_t s);
 // The rows-pass output of the last mixed apply: W (R x k, column-major, ld R) with
 // W[t, c] = s_t^2 sum_i (G_ti - mu_t)[observed] x_ic; nullptr before any mixed apply.
 const double* mixed_rows_output(const cs_kinship* op, int64_t* R, int64_t* k);
-// GenotypeMatrix half-passes on tensor cores over the view rows: U (R x k, row-major) = Z^T X,
-// and Y (rows x k, row-major) = Z V given W = s o V column-major (R x k).
-void mixed_multiply_zt(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* U,
-                       int64_t ldu, cudaStream_t s);
-void mixed_multiply_z(cs_kinship* op, const double* Wcol, int64_t k, double* Y, int64_t ldy,
-                      cudaStream_t s);
+// GenotypeMatrix half-passes on tensor cores: U (selected variants x k; rows of variants dropped
+// from the view are left alone) = Z^T X, and Y (rows x k) = Z V.
+void mixed_multiply_zt(cs_kinship* op, StridedIn X, int64_t k, StridedOut U, cudaStream_t s);
+void mixed_multiply_z(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cudaStream_t s);
 
 // Waits for the stream and fails if the operator's last FP64 tensor-core pass gave up waiting (its
 // results are NaN; kinship_slices.cu).

@@ -174,7 +174,7 @@ void kinship_apply_rowmajor(cs_kinship* op, const double* X, int64_t ldx, int64_
                             int64_t ldy, int precision, cudaStream_t s) {
     if (k <= 0) return;
     if (precision == CS_PRECISION_MIXED)
-        kinship_apply_mixed(op, X, ldx, k, Y, ldy, s);
+        kinship_apply_mixed(op, StridedIn{X, ldx, 1}, k, StridedOut{Y, ldy, 1}, s);
     else if (precision == CS_PRECISION_FP64)
         kinship_apply_fp64(op, X, ldx, k, Y, ldy, s);
     else
@@ -202,6 +202,13 @@ __global__ void k_f64row_to_f32col(const double* __restrict__ src, int64_t n, in
     }
 }
 
+// Whether two column-major blocks (ld, rows x k) share memory.
+template <class T>
+static bool overlap(const T* a, int64_t lda, int64_t rows_a, const T* b, int64_t ldb, int64_t rows_b,
+                    int64_t k) {
+    return a < b + (k - 1) * ldb + rows_b && b < a + (k - 1) * lda + rows_a;
+}
+
 // FP32 apply (device pointers): the inputs widened to FP64, the FP64 or mixed apply, the
 // result rounded to FP32.  Y may alias X.
 void kinship_apply_f32(cs_kinship* op, const float* X, int64_t ldx, int64_t k, float* Y,
@@ -211,6 +218,12 @@ void kinship_apply_f32(cs_kinship* op, const float* X, int64_t ldx, int64_t k, f
     if (ldx < op->rows || ldy < op->rows)
         fail(CS_ERR_INVALID_ARGUMENT, "PlinkKinshipOperator::apply: dimension mismatch");
     const int64_t n = op->rows;
+    // the tensor-core form reads and writes float columns itself
+    if (precision == CS_PRECISION_MIXED &&
+        ((X == Y && ldx == ldy) || !overlap(X, ldx, n, Y, ldy, n, k))) {
+        kinship_apply_mixed(op, Strided<const float>{X, 1, ldx}, k, Strided<float>{Y, 1, ldy}, s);
+        return;
+    }
     op->buf_x.resize(n * k);
     op->buf_y.resize(n * k);
     const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n * k + 255) / 256, 32LL * num_sms()));
@@ -227,13 +240,19 @@ void kinship_apply_f32(cs_kinship* op, const float* X, int64_t ldx, int64_t k, f
     }
 }
 
-// Whether two column-major blocks (ld, rows x k) share memory.
-static bool overlap(const double* a, int64_t lda, int64_t rows_a, const double* b, int64_t ldb,
-                    int64_t rows_b, int64_t k) {
-    return a < b + (k - 1) * ldb + rows_b && b < a + (k - 1) * lda + rows_a;
+// A column-major input as the kernels read it: as it is, or, where the output overlaps it (other
+// than in its place, with `in_place`), from a copy.
+static StridedIn apart(cs_kinship* op, const double* X, int64_t ldx, int64_t rows_x, const double* Y,
+                       int64_t ldy, int64_t rows_y, int64_t k, bool in_place, cudaStream_t s) {
+    if ((in_place && X == Y && ldx == ldy) || !overlap(X, ldx, rows_x, Y, ldy, rows_y, k))
+        return StridedIn{X, 1, ldx};
+    op->buf_x.resize(rows_x * k);
+    colmajor_to_rowmajor(X, ldx, rows_x, k, op->buf_x.get(), k, s);
+    return StridedIn{op->buf_x.get(), k, 1};
 }
 
-// Public column-major apply (device pointers): transposes in and out around the kernels.
+// Public column-major apply (device pointers).  The tensor-core kernels read and write column-major
+// blocks themselves; the FP64-pipe kernels work between transposes.
 void kinship_apply_colmajor(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* Y,
                             int64_t ldy, int precision, cudaStream_t s) {
     if (k < 0) fail(CS_ERR_INVALID_ARGUMENT, "negative column count");
@@ -241,12 +260,14 @@ void kinship_apply_colmajor(cs_kinship* op, const double* X, int64_t ldx, int64_
     if (ldx < op->rows || ldy < op->rows)
         fail(CS_ERR_INVALID_ARGUMENT, "PlinkKinshipOperator::apply: dimension mismatch");
     const int64_t n = op->rows;
-    // the slice kernels read and write column-major as it is (Y in X's place included; blocks that
-    // overlap in another way go through the copies below)
-    if (precision == CS_PRECISION_FP64 &&
-        ((X == Y && ldx == ldy) || !overlap(X, ldx, n, Y, ldy, n, k)) &&
-        kinship_apply_slices(op, StridedIn{X, 1, ldx}, k, StridedOut{Y, 1, ldy}, s))
-        return;
+    if (precision == CS_PRECISION_MIXED || precision == CS_PRECISION_FP64) {
+        const StridedIn x = apart(op, X, ldx, n, Y, ldy, n, k, true, s);
+        if (precision == CS_PRECISION_MIXED) {
+            kinship_apply_mixed(op, x, k, StridedOut{Y, 1, ldy}, s);
+            return;
+        }
+        if (kinship_apply_slices(op, x, k, StridedOut{Y, 1, ldy}, s)) return;
+    }
     op->buf_x.resize(n * k);
     op->buf_y.resize(n * k);
     colmajor_to_rowmajor(X, ldx, n, k, op->buf_x.get(), k, s);
@@ -272,21 +293,14 @@ __global__ void k_scatter_rows(const double* __restrict__ in, int64_t ldi, int64
     }
 }
 
-// FP64 operand: W[t * k + c] = V[pos[t] * ldv + c]; tensor-core operand (column-major,
-// s-scaled): W[c * R + t] = s_t V[pos[t] * ldv + c].
+// W[t * k + c] = V[pos[t] * ldv + c].
 __global__ void k_gather_rows(const double* __restrict__ V, int64_t ldv, int64_t R, int64_t k,
-                              const int32_t* __restrict__ pos, const double* __restrict__ s_row,
-                              double* __restrict__ W, int colmajor) {
+                              const int32_t* __restrict__ pos, double* __restrict__ W) {
     const int64_t total = R * k;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
-        if (colmajor) {
-            const int64_t c = idx / R, t = idx - c * R;
-            W[idx] = s_row[t] * V[(int64_t)pos[t] * ldv + c];
-        } else {
-            const int64_t t = idx / k, c = idx - t * k;
-            W[idx] = V[(int64_t)pos[t] * ldv + c];
-        }
+        const int64_t t = idx / k, c = idx - t * k;
+        W[idx] = V[(int64_t)pos[t] * ldv + c];
     }
 }
 
@@ -294,86 +308,85 @@ static unsigned grid_for(int64_t work) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + 255) / 256, 32LL * num_sms()));
 }
 
-// U (numVariants x k, row-major ldu) = Z^T X for X (rows x k, row-major ldx).
-void genotype_multiply_zt_rowmajor(cs_kinship* op, const double* X, int64_t ldx, int64_t k,
-                                   double* U, int64_t ldu, int precision, cudaStream_t s) {
-    const int64_t R = op->n_active, nv = op->num_variants;
-    CS_CUDA(cudaMemset2DAsync(U, ldu * 8, 0, k * 8, nv, s));
-    if (R == 0 || k == 0) return;
-    op->buf_u.resize(R * k);
-    if (precision == CS_PRECISION_MIXED)
-        mixed_multiply_zt(op, X, ldx, k, op->buf_u.get(), k, s);
-    else if (precision == CS_PRECISION_FP64)
-        decode_gemm_rows_fp64(op->view, op->d_lut.get(), X, ldx, k, op->buf_u.get(), k, op->ws, s);
-    else
-        fail(CS_ERR_INVALID_ARGUMENT, "unknown precision mode");
-    prof::Scope ps("scatter_rows", s, 0.0, 16.0 * R * k);
-    k_scatter_rows<<<grid_for(R * k), 256, 0, s>>>(op->buf_u.get(), k, R, k, op->d_view_pos.get(),
-                                                   U, ldu);
-    CS_LAUNCH("scatter_rows");
-}
-
-// Y (rows x k, row-major ldy) = Z V for V (numVariants x k, row-major ldv).
-void genotype_multiply_z_rowmajor(cs_kinship* op, const double* V, int64_t ldv, int64_t k,
-                                  double* Y, int64_t ldy, int precision, cudaStream_t s) {
-    const int64_t R = op->n_active;
-    if (k == 0) return;
-    if (R == 0) {
-        CS_CUDA(cudaMemset2DAsync(Y, ldy * 8, 0, k * 8, op->rows, s));
-        return;
-    }
+// Column-major public forms (device pointers), on the tensor cores or, where those kernels are not
+// available, the FP64 pipe between transposes.
+static void require_precision(int precision) {
     if (precision != CS_PRECISION_MIXED && precision != CS_PRECISION_FP64)
         fail(CS_ERR_INVALID_ARGUMENT, "unknown precision mode");
-    const bool mixed = precision == CS_PRECISION_MIXED;
-    op->buf_u.resize(R * k);
-    {
-        prof::Scope ps("gather_rows", s, 0.0, 16.0 * R * k);
-        k_gather_rows<<<grid_for(R * k), 256, 0, s>>>(V, ldv, R, k, op->d_view_pos.get(),
-                                                      op->d_inv_std.get(), op->buf_u.get(),
-                                                      mixed ? 1 : 0);
-        CS_LAUNCH("gather_rows");
-    }
-    if (mixed)
-        mixed_multiply_z(op, op->buf_u.get(), k, Y, ldy, s);
-    else
-        decode_gemm_samples_fp64(op->view, op->d_lut.get(), op->buf_u.get(), k, k, Y, ldy, 1.0,
-                                 op->ws, s);
 }
 
-// Column-major public forms (device pointers): transposes around the row-major passes.
+// U (numVariants x k) = Z^T X.
 void genotype_multiply_zt(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* U,
                           int64_t ldu, int precision, cudaStream_t s) {
     if (k < 0) fail(CS_ERR_INVALID_ARGUMENT, "negative column count");
     if (ldx < op->rows || ldu < op->num_variants)
         fail(CS_ERR_INVALID_ARGUMENT, "Dimension mismatch in multiply_Zt_v");
     if (k == 0) return;
-    const int64_t n = op->rows, nv = op->num_variants;
-    if (precision == CS_PRECISION_FP64 && !overlap(X, ldx, n, U, ldu, nv, k)) {
-        // rows of variants the view dropped (1/sd == 0) stay zero
-        if (op->n_active < nv) CS_CUDA(cudaMemset2DAsync(U, ldu * 8, 0, nv * 8, k, s));
-        if (multiply_zt_slices(op, StridedIn{X, 1, ldx}, k, StridedOut{U, 1, ldu}, s)) return;
+    const int64_t n = op->rows, nv = op->num_variants, R = op->n_active;
+    // rows of variants the view dropped (1/sd == 0) are zero
+    auto clear = [&] { CS_CUDA(cudaMemset2DAsync(U, ldu * 8, 0, nv * 8, k, s)); };
+    if (R == 0) {
+        clear();
+        return;
     }
-    op->buf_x.resize(n * k);
+    require_precision(precision);
+    const StridedIn x = apart(op, X, ldx, n, U, ldu, nv, k, false, s);
+    if (R < nv) clear();
+    if (precision == CS_PRECISION_MIXED) {
+        mixed_multiply_zt(op, x, k, StridedOut{U, 1, ldu}, s);
+        return;
+    }
+    if (multiply_zt_slices(op, x, k, StridedOut{U, 1, ldu}, s)) return;
+    if (x.rs == 1) {
+        op->buf_x.resize(n * k);
+        colmajor_to_rowmajor(X, ldx, n, k, op->buf_x.get(), k, s);
+    }
+    op->buf_u.resize(R * k);
     op->buf_y.resize(nv * k);
-    colmajor_to_rowmajor(X, ldx, n, k, op->buf_x.get(), k, s);
-    genotype_multiply_zt_rowmajor(op, op->buf_x.get(), k, k, op->buf_y.get(), k, precision, s);
+    decode_gemm_rows_fp64(op->view, op->d_lut.get(), op->buf_x.get(), k, k, op->buf_u.get(), k, op->ws, s);
+    CS_CUDA(cudaMemsetAsync(op->buf_y.get(), 0, 8 * nv * k, s));
+    {
+        prof::Scope ps("scatter_rows", s, 0.0, 16.0 * R * k);
+        k_scatter_rows<<<grid_for(R * k), 256, 0, s>>>(op->buf_u.get(), k, R, k, op->d_view_pos.get(),
+                                                       op->buf_y.get(), k);
+        CS_LAUNCH("scatter_rows");
+    }
     rowmajor_to_colmajor(op->buf_y.get(), k, nv, k, U, ldu, s);
 }
 
+// Y (rows x k) = Z V.
 void genotype_multiply_z(cs_kinship* op, const double* V, int64_t ldv, int64_t k, double* Y,
                          int64_t ldy, int precision, cudaStream_t s) {
     if (k < 0) fail(CS_ERR_INVALID_ARGUMENT, "negative column count");
     if (ldv < op->num_variants || ldy < op->rows)
         fail(CS_ERR_INVALID_ARGUMENT, "Dimension mismatch in multiply_Z_v");
     if (k == 0) return;
-    const int64_t n = op->rows, nv = op->num_variants;
-    if (precision == CS_PRECISION_FP64 && !overlap(V, ldv, nv, Y, ldy, n, k) &&
-        multiply_z_slices(op, StridedIn{V, 1, ldv}, k, StridedOut{Y, 1, ldy}, s))
+    const int64_t n = op->rows, nv = op->num_variants, R = op->n_active;
+    if (R == 0) {
+        CS_CUDA(cudaMemset2DAsync(Y, ldy * 8, 0, n * 8, k, s));
         return;
-    op->buf_x.resize(nv * k);
+    }
+    require_precision(precision);
+    const StridedIn v = apart(op, V, ldv, nv, Y, ldy, n, k, false, s);
+    if (precision == CS_PRECISION_MIXED) {
+        mixed_multiply_z(op, v, k, StridedOut{Y, 1, ldy}, s);
+        return;
+    }
+    if (multiply_z_slices(op, v, k, StridedOut{Y, 1, ldy}, s)) return;
+    if (v.rs == 1) {
+        op->buf_x.resize(nv * k);
+        colmajor_to_rowmajor(V, ldv, nv, k, op->buf_x.get(), k, s);
+    }
+    op->buf_u.resize(R * k);
     op->buf_y.resize(n * k);
-    colmajor_to_rowmajor(V, ldv, nv, k, op->buf_x.get(), k, s);
-    genotype_multiply_z_rowmajor(op, op->buf_x.get(), k, k, op->buf_y.get(), k, precision, s);
+    {
+        prof::Scope ps("gather_rows", s, 0.0, 16.0 * R * k);
+        k_gather_rows<<<grid_for(R * k), 256, 0, s>>>(op->buf_x.get(), k, R, k, op->d_view_pos.get(),
+                                                      op->buf_u.get());
+        CS_LAUNCH("gather_rows");
+    }
+    decode_gemm_samples_fp64(op->view, op->d_lut.get(), op->buf_u.get(), k, k, op->buf_y.get(), k, 1.0,
+                             op->ws, s);
     rowmajor_to_colmajor(op->buf_y.get(), k, n, k, Y, ldy, s);
 }
 

@@ -720,31 +720,28 @@ k_mixed_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
 }
 
 // ---------------------------------------------------------------- operand preparation
-// All reductions here are deterministic: block-level trees in a fixed order, per-block
-// partials summed in block order, and maxima through atomicMax on non-negative doubles
-// (order independent).  Tiles are 32 columns x 64 rows so that row-major FP64 inputs are
-// read with coalesced 256-byte rows and column-major outputs written with coalesced runs.
-constexpr int kPrepCols = 32, kPrepRows = 64;
+// All reductions here are deterministic: FP64 sums over fixed chunks in a fixed order (whatever the
+// column count and layout, so that a column's bits do not depend on its neighbours), integer sums
+// and maxima of non-negative doubles' bits through atomics (order independent).  Every kernel
+// moves each element once, 16 bytes at a time where the layout allows: at 266 columns, N=50k,
+// M=100k the operand and reduction kernels around the two passes take 0.24 ms of a 10 ms apply.
 
-// Quantises v (centred and multiplied by 127 / max) into three int8 pieces of base 254;
-// returns the represented value.
-__device__ __forceinline__ double quantise3(double v, int8_t& q1, int8_t& q2, int8_t& q3) {
+// Quantises v (centred and multiplied by 127 / max) into three int8 pieces of base 254.
+__device__ __forceinline__ void quantise3(double v, int& q1, int& q2, int& q3) {
     const double a = rint(v);
     const double r1 = (v - a) * kBase;
     const double b = rint(r1);
     const double r2 = (r1 - b) * kBase;
-    const double c = rint(r2);
-    q1 = (int8_t)a;
-    q2 = (int8_t)b;
-    q3 = (int8_t)c;
-    return a + b / kBase + c / (kBase * kBase);
+    q1 = (int)(int8_t)a;
+    q2 = (int)(int8_t)b;
+    q3 = (int)(int8_t)rint(r2);
 }
 
 // Two int8 pieces of base 254 (the residual operand of the samples pass, |v| <= 63.5).
-__device__ __forceinline__ void quantise2(double v, int8_t& q1, int8_t& q2) {
+__device__ __forceinline__ void quantise2(double v, int& q1, int& q2) {
     const double a = rint(v);
-    q1 = (int8_t)a;
-    q2 = (int8_t)rint((v - a) * kBase);
+    q1 = (int)(int8_t)a;
+    q2 = (int)(int8_t)rint((v - a) * kBase);
 }
 
 __device__ __forceinline__ double quant_factor(unsigned long long bits) {
@@ -752,214 +749,328 @@ __device__ __forceinline__ double quant_factor(unsigned long long bits) {
     return m > 0.0 ? 127.0 / m : 0.0;
 }
 
-// Per-column sums, minima and maxima of a row-major FP64 matrix over tiles of 64 rows x 32
-// columns (blockIdx.x, blockIdx.y): part[b][c], part[nb + b][c], part[2 nb + b][c], b the row
-// tile, nb = gridDim.x.  Warps read 32 consecutive columns of a row (256-byte segments).
+// Whether this block is the last of `n` to arrive at the counter (which wraps back to zero).
+// Every thread of the block calls it, after its own writes.
+__device__ __forceinline__ bool last_block(unsigned* counter, unsigned n) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(counter, n - 1) == n - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
+}
+
+// What the operand kernels of a call hand on: per column the mean and the bits of max |x - mean|
+// (rows operand), the integer sum of the quantised values in units of 1 / 254^2, the bits of
+// max |W| and max(|W|, |mu W|) (samples operand), and the counters of last_block.
+struct MixedColumns {
+    double* mean;
+    unsigned long long* max1;
+    unsigned long long* qsum;
+    unsigned long long* max_w;
+    unsigned long long* max_wmu;
+    unsigned* counter;
+};
+
+// Per-column sums, minima and maxima of X over chunks of 512 rows (8 interleaved lanes each, added
+// in lane order), then, in the last block of a column tile, mean[c] = (sum over chunks) / n and
+// max1[c] = the bits of max |x - mean| = max(max x - mean, mean - min x) (rounding is monotonic, so
+// this equals the maximum of the rounded differences); the column's other words are cleared.
+// A block covers kc columns (a power of two up to 32) x 32 / kc chunks.
+constexpr int kStatRows = 512;
+template <class T>
 __global__ void __launch_bounds__(256)
-k_col_stats(const double* __restrict__ X, int64_t ld, int64_t n, int64_t k, double* __restrict__ part) {
-    __shared__ double red[3][8][kPrepCols];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t c = (int64_t)blockIdx.y * kPrepCols + tx;
-    const int64_t r0 = (int64_t)blockIdx.x * kPrepRows;
+k_col_stats(const Strided<const T> X, int64_t n, int64_t k, int kc, int64_t nb,
+            double* __restrict__ part, const MixedColumns C) {
+    __shared__ double red[3][256];
+    // threads in the order of memory: columns fastest in row-major input, lanes in column-major
+    const int per = 256 / kc;  // 8 lanes x chunks
+    const int tc = X.rs == 1 ? threadIdx.x / per : threadIdx.x % kc;
+    const int tl = X.rs == 1 ? threadIdx.x % per : threadIdx.x / kc;
+    const int lane = tl & 7, ch = tl >> 3;
+    const int64_t c = (int64_t)blockIdx.y * kc + tc;
+    const int64_t b = (int64_t)blockIdx.x * (per >> 3) + ch;
     double sm = 0.0, mn = INFINITY, mx = -INFINITY;
-    if (c < k)
-        for (int64_t r = r0 + ty; r < min(n, r0 + kPrepRows); r += 8) {
-            const double v = X[r * ld + c];
+    if (c < k && b < nb) {
+        const int64_t r1 = min(n, (b + 1) * kStatRows);
+#pragma unroll 8
+        for (int64_t r = b * kStatRows + lane; r < r1; r += 8) {
+            const double v = (double)X.p[r * X.rs + c * X.cs];
             sm += v;
             mn = fmin(mn, v);
             mx = fmax(mx, v);
         }
-    red[0][ty][tx] = sm;
-    red[1][ty][tx] = mn;
-    red[2][ty][tx] = mx;
+    }
+    const int slot = (tc * (per >> 3) + ch) * 8 + lane;
+    red[0][slot] = sm;
+    red[1][slot] = mn;
+    red[2][slot] = mx;
     __syncthreads();
-    if (ty == 0 && c < k) {
-        for (int j = 1; j < 8; ++j) {
-            sm += red[0][j][tx];
-            mn = fmin(mn, red[1][j][tx]);
-            mx = fmax(mx, red[2][j][tx]);
+    if (threadIdx.x < 32) {  // one thread per (column, chunk)
+        const int oc = threadIdx.x / (per >> 3), och = threadIdx.x % (per >> 3);
+        const int64_t cc = (int64_t)blockIdx.y * kc + oc, bb = (int64_t)blockIdx.x * (per >> 3) + och;
+        if (cc < k && bb < nb) {
+            const int s0 = threadIdx.x * 8;
+            sm = red[0][s0];
+            mn = red[1][s0];
+            mx = red[2][s0];
+            for (int j = 1; j < 8; ++j) {
+                sm += red[0][s0 + j];
+                mn = fmin(mn, red[1][s0 + j]);
+                mx = fmax(mx, red[2][s0 + j]);
+            }
+            part[bb * k + cc] = sm;
+            part[(nb + bb) * k + cc] = mn;
+            part[(2 * nb + bb) * k + cc] = mx;
         }
-        const int64_t nb = gridDim.x;
-        part[(int64_t)blockIdx.x * k + c] = sm;
-        part[(nb + blockIdx.x) * k + c] = mn;
-        part[(2 * nb + blockIdx.x) * k + c] = mx;
+    }
+    if (!last_block(C.counter + blockIdx.y, gridDim.x)) return;
+    // one warp per column: lane l takes chunks l, l + 32, ..., then a fixed shuffle tree
+    const int wl = threadIdx.x & 31;
+    for (int j = threadIdx.x >> 5; j < kc; j += 8) {
+        const int64_t cc = (int64_t)blockIdx.y * kc + j;
+        if (cc >= k) break;
+        sm = 0.0;
+        mn = INFINITY;
+        mx = -INFINITY;
+        for (int64_t q = wl; q < nb; q += 32) {
+            sm += __ldcg(part + q * k + cc);
+            mn = fmin(mn, __ldcg(part + (nb + q) * k + cc));
+            mx = fmax(mx, __ldcg(part + (2 * nb + q) * k + cc));
+        }
+        for (int off = 16; off; off >>= 1) {
+            sm += __shfl_xor_sync(0xffffffffu, sm, off);
+            mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        }
+        if (wl == 0) {
+            const double m = sm / (double)n;
+            C.mean[cc] = m;
+            const double a = fmax(fmax(mx - m, m - mn), 0.0);
+            C.max1[cc] = (unsigned long long)__double_as_longlong(a);
+            C.qsum[cc] = 0;
+            C.max_w[cc] = 0;
+            C.max_wmu[cc] = 0;
+        }
     }
 }
 
-// mean[c] = (sum over row tiles) / n and maxbits[c] = the bits of max |x - mean[c]| =
-// max(max x - mean, mean - min x) (rounding is monotonic, so this equals the maximum of the
-// rounded differences).  One warp per column: lane l takes tiles l, l + 32, ..., then a fixed
-// shuffle tree (deterministic).
-__global__ void __launch_bounds__(256)
-k_col_finalize(const double* __restrict__ part, int nb, int64_t k, int64_t n,
-               double* __restrict__ mean, unsigned long long* __restrict__ maxbits) {
-    const int lane = threadIdx.x & 31;
-    const int64_t c = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (c >= k) return;
-    double sm = 0.0, mn = INFINITY, mx = -INFINITY;
-    for (int b = lane; b < nb; b += 32) {
-        sm += part[(int64_t)b * k + c];
-        mn = fmin(mn, part[(int64_t)(nb + b) * k + c]);
-        mx = fmax(mx, part[(int64_t)(2 * nb + b) * k + c]);
+// 16 int8 values (by K element) -> the 16 bytes of their K positions: interleaved as the decoded
+// tiles are, or in order.
+template <bool INTERLEAVE>
+__device__ __forceinline__ uint4 pack16(const int (&q)[16]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const int e0 = INTERLEAVE ? sample_at(4 * g) : 4 * g, e1 = INTERLEAVE ? sample_at(4 * g + 1) : 4 * g + 1;
+        const int e2 = INTERLEAVE ? sample_at(4 * g + 2) : 4 * g + 2, e3 = INTERLEAVE ? sample_at(4 * g + 3) : 4 * g + 3;
+        w[g] = __byte_perm(__byte_perm((uint32_t)q[e0], (uint32_t)q[e1], 0x0040),
+                           __byte_perm((uint32_t)q[e2], (uint32_t)q[e3], 0x0040), 0x5410);
     }
-    for (int off = 16; off; off >>= 1) {
-        sm += __shfl_xor_sync(0xffffffffu, sm, off);
-        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, off));
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    }
-    if (lane == 0) {
-        const double m = sm / (double)n;
-        mean[c] = m;
-        const double a = fmax(fmax(mx - m, m - mn), 0.0);
-        maxbits[c] = (unsigned long long)__double_as_longlong(a);
-    }
-}
-
-// out[c] = scale * sum_b part[b][c]: one warp per column, lane l takes b = l, l + 32, ...,
-// then a fixed shuffle tree (deterministic).  Launch with (k + 7) / 8 blocks of 256 threads.
-__global__ void __launch_bounds__(256)
-k_sum_partials(const double* __restrict__ part, int nb, int64_t k, double scale, double* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    const int64_t c = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (c >= k) return;
-    double sm = 0.0;
-    for (int b = lane; b < nb; b += 32) sm += part[(int64_t)b * k + c];
-    for (int off = 16; off; off >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, off);
-    if (lane == 0) out[c] = sm * scale;
+    return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // Rows-pass operand: B1[q*kp + c][pos(i)] (int8 pieces of (x_ic - mean_c) 127 / max_c, i < n_pad;
-// pos interleaves each group of 16 samples as the decoded tiles do) and per-tile sums of the
-// represented values qpart[blockIdx.x][c].
-__global__ void __launch_bounds__(256)
-k_split_rows_operand(const double* __restrict__ X, int64_t ld, int64_t n, int64_t k, int64_t kp,
-                     int64_t n_pad, const double* __restrict__ mean,
-                     const unsigned long long* __restrict__ maxbits, int8_t* __restrict__ B,
-                     double* __restrict__ qpart) {
-    __shared__ double tile[kPrepRows][kPrepCols + 1];
-    __shared__ double red[8][kPrepCols];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t c0 = (int64_t)blockIdx.y * kPrepCols, r0 = (int64_t)blockIdx.x * kPrepRows;
-    for (int rr = ty; rr < kPrepRows; rr += 8) {
-        const int64_t r = r0 + rr, c = c0 + tx;
-        tile[rr][tx] = (r < n && c < k) ? X[r * ld + c] : 0.0;
+// pos interleaves each group of 16 samples as the decoded tiles do) and the integer sums of the
+// quantised values.  A block takes COLS columns x ROWS rows through shared memory; a thread takes
+// 16 rows of a column.
+template <class T, int COLS, int ROWS>
+__global__ void __launch_bounds__(ROWS / 16 * COLS)
+k_split_rows_operand(const Strided<const T> X, int64_t n, int64_t k, int64_t kp, int64_t n_pad,
+                     const MixedColumns C, int8_t* __restrict__ B) {
+    constexpr int TH = ROWS / 16 * COLS;
+    __shared__ double tile[COLS][ROWS + ROWS / 16 + 1];  // one pad every 16 rows and one per column
+    const int64_t r0 = (int64_t)blockIdx.x * ROWS, c0 = (int64_t)blockIdx.y * COLS;
+    for (int e = threadIdx.x; e < ROWS * COLS; e += TH) {
+        const int rr = X.rs == 1 ? e % ROWS : e / COLS, cc = X.rs == 1 ? e / ROWS : e % COLS;
+        const int64_t r = r0 + rr, c = c0 + cc;
+        tile[cc][rr + (rr >> 4)] = (r < n && c < k) ? (double)X.p[r * X.rs + c * X.cs] : 0.0;
     }
     __syncthreads();
-    // each warp handles 4 columns; lane covers rows lane and lane + 32
-    double qs[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int cc = 0; cc < 4; ++cc) {
-        const int col = ty * 4 + cc;
-        const int64_t c = c0 + col;
-        if (c >= kp) continue;
-        const double f = c < k ? quant_factor(maxbits[c]) : 0.0;
-        const double mc = c < k ? mean[c] : 0.0;
-        for (int rr = tx; rr < kPrepRows; rr += 32) {
-            const int64_t i = r0 + rr;
-            if (i >= n_pad) continue;
-            int8_t q1 = 0, q2 = 0, q3 = 0;
-            if (c < k && i < n) qs[cc] += quantise3((tile[rr][col] - mc) * f, q1, q2, q3);
-            // K position of sample i: the decoded tiles interleave each group of 16 samples
-            const int64_t pos = (i & ~(int64_t)15) + position_of((int)(i & 15));
-            B[c * n_pad + pos] = q1;
-            B[(kp + c) * n_pad + pos] = q2;
-            B[(2 * kp + c) * n_pad + pos] = q3;
+    const int grp = threadIdx.x % (ROWS / 16), cc = threadIdx.x / (ROWS / 16);
+    const int64_t c = c0 + cc, i0 = r0 + 16 * grp;
+    const bool live = c < kp && i0 < n_pad;
+    long long sum = 0;
+    if (live) {
+        const double f = c < k ? quant_factor(C.max1[c]) : 0.0;
+        const double mc = c < k ? C.mean[c] : 0.0;
+        int q1[16], q2[16], q3[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            q1[j] = q2[j] = q3[j] = 0;
+            if (c < k && i0 + j < n) quantise3((tile[cc][17 * grp + j] - mc) * f, q1[j], q2[j], q3[j]);
+            sum += (long long)q1[j] * 64516 + q2[j] * 254 + q3[j];
         }
+        *reinterpret_cast<uint4*>(B + c * n_pad + i0) = pack16<true>(q1);
+        *reinterpret_cast<uint4*>(B + (kp + c) * n_pad + i0) = pack16<true>(q2);
+        *reinterpret_cast<uint4*>(B + (2 * kp + c) * n_pad + i0) = pack16<true>(q3);
     }
-    for (int cc = 0; cc < 4; ++cc) {
-        double v = qs[cc];
-        for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (tx == 0) red[0][ty * 4 + cc] = v;  // lane 0 of warp ty owns columns 4ty..4ty+3
-    }
-    __syncthreads();
-    if (threadIdx.x < kPrepCols) {
-        const int64_t c = c0 + threadIdx.x;
-        if (c < k) qpart[(int64_t)blockIdx.x * k + c] = red[0][threadIdx.x];
-    }
+    for (int off = 8; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if ((threadIdx.x & 15) == 0 && live && c < k) atomicAdd(C.qsum + c, (unsigned long long)sum);
 }
 
-// Rows-pass reduction, one column per blockIdx.y and 2048 rows per blockIdx.x:
-//   inner_tc = (sum_z part[z][c][t] - mu_t Q_c) / f_c + mean_c exc_t
-// out = inner * s_t^spow written column-major (out[c * out_ld + t]) or row-major
-// (out[t * out_ld + c]); optional maxima of |out| per column.
+// (sum_z part[z][c][t] - mu_t Q_c) / f_c + mean_c exc_t, the rows pass's centred product.
+struct RowsColumn {
+    double inv_f, mean, qsum;
+    __device__ __forceinline__ RowsColumn(const MixedColumns& C, int64_t c) {
+        const double f = quant_factor(C.max1[c]);
+        inv_f = f > 0.0 ? 1.0 / f : 0.0;
+        mean = C.mean[c];
+        qsum = (double)(long long)C.qsum[c] / (kBase * kBase);
+    }
+    __device__ __forceinline__ double value(double acc, double mu, double exc) const {
+        return (acc - mu * qsum) * inv_f + mean * exc;
+    }
+};
+
+// Rows-pass reduction for an apply: W^T (column-major, R per column) = s^2 o the product, with the
+// maxima of |W| and of max(|W|, |mu W|).  1024 SNPs per block, one column per blockIdx.y.
 __global__ void __launch_bounds__(256)
 k_reduce_rows(const double* __restrict__ part, int splits, int64_t kp, int64_t ld, int64_t R,
-              int64_t k, const double* __restrict__ s_row, int spow,
-              const double* __restrict__ exc_row, const double* __restrict__ mu,
-              const double* __restrict__ mean, const double* __restrict__ qsum,
-              const unsigned long long* __restrict__ maxbits_in, double* __restrict__ out,
-              int64_t out_ld, int colmajor, unsigned long long* __restrict__ max_w) {
-    __shared__ double red_w[8];
+              const double* __restrict__ s_row, const double* __restrict__ exc_row,
+              const double* __restrict__ mu, const MixedColumns C, double* __restrict__ out) {
+    __shared__ double red[2][8];
     const int64_t c = blockIdx.y;
-    const double f = quant_factor(maxbits_in[c]);
-    const double inv_f = f > 0.0 ? 1.0 / f : 0.0;
-    const double mc = mean[c], qc = qsum[c];
-    double mw = 0.0;
-    const int64_t t0 = (int64_t)blockIdx.x * 2048;
-    for (int64_t t = t0 + threadIdx.x; t < min(R, t0 + 2048); t += 256) {
-        double acc = 0.0;
-        for (int z = 0; z < splits; ++z) acc += part[((int64_t)z * kp + c) * ld + t];
-        double v = (acc - mu[t] * qc) * inv_f + mc * exc_row[t];
-        if (s_row) {
-            v *= s_row[t];
-            if (spow == 2) v *= s_row[t];
-        }
-        if (colmajor) out[c * out_ld + t] = v;
-        else out[t * out_ld + c] = v;
-        mw = fmax(mw, fabs(v));
+    const RowsColumn col(C, c);
+    double mw = 0.0, mm = 0.0;
+    const int64_t t0 = (int64_t)blockIdx.x * 1024 + threadIdx.x;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int z = 0; z < splits; ++z) {
+        const double* p = part + ((int64_t)z * kp + c) * ld + t0;  // ld >= R rounded up to 256
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (t0 + 256 * j < R) acc[j] += p[256 * j];
     }
-    if (max_w) {
-        for (int off = 16; off; off >>= 1) mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, off));
-        if ((threadIdx.x & 31) == 0) red_w[threadIdx.x >> 5] = mw;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int j = 1; j < 8; ++j) mw = fmax(mw, red_w[j]);
-            atomicMax(max_w + c, (unsigned long long)__double_as_longlong(mw));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int64_t t = t0 + 256 * j;
+        if (t < R) {
+            const double m = mu[t], s = s_row[t];
+            const double v = col.value(acc[j], m, exc_row[t]) * s * s;
+            out[c * R + t] = v;
+            mw = fmax(mw, fabs(v));
+            mm = fmax(mm, fmax(fabs(v), m * fabs(v)));
         }
+    }
+    for (int off = 16; off; off >>= 1) {
+        mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, off));
+        mm = fmax(mm, __shfl_xor_sync(0xffffffffu, mm, off));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = mw;
+        red[1][threadIdx.x >> 5] = mm;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int j = 1; j < 8; ++j) {
+            mw = fmax(mw, red[0][j]);
+            mm = fmax(mm, red[1][j]);
+        }
+        atomicMax(C.max_w + c, (unsigned long long)__double_as_longlong(mw));
+        atomicMax(C.max_wmu + c, (unsigned long long)__double_as_longlong(mm));
     }
 }
 
-// Samples-pass operand from W^T (column-major, k x R): three pieces of W f (rows q kp + c)
-// and two of (Q r o W) f (rows (3 + q) kp + c), t < r_pad, with ONE factor f = 127 / max|W|
-// per column so that both MMAs accumulate into the same TMEM columns (|Q r_t| <= 1/2); 1/(Q f)
-// per column; and per-block sums of mu_t W[t][c] (the centring term) in cpart[blockIdx.x][c].
-// `interleave` (A in TMEM, over the sample-major copy): SNP t sits at K position
-// (t & ~15) + position_of(t & 15), the order in which the decoder writes each group of 16, and
-// the residual pieces are negated (that decoder's missing-indicator tile holds -1).
-// Grid: (r_pad / 2048, kp).
+// Rows-pass reduction for a half-pass or a scan: out(row, c) = s_t o the product, row = pos[t] (or
+// t).  Tiles of 32 SNPs x 32 columns; a row-major result goes through shared memory, so that both
+// sides are coalesced.
 __global__ void __launch_bounds__(256)
+k_reduce_rows_out(const double* __restrict__ part, int splits, int64_t kp, int64_t ld, int64_t R,
+                  int64_t k, const double* __restrict__ s_row, const double* __restrict__ exc_row,
+                  const double* __restrict__ mu, const int32_t* __restrict__ pos, const MixedColumns C,
+                  StridedOut out) {
+    __shared__ double tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t t0 = (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
+    const int64_t t = t0 + tx;
+#pragma unroll
+    for (int cc = ty; cc < 32; cc += 8) {
+        const int64_t c = c0 + cc;
+        if (c >= k || t >= R) continue;
+        const RowsColumn col(C, c);
+        double acc = 0.0;
+        for (int z = 0; z < splits; ++z) acc += part[((int64_t)z * kp + c) * ld + t];
+        const double v = col.value(acc, mu[t], exc_row[t]) * s_row[t];
+        if (out.rs == 1) out.p[(pos ? (int64_t)pos[t] : t) + c * out.cs] = v;
+        else tile[cc][tx] = v;
+    }
+    if (out.rs == 1) return;
+    __syncthreads();
+    for (int tt = ty; tt < 32; tt += 8) {
+        const int64_t r = t0 + tt, c = c0 + tx;
+        if (r < R && c < k) out.p[(pos ? (int64_t)pos[r] : r) * out.rs + c * out.cs] = tile[tx][tt];
+    }
+}
+
+// Samples-pass operand from W^T (column-major, k x R), and the sums c0_c of mu_t W[t][c] (the
+// centring term): chunks of 2048 SNPs, added in chunk order by the last block of the column.
+//   SIX: pieces of W f (rows q kp + c) and of (mu o W) f (rows (3 + q) kp + c), f = 127 /
+//        max(|W|, |mu W|), at interleaved K positions;
+//   otherwise three pieces of W f and two of (Q r o W) f, f = 127 / max|W| (|Q r_t| <= 1/2), so
+//        that both MMAs accumulate into the same TMEM columns; INTERLEAVE (over the sample-major
+//        copy) also negates the residual pieces (that decoder's missing-indicator tile holds -1).
+// inv_f[c] scales the sums back.  A thread takes 16 SNPs of a column.  Grid: (chunks, kp).
+template <bool SIX, bool INTERLEAVE>
+__global__ void __launch_bounds__(128)
 k_split_samples_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int64_t kp,
                         int64_t r_pad, const double* __restrict__ mu,
-                        const double* __restrict__ resid,
-                        const unsigned long long* __restrict__ max_w, int interleave,
+                        const double* __restrict__ resid, const MixedColumns C,
                         int8_t* __restrict__ B, double* __restrict__ inv_f,
-                        double* __restrict__ cpart) {
-    __shared__ double red[8];
+                        double* __restrict__ cpart, double* __restrict__ c0) {
+    __shared__ double red[4];
+    // W and the second operand of 2048 SNPs, one pad every 16, read in the order of memory
+    __shared__ double sw[128 * 17], sb[128 * 17];
     const int64_t c = blockIdx.y;
-    const double f = c < k ? quant_factor(max_w[c]) : 0.0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) inv_f[c] = f > 0.0 ? 1.0 / (f * kImputeQ) : 0.0;
+    const double f = c < k ? quant_factor(SIX ? C.max_wmu[c] : C.max_w[c]) : 0.0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) inv_f[c] = f > 0.0 ? 1.0 / (SIX ? f : f * kImputeQ) : 0.0;
     double cs = 0.0;
-    const int64_t t0 = (int64_t)blockIdx.x * 2048;
-    for (int64_t t = t0 + threadIdx.x; t < min(r_pad, t0 + 2048); t += 256) {
-        int8_t a1 = 0, a2 = 0, a3 = 0, b1 = 0, b2 = 0;
+    const int64_t base = (int64_t)blockIdx.x * 2048;
+#pragma unroll 8
+    for (int e = threadIdx.x; e < 2048; e += 128) {
+        const int64_t t = base + e;
+        double w = 0.0, b = 0.0;
         if (c < k && t < R) {
-            const double w = Wt[c * R + t];
-            quantise3(w * f, a1, a2, a3);
-            quantise2((interleave ? -kImputeQ : kImputeQ) * resid[t] * w * f, b1, b2);
-            cs += mu[t] * w;
+            const double m = mu[t];
+            w = Wt[c * R + t];
+            b = SIX ? m * w : (INTERLEAVE ? -kImputeQ : kImputeQ) * resid[t] * w;
+            cs += m * w;
         }
-        const int64_t pos = interleave ? (t & ~(int64_t)15) + position_of((int)(t & 15)) : t;
-        B[c * r_pad + pos] = a1;
-        B[(kp + c) * r_pad + pos] = a2;
-        B[(2 * kp + c) * r_pad + pos] = a3;
-        B[(3 * kp + c) * r_pad + pos] = b1;
-        B[(4 * kp + c) * r_pad + pos] = b2;
+        sw[e + (e >> 4)] = w;
+        sb[e + (e >> 4)] = b;
     }
+    __syncthreads();
+    const int64_t t0 = base + 16 * threadIdx.x;
+    if (t0 < r_pad) {
+        int8_t* dst = B + c * r_pad + t0;
+        const int64_t step = kp * r_pad;
+        int q1[16], q2[16], q3[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) quantise3(sw[17 * threadIdx.x + j] * f, q1[j], q2[j], q3[j]);
+        *reinterpret_cast<uint4*>(dst) = pack16<INTERLEAVE>(q1);
+        *reinterpret_cast<uint4*>(dst + step) = pack16<INTERLEAVE>(q2);
+        *reinterpret_cast<uint4*>(dst + 2 * step) = pack16<INTERLEAVE>(q3);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const double v = sb[17 * threadIdx.x + j] * f;
+            if (SIX) quantise3(v, q1[j], q2[j], q3[j]);
+            else quantise2(v, q1[j], q2[j]);
+        }
+        *reinterpret_cast<uint4*>(dst + 3 * step) = pack16<INTERLEAVE>(q1);
+        *reinterpret_cast<uint4*>(dst + 4 * step) = pack16<INTERLEAVE>(q2);
+        if (SIX) *reinterpret_cast<uint4*>(dst + 5 * step) = pack16<INTERLEAVE>(q3);
+    }
+    if (c >= k) return;
     for (int off = 16; off; off >>= 1) cs += __shfl_xor_sync(0xffffffffu, cs, off);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = cs;
     __syncthreads();
-    if (threadIdx.x == 0 && c < k) {
-        for (int j = 1; j < 8; ++j) cs += red[j];
-        cpart[(int64_t)blockIdx.x * k + c] = cs;
+    if (threadIdx.x == 0) cpart[(int64_t)blockIdx.x * k + c] = (red[0] + red[1]) + (red[2] + red[3]);
+    if (!last_block(C.counter + c, gridDim.x)) return;
+    if (threadIdx.x < 32) {
+        double sm = 0.0;
+        for (int64_t b = threadIdx.x; b < gridDim.x; b += 32) sm += __ldcg(cpart + b * k + c);
+        for (int off = 16; off; off >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, off);
+        if (threadIdx.x == 0) c0[c] = sm;
     }
 }
 
@@ -995,79 +1106,56 @@ k_transpose_packed(const uint8_t* __restrict__ src, int64_t R, int64_t stride,
     *reinterpret_cast<uint4*>(d) = make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-// Column maxima of max(|W|, |mu o W|) for a column-major R x k W (the six-set samples operand).
+// The samples operand's W of a half-pass, W^T[c][t] = s_t V[pos[t]][c], and its maxima (cleared
+// before).  1024 SNPs per block, one column per blockIdx.y.
 __global__ void __launch_bounds__(256)
-k_col_absmax_mu(const double* __restrict__ W, int64_t R, const double* __restrict__ mu,
-                unsigned long long* __restrict__ max_w) {
-    __shared__ double red_w[8];
+k_gather_operand(const StridedIn V, int64_t R, const int32_t* __restrict__ pos,
+                 const double* __restrict__ s_row, const double* __restrict__ mu, const MixedColumns C,
+                 double* __restrict__ Wt) {
     const int64_t c = blockIdx.y;
-    double mw = 0.0;
-    const int64_t t0 = (int64_t)blockIdx.x * 2048;
-    for (int64_t t = t0 + threadIdx.x; t < min(R, t0 + 2048); t += 256) {
-        const double v = fabs(W[c * R + t]);
-        mw = fmax(mw, fmax(v, mu[t] * v));
+    double mw = 0.0, mm = 0.0;
+    const int64_t t0 = (int64_t)blockIdx.x * 1024;
+    for (int64_t t = t0 + threadIdx.x; t < min(R, t0 + 1024); t += 256) {
+        const double w = s_row[t] * V.p[(int64_t)pos[t] * V.rs + c * V.cs];
+        Wt[c * R + t] = w;
+        mw = fmax(mw, fabs(w));
+        mm = fmax(mm, fmax(fabs(w), mu[t] * fabs(w)));
     }
-    for (int off = 16; off; off >>= 1) mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, off));
-    if ((threadIdx.x & 31) == 0) red_w[threadIdx.x >> 5] = mw;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int j = 1; j < 8; ++j) mw = fmax(mw, red_w[j]);
-        atomicMax(max_w + c, (unsigned long long)__double_as_longlong(mw));
+    for (int off = 16; off; off >>= 1) {
+        mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, off));
+        mm = fmax(mm, __shfl_xor_sync(0xffffffffu, mm, off));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(C.max_w + c, (unsigned long long)__double_as_longlong(mw));
+        atomicMax(C.max_wmu + c, (unsigned long long)__double_as_longlong(mm));
     }
 }
 
-// Six-set samples operand (A in TMEM over the sample-major copy): pieces of W f (rows q kp + c)
-// and of (mu o W) f (rows (3 + q) kp + c) at the K positions of the decoded tiles (SNPs
-// interleaved within groups of 16 like samples in the rows pass), f = 127 / max(|W|, |mu W|)
-// per column; 1/f per column; per-block sums of mu_t W[t][c] in cpart[blockIdx.x][c].
-// Grid: (r_pad / 2048, kp).
+// Samples-pass reduction: Y[i][c] = (sum_z part[z][c][i] - c0_c) / M.  Tiles of 32 samples x 32
+// columns; a row-major result goes through shared memory, so that both sides are coalesced.
+template <class T>
 __global__ void __launch_bounds__(256)
-k_split_samples_t_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int64_t kp,
-                          int64_t r_pad, const double* __restrict__ mu,
-                          const unsigned long long* __restrict__ max_wmu, int8_t* __restrict__ B,
-                          double* __restrict__ inv_f, double* __restrict__ cpart) {
-    __shared__ double red[8];
-    const int64_t c = blockIdx.y;
-    const double f = c < k ? quant_factor(max_wmu[c]) : 0.0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) inv_f[c] = f > 0.0 ? 1.0 / f : 0.0;
-    double cs = 0.0;
-    const int64_t t0 = (int64_t)blockIdx.x * 2048;
-    for (int64_t t = t0 + threadIdx.x; t < min(r_pad, t0 + 2048); t += 256) {
-        int8_t a1 = 0, a2 = 0, a3 = 0, b1 = 0, b2 = 0, b3 = 0;
-        if (c < k && t < R) {
-            const double w = Wt[c * R + t];
-            quantise3(w * f, a1, a2, a3);
-            quantise3(mu[t] * w * f, b1, b2, b3);
-            cs += mu[t] * w;
-        }
-        const int64_t pos = (t & ~(int64_t)15) + position_of((int)(t & 15));
-        B[c * r_pad + pos] = a1;
-        B[(kp + c) * r_pad + pos] = a2;
-        B[(2 * kp + c) * r_pad + pos] = a3;
-        B[(3 * kp + c) * r_pad + pos] = b1;
-        B[(4 * kp + c) * r_pad + pos] = b2;
-        B[(5 * kp + c) * r_pad + pos] = b3;
-    }
-    for (int off = 16; off; off >>= 1) cs += __shfl_xor_sync(0xffffffffu, cs, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = cs;
-    __syncthreads();
-    if (threadIdx.x == 0 && c < k) {
-        for (int j = 1; j < 8; ++j) cs += red[j];
-        cpart[(int64_t)blockIdx.x * k + c] = cs;
-    }
-}
-
-// Samples-pass reduction: Y[i][c] = (sum_z part[z][c][i] - c0_c) / M.
-__global__ void k_reduce_samples(const double* __restrict__ part, int splits, int64_t kp,
-                                 int64_t ld, int64_t n, int64_t k, const double* __restrict__ c0,
-                                 double inv_m, double* __restrict__ Y, int64_t ldy) {
-    const int64_t total = n * k;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = idx / k, c = idx - i * k;  // c fastest: coalesced Y rows
+k_reduce_samples(const double* __restrict__ part, int splits, int64_t kp, int64_t ld, int64_t n,
+                 int64_t k, const double* __restrict__ c0v, double inv_m, const Strided<T> Y) {
+    __shared__ double tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t i0 = (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
+    const int64_t i = i0 + tx;
+#pragma unroll
+    for (int cc = ty; cc < 32; cc += 8) {
+        const int64_t c = c0 + cc;
+        if (c >= k || i >= n) continue;
         double acc = 0.0;
         for (int z = 0; z < splits; ++z) acc += part[((int64_t)z * kp + c) * ld + i];
-        Y[i * ldy + c] = (acc - c0[c]) * inv_m;
+        const double v = (acc - c0v[c]) * inv_m;
+        if (Y.rs == 1) Y.p[i + c * Y.cs] = (T)v;
+        else tile[cc][tx] = v;
+    }
+    if (Y.rs == 1) return;
+    __syncthreads();
+    for (int ii = ty; ii < 32; ii += 8) {
+        const int64_t r = i0 + ii, c = c0 + tx;
+        if (r < n && c < k) Y.p[r * Y.rs + c * Y.cs] = (T)tile[tx][ii];
     }
 }
 
@@ -1227,8 +1315,22 @@ int choose_splits(int64_t units_per_split, int kb_total, int64_t target) {
 
 struct MixedWorkspace {
     DeviceBuffer<int8_t> b1, b2;
-    DeviceBuffer<double> part, colpart, mean1, qsum, c0, W, inv_f;
-    DeviceBuffer<unsigned long long> max1, max_w, max_wmu;
+    DeviceBuffer<double> part, colpart, mean1, c0, W, inv_f;
+    DeviceBuffer<unsigned long long> max1, qsum, max_w, max_wmu;
+    DeviceBuffer<unsigned> counter;
+    // the column words of a call on k columns (new counters start at zero)
+    MixedColumns columns(int64_t k, cudaStream_t s) {
+        mean1.resize(k);
+        max1.resize(k);
+        qsum.resize(k);
+        max_w.resize(k);
+        max_wmu.resize(k);
+        if (counter.count < (size_t)k) {
+            counter.resize(k);
+            CS_CUDA(cudaMemsetAsync(counter.get(), 0, 4 * counter.count, s));
+        }
+        return MixedColumns{mean1.get(), max1.get(), qsum.get(), max_w.get(), max_wmu.get(), counter.get()};
+    }
     CUtensorMap tm_b1{}, tm_b2{};
     CUtensorMap tm_b1t{}, tm_b2t{};  // boxes of the last column tile's width
     const void* tm_b1_base = nullptr;
@@ -1625,13 +1727,13 @@ PassPlan choose_plan(bool rows, bool allow, int64_t R, int64_t n, int64_t k, int
     return best.plan;
 }
 
-// Rows pass over a MixedRows context: for X (n x k, row-major ldx),
-//   out_tc = s_t^spow ( sum_i (G_ti - mu_t)[obs] x_ic )  (mean-imputed centred dosages)
-// written column-major (out[c * out_ld + t]) or row-major.  With want_max, also the
-// per-column maxima of |out| and |mu out| (samples-pass operand scales).
-void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, const double* X,
-                    int64_t ldx, int64_t k, double* out, int64_t out_ld, bool colmajor, int spow,
-                    bool want_max, cudaStream_t s) {
+// Rows pass over a MixedRows context on X (n x k):
+//   u_tc = sum_i (G_ti - mu_t)[obs] x_ic  (mean-imputed centred dosages)
+// With Wt: W^T (column-major, R per column) = s_t^2 u and its maxima for the samples operand;
+// otherwise out(pos[t] or t, c) = s_t u.
+template <class T>
+void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, Strided<const T> X,
+                    int64_t k, double* Wt, const int32_t* pos, StridedOut out, cudaStream_t s) {
     const int64_t tiles = r.r_pad / kTile;
     const bool pairs = plan.pairs;
     const Tiling tl = tiling_for(k, plan.max_w);
@@ -1640,15 +1742,11 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, cons
     const int kbs = (kb + plan.splits - 1) / plan.splits;
     const int splits = (kb + kbs - 1) / kbs;  // no empty slice
     if (kbs > kMaxKbPerAccum) fail(CS_ERR_UNSUPPORTED, "rows pass: K slice exceeds the exact int32 range");
-    const int rt = (int)((n_pad + kPrepRows - 1) / kPrepRows);
-    const int nst = (int)((n + kPrepRows - 1) / kPrepRows);  // row tiles of the column stats
+    const int64_t nst = (n + kStatRows - 1) / kStatRows;  // chunks of the column stats
     ws.b1.resize(3 * kp * n_pad);
     ws.part.resize((int64_t)splits * kp * r_pad);
-    ws.colpart.resize((int64_t)std::max(rt, 3 * nst) * k);
-    ws.mean1.resize(k);
-    ws.qsum.resize(k);
-    ws.max1.resize(k);
-    ws.max_w.resize(k);
+    ws.colpart.resize(3 * nst * k);
+    const MixedColumns C = ws.columns(k, s);
     if (!ws.status.get()) {
         ws.status.resize(1);
         // on the pass's own stream, so the kernel never reads the pool's previous contents
@@ -1665,14 +1763,17 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, cons
     }
     {
         prof::Scope ps("mixed_prep_rows_operand", s, 0.0, 24.0 * n * k + 3.0 * kp * n_pad);
-        dim3 g1((unsigned)nst, (unsigned)((k + kPrepCols - 1) / kPrepCols));
-        k_col_stats<<<g1, 256, 0, s>>>(X, ldx, n, k, ws.colpart.get());
-        k_col_finalize<<<(unsigned)((k + 7) / 8), 256, 0, s>>>(ws.colpart.get(), nst, k, n,
-                                                               ws.mean1.get(), ws.max1.get());
-        dim3 g2((unsigned)rt, (unsigned)((kp + kPrepCols - 1) / kPrepCols));
-        k_split_rows_operand<<<g2, 256, 0, s>>>(X, ldx, n, k, kp, n_pad, ws.mean1.get(),
-                                                ws.max1.get(), ws.b1.get(), ws.colpart.get());
-        k_sum_partials<<<(unsigned)((k + 7) / 8), 256, 0, s>>>(ws.colpart.get(), rt, k, 1.0, ws.qsum.get());
+        int kc = 1;
+        while (X.rs != 1 && kc < k && kc < 32) kc *= 2;
+        const int64_t per = 32 / kc;  // chunks per block
+        k_col_stats<T><<<dim3((unsigned)((nst + per - 1) / per), (unsigned)((k + kc - 1) / kc)), 256, 0, s>>>(
+            X, n, k, kc, nst, ws.colpart.get(), C);
+        if (kp <= 16)
+            k_split_rows_operand<T, 4, 512><<<dim3((unsigned)((n_pad + 511) / 512), (unsigned)((kp + 3) / 4)),
+                                              128, 0, s>>>(X, n, k, kp, n_pad, C, ws.b1.get());
+        else
+            k_split_rows_operand<T, 16, 256><<<dim3((unsigned)(n_pad / 256), (unsigned)((kp + 15) / 16)), 256,
+                                               0, s>>>(X, n, k, kp, n_pad, C, ws.b1.get());
         CS_LAUNCH("mixed rows operand");
     }
     PassArgs P{};
@@ -1710,22 +1811,23 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, cons
             launch_pass<true, false>(r.tm, ws.tm_b1, ws.tm_b1t, P, s);
         CS_LAUNCH("kinship_rows_tc");
     }
-    if (want_max) CS_CUDA(cudaMemsetAsync(ws.max_w.get(), 0, 8 * k, s));
     {
         prof::Scope ps("mixed_reduce_rows", s, 0.0, 8.0 * splits * kp * R + 8.0 * R * k);
-        dim3 g((unsigned)((R + 2047) / 2048), (unsigned)k);
-        k_reduce_rows<<<g, 256, 0, s>>>(ws.part.get(), splits, kp, r_pad, R, k, r.s.get(), spow,
-                                        r.exc.get(), r.mu.get(), ws.mean1.get(), ws.qsum.get(),
-                                        ws.max1.get(), out, out_ld, colmajor ? 1 : 0,
-                                        want_max ? ws.max_w.get() : nullptr);
+        if (Wt)
+            k_reduce_rows<<<dim3((unsigned)((R + 1023) / 1024), (unsigned)k), 256, 0, s>>>(
+                ws.part.get(), splits, kp, r_pad, R, r.s.get(), r.exc.get(), r.mu.get(), C, Wt);
+        else
+            k_reduce_rows_out<<<dim3((unsigned)((R + 31) / 32), (unsigned)((k + 31) / 32)), 256, 0, s>>>(
+                ws.part.get(), splits, kp, r_pad, R, k, r.s.get(), r.exc.get(), r.mu.get(), pos, C, out);
         CS_LAUNCH("reduce_rows");
     }
 }
 
-// Samples pass: Y (n x k, row-major ldy) = (Z W) / M for W^T (k x R, column-major) with the
-// per-column maxima computed by rows_pass(want_max).
+// Samples pass: Y (n x k) = (Z W) / M for W^T (k x R, column-major) with the per-column maxima that
+// the rows pass (or the gather) left.
+template <class T>
 void samples_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, const double* Wt,
-                       int64_t k, double inv_m, double* Y, int64_t ldy, cudaStream_t s) {
+                       int64_t k, double inv_m, Strided<T> Y, cudaStream_t s) {
     const int64_t tiles = r.n_pad / kTile;
     const bool pairs = plan.pairs;
     const Tiling tl = tiling_for(k, plan.max_w);
@@ -1757,21 +1859,15 @@ void samples_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, c
     }
     {
         prof::Scope ps("mixed_prep_samples_operand", s, 0.0, 8.0 * R * k + pieces * kp * r_pad);
-        dim3 g((unsigned)nrb, (unsigned)kp);
-        if (six) {
-            ws.max_wmu.resize(k);
-            CS_CUDA(cudaMemsetAsync(ws.max_wmu.get(), 0, 8 * k, s));
-            k_col_absmax_mu<<<dim3((unsigned)nrb, (unsigned)k), 256, 0, s>>>(Wt, R, r.mu.get(),
-                                                                            ws.max_wmu.get());
-            k_split_samples_t_operand<<<g, 256, 0, s>>>(Wt, R, k, kp, r_pad, r.mu.get(),
-                                                        ws.max_wmu.get(), ws.b2.get(),
-                                                        ws.inv_f.get(), ws.colpart.get());
-        } else {
-            k_split_samples_operand<<<g, 256, 0, s>>>(Wt, R, k, kp, r_pad, r.mu.get(), r.resid.get(),
-                                                      ws.max_w.get(), tmem_a ? 1 : 0, ws.b2.get(),
-                                                      ws.inv_f.get(), ws.colpart.get());
-        }
-        k_sum_partials<<<(unsigned)((k + 7) / 8), 256, 0, s>>>(ws.colpart.get(), nrb, k, 1.0, ws.c0.get());
+        const dim3 g((unsigned)nrb, (unsigned)kp);
+        const MixedColumns C = ws.columns(k, s);
+        auto split = [&](auto kern) {
+            kern<<<g, 128, 0, s>>>(Wt, R, k, kp, r_pad, r.mu.get(), r.resid.get(), C, ws.b2.get(),
+                                   ws.inv_f.get(), ws.colpart.get(), ws.c0.get());
+        };
+        if (six) split(k_split_samples_operand<true, true>);
+        else if (tmem_a) split(k_split_samples_operand<false, true>);
+        else split(k_split_samples_operand<false, false>);
         CS_LAUNCH("mixed samples operand");
     }
     PassArgs P{};
@@ -1813,30 +1909,31 @@ void samples_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, c
     }
     {
         prof::Scope ps("mixed_reduce_samples", s, 0.0, 8.0 * splits * kp * n + 8.0 * n * k);
-        k_reduce_samples<<<blocks_for(n * k), 256, 0, s>>>(ws.part.get(), splits, kp, n_pad, n, k,
-                                                           ws.c0.get(), inv_m, Y, ldy);
+        k_reduce_samples<T><<<dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)), 256, 0, s>>>(
+            ws.part.get(), splits, kp, n_pad, n, k, ws.c0.get(), inv_m, Y);
         CS_LAUNCH("reduce_samples");
     }
 }
 
-void rows_pass(MixedRows& r, MixedWorkspace& ws, const double* X, int64_t ldx, int64_t k,
-               double* out, int64_t out_ld, bool colmajor, int spow, bool want_max,
-               cudaStream_t s, bool allow_tune) {
+template <class T>
+void rows_pass(MixedRows& r, MixedWorkspace& ws, Strided<const T> X, int64_t k, double* Wt,
+               const int32_t* pos, StridedOut out, cudaStream_t s, bool allow_tune) {
     const int64_t tiles = r.r_pad / kTile;
     const int kb = (int)(r.n_pad / kKBlock);
     const PassPlan plan = choose_plan(true, allow_tune, r.R, r.n, k, tiles, kb, s, [&](const PassPlan& p) {
-        rows_pass_plan(p, r, ws, X, ldx, k, out, out_ld, colmajor, spow, want_max, s);
+        rows_pass_plan(p, r, ws, X, k, Wt, pos, out, s);
     });
-    rows_pass_plan(plan, r, ws, X, ldx, k, out, out_ld, colmajor, spow, want_max, s);
+    rows_pass_plan(plan, r, ws, X, k, Wt, pos, out, s);
 }
 
+template <class T>
 void samples_pass(MixedRows& r, MixedWorkspace& ws, const double* Wt, int64_t k, double inv_m,
-                  double* Y, int64_t ldy, cudaStream_t s, bool allow_tune, bool sample_major_copy) {
+                  Strided<T> Y, cudaStream_t s, bool allow_tune, bool sample_major_copy) {
     const int64_t tiles = r.n_pad / kTile;
     const int kb = (int)(r.r_pad / kKBlock);
     PassPlan plan = choose_plan(false, allow_tune && sample_major_copy, r.R, r.n, k, tiles, kb, s,
                                 [&](const PassPlan& p) {
-                                    samples_pass_plan(p, r, ws, Wt, k, inv_m, Y, ldy, s);
+                                    samples_pass_plan(p, r, ws, Wt, k, inv_m, Y, s);
                                 });
     if (!sample_major_copy && plan.tmem_a) {
         // A in shared memory (narrow up to 32 columns, otherwise the general layouts): the same
@@ -1848,7 +1945,7 @@ void samples_pass(MixedRows& r, MixedWorkspace& ws, const double* Wt, int64_t k,
             plan.max_w = plan.pairs ? kPairSamplesW : kSamplesW;
         }
     }
-    samples_pass_plan(plan, r, ws, Wt, k, inv_m, Y, ldy, s);
+    samples_pass_plan(plan, r, ws, Wt, k, inv_m, Y, s);
 }
 
 }  // namespace
@@ -1868,76 +1965,62 @@ static MixedOperator* mixed_for(cs_kinship* op) {
 
 MixedRows& mixed_rows_for(cs_kinship* op) { return mixed_for(op)->rows; }
 
-void kinship_apply_mixed(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* Y,
-                         int64_t ldy, cudaStream_t s) {
+template <class T>
+void kinship_apply_mixed(cs_kinship* op, Strided<const T> X, int64_t k, Strided<T> Y, cudaStream_t s) {
     if (k <= 0) return;
     const int64_t n = op->rows, R = op->n_active;
     if (R == 0) {
-        CS_CUDA(cudaMemset2DAsync(Y, ldy * 8, 0, k * 8, n, s));
+        const bool cm = Y.rs == 1;
+        CS_CUDA(cudaMemset2DAsync(Y.p, sizeof(T) * (cm ? Y.cs : Y.rs), 0, sizeof(T) * (cm ? n : k),
+                                  cm ? k : n, s));
         return;
     }
     MixedOperator* m = mixed_for(op);
     m->ws.W.resize(R * k);
     // W^T = s o s o (Z-centred)^T X: the rows pass output already scaled for the samples pass
     m->last_k = 0;
-    rows_pass(m->rows, m->ws, X, ldx, k, m->ws.W.get(), R, true, 2, true, s, op->autotune);
-    samples_pass(m->rows, m->ws, m->ws.W.get(), k, 1.0 / (double)op->num_variants, Y, ldy, s,
-                 op->autotune, op->sample_major_copy);
+    rows_pass(m->rows, m->ws, X, k, m->ws.W.get(), nullptr, StridedOut{}, s, op->autotune);
+    samples_pass(m->rows, m->ws, m->ws.W.get(), k, 1.0 / (double)op->num_variants, Y, s, op->autotune,
+                 op->sample_major_copy);
     check_status(m->ws, s);
     m->last_k = k;
 }
+template void kinship_apply_mixed<double>(cs_kinship*, Strided<const double>, int64_t, Strided<double>,
+                                          cudaStream_t);
+template void kinship_apply_mixed<float>(cs_kinship*, Strided<const float>, int64_t, Strided<float>,
+                                         cudaStream_t);
 
-// Column maxima of |W| for a column-major R x k W (the samples-pass operand scales):
-// atomicMax on the bits of non-negative doubles (order independent).
-__global__ void __launch_bounds__(256)
-k_col_absmax(const double* __restrict__ W, int64_t R, int64_t k, unsigned long long* __restrict__ max_w) {
-    __shared__ double red_w[8];
-    const int64_t c = blockIdx.y;
-    double mw = 0.0;
-    const int64_t t0 = (int64_t)blockIdx.x * 2048;
-    for (int64_t t = t0 + threadIdx.x; t < min(R, t0 + 2048); t += 256) mw = fmax(mw, fabs(W[c * R + t]));
-    for (int off = 16; off; off >>= 1) mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, off));
-    if ((threadIdx.x & 31) == 0) red_w[threadIdx.x >> 5] = mw;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int j = 1; j < 8; ++j) mw = fmax(mw, red_w[j]);
-        atomicMax(max_w + c, (unsigned long long)__double_as_longlong(mw));
-    }
-}
-
-// GenotypeMatrix::multiply_Zt_v on tensor cores: U (R x k, row-major ldu) = Z^T X over the
-// operator's view rows, X (rows x k, row-major ldx).
-void mixed_multiply_zt(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* U,
-                       int64_t ldu, cudaStream_t s) {
+// GenotypeMatrix::multiply_Zt_v on tensor cores.
+void mixed_multiply_zt(cs_kinship* op, StridedIn X, int64_t k, StridedOut U, cudaStream_t s) {
     if (k <= 0 || op->n_active == 0) return;
     MixedOperator* m = mixed_for(op);
     m->last_k = 0;
-    rows_pass(m->rows, m->ws, X, ldx, k, U, ldu, false, 1, false, s, op->autotune);
+    rows_pass(m->rows, m->ws, X, k, nullptr, op->d_view_pos.get(), U, s, op->autotune);
     check_status(m->ws, s);
 }
 
-// GenotypeMatrix::multiply_Z_v on tensor cores: Y (rows x k, row-major ldy) = Z V with
-// W = s o V over the view rows given column-major (R x k, leading dimension R).
-void mixed_multiply_z(cs_kinship* op, const double* Wcol, int64_t k, double* Y, int64_t ldy,
-                      cudaStream_t s) {
+// GenotypeMatrix::multiply_Z_v on tensor cores.
+void mixed_multiply_z(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cudaStream_t s) {
     if (k <= 0) return;
     const int64_t R = op->n_active;
     MixedOperator* m = mixed_for(op);
     m->last_k = 0;
     MixedWorkspace& ws = m->ws;
-    ws.max_w.resize(k);
     if (!ws.status.get()) {
         ws.status.resize(1);
         CS_CUDA(cudaMemsetAsync(ws.status.get(), 0, sizeof(int), s));
     }
-    CS_CUDA(cudaMemsetAsync(ws.max_w.get(), 0, 8 * k, s));
+    ws.W.resize(R * k);
+    const MixedColumns C = ws.columns(k, s);
+    CS_CUDA(cudaMemsetAsync(C.max_w, 0, 8 * k, s));
+    CS_CUDA(cudaMemsetAsync(C.max_wmu, 0, 8 * k, s));
     {
-        prof::Scope ps("mixed_col_absmax", s, 0.0, 8.0 * R * k);
-        dim3 g((unsigned)((R + 2047) / 2048), (unsigned)k);
-        k_col_absmax<<<g, 256, 0, s>>>(Wcol, R, k, ws.max_w.get());
-        CS_LAUNCH("col_absmax");
+        prof::Scope ps("mixed_gather_operand", s, 0.0, 16.0 * R * k);
+        k_gather_operand<<<dim3((unsigned)((R + 1023) / 1024), (unsigned)k), 256, 0, s>>>(
+            V, R, op->d_view_pos.get(), m->rows.s.get(), m->rows.mu.get(), C, ws.W.get());
+        CS_LAUNCH("gather_operand");
     }
-    samples_pass(m->rows, ws, Wcol, k, 1.0, Y, ldy, s, op->autotune, op->sample_major_copy);
+    samples_pass(m->rows, ws, ws.W.get(), k, 1.0, Y, s, op->autotune, op->sample_major_copy);
     check_status(ws, s);
 }
 
@@ -1996,7 +2079,7 @@ void mixed_scan_destroy(MixedScan* m) { delete m; }
 
 void mixed_scan_project(MixedScan* m, const double* B, int64_t ldb, int64_t k, double* T,
                         int64_t ldt, cudaStream_t s) {
-    rows_pass(m->rows, m->ws, B, ldb, k, T, ldt, false, 1, false, s, true);
+    rows_pass(m->rows, m->ws, StridedIn{B, ldb, 1}, k, nullptr, nullptr, StridedOut{T, ldt, 1}, s, true);
     check_status(m->ws, s);
 }
 

@@ -795,25 +795,35 @@ __global__ void __launch_bounds__(128)
 k_slice_samples_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int64_t r_pad,
                         int slice_rows, const double* __restrict__ mu, const SliceSums S, BLayout B,
                         int8_t* __restrict__ out) {
-    const int64_t c = blockIdx.y;
-    const int64_t t0 = ((int64_t)blockIdx.x * 128 + threadIdx.x) * 16;
+    // w and mu o w of 2048 SNPs, one pad every 16, read in the order of memory
+    __shared__ double sw[128 * 17], sb[128 * 17];
+    const int64_t c = blockIdx.y, base = (int64_t)blockIdx.x * 2048;
+#pragma unroll 8
+    for (int e = threadIdx.x; e < 2048; e += 128) {
+        const int64_t t = base + e;
+        const double w = (c < k && t < R) ? Wt[c * R + t] : 0.0;
+        sw[e + (e >> 4)] = w;
+        sb[e + (e >> 4)] = t < R ? mu[t] * w : 0.0;
+    }
+    __syncthreads();
+    const int64_t t0 = base + 16 * threadIdx.x;
     const bool live = t0 < r_pad;
     int64_t sh = 0, sl = 0;
     if (live) {
         const double f = c < k ? pow2(slice_exponent(S.range_w[c].max_bits)) : 0.0;
-        int64_t v[16], m[16];
+        int64_t v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = __double2ll_rn(sw[17 * threadIdx.x + j] * f);
+        emit_digits(v, B, c, 0, t0, r_pad, out);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            const double w = (c < k && t0 + j < R) ? Wt[c * R + t0 + j] : 0.0;
-            v[j] = __double2ll_rn(w * f);
-            m[j] = __double2ll_rn((mu[t0 + j] * w) * f);
+            v[j] = __double2ll_rn(sb[17 * threadIdx.x + j] * f);
             int64_t h, l;
-            split_value(m[j], h, l);
+            split_value(v[j], h, l);
             sh += h;
             sl += l;
         }
-        emit_digits(v, B, c, 0, t0, r_pad, out);
-        emit_digits(m, B, c, 1, t0, r_pad, out);
+        emit_digits(v, B, c, 1, t0, r_pad, out);
     }
     // 16 threads hold 256 SNPs, which lie in one slice
     sh = shfl_sum(sh, 16);

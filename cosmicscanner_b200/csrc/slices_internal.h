@@ -38,17 +38,6 @@ __device__ __forceinline__ bool range_excluded(const ColumnRange& r) {
 struct SliceOperator;
 void destroy_slices(SliceOperator* s);
 
-// A matrix operand with element (i, c) at p[i * rs + c * cs]: row-major (cs = 1) or column-major
-// (rs = 1).
-struct StridedIn {
-    const double* p;
-    int64_t rs, cs;
-};
-struct StridedOut {
-    double* p;
-    int64_t rs, cs;
-};
-
 // FP64 products through the slices where the operator has (or may have) a sample-major copy and
 // the shape is large enough; false when the FP64-pipe kernels are to be used.  Results may
 // overwrite the input.
