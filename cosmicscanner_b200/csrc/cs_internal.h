@@ -147,6 +147,8 @@ struct MixedOperator;  // tensor-core form (kinship_mixed.cu)
 void destroy_mixed(MixedOperator* m);
 struct SliceOperator;  // FP64 on the tensor cores (kinship_slices.cu)
 void destroy_slices(SliceOperator* s);
+struct PcgWorkspace;  // pcg.cu
+void destroy_pcg(PcgWorkspace* w);
 }  // namespace cs
 
 // Kinship operator over a (keep, variants) selection of a cs_genotypes matrix.
@@ -173,6 +175,8 @@ struct cs_kinship {
     cs::MixedOperator* mixed = nullptr;
     cs::SliceOperator* slices = nullptr;
     bool slices_unavailable = false;  // no device memory for them: FP64-pipe kernels only
+    bool defer_checks = false;        // a solver's loop checks its passes itself (kinship_check)
+    cs::PcgWorkspace* pcg = nullptr;  // kept from one solve on this operator to the next (pcg.cu)
     bool autotune = true;  // the tensor-core passes may tune their plan on new shapes
     // the samples pass may keep a sample-major copy of the packed view (one more packed matrix
     // in HBM) and read its A operand from tensor memory (six operand sets at the widths where
@@ -180,6 +184,7 @@ struct cs_kinship {
     // five-set form, so a column's result does not depend on how many columns share its apply
     bool sample_major_copy = true;
     ~cs_kinship() {
+        cs::destroy_pcg(pcg);
         cs::destroy_slices(slices);
         cs::destroy_mixed(mixed);
     }
@@ -214,8 +219,13 @@ void mixed_multiply_zt(cs_kinship* op, StridedIn X, int64_t k, StridedOut U, cud
 void mixed_multiply_z(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cudaStream_t s);
 
 // Waits for the stream and fails if the operator's last FP64 tensor-core pass gave up waiting (its
-// results are NaN; kinship_slices.cu).
+// results are NaN; kinship_slices.cu), or a mixed one has (kinship_mixed.cu), or either.
 void check_slices(cs_kinship* op, cudaStream_t s);
+void check_mixed(cs_kinship* op, cudaStream_t s);
+inline void kinship_check(cs_kinship* op, cudaStream_t s) {
+    check_mixed(op, s);
+    check_slices(op, s);
+}
 
 // The reference's Gaussian test matrix (std::normal_distribution over std::mt19937_64) on the
 // device, written row-major n x ld (omega.cu).

@@ -1982,9 +1982,13 @@ void kinship_apply_mixed(cs_kinship* op, Strided<const T> X, int64_t k, Strided<
     rows_pass(m->rows, m->ws, X, k, m->ws.W.get(), nullptr, StridedOut{}, s, op->autotune);
     samples_pass(m->rows, m->ws, m->ws.W.get(), k, 1.0 / (double)op->num_variants, Y, s, op->autotune,
                  op->sample_major_copy);
-    check_status(m->ws, s);
+    if (!op->defer_checks) check_status(m->ws, s);
     m->last_k = k;
 }
+void check_mixed(cs_kinship* op, cudaStream_t s) {
+    if (op->mixed && op->mixed->ws.status.get()) check_status(op->mixed->ws, s);
+}
+
 template void kinship_apply_mixed<double>(cs_kinship*, Strided<const double>, int64_t, Strided<double>,
                                           cudaStream_t);
 template void kinship_apply_mixed<float>(cs_kinship*, Strided<const float>, int64_t, Strided<float>,

@@ -20,98 +20,231 @@ namespace cs {
 
 namespace {
 
-constexpr int kColTile = 32, kRowLanes = 8;
+// ---------------------------------------------------------------- column sums
+// Sums over the rows of n x k blocks, NV per column, in an order that depends on n alone: chunks of
+// `chunk` rows, eight interleaved lanes in each, lanes added in order, then the chunks by one
+// warp's strided sums and a shuffle tree.  A block covers kc columns (a power of two up to 32) x
+// 32 / kc chunks; the last block of a column tile finishes its columns, so that what follows from
+// the sums (a step length, a coefficient) needs no kernel of its own.  Chunks of 64 rows keep the
+// chain of dependent loads short: at n=2000 and 34 columns a sum took 14 us with 512-row chunks
+// in 8 blocks and takes 4 us with these.
+constexpr int kChunkRows = 64, kMaxChunks = 512;
+int64_t chunk_rows(int64_t n) {
+    return kChunkRows * std::max<int64_t>(1, (n + (int64_t)kChunkRows * kMaxChunks - 1) /
+                                                 ((int64_t)kChunkRows * kMaxChunks));
+}
+int64_t chunk_count(int64_t n) { return std::max<int64_t>(1, (n + chunk_rows(n) - 1) / chunk_rows(n)); }
 
-int64_t reduction_chunks(int64_t n) { return std::min<int64_t>(128, std::max<int64_t>(1, (n + 511) / 512)); }
-
-// partial[b * k + c] = sum over rows of chunk b of A[r, c] * B[r, c]
-__global__ void k_dot_partial(const double* __restrict__ A, int64_t lda, const double* __restrict__ B,
-                              int64_t ldb, int64_t n, int64_t k, int64_t chunk,
-                              double* __restrict__ partial) {
-    __shared__ double red[kRowLanes][kColTile];
-    const int64_t c = (int64_t)blockIdx.y * kColTile + threadIdx.x;
-    const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = min(n, r0 + chunk);
-    double acc = 0.0;
-    if (c < k)
-        for (int64_t r = r0 + threadIdx.y; r < r1; r += kRowLanes) acc += A[r * lda + c] * B[r * ldb + c];
-    red[threadIdx.y][threadIdx.x] = acc;
+template <int NV, class Elem, class Finish>
+__global__ void __launch_bounds__(256)
+k_column_reduce(int64_t n, int64_t k, int64_t chunk, int64_t nb, int kc, double* __restrict__ part,
+                unsigned* __restrict__ counter, const Elem elem, const Finish finish) {
+    __shared__ double red[NV][256];
+    __shared__ int last;
+    const int chunks = 32 / kc;
+    const int tc = threadIdx.x % kc, tl = threadIdx.x / kc;
+    const int lane = tl & 7, ch = tl >> 3;
+    const int64_t c = (int64_t)blockIdx.y * kc + tc;
+    const int64_t b = (int64_t)blockIdx.x * chunks + ch;
+    double v[NV] = {};
+    if (c < k && b < nb) {
+        const int64_t r1 = min(n, (b + 1) * chunk);
+#pragma unroll 4
+        for (int64_t r = b * chunk + lane; r < r1; r += 8) elem(r, c, v);
+    }
+    const int slot = (tc * chunks + ch) * 8 + lane;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) red[q][slot] = v[q];
     __syncthreads();
-    if (threadIdx.y == 0 && c < k) {
-        double s = red[0][threadIdx.x];
-        for (int q = 1; q < kRowLanes; ++q) s += red[q][threadIdx.x];
-        partial[blockIdx.x * k + c] = s;
+    if (threadIdx.x < 32) {  // one thread per (column, chunk)
+        const int64_t oc = (int64_t)blockIdx.y * kc + threadIdx.x / chunks;
+        const int64_t ob = (int64_t)blockIdx.x * chunks + threadIdx.x % chunks;
+        if (oc < k && ob < nb)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                double t = red[q][threadIdx.x * 8];
+                for (int j = 1; j < 8; ++j) t += red[q][threadIdx.x * 8 + j];
+                part[((int64_t)q * nb + ob) * k + oc] = t;
+            }
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(counter + blockIdx.y, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int wl = threadIdx.x & 31;
+    for (int j = threadIdx.x >> 5; j < kc; j += 8) {
+        const int64_t oc = (int64_t)blockIdx.y * kc + j;
+        if (oc >= k) break;
+        double tot[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            double t = 0.0;
+            for (int64_t ob = wl; ob < nb; ob += 32) t += __ldcg(part + ((int64_t)q * nb + ob) * k + oc);
+            for (int off = 16; off; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+            tot[q] = t;
+        }
+        if (wl == 0) finish(oc, tot);
     }
 }
 
-__global__ void k_sum_partials(const double* __restrict__ partial, int64_t nb, int64_t k,
-                               double* __restrict__ out) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= k) return;
-    double s = 0.0;
-    for (int64_t b = 0; b < nb; ++b) s += partial[b * k + c];
-    out[c] = s;
+template <int NV, class Elem, class Finish>
+void column_reduce(int64_t n, int64_t k, const Elem& elem, const Finish& finish, PcgWorkspace& ws,
+                   cudaStream_t s) {
+    ws.reserve_reduction(n, k, s);
+    int kc = 1;
+    while (kc < k && kc < 32) kc *= 2;
+    const int64_t nb = chunk_count(n), chunks = 32 / kc;
+    k_column_reduce<NV, Elem, Finish>
+        <<<dim3((unsigned)((nb + chunks - 1) / chunks), (unsigned)((k + kc - 1) / kc)), 256, 0, s>>>(
+            n, k, chunk_rows(n), nb, kc, ws.partial.get(), ws.counter.get(), elem, finish);
+    CS_LAUNCH("column_reduce");
 }
 
-// alpha_c = rsold_c / (p . Ap)_c
-__global__ void k_alpha(const double* __restrict__ partial, int64_t nb, int64_t k,
-                        const double* __restrict__ rsold, double* __restrict__ alpha) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= k) return;
-    double s = 0.0;
-    for (int64_t b = 0; b < nb; ++b) s += partial[b * k + c];
-    alpha[c] = rsold[c] / s;
-}
-
-// x += alpha p, r -= alpha Ap; partial sums of r.r and r.z with z = r / diag
-__global__ void k_cg_update(double* __restrict__ X, int64_t ldx, const int32_t* __restrict__ map,
-                            const double* __restrict__ P, const double* __restrict__ AP,
-                            double* __restrict__ R, int64_t ld, int64_t n, int64_t k, int64_t chunk,
-                            const double* __restrict__ alpha, double diag,
-                            double* __restrict__ part_rr, double* __restrict__ part_rz) {
-    __shared__ double red_a[kRowLanes][kColTile], red_b[kRowLanes][kColTile];
-    const int64_t c = (int64_t)blockIdx.y * kColTile + threadIdx.x;
-    const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = min(n, r0 + chunk);
-    double rr = 0.0, rz = 0.0;
-    if (c < k) {
+struct StoreSum {
+    double* out;
+    __device__ void operator()(int64_t c, const double (&t)[1]) const { out[c] = t[0]; }
+};
+struct StoreTwo {
+    double *a, *b;
+    __device__ void operator()(int64_t c, const double (&t)[2]) const {
+        a[c] = t[0];
+        b[c] = t[1];
+    }
+};
+struct Dot {
+    const double* A;
+    int64_t lda;
+    const double* B;
+    int64_t ldb;
+    __device__ void operator()(int64_t r, int64_t c, double (&v)[1]) const {
+        v[0] += A[r * lda + c] * B[r * ldb + c];
+    }
+};
+// R = B (columns idx), P = B / diag; r . r and r . p
+struct CgInit {
+    const double* B;
+    int64_t ldb;
+    const int32_t* idx;
+    double *R, *P;
+    int64_t ld;
+    double diag;
+    __device__ void operator()(int64_t r, int64_t c, double (&v)[2]) const {
+        const double b = B[r * ldb + idx[c]], p = b / diag;
+        R[r * ld + c] = b;
+        P[r * ld + c] = p;
+        v[0] += b * b;
+        v[1] += b * p;
+    }
+};
+// out = vg * fac * KU[row(r)] + vpe * U[row(r)] + ve * V[r]   (stcg_vce.cpp:103-115)
+struct Covariance {
+    const double *V, *KU, *U;
+    int64_t ldv, ldk, ldu;
+    const int32_t* rec_to_row;
+    double vg, fac, vpe, ve;
+    int with_pe;
+    __device__ double operator()(int64_t r, int64_t c) const {
+        const int64_t i = rec_to_row ? rec_to_row[r] : r;
+        double g = 0.0, pe = 0.0;
+        if (i >= 0) {
+            g = KU[i * ldk + c];
+            if (fac != 1.0) g *= fac;
+            if (with_pe) pe = U[i * ldu + c];
+        }
+        double o = vg * g;
+        if (with_pe) o += vpe * pe;
+        return o + ve * V[r * ldv + c];
+    }
+};
+// AP = V p and p . AP
+struct CgProduct {
+    Covariance cov;
+    double* out;
+    int64_t ldo;
+    __device__ void operator()(int64_t r, int64_t c, double (&v)[1]) const {
+        const double o = cov(r, c);
+        out[r * ldo + c] = o;
+        v[0] += cov.V[r * cov.ldv + c] * o;
+    }
+};
+// alpha = rsold / (p . Ap)
+struct CgAlpha {
+    const double* rsold;
+    double* alpha;
+    __device__ void operator()(int64_t c, const double (&t)[1]) const { alpha[c] = rsold[c] / t[0]; }
+};
+// x += alpha p, r -= alpha Ap; r . r and r . z with z = r / diag
+struct CgUpdate {
+    double* X;
+    int64_t ldx;
+    const int32_t* map;
+    const double *P, *AP;
+    double* R;
+    int64_t ld;
+    const double* alpha;
+    double diag;
+    __device__ void operator()(int64_t r, int64_t c, double (&v)[2]) const {
         const double a = alpha[c];
-        const int64_t xc = map[c];
-        for (int64_t r = r0 + threadIdx.y; r < r1; r += kRowLanes) {
-            X[r * ldx + xc] += a * P[r * ld + c];
-            const double rv = R[r * ld + c] - a * AP[r * ld + c];
-            R[r * ld + c] = rv;
-            rr += rv * rv;
-            rz += rv * (rv / diag);
+        X[r * ldx + map[c]] += a * P[r * ld + c];
+        const double rv = R[r * ld + c] - a * AP[r * ld + c];
+        R[r * ld + c] = rv;
+        v[0] += rv * rv;
+        v[1] += rv * (rv / diag);
+    }
+};
+// beta = rz / rsold, rsold = rz; the squared residual (and rz) to the host
+struct CgBeta {
+    double *rsold, *beta, *rr_host, *rz_host;
+    __device__ void operator()(int64_t c, const double (&t)[2]) const {
+        rr_host[c] = t[0];
+        rz_host[c] = t[1];
+        beta[c] = t[1] / rsold[c];
+        rsold[c] = t[1];
+    }
+};
+struct CgBetaZ {
+    double *rsold, *beta, *rz_host;
+    __device__ void operator()(int64_t c, const double (&t)[1]) const {
+        rz_host[c] = t[0];
+        beta[c] = t[0] / rsold[c];
+        rsold[c] = t[0];
+    }
+};
+struct LanczosElem {
+    double* w;
+    const double *sub, *dot, *coef;
+    int64_t ld;
+    __device__ void operator()(int64_t r, int64_t c, double (&v)[1]) const {
+        double x = w[r * ld + c];
+        if (sub) {
+            x -= coef[c] * sub[r * ld + c];
+            w[r * ld + c] = x;
         }
+        v[0] += x * (dot ? dot[r * ld + c] : x);
     }
-    red_a[threadIdx.y][threadIdx.x] = rr;
-    red_b[threadIdx.y][threadIdx.x] = rz;
-    __syncthreads();
-    if (threadIdx.y == 0 && c < k) {
-        double sa = red_a[0][threadIdx.x], sb = red_b[0][threadIdx.x];
-        for (int q = 1; q < kRowLanes; ++q) {
-            sa += red_a[q][threadIdx.x];
-            sb += red_b[q][threadIdx.x];
+};
+struct LanczosFinish {
+    LanczosState st;
+    LanczosMode mode;
+    int step;
+    __device__ void operator()(int64_t c, const double (&t)[1]) const {
+        const bool done = st.done[c] != 0;
+        double coef = done ? 0.0 : t[0];
+        if (!done && mode == LanczosMode::kAlpha) st.alpha[c] = t[0];
+        if (!done && mode == LanczosMode::kBeta) {
+            coef = sqrt(t[0]);
+            st.beta[c] = coef;
+            if (coef < 1e-12) {
+                st.steps[c] = step + 1;
+                st.done[c] = 1;
+                coef = 0.0;
+            }
         }
-        part_rr[blockIdx.x * k + c] = sa;
-        part_rz[blockIdx.x * k + c] = sb;
+        st.coef[c] = coef;
     }
-}
-
-// rr_c, rz_c; beta_c = rz_c / rsold_c; rsold_c = rz_c
-__global__ void k_beta(const double* __restrict__ part_rr, const double* __restrict__ part_rz,
-                       int64_t nb, int64_t k, double* __restrict__ rsold, double* __restrict__ beta,
-                       double* __restrict__ rr_out) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= k) return;
-    double a = 0.0, b = 0.0;
-    for (int64_t q = 0; q < nb; ++q) {
-        a += part_rr[q * k + c];
-        b += part_rz[q * k + c];
-    }
-    rr_out[c] = a;
-    beta[c] = b / rsold[c];
-    rsold[c] = b;
-}
+};
 
 // p = z + beta p
 __global__ void k_direction_z(double* __restrict__ P, const double* __restrict__ Z, int64_t ld,
@@ -132,20 +265,6 @@ __global__ void k_direction(double* __restrict__ P, const double* __restrict__ R
          e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = e / k, c = e - r * k;
         P[r * ld + c] = R[r * ld + c] / diag + beta[c] * P[r * ld + c];
-    }
-}
-
-// R = B (columns idx), P = B / diag
-__global__ void k_cg_init(const double* __restrict__ B, int64_t ldb, const int32_t* __restrict__ idx,
-                          double* __restrict__ R, double* __restrict__ P, int64_t ld, int64_t n,
-                          int64_t k, double diag) {
-    const int64_t total = n * k;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = e / k, c = e - r * k;
-        const double b = B[r * ldb + idx[c]];
-        R[r * ld + c] = b;
-        P[r * ld + c] = b / diag;
     }
 }
 
@@ -175,26 +294,13 @@ __global__ void k_records_to_rows(const double* __restrict__ V, int64_t ldv, int
     }
 }
 
-// out = vg * fac * KU[row(r)] + vpe * U[row(r)] + ve * V[r]   (stcg_vce.cpp:103-115)
-__global__ void k_combine(double* __restrict__ out, int64_t ldo, const double* __restrict__ V,
-                          int64_t ldv, const double* __restrict__ KU, int64_t ldk,
-                          const double* __restrict__ U, int64_t ldu,
-                          const int32_t* __restrict__ rec_to_row, int64_t n_rec, int64_t k,
-                          double vg, double fac, double vpe, double ve, int with_pe) {
+__global__ void k_combine(double* __restrict__ out, int64_t ldo, const Covariance cov, int64_t n_rec,
+                          int64_t k) {
     const int64_t total = n_rec * k;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = e / k, c = e - r * k;
-        const int64_t i = rec_to_row ? rec_to_row[r] : r;
-        double g = 0.0, pe = 0.0;
-        if (i >= 0) {
-            g = KU[i * ldk + c];
-            if (fac != 1.0) g *= fac;
-            pe = U[i * ldu + c];
-        }
-        double o = vg * g;
-        if (with_pe) o += vpe * pe;
-        out[r * ldo + c] = o + ve * V[r * ldv + c];
+        out[r * ldo + c] = cov(r, c);
     }
 }
 
@@ -285,20 +391,36 @@ const double* VOperator::gather(const double* in, int64_t ldi, int64_t k, cudaSt
     return u.get();
 }
 
-void VOperator::apply(const double* in, int64_t ldi, int64_t k, double* out, int64_t ldo,
-                      cudaStream_t s) {
-    if (k <= 0) return;
+const double* VOperator::kinship(const double* in, int64_t ldi, int64_t k, int64_t& ldu, cudaStream_t s) {
     const double* U = gather(in, ldi, k, s);
-    const int64_t ldu = rm->identity ? ldi : k;
+    ldu = rm->identity ? ldi : k;
     ku.resize(std::max<int64_t>(1, rm->n_rows * k));
     kinship_apply_rowmajor(op, U, ldu, k, ku.get(), k, precision, s);
     ++applies;
     apply_cols += k;
+    return U;
+}
+
+void VOperator::apply(const double* in, int64_t ldi, int64_t k, double* out, int64_t ldo,
+                      cudaStream_t s) {
+    if (k <= 0) return;
+    int64_t ldu = 0;
+    const double* U = kinship(in, ldi, k, ldu, s);
+    const Covariance cov{in, ku.get(), U, ldi, k, ldu, rm->identity ? nullptr : rm->d_rec_to_row.get(),
+                         vg, fac, vpe, ve, with_pe ? 1 : 0};
     prof::Scope ps("covariance_combine", s, 0.0, 8.0 * 3.0 * (double)rm->n_rec * k);
-    k_combine<<<grid_for(rm->n_rec * k), 256, 0, s>>>(
-        out, ldo, in, ldi, ku.get(), k, U, ldu, rm->identity ? nullptr : rm->d_rec_to_row.get(),
-        rm->n_rec, k, vg, fac, vpe, ve, with_pe ? 1 : 0);
+    k_combine<<<grid_for(rm->n_rec * k), 256, 0, s>>>(out, ldo, cov, rm->n_rec, k);
     CS_LAUNCH("covariance_combine");
+}
+
+void VOperator::apply_alpha(const double* p, int64_t k, double* out, const double* rsold, double* alpha,
+                            PcgWorkspace& ws, cudaStream_t s) {
+    int64_t ldu = 0;
+    const double* U = kinship(p, k, k, ldu, s);
+    const Covariance cov{p, ku.get(), U, k, k, ldu, rm->identity ? nullptr : rm->d_rec_to_row.get(),
+                         vg, fac, vpe, ve, with_pe ? 1 : 0};
+    prof::Scope ps("covariance_combine", s, 2.0 * (double)rm->n_rec * k, 8.0 * 3.0 * (double)rm->n_rec * k);
+    column_reduce<1>(rm->n_rec, k, CgProduct{cov, out, k}, CgAlpha{rsold, alpha}, ws, s);
 }
 
 void VOperator::derivatives(const double* in, int64_t ldi, int64_t k, double* g_out, int64_t ldg,
@@ -336,23 +458,33 @@ void VOperator::genetic_rows(const double* in, int64_t ldi, int64_t k, double* r
 }
 
 // ---------------------------------------------------------------- dots
+void PcgWorkspace::reserve_reduction(int64_t n, int64_t k, cudaStream_t s) {
+    partial.resize(2 * chunk_count(n) * std::max<int64_t>(1, k));
+    host.resize(2 * std::max<int64_t>(1, k));
+    if (counter.count < (size_t)k) {
+        counter.resize(k);
+        CS_CUDA(cudaMemsetAsync(counter.get(), 0, sizeof(unsigned) * counter.count, s));
+    }
+}
+
+void destroy_pcg(PcgWorkspace* w) { delete w; }
+
 void column_dots(const double* A, int64_t lda, const double* B, int64_t ldb, int64_t n, int64_t k,
                  double* out_host, PcgWorkspace& ws, cudaStream_t s) {
     if (k <= 0) return;
-    const int64_t nb = reduction_chunks(n), chunk = (n + nb - 1) / nb;
-    ws.partial_a.resize(nb * k);
-    ws.rr.resize(std::max<int64_t>(k, 1));
+    ws.reserve_reduction(n, k, s);
     {
         prof::Scope ps("column_dots", s, 2.0 * n * k, 16.0 * n * k);
-        k_dot_partial<<<dim3((unsigned)nb, (unsigned)((k + kColTile - 1) / kColTile)),
-                        dim3(kColTile, kRowLanes), 0, s>>>(A, lda, B, ldb, n, k, chunk,
-                                                            ws.partial_a.get());
-        CS_LAUNCH("column_dots");
+        column_reduce<1>(n, k, Dot{A, lda, B, ldb}, StoreSum{ws.host.ptr}, ws, s);
     }
-    k_sum_partials<<<(unsigned)((k + 127) / 128), 128, 0, s>>>(ws.partial_a.get(), nb, k, ws.rr.get());
-    CS_LAUNCH("sum_partials");
-    CS_CUDA(cudaMemcpyAsync(out_host, ws.rr.get(), 8 * k, cudaMemcpyDeviceToHost, s));
     CS_CUDA(cudaStreamSynchronize(s));
+    std::copy(ws.host.ptr, ws.host.ptr + k, out_host);
+}
+
+void lanczos_step(double* w, const double* sub, const double* dot, int64_t n, int64_t k,
+                  const LanczosState& st, LanczosMode mode, int step, PcgWorkspace& ws, cudaStream_t s) {
+    prof::Scope ps("lanczos_step", s, 4.0 * n * k, 8.0 * (sub ? 4.0 : 2.0) * n * k);
+    column_reduce<1>(n, k, LanczosElem{w, sub, dot, st.coef, k}, LanczosFinish{st, mode, step}, ws, s);
 }
 
 // ---------------------------------------------------------------- low-rank preconditioner
@@ -395,31 +527,31 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
     st.column_iterations = 0;
     if (k <= 0) return;
     const int64_t n = A.rm->n_rec;
+    const DeferChecks defer(A.op);
     CS_CUDA(cudaMemset2DAsync(X, ldx * 8, 0, k * 8, n, s));
-    const int64_t nb = reduction_chunks(n), chunk = (n + nb - 1) / nb;
     ws.R.resize(n * k);
     ws.P.resize(n * k);
     ws.AP.resize(n * k);
     ws.T.resize(n * k);
-    ws.partial_a.resize(nb * k);
-    ws.partial_b.resize(nb * k);
-    for (auto* b : {&ws.alpha, &ws.beta, &ws.rsold, &ws.rr, &ws.rz}) b->resize(k);
+    ws.reserve_reduction(n, k, s);
+    for (auto* b : {&ws.alpha, &ws.beta, &ws.rsold}) b->resize(k);
     ws.map.resize(k);
     ws.idx.resize(k);
+    double* const rr_h = ws.host.ptr;      // squared residuals and r . z of the live columns, written
+    double* const rz_h = ws.host.ptr + k;  // by the kernels, read after a synchronisation
     std::vector<int32_t> map(k);
     for (int64_t c = 0; c < k; ++c) map[c] = (int32_t)c;
     CS_CUDA(cudaMemcpyAsync(ws.idx.get(), map.data(), 4 * k, cudaMemcpyHostToDevice, s));
-    k_cg_init<<<grid_for(n * k), 256, 0, s>>>(B, ldb, ws.idx.get(), ws.R.get(), ws.P.get(), k, n, k,
-                                              diag);
-    CS_LAUNCH("cg_init");
+    column_reduce<2>(n, k, CgInit{B, ldb, ws.idx.get(), ws.R.get(), ws.P.get(), k, diag},
+                     StoreTwo{rr_h, rz_h}, ws, s);
     if (M) {
         ws.Zp.resize(n * k);
         M->apply(ws.R.get(), k, k, ws.P.get(), k, s);  // p0 = z0 = M^-1 r0
+        column_reduce<1>(n, k, Dot{ws.R.get(), k, ws.P.get(), k}, StoreSum{rz_h}, ws, s);
     }
     // ||b||^2 and rsold = r . z
-    std::vector<double> rr(k), rs(k);
-    column_dots(ws.R.get(), k, ws.R.get(), k, n, k, rr.data(), ws, s);
-    column_dots(ws.R.get(), k, ws.P.get(), k, n, k, rs.data(), ws, s);
+    CS_CUDA(cudaStreamSynchronize(s));
+    std::vector<double> rr(rr_h, rr_h + k), rs(rz_h, rz_h + k);
     std::vector<double> tol_c(k);
     for (int64_t c = 0; c < k; ++c) tol_c[c] = relative ? tol * std::sqrt(rr[c]) : tol;
     // columns already solved by x = 0 (matrix_free_pcg.h:32)
@@ -453,47 +585,25 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
         CS_CUDA(cudaMemcpyAsync(ws.rsold.get(), rs.data(), 8 * k, cudaMemcpyHostToDevice, s));
     }
     CS_CUDA(cudaMemcpyAsync(ws.map.get(), map.data(), 4 * ka, cudaMemcpyHostToDevice, s));
-    std::vector<double> rr_h(k), rs_h(k);
     for (int it = 0; it < max_iter && ka > 0; ++it) {
-        A.apply(ws.P.get(), ka, ka, ws.AP.get(), ka, s);
+        A.apply_alpha(ws.P.get(), ka, ws.AP.get(), ws.rsold.get(), ws.alpha.get(), ws, s);
         ++st.sweeps;
         st.column_iterations += ka;
-        const dim3 grid((unsigned)nb, (unsigned)((ka + kColTile - 1) / kColTile));
-        const dim3 block(kColTile, kRowLanes);
+        const CgUpdate update{X, ldx, ws.map.get(), ws.P.get(), ws.AP.get(), ws.R.get(), ka, ws.alpha.get(), diag};
         {
-            prof::Scope ps("cg_step", s, 6.0 * n * ka, 8.0 * 7.0 * n * ka);
-            k_dot_partial<<<grid, block, 0, s>>>(ws.P.get(), ka, ws.AP.get(), ka, n, ka, chunk,
-                                                 ws.partial_a.get());
-            CS_LAUNCH("cg_dot");
-            k_alpha<<<(unsigned)((ka + 127) / 128), 128, 0, s>>>(ws.partial_a.get(), nb, ka,
-                                                                 ws.rsold.get(), ws.alpha.get());
-            CS_LAUNCH("cg_alpha");
-            k_cg_update<<<grid, block, 0, s>>>(X, ldx, ws.map.get(), ws.P.get(), ws.AP.get(),
-                                               ws.R.get(), ka, n, ka, chunk, ws.alpha.get(), diag,
-                                               ws.partial_a.get(), ws.partial_b.get());
-            CS_LAUNCH("cg_update");
+            prof::Scope ps("cg_step", s, 6.0 * n * ka, 8.0 * 6.0 * n * ka);
             if (M) {
                 // z = M^-1 r and r . z in place of the scalar form's r . r / diag
+                column_reduce<2>(n, ka, update, StoreTwo{rr_h, rz_h}, ws, s);
                 M->apply(ws.R.get(), ka, ka, ws.Zp.get(), ka, s);
-                k_dot_partial<<<grid, block, 0, s>>>(ws.R.get(), ka, ws.Zp.get(), ka, n, ka, chunk,
-                                                     ws.partial_b.get());
-                CS_LAUNCH("cg_rz");
+                column_reduce<1>(n, ka, Dot{ws.R.get(), ka, ws.Zp.get(), ka},
+                                 CgBetaZ{ws.rsold.get(), ws.beta.get(), rz_h}, ws, s);
+            } else {
+                column_reduce<2>(n, ka, update, CgBeta{ws.rsold.get(), ws.beta.get(), rr_h, rz_h}, ws, s);
             }
-            k_beta<<<(unsigned)((ka + 127) / 128), 128, 0, s>>>(ws.partial_a.get(), ws.partial_b.get(),
-                                                                nb, ka, ws.rsold.get(), ws.beta.get(),
-                                                                ws.rr.get());
-            CS_LAUNCH("cg_beta");
         }
-        CS_CUDA(cudaMemcpyAsync(rr_h.data(), ws.rr.get(), 8 * ka, cudaMemcpyDeviceToHost, s));
-        CS_CUDA(cudaStreamSynchronize(s));
-        for (int64_t c = 0; c < ka; ++c)
-            if (std::isnan(rr_h[c])) check_slices(A.op, s);  // an apply that gave up leaves NaN
-        std::vector<int32_t> keep_pos;
-        for (int64_t c = 0; c < ka; ++c) {
-            st.iterations[map[c]] = it + 1;
-            if (!(std::sqrt(rr_h[c]) < tol_c[map[c]])) keep_pos.push_back((int32_t)c);
-        }
-        if (keep_pos.empty()) break;
+        // the next direction of every column (also of those that turn out to be done), so that the
+        // device has it under way while the host looks at the residuals
         {
             prof::Scope ps("cg_direction", s, 2.0 * n * ka, 24.0 * n * ka);
             if (M)
@@ -504,13 +614,25 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
                                                              diag, ws.beta.get());
             CS_LAUNCH("cg_direction");
         }
+        CS_CUDA(cudaStreamSynchronize(s));
+        for (int64_t c = 0; c < ka; ++c)
+            if (std::isnan(rr_h[c])) {  // an apply that gave up leaves NaN
+                kinship_check(A.op, s);
+                break;
+            }
+        std::vector<int32_t> keep_pos;
+        for (int64_t c = 0; c < ka; ++c) {
+            st.iterations[map[c]] = it + 1;
+            if (!(std::sqrt(rr_h[c]) < tol_c[map[c]])) keep_pos.push_back((int32_t)c);
+        }
+        if (keep_pos.empty()) break;
         if ((int64_t)keep_pos.size() < ka) {
-            CS_CUDA(cudaMemcpyAsync(rs_h.data(), ws.rsold.get(), 8 * ka, cudaMemcpyDeviceToHost, s));
-            CS_CUDA(cudaStreamSynchronize(s));
+            std::vector<double> rs_h(rz_h, rz_h + ka);
             compact(keep_pos, rs_h);
             CS_CUDA(cudaMemcpyAsync(ws.map.get(), map.data(), 4 * ka, cudaMemcpyHostToDevice, s));
         }
     }
+    kinship_check(A.op, s);
     CS_CUDA(cudaStreamSynchronize(s));
 }
 

@@ -56,17 +56,6 @@ __global__ void k_copy_cols(const double* __restrict__ src, int64_t lds, int64_t
     }
 }
 
-// W[:, c] -= coef[c] * V[:, c]
-__global__ void k_axpy_cols(double* __restrict__ Wm, const double* __restrict__ Vm, int64_t ld,
-                            int64_t n, int64_t k, const double* __restrict__ coef) {
-    const int64_t total = n * k;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = e / k, c = e - r * k;
-        Wm[r * ld + c] -= coef[c] * Vm[r * ld + c];
-    }
-}
-
 // Vn[:, c] = W[:, c] * inv[c]
 __global__ void k_scale_cols(double* __restrict__ Vn, const double* __restrict__ Wm, int64_t ld,
                              int64_t n, int64_t k, const double* __restrict__ inv, int divide) {
@@ -218,62 +207,43 @@ static double slq_logdet(cs_vce* v, int probes, int steps, uint64_t seed, cudaSt
     CS_CUDA(cudaMemcpyAsync(dcoef.get(), inv.data(), 8 * k, cudaMemcpyHostToDevice, s));
     k_scale_cols<<<grid_1d(n * k), 256, 0, s>>>(Vj(0), v->lw.get(), k, n, k, dcoef.get(), 0);
     CS_LAUNCH("scale_cols");
-    std::vector<std::vector<double>> alpha(k, std::vector<double>(m, 0.0)), beta(k, std::vector<double>(m, 0.0));
-    std::vector<int> actual(k, m);
-    std::vector<char> done(k, 0);
-    std::vector<double> coef(k), dots(k);
-    auto axpy = [&](const double* Vm, const std::vector<double>& c) {
-        CS_CUDA(cudaMemcpyAsync(dcoef.get(), c.data(), 8 * k, cudaMemcpyHostToDevice, s));
-        k_axpy_cols<<<grid_1d(n * k), 256, 0, s>>>(v->lw.get(), Vm, k, n, k, dcoef.get());
-        CS_LAUNCH("axpy_cols");
-    };
+    // the recurrences stay on the device: alpha and beta by step (m x k), the coefficients of the
+    // axpy that follows, and which columns have broken down after how many steps
+    DeviceBuffer<double> d_ab;
+    DeviceBuffer<int32_t> d_done;
+    d_ab.resize(2 * (int64_t)m * k);
+    d_done.resize(2 * k);
+    std::vector<int32_t> actual(2 * k, 0);
+    std::fill(actual.begin() + k, actual.end(), m);
+    CS_CUDA(cudaMemsetAsync(d_ab.get(), 0, 16 * (int64_t)m * k, s));
+    CS_CUDA(cudaMemcpyAsync(d_done.get(), actual.data(), 8 * k, cudaMemcpyHostToDevice, s));
+    const DeferChecks defer(v->V.op);
     for (int j = 0; j < m; ++j) {
-        v->V.apply(Vj(j), k, k, v->lw.get(), k, s);
-        if (j > 0) {
-            for (int64_t c = 0; c < k; ++c) coef[c] = done[c] ? 0.0 : beta[c][j - 1];
-            axpy(Vj(j - 1), coef);
-        }
-        column_dots(v->lw.get(), k, Vj(j), k, n, k, dots.data(), v->pw, s);
-        for (int64_t c = 0; c < k; ++c) {
-            if (!done[c]) alpha[c][j] = dots[c];
-            coef[c] = done[c] ? 0.0 : dots[c];
-        }
-        axpy(Vj(j), coef);
-        // full reorthogonalisation
-        for (int q = 0; q <= j; ++q) {
-            column_dots(v->lw.get(), k, Vj(q), k, n, k, dots.data(), v->pw, s);
-            for (int64_t c = 0; c < k; ++c) coef[c] = done[c] ? 0.0 : dots[c];
-            axpy(Vj(q), coef);
-        }
-        column_dots(v->lw.get(), k, v->lw.get(), k, n, k, dots.data(), v->pw, s);
-        for (int64_t c = 0; c < k; ++c) {
-            if (done[c]) {
-                coef[c] = 0.0;
-                continue;
-            }
-            beta[c][j] = std::sqrt(dots[c]);
-            if (beta[c][j] < 1e-12) {
-                actual[c] = j + 1;
-                done[c] = 1;
-                coef[c] = 0.0;
-            } else {
-                coef[c] = beta[c][j];
-            }
-        }
-        if (j + 1 <= m) {
-            CS_CUDA(cudaMemcpyAsync(dcoef.get(), coef.data(), 8 * k, cudaMemcpyHostToDevice, s));
-            k_scale_cols<<<grid_1d(n * k), 256, 0, s>>>(Vj(j + 1), v->lw.get(), k, n, k, dcoef.get(), 1);
-            CS_LAUNCH("scale_cols");
-        }
+        const LanczosState st{dcoef.get(), d_ab.get() + (int64_t)j * k, d_ab.get() + (int64_t)(m + j) * k,
+                              d_done.get(), d_done.get() + k};
+        double* w = v->lw.get();
+        v->V.apply(Vj(j), k, k, w, k, s);
+        // w -= beta_{j-1} v_{j-1}; alpha_j = w . v_j; w -= alpha_j v_j; full reorthogonalisation
+        // against v_0 .. v_j; beta_j = |w|: each kernel subtracts what the one before it measured
+        lanczos_step(w, j > 0 ? Vj(j - 1) : nullptr, Vj(j), n, k, st, LanczosMode::kAlpha, j, v->pw, s);
+        for (int q = 0; q <= j; ++q)
+            lanczos_step(w, q == 0 ? Vj(j) : Vj(q - 1), Vj(q), n, k, st, LanczosMode::kReorth, j, v->pw, s);
+        lanczos_step(w, Vj(j), nullptr, n, k, st, LanczosMode::kBeta, j, v->pw, s);
+        k_scale_cols<<<grid_1d(n * k), 256, 0, s>>>(Vj(j + 1), w, k, n, k, dcoef.get(), 1);
+        CS_LAUNCH("scale_cols");
     }
+    std::vector<double> ab(2 * (int64_t)m * k);
+    CS_CUDA(cudaMemcpyAsync(ab.data(), d_ab.get(), 8 * ab.size(), cudaMemcpyDeviceToHost, s));
+    CS_CUDA(cudaMemcpyAsync(actual.data(), d_done.get(), 8 * k, cudaMemcpyDeviceToHost, s));
+    kinship_check(v->V.op, s);
     CS_CUDA(cudaStreamSynchronize(s));
     double total = 0.0;
     for (int64_t c = 0; c < k; ++c) {
-        const int a = actual[c];
+        const int a = actual[k + c];
         std::vector<double> T(a * a, 0.0), ev, vec;
         for (int j = 0; j < a; ++j) {
-            T[j + j * a] = alpha[c][j];
-            if (j + 1 < a) T[(j + 1) + j * a] = T[j + (j + 1) * a] = beta[c][j];
+            T[j + j * a] = ab[(int64_t)j * k + c];
+            if (j + 1 < a) T[(j + 1) + j * a] = T[j + (j + 1) * a] = ab[(int64_t)(m + j) * k + c];
         }
         if (!la::eigh(T, a, ev, vec)) fail(CS_ERR_NUMERIC, "SLQ tridiagonal eigensolver failed");
         double ss = 0.0;
@@ -634,6 +604,19 @@ void vce_history(const cs_vce* v, double* out, int64_t* n_iter) {
     if (out) std::copy(v->hist.begin(), v->hist.end(), out);
 }
 
+// The operator's workspace for public solves: kept between them (sixteen allocations and as many
+// waits of the allocator a solve otherwise), unless it has grown past a gigabyte.
+static PcgWorkspace& solve_workspace(cs_kinship* op) {
+    if (!op->pcg) op->pcg = new PcgWorkspace();
+    return *op->pcg;
+}
+static void trim_workspace(cs_kinship* op) {
+    if (op->pcg && op->pcg->bytes() > (size_t(1) << 30)) {
+        destroy_pcg(op->pcg);
+        op->pcg = nullptr;
+    }
+}
+
 // Public multi-RHS solve of (sg2 K + se2 I) X = B on device column-major blocks.
 void pcg_solve_public(cs_kinship* op, double divisor, double sg2, double se2, const double* B,
                       int64_t ldb, int64_t k, double* X, int64_t ldx, double tol, int relative,
@@ -652,16 +635,16 @@ void pcg_solve_public(cs_kinship* op, double divisor, double sg2, double se2, co
     V.vg = sg2;
     V.ve = se2;
     V.precision = precision;
-    PcgWorkspace ws;
+    PcgWorkspace& ws = solve_workspace(op);
     PcgStats st;
-    DeviceBuffer<double> b, x;
-    b.resize(n * k);
-    x.resize(n * k);
-    colmajor_to_rowmajor(B, ldb, n, k, b.get(), k, s);
+    ws.b.resize(n * k);
+    ws.x.resize(n * k);
+    colmajor_to_rowmajor(B, ldb, n, k, ws.b.get(), k, s);
     const double diag = std::max(se2, 1e-12) + std::max(sg2, 1e-12);
-    pcg_solve_block(V, diag, b.get(), k, k, x.get(), k, tol, relative != 0, max_iter, ws, st, s);
-    rowmajor_to_colmajor(x.get(), k, n, k, X, ldx, s);
+    pcg_solve_block(V, diag, ws.b.get(), k, k, ws.x.get(), k, tol, relative != 0, max_iter, ws, st, s);
+    rowmajor_to_colmajor(ws.x.get(), k, n, k, X, ldx, s);
     CS_CUDA(cudaStreamSynchronize(s));
+    trim_workspace(op);
     if (iterations) std::copy(st.iterations.begin(), st.iterations.end(), iterations);
 }
 
@@ -687,17 +670,17 @@ void pcg_solve_records_public(cs_kinship* op, double divisor, const int32_t* rec
     V.ve = se2;
     V.with_pe = with_pe;
     V.precision = precision;
-    PcgWorkspace ws;
+    PcgWorkspace& ws = solve_workspace(op);
     PcgStats st;
-    DeviceBuffer<double> b, x;
-    b.resize(n_rec * k);
-    x.resize(n_rec * k);
-    colmajor_to_rowmajor(B, ldb, n_rec, k, b.get(), k, s);
+    ws.b.resize(n_rec * k);
+    ws.x.resize(n_rec * k);
+    colmajor_to_rowmajor(B, ldb, n_rec, k, ws.b.get(), k, s);
     double diag = std::max(se2, 1e-12) + std::max(sg2, 1e-12);
     if (with_pe) diag += std::max(spe2, 1e-12);
-    pcg_solve_block(V, diag, b.get(), k, k, x.get(), k, tol, relative != 0, max_iter, ws, st, s);
-    rowmajor_to_colmajor(x.get(), k, n_rec, k, X, ldx, s);
+    pcg_solve_block(V, diag, ws.b.get(), k, k, ws.x.get(), k, tol, relative != 0, max_iter, ws, st, s);
+    rowmajor_to_colmajor(ws.x.get(), k, n_rec, k, X, ldx, s);
     CS_CUDA(cudaStreamSynchronize(s));
+    trim_workspace(op);
     if (iterations) std::copy(st.iterations.begin(), st.iterations.end(), iterations);
 }
 

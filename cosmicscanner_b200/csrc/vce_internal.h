@@ -6,6 +6,7 @@
 #include <cublas_v2.h>
 #include <cusolverDn.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "cs_internal.h"
@@ -31,6 +32,8 @@ cusolverDnHandle_t shared_solver();
 
 // Records -> genotype rows (libCosmicCore/src/stcg_vce.cpp:17-38, 64-78).  Identity when
 // every record is its own genotype row, in order.
+struct PcgWorkspace;
+
 struct RecordMap {
     int64_t n_rec = 0, n_rows = 0;
     bool identity = true;
@@ -54,6 +57,9 @@ struct VOperator {
 
     // out (n_rec x ldo) = V * in (n_rec x ldi), k columns.
     void apply(const double* in, int64_t ldi, int64_t k, double* out, int64_t ldo, cudaStream_t s);
+    // The same for CG (out = V p), with alpha[c] = rsold[c] / (p . V p)[c].
+    void apply_alpha(const double* p, int64_t k, double* out, const double* rsold, double* alpha,
+                     PcgWorkspace& ws, cudaStream_t s);
     // g_out = Zr K Zr^T in (dV/d sigma2_g); pe_out (optional) = Zr Zr^T in.
     void derivatives(const double* in, int64_t ldi, int64_t k, double* g_out, int64_t ldg,
                      double* pe_out, int64_t ldp, cudaStream_t s);
@@ -62,6 +68,7 @@ struct VOperator {
                       double* zt_out, int64_t ldz, cudaStream_t s);
 
    private:
+    const double* kinship(const double* in, int64_t ldi, int64_t k, int64_t& ldu, cudaStream_t s);
     const double* gather(const double* in, int64_t ldi, int64_t k, cudaStream_t s);
 };
 
@@ -83,10 +90,52 @@ struct LowRankPreconditioner {
     void apply(const double* R, int64_t ldr, int64_t k, double* Z, int64_t ldz, cudaStream_t s);
 };
 
+// Host memory that kernels write directly: a reduction's few results are there when its stream has
+// been waited for, without a copy of their own.
+struct HostMapped {
+    double* ptr = nullptr;
+    size_t count = 0;
+    HostMapped() = default;
+    HostMapped(const HostMapped&) = delete;
+    HostMapped& operator=(const HostMapped&) = delete;
+    ~HostMapped() {
+        if (ptr) cudaFreeHost(ptr);
+    }
+    void resize(size_t n) {
+        if (n <= count) return;
+        if (ptr) cudaFreeHost(ptr);
+        ptr = nullptr;
+        count = 0;
+        n = std::max<size_t>(n, 64);
+        CS_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&ptr), n * sizeof(double),
+                              cudaHostAllocMapped | cudaHostAllocPortable));
+        count = n;
+    }
+};
+
 struct PcgWorkspace {
-    DeviceBuffer<double> R, P, AP, T, Zp, partial_a, partial_b;
-    DeviceBuffer<double> alpha, beta, rsold, rr, rz;
+    DeviceBuffer<double> R, P, AP, T, Zp, partial;
+    DeviceBuffer<double> alpha, beta, rsold;
     DeviceBuffer<int32_t> map, idx;
+    DeviceBuffer<unsigned> counter;  // column_reduce's, zero between kernels
+    HostMapped host;                 // reductions read by the host: two values a column
+    DeviceBuffer<double> b, x;       // a public solve's row-major blocks
+    // room for reductions over n rows of k columns
+    void reserve_reduction(int64_t n, int64_t k, cudaStream_t s);
+    size_t bytes() const {
+        return 8 * (R.count + P.count + AP.count + T.count + Zp.count + partial.count + b.count + x.count);
+    }
+};
+
+// Applies inside a solver's loop leave the check for a pass that gave up waiting to the loop's own
+// synchronisations (kinship_check), instead of waiting for the stream after each apply.
+struct DeferChecks {
+    cs_kinship* op;
+    bool before;
+    explicit DeferChecks(cs_kinship* o) : op(o), before(o->defer_checks) { op->defer_checks = true; }
+    ~DeferChecks() { op->defer_checks = before; }
+    DeferChecks(const DeferChecks&) = delete;
+    DeferChecks& operator=(const DeferChecks&) = delete;
 };
 
 struct PcgStats {
@@ -109,6 +158,20 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
 // in a fixed summation order.
 void column_dots(const double* A, int64_t lda, const double* B, int64_t ldb, int64_t n, int64_t k,
                  double* out_host, PcgWorkspace& ws, cudaStream_t s);
+
+// One step of the Lanczos recurrences' vector work on row-major n x k blocks: w -= coef o sub (sub
+// null: nothing), then the column sums of w * dot (dot null: of w * w), from which `mode` leaves
+//   kAlpha   alpha[c] = the sum, coef[c] = the sum     kReorth  coef[c] = the sum
+//   kBeta    beta[c] = coef[c] = its square root, or, where that is below 1e-12, steps[c] = step + 1
+//            and the column done
+// (a done column keeps its alpha and beta, and its coef is zero).
+struct LanczosState {
+    double *coef, *alpha, *beta;
+    int32_t *done, *steps;
+};
+enum class LanczosMode { kAlpha, kReorth, kBeta };
+void lanczos_step(double* w, const double* sub, const double* dot, int64_t n, int64_t k,
+                  const LanczosState& st, LanczosMode mode, int step, PcgWorkspace& ws, cudaStream_t s);
 
 // The mt19937_64 stream on the device (omega.cu).
 void mt64_seed_device(uint64_t seed, uint64_t* d_state, cudaStream_t s);
