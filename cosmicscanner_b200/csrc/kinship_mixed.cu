@@ -720,21 +720,36 @@ k_mixed_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
 }
 
 // ---------------------------------------------------------------- operand preparation
-// All reductions here are deterministic: FP64 sums over fixed chunks in a fixed order (whatever the
-// column count and layout, so that a column's bits do not depend on its neighbours), integer sums
-// and maxima of non-negative doubles' bits through atomics (order independent).  Every kernel
-// moves each element once, 16 bytes at a time where the layout allows: at 266 columns, N=50k,
-// M=100k the operand and reduction kernels around the two passes take 0.24 ms of a 10 ms apply.
+// All reductions here are deterministic: FP64 sums over fixed tiles in a fixed order (whatever the
+// column count and layout, so that a column's bits do not depend on its neighbours) and maxima of
+// non-negative doubles' bits through atomics (order independent).  The order matters beyond that:
+// a quantised digit flips where a sum's last bit moves it over a half, so that an iteration on the
+// mixed form (the low-rank sketch) moves by 1e-8 when the order of one of these sums changes.
+// Every kernel moves each element once, 16 bytes at a time where the layout allows: at 266 columns,
+// N=50k, M=100k the operand and reduction kernels around the two passes take 0.44 ms of a 10 ms apply.
 
 // Quantises v (centred and multiplied by 127 / max) into three int8 pieces of base 254.
-__device__ __forceinline__ void quantise3(double v, int& q1, int& q2, int& q3) {
-    const double a = rint(v);
+__device__ __forceinline__ void quantise3(double v, double& a, double& b, double& c) {
+    a = rint(v);
     const double r1 = (v - a) * kBase;
-    const double b = rint(r1);
-    const double r2 = (r1 - b) * kBase;
+    b = rint(r1);
+    c = rint((r1 - b) * kBase);
+}
+__device__ __forceinline__ void quantise3(double v, int& q1, int& q2, int& q3) {
+    double a, b, c;
+    quantise3(v, a, b, c);
     q1 = (int)(int8_t)a;
     q2 = (int)(int8_t)b;
-    q3 = (int)(int8_t)rint(r2);
+    q3 = (int)(int8_t)c;
+}
+
+// x / d for an integer |x| <= 128 and d = 254 or 254^2: one correction of x (1 / d) gives the
+// correctly rounded quotient (true for all of these x, checked one by one).
+template <int D>
+__device__ __forceinline__ double small_quotient(double x) {
+    constexpr double r = 1.0 / D;
+    const double q = x * r;
+    return fma(fma(-(double)D, q, x), r, q);
 }
 
 // Two int8 pieces of base 254 (the residual operand of the samples pass, |v| <= 63.5).
@@ -762,28 +777,54 @@ __device__ __forceinline__ bool last_block(unsigned* counter, unsigned n) {
 }
 
 // What the operand kernels of a call hand on: per column the mean and the bits of max |x - mean|
-// (rows operand), the integer sum of the quantised values in units of 1 / 254^2, the bits of
-// max |W| and max(|W|, |mu W|) (samples operand), and the counters of last_block.
+// (rows operand), the sum of the quantised values, the bits of max |W| and max(|W|, |mu W|) (samples
+// operand), and the counters of last_block.
 struct MixedColumns {
     double* mean;
     unsigned long long* max1;
-    unsigned long long* qsum;
+    double* qsum;
     unsigned long long* max_w;
     unsigned long long* max_wmu;
     unsigned* counter;
 };
 
-// Per-column sums, minima and maxima of X over chunks of 512 rows (8 interleaved lanes each, added
-// in lane order), then, in the last block of a column tile, mean[c] = (sum over chunks) / n and
-// max1[c] = the bits of max |x - mean| = max(max x - mean, mean - min x) (rounding is monotonic, so
-// this equals the maximum of the rounded differences); the column's other words are cleared.
-// A block covers kc columns (a power of two up to 32) x 32 / kc chunks.
-constexpr int kStatRows = 512;
+// Sums over tiles in the order every column sum of these kernels has: part[t * ld + c] for tiles
+// t = l, l + 32, ... by lane l, then the 32 lanes in a shuffle tree.  A block sums `cols` columns (a
+// power of two up to 32) from c0 on; a warp calls out(j, sum) for column c0 + j; sh: 32 x 33 doubles.
+// Columns are the fastest thread index, so that the partials are read in the order of memory.
+template <int THREADS, class Out>
+__device__ __forceinline__ void sum_tiles(const double* __restrict__ part, int64_t nt, int64_t ld, int64_t c0,
+                                          int cols, int64_t k, double* sh, Out&& out) {
+    const int cc = threadIdx.x % cols, slot = threadIdx.x / cols, slots = min(32, THREADS / cols);
+    if (slot < slots)
+        for (int l = slot; l < 32; l += slots) {
+            double sm = 0.0;
+            if (c0 + cc < k) {
+#pragma unroll 8
+                for (int64_t t = l; t < nt; t += 32) sm += __ldcg(part + t * ld + c0 + cc);
+            }
+            sh[l * 33 + cc] = sm;
+        }
+    __syncthreads();
+    const int wl = threadIdx.x & 31;
+    for (int j = threadIdx.x >> 5; j < cols; j += THREADS / 32) {
+        double sm = sh[wl * 33 + j];
+        for (int off = 16; off; off >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, off);
+        if (c0 + j < k) out(j, sm);
+    }
+}
+
+// Per-column sums over tiles of 64 rows (8 interleaved lanes each, added in lane order) and minima
+// and maxima over chunks of 512, then, in the last block of a column tile, mean[c] = (sum over
+// tiles) / n and max1[c] = the bits of max |x - mean| = max(max x - mean, mean - min x) (rounding is
+// monotonic, so this equals the maximum of the rounded differences); the column's maxima of W are
+// cleared.  A block covers kc columns (a power of two up to 32) x 32 / kc chunks.
+constexpr int kStatTile = 64, kStatRows = 8 * kStatTile;
 template <class T>
 __global__ void __launch_bounds__(256)
 k_col_stats(const Strided<const T> X, int64_t n, int64_t k, int kc, int64_t nb,
             double* __restrict__ part, const MixedColumns C) {
-    __shared__ double red[3][256];
+    __shared__ double red[10][32 * 9];  // eight tiles' sums, minima, maxima; 8 lanes and a pad per (column, chunk)
     // threads in the order of memory: columns fastest in row-major input, lanes in column-major
     const int per = 256 / kc;  // 8 lanes x chunks
     const int tc = X.rs == 1 ? threadIdx.x / per : threadIdx.x % kc;
@@ -791,69 +832,82 @@ k_col_stats(const Strided<const T> X, int64_t n, int64_t k, int kc, int64_t nb,
     const int lane = tl & 7, ch = tl >> 3;
     const int64_t c = (int64_t)blockIdx.y * kc + tc;
     const int64_t b = (int64_t)blockIdx.x * (per >> 3) + ch;
-    double sm = 0.0, mn = INFINITY, mx = -INFINITY;
-    if (c < k && b < nb) {
-        const int64_t r1 = min(n, (b + 1) * kStatRows);
-#pragma unroll 8
-        for (int64_t r = b * kStatRows + lane; r < r1; r += 8) {
-            const double v = (double)X.p[r * X.rs + c * X.cs];
-            sm += v;
-            mn = fmin(mn, v);
-            mx = fmax(mx, v);
+    const int64_t nt = (n + kStatTile - 1) / kStatTile;
+    const int slot = (tc * (per >> 3) + ch) * 9 + lane;
+    double mn = INFINITY, mx = -INFINITY;
+#pragma unroll 4
+    for (int j = 0; j < 8; ++j) {
+        double sm = 0.0;
+        if (c < k && b < nb) {
+            const int64_t r0 = b * kStatRows + j * kStatTile + lane;
+#pragma unroll
+            for (int q = 0; q < kStatTile; q += 8)
+                if (r0 + q < n) {
+                    const double v = (double)X.p[(r0 + q) * X.rs + c * X.cs];
+                    sm += v;
+                    mn = fmin(mn, v);
+                    mx = fmax(mx, v);
+                }
         }
+        red[j][slot] = sm;
     }
-    const int slot = (tc * (per >> 3) + ch) * 8 + lane;
-    red[0][slot] = sm;
-    red[1][slot] = mn;
-    red[2][slot] = mx;
+    red[8][slot] = mn;
+    red[9][slot] = mx;
     __syncthreads();
-    if (threadIdx.x < 32) {  // one thread per (column, chunk)
-        const int oc = threadIdx.x / (per >> 3), och = threadIdx.x % (per >> 3);
+    {   // one thread per (column, chunk) and tile
+        const int pair = threadIdx.x & 31, j = threadIdx.x >> 5;
+        const int oc = pair / (per >> 3), och = pair % (per >> 3);
         const int64_t cc = (int64_t)blockIdx.y * kc + oc, bb = (int64_t)blockIdx.x * (per >> 3) + och;
         if (cc < k && bb < nb) {
-            const int s0 = threadIdx.x * 8;
-            sm = red[0][s0];
-            mn = red[1][s0];
-            mx = red[2][s0];
-            for (int j = 1; j < 8; ++j) {
-                sm += red[0][s0 + j];
-                mn = fmin(mn, red[1][s0 + j]);
-                mx = fmax(mx, red[2][s0 + j]);
+            double sm = red[j][9 * pair];
+            for (int q = 1; q < 8; ++q) sm += red[j][9 * pair + q];
+            if (8 * bb + j < nt) part[(8 * bb + j) * k + cc] = sm;
+            if (j == 0) {
+                mn = INFINITY;
+                mx = -INFINITY;
+                for (int q = 0; q < 8; ++q) {
+                    mn = fmin(mn, red[8][9 * pair + q]);
+                    mx = fmax(mx, red[9][9 * pair + q]);
+                }
+                part[(nt + bb) * k + cc] = mn;
+                part[(nt + nb + bb) * k + cc] = mx;
             }
-            part[bb * k + cc] = sm;
-            part[(nb + bb) * k + cc] = mn;
-            part[(2 * nb + bb) * k + cc] = mx;
         }
     }
     if (!last_block(C.counter + blockIdx.y, gridDim.x)) return;
-    // one warp per column: lane l takes chunks l, l + 32, ..., then a fixed shuffle tree
-    const int wl = threadIdx.x & 31;
-    for (int j = threadIdx.x >> 5; j < kc; j += 8) {
-        const int64_t cc = (int64_t)blockIdx.y * kc + j;
-        if (cc >= k) break;
-        sm = 0.0;
+    double* const sh = &red[0][0];
+    double *const smn = sh + 32 * 33, *const smx = smn + 256;
+    const int64_t c0 = (int64_t)blockIdx.y * kc;
+    const int cc = threadIdx.x % kc, sl = threadIdx.x / kc, slots = min(32, 256 / kc);
+    if (sl < slots) {
         mn = INFINITY;
         mx = -INFINITY;
-        for (int64_t q = wl; q < nb; q += 32) {
-            sm += __ldcg(part + q * k + cc);
-            mn = fmin(mn, __ldcg(part + (nb + q) * k + cc));
-            mx = fmax(mx, __ldcg(part + (2 * nb + q) * k + cc));
+        if (c0 + cc < k) {
+#pragma unroll 4
+            for (int64_t q = sl; q < nb; q += slots) {
+                mn = fmin(mn, __ldcg(part + (nt + q) * k + c0 + cc));
+                mx = fmax(mx, __ldcg(part + (nt + nb + q) * k + c0 + cc));
+            }
         }
+        smn[sl * kc + cc] = mn;
+        smx[sl * kc + cc] = mx;
+    }
+    sum_tiles<256>(part, nt, k, c0, kc, k, sh, [&](int j, double sm) {
+        const int wl = threadIdx.x & 31;
+        double lo = wl < slots ? smn[wl * kc + j] : INFINITY, hi = wl < slots ? smx[wl * kc + j] : -INFINITY;
         for (int off = 16; off; off >>= 1) {
-            sm += __shfl_xor_sync(0xffffffffu, sm, off);
-            mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, off));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+            lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+            hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, off));
         }
         if (wl == 0) {
             const double m = sm / (double)n;
-            C.mean[cc] = m;
-            const double a = fmax(fmax(mx - m, m - mn), 0.0);
-            C.max1[cc] = (unsigned long long)__double_as_longlong(a);
-            C.qsum[cc] = 0;
-            C.max_w[cc] = 0;
-            C.max_wmu[cc] = 0;
+            C.mean[c0 + j] = m;
+            const double a = fmax(fmax(hi - m, m - lo), 0.0);
+            C.max1[c0 + j] = (unsigned long long)__double_as_longlong(a);
+            C.max_w[c0 + j] = 0;
+            C.max_wmu[c0 + j] = 0;
         }
-    }
+    });
 }
 
 // 16 int8 values (by K element) -> the 16 bytes of their K positions: interleaved as the decoded
@@ -872,42 +926,72 @@ __device__ __forceinline__ uint4 pack16(const int (&q)[16]) {
 }
 
 // Rows-pass operand: B1[q*kp + c][pos(i)] (int8 pieces of (x_ic - mean_c) 127 / max_c, i < n_pad;
-// pos interleaves each group of 16 samples as the decoded tiles do) and the integer sums of the
-// quantised values.  A block takes COLS columns x ROWS rows through shared memory; a thread takes
-// 16 rows of a column.
+// pos interleaves each group of 16 samples as the decoded tiles do) and the sums Q_c of the
+// represented values: in tiles of 64 rows (rows i and i + 32, then the 32 pairs in a tree), the
+// tiles by the last block of a column group.  A block takes COLS columns x ROWS rows through shared
+// memory; a thread takes 16 rows of a column, four threads a tile.
 template <class T, int COLS, int ROWS>
 __global__ void __launch_bounds__(ROWS / 16 * COLS)
 k_split_rows_operand(const Strided<const T> X, int64_t n, int64_t k, int64_t kp, int64_t n_pad,
-                     const MixedColumns C, int8_t* __restrict__ B) {
+                     const MixedColumns C, int8_t* __restrict__ B, double* __restrict__ part) {
     constexpr int TH = ROWS / 16 * COLS;
-    __shared__ double tile[COLS][ROWS + ROWS / 16 + 1];  // one pad every 16 rows and one per column
+    constexpr int kPitch = ROWS + ROWS / 16 + 1;  // one pad every 16 rows and one per column
+    static_assert(COLS * kPitch >= 32 * 33, "sum_tiles's scratch");
+    __shared__ double tile[COLS * kPitch];
     const int64_t r0 = (int64_t)blockIdx.x * ROWS, c0 = (int64_t)blockIdx.y * COLS;
     for (int e = threadIdx.x; e < ROWS * COLS; e += TH) {
         const int rr = X.rs == 1 ? e % ROWS : e / COLS, cc = X.rs == 1 ? e / ROWS : e % COLS;
         const int64_t r = r0 + rr, c = c0 + cc;
-        tile[cc][rr + (rr >> 4)] = (r < n && c < k) ? (double)X.p[r * X.rs + c * X.cs] : 0.0;
+        tile[cc * kPitch + rr + (rr >> 4)] = (r < n && c < k) ? (double)X.p[r * X.rs + c * X.cs] : 0.0;
     }
     __syncthreads();
     const int grp = threadIdx.x % (ROWS / 16), cc = threadIdx.x / (ROWS / 16);
     const int64_t c = c0 + cc, i0 = r0 + 16 * grp;
-    const bool live = c < kp && i0 < n_pad;
-    long long sum = 0;
-    if (live) {
+    double val[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) val[j] = 0.0;
+    if (c < kp && i0 < n_pad) {
         const double f = c < k ? quant_factor(C.max1[c]) : 0.0;
         const double mc = c < k ? C.mean[c] : 0.0;
         int q1[16], q2[16], q3[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             q1[j] = q2[j] = q3[j] = 0;
-            if (c < k && i0 + j < n) quantise3((tile[cc][17 * grp + j] - mc) * f, q1[j], q2[j], q3[j]);
-            sum += (long long)q1[j] * 64516 + q2[j] * 254 + q3[j];
+            if (c < k && i0 + j < n) {
+                double a, b, d;
+                quantise3((tile[cc * kPitch + 17 * grp + j] - mc) * f, a, b, d);
+                q1[j] = (int)(int8_t)a;
+                q2[j] = (int)(int8_t)b;
+                q3[j] = (int)(int8_t)d;
+                val[j] = a + small_quotient<254>(b) + small_quotient<64516>(d);
+            }
         }
         *reinterpret_cast<uint4*>(B + c * n_pad + i0) = pack16<true>(q1);
         *reinterpret_cast<uint4*>(B + (kp + c) * n_pad + i0) = pack16<true>(q2);
         *reinterpret_cast<uint4*>(B + (2 * kp + c) * n_pad + i0) = pack16<true>(q3);
     }
-    for (int off = 8; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    if ((threadIdx.x & 15) == 0 && live && c < k) atomicAdd(C.qsum + c, (unsigned long long)sum);
+    // rows 16 g + j of a tile, g = the thread's place among its four: + 32, + 16, + 8, + 4, + 2, + 1,
+    // each thread keeping the half that it needs
+    const bool hi = grp & 2, lo = grp & 1;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {  // j = 2 m + hi
+        const double keep = hi ? val[2 * m + 1] : val[2 * m], send = hi ? val[2 * m] : val[2 * m + 1];
+        val[m] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {  // j = 4 m + 2 lo + hi
+        const double keep = lo ? val[2 * m + 1] : val[2 * m], send = lo ? val[2 * m] : val[2 * m + 1];
+        val[m] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+    }
+    double sum = (val[0] + val[2]) + (val[1] + val[3]);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    const int64_t nt = (n + 63) / 64;
+    if ((grp & 3) == 0 && c < k && i0 < n) part[(i0 >> 6) * k + c] = sum;
+    if (c0 >= k || !last_block(C.counter + blockIdx.y, gridDim.x)) return;
+    sum_tiles<TH>(part, nt, k, c0, COLS, k, tile, [&](int j, double sm) {
+        if ((threadIdx.x & 31) == 0) C.qsum[c0 + j] = sm;
+    });
 }
 
 // (sum_z part[z][c][t] - mu_t Q_c) / f_c + mean_c exc_t, the rows pass's centred product.
@@ -917,10 +1001,10 @@ struct RowsColumn {
         const double f = quant_factor(C.max1[c]);
         inv_f = f > 0.0 ? 1.0 / f : 0.0;
         mean = C.mean[c];
-        qsum = (double)(long long)C.qsum[c] / (kBase * kBase);
+        qsum = C.qsum[c];
     }
     __device__ __forceinline__ double value(double acc, double mu, double exc) const {
-        return (acc - mu * qsum) * inv_f + mean * exc;
+        return fma(mean, exc, __dmul_rn(fma(-mu, qsum, acc), inv_f));
     }
 };
 
@@ -1018,23 +1102,24 @@ k_split_samples_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int
                         const double* __restrict__ resid, const MixedColumns C,
                         int8_t* __restrict__ B, double* __restrict__ inv_f,
                         double* __restrict__ cpart, double* __restrict__ c0) {
-    __shared__ double red[4];
+    __shared__ double red[8];
     // W and the second operand of 2048 SNPs, one pad every 16, read in the order of memory
     __shared__ double sw[128 * 17], sb[128 * 17];
     const int64_t c = blockIdx.y;
     const double f = c < k ? quant_factor(SIX ? C.max_wmu[c] : C.max_w[c]) : 0.0;
     if (blockIdx.x == 0 && threadIdx.x == 0) inv_f[c] = f > 0.0 ? 1.0 / (SIX ? f : f * kImputeQ) : 0.0;
-    double cs = 0.0;
+    double cs[2] = {0.0, 0.0};  // a chunk is summed by 256 lanes, two to a thread
     const int64_t base = (int64_t)blockIdx.x * 2048;
-#pragma unroll 8
-    for (int e = threadIdx.x; e < 2048; e += 128) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+        const int e = threadIdx.x + 128 * q;
         const int64_t t = base + e;
         double w = 0.0, b = 0.0;
         if (c < k && t < R) {
             const double m = mu[t];
             w = Wt[c * R + t];
-            b = SIX ? m * w : (INTERLEAVE ? -kImputeQ : kImputeQ) * resid[t] * w;
-            cs += m * w;
+            b = SIX ? __dmul_rn(m, w) : (INTERLEAVE ? -kImputeQ : kImputeQ) * resid[t] * w;
+            cs[q & 1] = SIX ? __dadd_rn(cs[q & 1], b) : fma(m, w, cs[q & 1]);
         }
         sw[e + (e >> 4)] = w;
         sb[e + (e >> 4)] = b;
@@ -1061,10 +1146,20 @@ k_split_samples_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int
         if (SIX) *reinterpret_cast<uint4*>(dst + 5 * step) = pack16<INTERLEAVE>(q3);
     }
     if (c >= k) return;
-    for (int off = 16; off; off >>= 1) cs += __shfl_xor_sync(0xffffffffu, cs, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = cs;
+    for (int off = 16; off; off >>= 1) {
+        cs[0] += __shfl_xor_sync(0xffffffffu, cs[0], off);
+        cs[1] += __shfl_xor_sync(0xffffffffu, cs[1], off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        red[threadIdx.x >> 5] = cs[0];
+        red[4 + (threadIdx.x >> 5)] = cs[1];
+    }
     __syncthreads();
-    if (threadIdx.x == 0) cpart[(int64_t)blockIdx.x * k + c] = (red[0] + red[1]) + (red[2] + red[3]);
+    if (threadIdx.x == 0) {
+        double sm = red[0];
+        for (int j = 1; j < 8; ++j) sm += red[j];
+        cpart[(int64_t)blockIdx.x * k + c] = sm;
+    }
     if (!last_block(C.counter + c, gridDim.x)) return;
     if (threadIdx.x < 32) {
         double sm = 0.0;
@@ -1315,8 +1410,8 @@ int choose_splits(int64_t units_per_split, int kb_total, int64_t target) {
 
 struct MixedWorkspace {
     DeviceBuffer<int8_t> b1, b2;
-    DeviceBuffer<double> part, colpart, mean1, c0, W, inv_f;
-    DeviceBuffer<unsigned long long> max1, qsum, max_w, max_wmu;
+    DeviceBuffer<double> part, colpart, mean1, qsum, c0, W, inv_f;
+    DeviceBuffer<unsigned long long> max1, max_w, max_wmu;
     DeviceBuffer<unsigned> counter;
     // the column words of a call on k columns (new counters start at zero)
     MixedColumns columns(int64_t k, cudaStream_t s) {
@@ -1745,7 +1840,7 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, Stri
     const int64_t nst = (n + kStatRows - 1) / kStatRows;  // chunks of the column stats
     ws.b1.resize(3 * kp * n_pad);
     ws.part.resize((int64_t)splits * kp * r_pad);
-    ws.colpart.resize(3 * nst * k);
+    ws.colpart.resize(((n + kStatTile - 1) / kStatTile + 2 * nst) * k);
     const MixedColumns C = ws.columns(k, s);
     if (!ws.status.get()) {
         ws.status.resize(1);
@@ -1770,10 +1865,10 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, Stri
             X, n, k, kc, nst, ws.colpart.get(), C);
         if (kp <= 16)
             k_split_rows_operand<T, 4, 512><<<dim3((unsigned)((n_pad + 511) / 512), (unsigned)((kp + 3) / 4)),
-                                              128, 0, s>>>(X, n, k, kp, n_pad, C, ws.b1.get());
+                                              128, 0, s>>>(X, n, k, kp, n_pad, C, ws.b1.get(), ws.colpart.get());
         else
             k_split_rows_operand<T, 16, 256><<<dim3((unsigned)(n_pad / 256), (unsigned)((kp + 15) / 16)), 256,
-                                               0, s>>>(X, n, k, kp, n_pad, C, ws.b1.get());
+                                               0, s>>>(X, n, k, kp, n_pad, C, ws.b1.get(), ws.colpart.get());
         CS_LAUNCH("mixed rows operand");
     }
     PassArgs P{};
