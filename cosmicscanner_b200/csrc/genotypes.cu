@@ -90,10 +90,54 @@ __global__ void k_sanitize_tail(uint8_t* rows, int64_t n_rows, int64_t stride, i
     rows[t * stride + last_byte] = b;
 }
 
-__global__ void k_repack(const uint8_t* __restrict__ src, int64_t src_stride,
-                         const int32_t* __restrict__ rows, int64_t n_rows,
-                         const int32_t* __restrict__ keep, int64_t n_keep,
-                         uint8_t* __restrict__ dst, int64_t dst_stride) {
+// dst row t = src row rows[t] (or t) restricted to the samples keep (or the first n_keep), packed and
+// padded with the missing code.  A block takes kRows rows: they go through shared memory whole
+// (a keep list may name samples anywhere in the row, in any order), and a thread makes 16 output
+// codes of each from one reading of its 16 indices.
+template <int kRows>
+__global__ void __launch_bounds__(256)
+k_repack(const uint8_t* __restrict__ src, int64_t src_stride, const int32_t* __restrict__ rows,
+         int64_t n_rows, const int32_t* __restrict__ keep, int64_t n_keep,
+         uint8_t* __restrict__ dst, int64_t dst_stride) {
+    extern __shared__ __align__(16) uint8_t packed[];  // [kRows][src_stride]
+    const int64_t t0 = (int64_t)blockIdx.x * kRows;
+    const int here = (int)min((int64_t)kRows, n_rows - t0);
+    for (int r = 0; r < here; ++r) {
+        const uint4* s = reinterpret_cast<const uint4*>(src + (int64_t)(rows ? rows[t0 + r] : t0 + r) * src_stride);
+        for (int64_t q = threadIdx.x; q < src_stride / 16; q += 256)
+            reinterpret_cast<uint4*>(packed + r * src_stride)[q] = __ldg(s + q);
+    }
+    __syncthreads();
+    for (int64_t w = threadIdx.x; w < dst_stride / 4; w += 256) {
+        uint32_t out[kRows];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) out[r] = 0x55555555u;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const int64_t i = 16 * w + j;
+            if (i < n_keep) {
+                const int32_t k = keep ? __ldg(keep + i) : (int32_t)i;
+                const int sh = (k & 3) * 2;
+#pragma unroll
+                for (int r = 0; r < kRows; ++r) {
+                    if (r < here) {
+                        const uint32_t code = ((uint32_t)packed[r * src_stride + (k >> 2)] >> sh) & 3u;
+                        out[r] = (out[r] & ~(3u << (2 * j))) | (code << (2 * j));
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r)
+            if (r < here) reinterpret_cast<uint32_t*>(dst + (t0 + r) * dst_stride)[w] = out[r];
+    }
+}
+
+// The same a byte at a time from global memory, for rows that do not fit shared memory.
+__global__ void k_repack_long(const uint8_t* __restrict__ src, int64_t src_stride,
+                              const int32_t* __restrict__ rows, int64_t n_rows,
+                              const int32_t* __restrict__ keep, int64_t n_keep,
+                              uint8_t* __restrict__ dst, int64_t dst_stride) {
     const int64_t total = n_rows * dst_stride;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
@@ -167,8 +211,25 @@ void repack(const uint8_t* src, int64_t src_stride, const int32_t* d_rows, int64
             cudaStream_t s) {
     if (n_rows == 0) return;
     prof::Scope ps("repack", s, 0.0, (double)n_rows * dst_stride);
-    k_repack<<<grid_for(n_rows * dst_stride, 256), 256, 0, s>>>(src, src_stride, d_rows, n_rows,
-                                                               d_keep, n_keep, dst, dst_stride);
+    // as many rows a block as keep two blocks on an SM, four where one block must do (every row then
+    // still shares the indices with three others)
+    constexpr int64_t kHalf = 110 * 1024, kWhole = 220 * 1024;
+    static PerDeviceOnce configured;
+    once_per_device(configured, [] {
+        cudaError_t e = cudaFuncSetAttribute(k_repack<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHalf);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_repack<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWhole);
+        return e;
+    }, "configure repack kernels");
+    if (8 * src_stride <= kHalf)
+        k_repack<8><<<(unsigned)((n_rows + 7) / 8), 256, 8 * src_stride, s>>>(
+            src, src_stride, d_rows, n_rows, d_keep, n_keep, dst, dst_stride);
+    else if (4 * src_stride <= kWhole)
+        k_repack<4><<<(unsigned)((n_rows + 3) / 4), 256, 4 * src_stride, s>>>(
+            src, src_stride, d_rows, n_rows, d_keep, n_keep, dst, dst_stride);
+    else
+        k_repack_long<<<grid_for(n_rows * dst_stride, 256), 256, 0, s>>>(
+            src, src_stride, d_rows, n_rows, d_keep, n_keep, dst, dst_stride);
     CS_LAUNCH("repack");
 }
 
