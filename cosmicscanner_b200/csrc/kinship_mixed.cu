@@ -726,21 +726,34 @@ k_mixed_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
 // a quantised digit flips where a sum's last bit moves it over a half, so that an iteration on the
 // mixed form (the low-rank sketch) moves by 1e-8 when the order of one of these sums changes.
 // Every kernel moves each element once, 16 bytes at a time where the layout allows: at 266 columns,
-// N=50k, M=100k the operand and reduction kernels around the two passes take 0.44 ms of a 10 ms apply.
+// N=50k, M=100k the operand and reduction kernels around the two passes take 0.39 ms of a 9.9 ms apply.
 
-// Quantises v (centred and multiplied by 127 / max) into three int8 pieces of base 254.
-__device__ __forceinline__ void quantise3(double v, double& a, double& b, double& c) {
-    a = rint(v);
-    const double r1 = (v - a) * kBase;
-    b = rint(r1);
-    c = rint((r1 - b) * kBase);
+// Round to nearest even of |v| < 2^31 by adding 1.5 * 2^52: the sum's low word is the integer, two
+// additions give it back as a double.  rint and a conversion are both quarter-rate instructions.
+__device__ __forceinline__ double round_to(double v, int& q) {
+    constexpr double kMagic = 6755399441055744.0;
+    const double t = __dadd_rn(v, kMagic);
+    q = __double2loint(t);
+    return __dadd_rn(t, -kMagic);
+}
+// Quantises v (centred and multiplied by 127 / max) into three pieces of base 254, of which the low
+// bytes are the int8 digits; the products round before the differences (no contraction), whichever
+// kernel this is inlined in.
+__device__ __forceinline__ void quantise3(double v, double& a, double& b, double& c, int& q1, int& q2, int& q3) {
+    a = round_to(v, q1);
+    const double r1 = __dmul_rn(__dsub_rn(v, a), kBase);
+    b = round_to(r1, q2);
+    c = round_to(__dmul_rn(__dsub_rn(r1, b), kBase), q3);
 }
 __device__ __forceinline__ void quantise3(double v, int& q1, int& q2, int& q3) {
     double a, b, c;
-    quantise3(v, a, b, c);
-    q1 = (int)(int8_t)a;
-    q2 = (int)(int8_t)b;
-    q3 = (int)(int8_t)c;
+    quantise3(v, a, b, c, q1, q2, q3);
+}
+
+// Two pieces of base 254 (the residual operand of the samples pass, |v| <= 63.5).
+__device__ __forceinline__ void quantise2(double v, int& q1, int& q2) {
+    const double a = round_to(v, q1);
+    round_to(__dmul_rn(__dsub_rn(v, a), kBase), q2);
 }
 
 // x / d for an integer |x| <= 128 and d = 254 or 254^2: one correction of x (1 / d) gives the
@@ -750,13 +763,6 @@ __device__ __forceinline__ double small_quotient(double x) {
     constexpr double r = 1.0 / D;
     const double q = x * r;
     return fma(fma(-(double)D, q, x), r, q);
-}
-
-// Two int8 pieces of base 254 (the residual operand of the samples pass, |v| <= 63.5).
-__device__ __forceinline__ void quantise2(double v, int& q1, int& q2) {
-    const double a = rint(v);
-    q1 = (int)(int8_t)a;
-    q2 = (int)(int8_t)rint((v - a) * kBase);
 }
 
 __device__ __forceinline__ double quant_factor(unsigned long long bits) {
@@ -925,13 +931,20 @@ __device__ __forceinline__ uint4 pack16(const int (&q)[16]) {
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// Byte p of w = the low byte of q (p known at compile time).
+__device__ __forceinline__ void put_byte(uint32_t (&w)[4], int p, int q) {
+    w[p >> 2] = __byte_perm(w[p >> 2], (uint32_t)q, 0x3210 ^ (((p & 3) ^ 4) << (4 * (p & 3))));
+}
+
 // Rows-pass operand: B1[q*kp + c][pos(i)] (int8 pieces of (x_ic - mean_c) 127 / max_c, i < n_pad;
 // pos interleaves each group of 16 samples as the decoded tiles do) and the sums Q_c of the
 // represented values: in tiles of 64 rows (rows i and i + 32, then the 32 pairs in a tree), the
 // tiles by the last block of a column group.  A block takes COLS columns x ROWS rows through shared
-// memory; a thread takes 16 rows of a column, four threads a tile.
+// memory; a thread takes 16 rows of a column, four threads a tile.  Loads and arithmetic overlap only
+// between blocks, so the registers are held to 64 for 1024 threads an SM: 79 us at 266 columns, N=50k,
+// against 160 with 128 registers.
 template <class T, int COLS, int ROWS>
-__global__ void __launch_bounds__(ROWS / 16 * COLS)
+__global__ void __launch_bounds__(ROWS / 16 * COLS, 1024 / (ROWS / 16 * COLS))
 k_split_rows_operand(const Strided<const T> X, int64_t n, int64_t k, int64_t kp, int64_t n_pad,
                      const MixedColumns C, int8_t* __restrict__ B, double* __restrict__ part) {
     constexpr int TH = ROWS / 16 * COLS;
@@ -947,41 +960,37 @@ k_split_rows_operand(const Strided<const T> X, int64_t n, int64_t k, int64_t kp,
     __syncthreads();
     const int grp = threadIdx.x % (ROWS / 16), cc = threadIdx.x / (ROWS / 16);
     const int64_t c = c0 + cc, i0 = r0 + 16 * grp;
-    double val[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) val[j] = 0.0;
-    if (c < kp && i0 < n_pad) {
-        const double f = c < k ? quant_factor(C.max1[c]) : 0.0;
-        const double mc = c < k ? C.mean[c] : 0.0;
-        int q1[16], q2[16], q3[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            q1[j] = q2[j] = q3[j] = 0;
-            if (c < k && i0 + j < n) {
-                double a, b, d;
-                quantise3((tile[cc * kPitch + 17 * grp + j] - mc) * f, a, b, d);
-                q1[j] = (int)(int8_t)a;
-                q2[j] = (int)(int8_t)b;
-                q3[j] = (int)(int8_t)d;
-                val[j] = a + small_quotient<254>(b) + small_quotient<64516>(d);
-            }
-        }
-        *reinterpret_cast<uint4*>(B + c * n_pad + i0) = pack16<true>(q1);
-        *reinterpret_cast<uint4*>(B + (kp + c) * n_pad + i0) = pack16<true>(q2);
-        *reinterpret_cast<uint4*>(B + (2 * kp + c) * n_pad + i0) = pack16<true>(q3);
-    }
-    // rows 16 g + j of a tile, g = the thread's place among its four: + 32, + 16, + 8, + 4, + 2, + 1,
-    // each thread keeping the half that it needs
+    // rows 16 g + j of a tile, g = the thread's place among its four: + 32 and + 16 as the values come,
+    // each thread keeping a quarter (j = 4 m + 2 lo + hi), then + 8, + 4, + 2, + 1
     const bool hi = grp & 2, lo = grp & 1;
+    const double f = c < k ? quant_factor(C.max1[c]) : 0.0;
+    const double mc = c < k ? C.mean[c] : 0.0;
+    const double* const mine = tile + cc * kPitch + 17 * grp;
+    const int rows = c < k ? (int)min((int64_t)16, n - i0) : 0;  // may be negative
+    uint32_t w1[4] = {}, w2[4] = {}, w3[4] = {};  // the 16 bytes of each piece at their K positions
+    double val[4];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {  // j = 2 m + hi
-        const double keep = hi ? val[2 * m + 1] : val[2 * m], send = hi ? val[2 * m] : val[2 * m + 1];
-        val[m] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+    for (int m = 0; m < 4; ++m) {
+        double v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int j = 4 * m + q;
+            double a, b, d;
+            int q1, q2, q3;
+            quantise3(j < rows ? __dmul_rn(mine[j] - mc, f) : 0.0, a, b, d, q1, q2, q3);
+            put_byte(w1, position_of(j), q1);
+            put_byte(w2, position_of(j), q2);
+            put_byte(w3, position_of(j), q3);
+            v[q] = a + small_quotient<254>(b) + small_quotient<64516>(d);
+        }
+        const double x0 = (hi ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[1], 2);
+        const double x1 = (hi ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, hi ? v[2] : v[3], 2);
+        val[m] = (lo ? x1 : x0) + __shfl_xor_sync(0xffffffffu, lo ? x0 : x1, 1);
     }
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {  // j = 4 m + 2 lo + hi
-        const double keep = lo ? val[2 * m + 1] : val[2 * m], send = lo ? val[2 * m] : val[2 * m + 1];
-        val[m] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+    if (c < kp && i0 < n_pad) {
+        *reinterpret_cast<uint4*>(B + c * n_pad + i0) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+        *reinterpret_cast<uint4*>(B + (kp + c) * n_pad + i0) = make_uint4(w2[0], w2[1], w2[2], w2[3]);
+        *reinterpret_cast<uint4*>(B + (2 * kp + c) * n_pad + i0) = make_uint4(w3[0], w3[1], w3[2], w3[3]);
     }
     double sum = (val[0] + val[2]) + (val[1] + val[3]);
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
@@ -1131,13 +1140,13 @@ k_split_samples_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int
         const int64_t step = kp * r_pad;
         int q1[16], q2[16], q3[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) quantise3(sw[17 * threadIdx.x + j] * f, q1[j], q2[j], q3[j]);
+        for (int j = 0; j < 16; ++j) quantise3(__dmul_rn(sw[17 * threadIdx.x + j], f), q1[j], q2[j], q3[j]);
         *reinterpret_cast<uint4*>(dst) = pack16<INTERLEAVE>(q1);
         *reinterpret_cast<uint4*>(dst + step) = pack16<INTERLEAVE>(q2);
         *reinterpret_cast<uint4*>(dst + 2 * step) = pack16<INTERLEAVE>(q3);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            const double v = sb[17 * threadIdx.x + j] * f;
+            const double v = __dmul_rn(sb[17 * threadIdx.x + j], f);
             if (SIX) quantise3(v, q1[j], q2[j], q3[j]);
             else quantise2(v, q1[j], q2[j]);
         }
