@@ -188,7 +188,11 @@ int cs_genotypes_stats(const cs_genotypes* g, double* mean, double* inv_std, int
     });
 }
 
-void cs_genotypes_destroy(cs_genotypes* g) { delete g; }
+void cs_genotypes_destroy(cs_genotypes* g) {
+    if (!g) return;
+    cs::FreeScope fs;
+    delete g;
+}
 
 int cs_kinship_create(const cs_genotypes* g, const int32_t* keep, int64_t n_keep,
                       const int32_t* variants, int64_t n_variants, cs_kinship** out) {
@@ -316,7 +320,11 @@ int cs_kinship_diagonal(cs_kinship* op, double* diag) {
     });
 }
 
-void cs_kinship_destroy(cs_kinship* op) { delete op; }
+void cs_kinship_destroy(cs_kinship* op) {
+    if (!op) return;
+    cs::FreeScope fs;
+    delete op;
+}
 
 int cs_lmm_create(cs_lmm** out) {
     return guarded([&] {

@@ -82,6 +82,23 @@ void device_free(void* p) noexcept;
 // waiting for the whole device, so a buffer is only reused after the work queued before its
 // release has finished.  nullptr restores the device-wide synchronisation.
 void set_thread_free_stream(cudaStream_t s);
+// While one of these lives, the thread's frees do not each wait for the device: the first one's
+// construction has.  For the destruction of a handle, whose buffers nothing queued later may use
+// (a handle's thirty buffers each waited 10 us to 50 us).
+struct FreeScope {
+    FreeScope();
+    ~FreeScope();
+    FreeScope(const FreeScope&) = delete;
+    FreeScope& operator=(const FreeScope&) = delete;
+};
+// Waits for the work that a buffer about to be given back may still serve, as device_free does.
+void wait_before_free() noexcept;
+// Page-locked host memory, mapped and portable.  cudaHostAlloc and cudaFreeHost take milliseconds
+// each in a process that holds a cohort, so up to 32 MiB of freed blocks are kept for the next
+// caller (any thread, any device) and given back when the device runs out of memory.  No work in
+// flight may use a block that is freed.
+void* pinned_alloc(size_t bytes);
+void pinned_free(void* p, size_t bytes) noexcept;
 // Gives the calling thread's cuBLAS / cuSOLVER handles (created on first use per thread and
 // device) back to a free list that later threads take them from; threads that end while the
 // process goes on (the serving workers) call it last.
@@ -122,6 +139,7 @@ struct cs_genotypes {
     cs::DeviceBuffer<uint8_t> packed;
     // per-SNP statistics over all samples (plink_reader.cpp:187-239), device + host
     cs::DeviceBuffer<double> d_mean, d_inv_std;
+    cs::DeviceBuffer<int32_t> d_code_counts;
     std::vector<double> mean, inv_std;
     std::vector<int32_t> count;
     std::vector<double> sum;
@@ -168,7 +186,7 @@ struct cs_kinship {
     cs::DeviceBuffer<double> d_lut;        // per view row: {(2-mu)s, 0, (1-mu)s, -mu s}
     cs::DeviceBuffer<double> d_lut_sq;     // squared entries (diagonal)
     cs::DeviceBuffer<double> d_mean, d_inv_std;
-    cs::DeviceBuffer<int32_t> d_counts;
+    cs::DeviceBuffer<int32_t> d_counts;    // `counts` on the device
     double trace = 0.0;
     cs::Workspace ws;
     cs::DeviceBuffer<double> buf_x, buf_u, buf_y;

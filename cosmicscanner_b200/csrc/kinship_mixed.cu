@@ -1566,8 +1566,36 @@ void launch_pass(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
 // optional multiplier s_t, and the imputed-code table: codes 00 / 01 (missing) / 10 / 11 ->
 // 2Q / q_t / Q / 0 with q_t = rint(Q mu_t), and the residual r_t = mu_t - q_t / Q.  Padding
 // rows decode to zeros.
+__global__ void __launch_bounds__(256)
+k_row_tables(int64_t R, const double* __restrict__ mean, const int32_t* __restrict__ counts,
+             const double* __restrict__ s, double* __restrict__ mu, double* __restrict__ exc,
+             double* __restrict__ sv, double* __restrict__ resid, uint32_t* __restrict__ lut,
+             uint8_t* __restrict__ qperm) {
+    const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;  // r_pad is a multiple of 256
+    double mt = 0.0, ex = 0.0, sc = 0.0, rs = 0.0;
+    uint32_t q = 0, l = 0;
+    if (t < R) {
+        mt = mean[t];
+        const bool ok = isfinite(mt);
+        q = (uint32_t)fmin(fmax(ok ? rint(kImputeQ * mt) : 0.0, 0.0), 2.0 * kImputeQ);
+        l = (uint32_t)(2 * kImputeQ) | (q << 8) | ((uint32_t)kImputeQ << 16);
+        rs = ok ? __dsub_rn(mt, (double)q / kImputeQ) : 0.0;
+        const int64_t c00 = counts[4 * t], c10 = counts[4 * t + 2], c11 = counts[4 * t + 3];
+        ex = __dsub_rn((double)(2 * c00 + c10), __dmul_rn(mt, (double)(c00 + c10 + c11)));
+        sc = s ? s[t] : 1.0;
+    }
+    mu[t] = mt;
+    exc[t] = ex;
+    sv[t] = sc;
+    resid[t] = rs;
+    lut[t] = l;
+    qperm[(t & ~(int64_t)15) + position_of((int)(t & 15))] = (uint8_t)q;
+}
+
+// mean, counts and s on the device
 void init_rows(MixedRows& r, const cs_packed_view& v, const double* mean, const int32_t* counts,
                const double* s_or_null) {
+    const cudaStream_t st = 0;
     configure_kernels();
     r.R = v.n_rows;
     r.n = v.n_samples;
@@ -1576,33 +1604,17 @@ void init_rows(MixedRows& r, const cs_packed_view& v, const double* mean, const 
     // samples padded to 256: the samples pass runs on pairs of 128-sample tiles (packed rows
     // hold a multiple of 256 samples, so the padding tiles read missing codes)
     r.n_pad = round_up(std::max<int64_t>(r.n, 1), 2 * kTile);
-    std::vector<double> mu(r.r_pad, 0.0), ex(r.r_pad, 0.0), sv(r.r_pad, 0.0), rs(r.r_pad, 0.0);
-    std::vector<uint32_t> lut(r.r_pad, 0u);
-    std::vector<uint8_t> qp(r.r_pad, 0u);
-    for (int64_t t = 0; t < r.R; ++t) {
-        const double mt = mean[t];
-        mu[t] = mt;
-        const double qd = std::isfinite(mt) ? std::rint(kImputeQ * mt) : 0.0;
-        const uint32_t q = (uint32_t)std::min(std::max(qd, 0.0), 2.0 * kImputeQ);
-        lut[t] = (uint32_t)(2 * kImputeQ) | (q << 8) | ((uint32_t)kImputeQ << 16);
-        qp[(t & ~(int64_t)15) + position_of((int)(t & 15))] = (uint8_t)q;
-        rs[t] = std::isfinite(mt) ? mt - (double)q / kImputeQ : 0.0;
-        const int64_t c00 = counts[4 * t], c10 = counts[4 * t + 2], c11 = counts[4 * t + 3];
-        ex[t] = (double)(2 * c00 + c10) - mt * (double)(c00 + c10 + c11);
-        sv[t] = s_or_null ? s_or_null[t] : 1.0;
-    }
     r.mu.resize(r.r_pad);
     r.exc.resize(r.r_pad);
     r.s.resize(r.r_pad);
     r.resid.resize(r.r_pad);
     r.lut.resize(r.r_pad);
     r.qperm.resize(r.r_pad / 16);
-    CS_CUDA(cudaMemcpy(r.resid.get(), rs.data(), 8 * r.r_pad, cudaMemcpyHostToDevice));
-    CS_CUDA(cudaMemcpy(r.lut.get(), lut.data(), 4 * r.r_pad, cudaMemcpyHostToDevice));
-    CS_CUDA(cudaMemcpy(r.qperm.get(), qp.data(), r.r_pad, cudaMemcpyHostToDevice));
-    CS_CUDA(cudaMemcpy(r.mu.get(), mu.data(), 8 * r.r_pad, cudaMemcpyHostToDevice));
-    CS_CUDA(cudaMemcpy(r.exc.get(), ex.data(), 8 * r.r_pad, cudaMemcpyHostToDevice));
-    CS_CUDA(cudaMemcpy(r.s.get(), sv.data(), 8 * r.r_pad, cudaMemcpyHostToDevice));
+    k_row_tables<<<(unsigned)(r.r_pad / 256), 256, 0, st>>>(
+        r.R, mean, counts, s_or_null, r.mu.get(), r.exc.get(), r.s.get(), r.resid.get(), r.lut.get(),
+        reinterpret_cast<uint8_t*>(r.qperm.get()));
+    CS_LAUNCH("row_tables");
+    CS_CUDA(cudaStreamSynchronize(st));  // ready for whichever stream applies first
     // packed tiles: 32 bytes (128 samples) x 128 SNP rows; rows past R read as zeros and
     // either land in discarded output rows (rows pass) or meet zero B rows (samples pass)
     r.tm = make_map_u8(v.rows, v.stride, std::max<int64_t>(r.R, 1), v.stride, 32, kTile, false);
@@ -2087,7 +2099,7 @@ static MixedOperator* mixed_for(cs_kinship* op) {
     if (op->mixed) return op->mixed;
     auto* m = new MixedOperator();
     try {
-        init_rows(m->rows, op->view, op->mean.data(), op->counts.data(), op->inv_std.data());
+        init_rows(m->rows, op->view, op->d_mean.get(), op->d_counts.get(), op->d_inv_std.get());
     } catch (...) {
         delete m;
         throw;
@@ -2204,7 +2216,13 @@ struct MixedScan {
 MixedScan* mixed_scan_create(const cs_packed_view& v, const double* row_mean, const int32_t* counts) {
     auto* m = new MixedScan();
     try {
-        init_rows(m->rows, v, row_mean, counts, nullptr);
+        DeviceBuffer<double> d_mean;
+        DeviceBuffer<int32_t> d_counts;
+        d_mean.resize(std::max<int64_t>(1, v.n_rows));
+        d_counts.resize(std::max<int64_t>(1, 4 * v.n_rows));
+        CS_CUDA(cudaMemcpy(d_mean.get(), row_mean, 8 * v.n_rows, cudaMemcpyHostToDevice));
+        CS_CUDA(cudaMemcpy(d_counts.get(), counts, 16 * v.n_rows, cudaMemcpyHostToDevice));
+        init_rows(m->rows, v, d_mean.get(), d_counts.get(), nullptr);
     } catch (...) {
         delete m;
         throw;

@@ -723,6 +723,8 @@ cs_lmm* lmm_create() {
 
 void lmm_destroy(cs_lmm* l) {
     prof::HostScope hs("lmm_destroy");
+    if (!l) return;
+    FreeScope fs;
     delete l;
 }
 

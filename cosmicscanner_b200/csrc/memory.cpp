@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "cs_internal.h"
@@ -46,6 +47,25 @@ std::mutex g_handle_mu;
 std::vector<cublasHandle_t> g_free_blas[kMaxDevices];
 std::vector<cusolverDnHandle_t> g_free_solver[kMaxDevices];
 
+// Free page-locked blocks, by size (a power of two), at most kPinnedKeep bytes of them.
+constexpr size_t kPinnedKeep = size_t(32) << 20;
+std::mutex g_pinned_mu;
+std::vector<std::pair<size_t, void*>> g_pinned;
+size_t g_pinned_bytes = 0;
+
+void trim_pinned() {
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    for (auto& b : g_pinned) cudaFreeHost(b.second);
+    g_pinned.clear();
+    g_pinned_bytes = 0;
+}
+
+size_t pinned_size(size_t bytes) {
+    size_t n = 4096;
+    while (n < bytes) n *= 2;
+    return n;
+}
+
 // Gives the pool's reserved free blocks back to the device (after the device has finished
 // with them), when an allocation found no room: the pool keeps freed blocks reserved, which
 // neither a block of another size nor the libraries' own allocations can use.
@@ -54,6 +74,7 @@ void trim_pool(int dev) {
     if (cudaDeviceSynchronize() == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
         cudaMemPoolTrimTo(pool, 0);
     cudaGetLastError();
+    trim_pinned();
 }
 }  // namespace
 
@@ -79,6 +100,44 @@ void* device_alloc(size_t bytes) {
     // usable from every stream once the allocation is ordered on the legacy stream
     CS_CUDA(cudaStreamSynchronize(0));
     return p;
+}
+
+void* pinned_alloc(size_t bytes) {
+    const size_t n = pinned_size(bytes);
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        for (size_t i = 0; i < g_pinned.size(); ++i)
+            if (g_pinned[i].first == n) {
+                void* p = g_pinned[i].second;
+                g_pinned[i] = g_pinned.back();
+                g_pinned.pop_back();
+                g_pinned_bytes -= n;
+                return p;
+            }
+    }
+    void* p = nullptr;
+    const cudaError_t e = cudaHostAlloc(&p, n, cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        fail(CS_ERR_CUDA, std::string("page-locked allocation of ") + std::to_string(n) +
+                              " bytes failed: " + cudaGetErrorString(e));
+    }
+    return p;
+}
+
+void pinned_free(void* p, size_t bytes) noexcept {
+    if (!p) return;
+    const size_t n = pinned_size(bytes);
+    try {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        if (g_pinned_bytes + n <= kPinnedKeep) {
+            g_pinned.emplace_back(n, p);
+            g_pinned_bytes += n;
+            return;
+        }
+    } catch (...) {
+    }
+    cudaFreeHost(p);
 }
 
 cublasHandle_t shared_blas() {
@@ -149,6 +208,20 @@ thread_local cudaStream_t g_free_stream = nullptr;
 
 void set_thread_free_stream(cudaStream_t s) { g_free_stream = s; }
 
+namespace {
+thread_local int t_free_scopes = 0;
+}
+
+FreeScope::FreeScope() {
+    if (t_free_scopes++ == 0 && !g_free_stream) cudaDeviceSynchronize();
+}
+FreeScope::~FreeScope() { --t_free_scopes; }
+
+void wait_before_free() noexcept {
+    if (g_free_stream) cudaStreamSynchronize(g_free_stream);
+    else if (!t_free_scopes) cudaDeviceSynchronize();
+}
+
 void device_free(void* p) noexcept {
     if (!p) return;
     if (g_free_stream) {
@@ -157,7 +230,7 @@ void device_free(void* p) noexcept {
         cudaFreeAsync(p, g_free_stream);
         return;
     }
-    cudaDeviceSynchronize();
+    if (!t_free_scopes) cudaDeviceSynchronize();
     cudaFreeAsync(p, 0);
 }
 

@@ -242,7 +242,7 @@ void omega_begin(uint64_t seed, int64_t total_count, OmegaWorkspace& ws, cudaStr
 
 OmegaWorkspace::~OmegaWorkspace() {
     if (counted) cudaEventSynchronize(counted);
-    if (h_counts) cudaFreeHost(h_counts);
+    if (h_counts) pinned_free(h_counts, 4 * (size_t)h_counts_cap);
     if (counted) cudaEventDestroy(counted);
 }
 
@@ -263,10 +263,10 @@ void omega_draw(OmegaWorkspace& ws, int64_t pairs_needed, cudaStream_t s) {
         ws.counts.resize(blocks);
         ws.offsets.resize(blocks);
         if (ws.h_counts_cap < blocks) {
-            if (ws.h_counts) CS_CUDA(cudaFreeHost(ws.h_counts));
+            if (ws.h_counts) pinned_free(ws.h_counts, 4 * (size_t)ws.h_counts_cap);
             ws.h_counts = nullptr;
             ws.h_counts_cap = 0;
-            CS_CUDA(cudaMallocHost(&ws.h_counts, 4 * blocks));
+            ws.h_counts = static_cast<int32_t*>(pinned_alloc(4 * (size_t)blocks));
             ws.h_counts_cap = blocks;
         }
     }

@@ -589,7 +589,11 @@ void vce_solve_stcg(cs_vce* v, cs_kinship* op, double divisor, const int32_t* re
     v->solved = true;
 }
 
-void vce_destroy(cs_vce* v) { delete v; }
+void vce_destroy(cs_vce* v) {
+    if (!v) return;
+    FreeScope fs;
+    delete v;
+}
 
 void vce_solution(const cs_vce* v, double* beta, double* a_rows, double* pe_rows) {
     if (!v->solved) fail(CS_ERR_INVALID_ARGUMENT, "STCG_VCE: solve() has not run");

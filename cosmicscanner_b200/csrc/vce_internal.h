@@ -98,17 +98,19 @@ struct HostMapped {
     HostMapped() = default;
     HostMapped(const HostMapped&) = delete;
     HostMapped& operator=(const HostMapped&) = delete;
-    ~HostMapped() {
-        if (ptr) cudaFreeHost(ptr);
+    ~HostMapped() { release(); }
+    void release() {
+        if (!ptr) return;
+        wait_before_free();
+        pinned_free(ptr, count * sizeof(double));
+        ptr = nullptr;
+        count = 0;
     }
     void resize(size_t n) {
         if (n <= count) return;
-        if (ptr) cudaFreeHost(ptr);
-        ptr = nullptr;
-        count = 0;
+        release();
         n = std::max<size_t>(n, 64);
-        CS_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&ptr), n * sizeof(double),
-                              cudaHostAllocMapped | cudaHostAllocPortable));
+        ptr = static_cast<double*>(pinned_alloc(n * sizeof(double)));
         count = n;
     }
 };
