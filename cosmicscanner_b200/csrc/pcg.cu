@@ -18,16 +18,42 @@
 
 namespace cs {
 
+// out = vg * fac * KU[row(r)] + vpe * U[row(r)] + ve * V[r]   (stcg_vce.cpp:103-115)
+struct Covariance {
+    const double *V, *KU, *U;
+    int64_t ldv, ldk, ldu;
+    const int32_t* rec_to_row;
+    double vg, fac, vpe, ve;
+    int with_pe;
+    struct In {
+        double g, pe, v;
+    };
+    __device__ In load(int64_t r, int64_t c) const {
+        const int64_t i = rec_to_row ? rec_to_row[r] : r;
+        return {i >= 0 ? KU[i * ldk + c] : 0.0, i >= 0 && with_pe ? U[i * ldu + c] : 0.0, V[r * ldv + c]};
+    }
+    __device__ double value(const In& in) const {
+        double g = in.g;
+        if (fac != 1.0) g *= fac;
+        double o = vg * g;
+        if (with_pe) o += vpe * in.pe;
+        return o + ve * in.v;
+    }
+    __device__ double operator()(int64_t r, int64_t c) const { return value(load(r, c)); }
+};
+
 namespace {
 
 // ---------------------------------------------------------------- column sums
 // Sums over the rows of n x k blocks, NV per column, in an order that depends on n alone: chunks of
-// `chunk` rows, eight interleaved lanes in each, lanes added in order, then the chunks by one
-// warp's strided sums and a shuffle tree.  A block covers kc columns (a power of two up to 32) x
-// 32 / kc chunks; the last block of a column tile finishes its columns, so that what follows from
-// the sums (a step length, a coefficient) needs no kernel of its own.  Chunks of 64 rows keep the
-// chain of dependent loads short: at n=2000 and 34 columns a sum took 14 us with 512-row chunks
-// in 8 blocks and takes 4 us with these.
+// `chunk` rows, eight interleaved lanes in each, lanes added in order, then the chunks by 32 lanes'
+// strided sums and a tree (more than two sums a column: the chunks in order).  A block covers kc
+// columns (a power of two up to 32) x 32 / kc chunks; the last block of a column tile finishes its
+// columns, so that what follows from the sums (a step length, a coefficient) needs no kernel of its
+// own.  What bounds it is the chain of dependent loads: a lane reads its rows' operands together
+// before it uses them, and the last block reads the partials in the order of memory, several at
+// once.  CG's update (n=20000, 34 columns) takes 23 us, 31 with one row at a time and a warp to a
+// column; n=2000 9.3 us against 12.5.
 constexpr int kChunkRows = 64, kMaxChunks = 512;
 int64_t chunk_rows(int64_t n) {
     return kChunkRows * std::max<int64_t>(1, (n + (int64_t)kChunkRows * kMaxChunks - 1) /
@@ -35,68 +61,102 @@ int64_t chunk_rows(int64_t n) {
 }
 int64_t chunk_count(int64_t n) { return std::max<int64_t>(1, (n + chunk_rows(n) - 1) / chunk_rows(n)); }
 
-template <int NV, class Elem, class Finish>
+// Elem: In load(r, c) reads what element (r, c) needs, use(in, r, c, v) adds it to the sums (and may
+// write the element); Batch rows are loaded at once.
+template <int NV, int Batch, class Elem, class Finish>
 __global__ void __launch_bounds__(256)
 k_column_reduce(int64_t n, int64_t k, int64_t chunk, int64_t nb, int kc, double* __restrict__ part,
                 unsigned* __restrict__ counter, const Elem elem, const Finish finish) {
-    __shared__ double red[NV][256];
+    constexpr int kScratch = NV <= 2 ? NV * 32 * 33 : NV * 256;
+    __shared__ double sh[kScratch];  // lanes' sums [NV][256], then the finish
     __shared__ int last;
     const int chunks = 32 / kc;
     const int tc = threadIdx.x % kc, tl = threadIdx.x / kc;
     const int lane = tl & 7, ch = tl >> 3;
-    const int64_t c = (int64_t)blockIdx.y * kc + tc;
+    const int64_t c0 = (int64_t)blockIdx.y * kc, c = c0 + tc;
     const int64_t b = (int64_t)blockIdx.x * chunks + ch;
     double v[NV] = {};
     if (c < k && b < nb) {
         const int64_t r1 = min(n, (b + 1) * chunk);
-#pragma unroll 4
-        for (int64_t r = b * chunk + lane; r < r1; r += 8) elem(r, c, v);
+        for (int64_t r = b * chunk + lane; r < r1; r += 8 * Batch) {
+            typename Elem::In in[Batch];
+#pragma unroll
+            for (int q = 0; q < Batch; ++q)
+                if (r + 8 * q < r1) in[q] = elem.load(r + 8 * q, c);
+#pragma unroll
+            for (int q = 0; q < Batch; ++q)
+                if (r + 8 * q < r1) elem.use(in[q], r + 8 * q, c, v);
+        }
     }
     const int slot = (tc * chunks + ch) * 8 + lane;
 #pragma unroll
-    for (int q = 0; q < NV; ++q) red[q][slot] = v[q];
+    for (int q = 0; q < NV; ++q) sh[q * 256 + slot] = v[q];
     __syncthreads();
-    if (threadIdx.x < 32) {  // one thread per (column, chunk)
-        const int64_t oc = (int64_t)blockIdx.y * kc + threadIdx.x / chunks;
-        const int64_t ob = (int64_t)blockIdx.x * chunks + threadIdx.x % chunks;
-        if (oc < k && ob < nb)
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                double t = red[q][threadIdx.x * 8];
-                for (int j = 1; j < 8; ++j) t += red[q][threadIdx.x * 8 + j];
-                part[((int64_t)q * nb + ob) * k + oc] = t;
-            }
-    }
+    // one thread per (column, chunk)
+    const int oc = threadIdx.x & 31;
+    const int64_t pc = c0 + oc / chunks, ob = (int64_t)blockIdx.x * chunks + oc % chunks;
+    for (int q = threadIdx.x >> 5; q < NV; q += 8)
+        if (pc < k && ob < nb) {
+            double t = sh[q * 256 + oc * 8];
+            for (int j = 1; j < 8; ++j) t += sh[q * 256 + oc * 8 + j];
+            part[((int64_t)q * nb + ob) * k + pc] = t;
+        }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = atomicInc(counter + blockIdx.y, gridDim.x - 1) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
-    const int wl = threadIdx.x & 31;
-    for (int j = threadIdx.x >> 5; j < kc; j += 8) {
-        const int64_t oc = (int64_t)blockIdx.y * kc + j;
-        if (oc >= k) break;
-        double tot[NV];
+    if constexpr (NV <= 2) {
+        const int slots = min(32, 256 / kc);
+        if (tl < slots && c < k)
 #pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            double t = 0.0;
-            for (int64_t ob = wl; ob < nb; ob += 32) t += __ldcg(part + ((int64_t)q * nb + ob) * k + oc);
-            for (int off = 16; off; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
-            tot[q] = t;
+            for (int q = 0; q < NV; ++q)
+                for (int l = tl; l < 32; l += slots) {
+                    double t = 0.0;
+#pragma unroll 8
+                    for (int64_t i = l; i < nb; i += 32) t += __ldcg(part + ((int64_t)q * nb + i) * k + c);
+                    sh[(q * 32 + l) * 33 + tc] = t;
+                }
+        __syncthreads();
+        const int wl = threadIdx.x & 31;
+        for (int j = threadIdx.x >> 5; j < kc && c0 + j < k; j += 8) {
+            double tot[NV];
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                tot[q] = sh[(q * 32 + wl) * 33 + j];
+                for (int off = 16; off; off >>= 1) tot[q] += __shfl_xor_sync(0xffffffffu, tot[q], off);
+            }
+            if (wl == 0) finish(c0 + j, tot);
         }
-        if (wl == 0) finish(oc, tot);
+    } else {
+        for (int p = threadIdx.x; p < NV * kc; p += 256) {
+            const int q = p / kc, j = p % kc;
+            double t = 0.0;
+            if (c0 + j < k) {
+#pragma unroll 16
+                for (int64_t i = 0; i < nb; ++i) t += __ldcg(part + ((int64_t)q * nb + i) * k + c0 + j);
+            }
+            sh[q * 32 + j] = t;
+        }
+        __syncthreads();
+        if (threadIdx.x < kc && c0 + threadIdx.x < k) {
+            double tot[NV];
+#pragma unroll
+            for (int q = 0; q < NV; ++q) tot[q] = sh[q * 32 + threadIdx.x];
+            finish(c0 + threadIdx.x, tot);
+        }
     }
 }
 
-template <int NV, class Elem, class Finish>
+template <int NV, int Batch = 8, class Elem, class Finish>
 void column_reduce(int64_t n, int64_t k, const Elem& elem, const Finish& finish, PcgWorkspace& ws,
                    cudaStream_t s) {
-    ws.reserve_reduction(n, k, s);
+    ws.reserve_reduction(n, k, NV, s);
     int kc = 1;
     while (kc < k && kc < 32) kc *= 2;
     const int64_t nb = chunk_count(n), chunks = 32 / kc;
-    k_column_reduce<NV, Elem, Finish>
+    k_column_reduce<NV, Batch, Elem, Finish>
         <<<dim3((unsigned)((nb + chunks - 1) / chunks), (unsigned)((k + kc - 1) / kc)), 256, 0, s>>>(
             n, k, chunk_rows(n), nb, kc, ws.partial.get(), ws.counter.get(), elem, finish);
     CS_LAUNCH("column_reduce");
@@ -118,9 +178,11 @@ struct Dot {
     int64_t lda;
     const double* B;
     int64_t ldb;
-    __device__ void operator()(int64_t r, int64_t c, double (&v)[1]) const {
-        v[0] += A[r * lda + c] * B[r * ldb + c];
-    }
+    struct In {
+        double a, b;
+    };
+    __device__ In load(int64_t r, int64_t c) const { return {A[r * lda + c], B[r * ldb + c]}; }
+    __device__ void use(const In& in, int64_t, int64_t, double (&v)[1]) const { v[0] += in.a * in.b; }
 };
 // R = B (columns idx), P = B / diag; r . r and r . p
 struct CgInit {
@@ -130,32 +192,16 @@ struct CgInit {
     double *R, *P;
     int64_t ld;
     double diag;
-    __device__ void operator()(int64_t r, int64_t c, double (&v)[2]) const {
-        const double b = B[r * ldb + idx[c]], p = b / diag;
+    struct In {
+        double b;
+    };
+    __device__ In load(int64_t r, int64_t c) const { return {B[r * ldb + idx[c]]}; }
+    __device__ void use(const In& in, int64_t r, int64_t c, double (&v)[2]) const {
+        const double b = in.b, p = b / diag;
         R[r * ld + c] = b;
         P[r * ld + c] = p;
         v[0] += b * b;
         v[1] += b * p;
-    }
-};
-// out = vg * fac * KU[row(r)] + vpe * U[row(r)] + ve * V[r]   (stcg_vce.cpp:103-115)
-struct Covariance {
-    const double *V, *KU, *U;
-    int64_t ldv, ldk, ldu;
-    const int32_t* rec_to_row;
-    double vg, fac, vpe, ve;
-    int with_pe;
-    __device__ double operator()(int64_t r, int64_t c) const {
-        const int64_t i = rec_to_row ? rec_to_row[r] : r;
-        double g = 0.0, pe = 0.0;
-        if (i >= 0) {
-            g = KU[i * ldk + c];
-            if (fac != 1.0) g *= fac;
-            if (with_pe) pe = U[i * ldu + c];
-        }
-        double o = vg * g;
-        if (with_pe) o += vpe * pe;
-        return o + ve * V[r * ldv + c];
     }
 };
 // AP = V p and p . AP
@@ -163,10 +209,12 @@ struct CgProduct {
     Covariance cov;
     double* out;
     int64_t ldo;
-    __device__ void operator()(int64_t r, int64_t c, double (&v)[1]) const {
-        const double o = cov(r, c);
+    using In = Covariance::In;
+    __device__ In load(int64_t r, int64_t c) const { return cov.load(r, c); }
+    __device__ void use(const In& in, int64_t r, int64_t c, double (&v)[1]) const {
+        const double o = cov.value(in);
         out[r * ldo + c] = o;
-        v[0] += cov.V[r * cov.ldv + c] * o;
+        v[0] += in.v * o;
     }
 };
 // alpha = rsold / (p . Ap)
@@ -185,10 +233,16 @@ struct CgUpdate {
     int64_t ld;
     const double* alpha;
     double diag;
-    __device__ void operator()(int64_t r, int64_t c, double (&v)[2]) const {
+    struct In {
+        double x, p, r, ap;
+    };
+    __device__ In load(int64_t r, int64_t c) const {
+        return {X[r * ldx + map[c]], P[r * ld + c], R[r * ld + c], AP[r * ld + c]};
+    }
+    __device__ void use(const In& in, int64_t r, int64_t c, double (&v)[2]) const {
         const double a = alpha[c];
-        X[r * ldx + map[c]] += a * P[r * ld + c];
-        const double rv = R[r * ld + c] - a * AP[r * ld + c];
+        X[r * ldx + map[c]] = in.x + a * in.p;
+        const double rv = in.r - a * in.ap;
         R[r * ld + c] = rv;
         v[0] += rv * rv;
         v[1] += rv * (rv / diag);
@@ -212,19 +266,60 @@ struct CgBetaZ {
         rsold[c] = t[0];
     }
 };
+// w -= sum_q coef[q] o sub[q] (blocks of n x k), then NV sums: w . dot[q], or w . w without dot
+constexpr int kLanczosGroup = kLanczosCoef;
+template <int NV>
 struct LanczosElem {
     double* w;
     const double *sub, *dot, *coef;
-    int64_t ld;
-    __device__ void operator()(int64_t r, int64_t c, double (&v)[1]) const {
-        double x = w[r * ld + c];
-        if (sub) {
-            x -= coef[c] * sub[r * ld + c];
-            w[r * ld + c] = x;
+    int n_sub, n_dot;
+    int64_t ld, block;
+    struct In {
+        double x, d[NV];
+    };
+    __device__ In load(int64_t r, int64_t c) const {
+        In in;
+        in.x = w[r * ld + c];
+        double s[8];
+        for (int q0 = 0; q0 < n_sub; q0 += 8) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) s[q] = q0 + q < n_sub ? sub[(q0 + q) * block + r * ld + c] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (q0 + q < n_sub) in.x -= coef[(q0 + q) * ld + c] * s[q];
         }
-        v[0] += x * (dot ? dot[r * ld + c] : x);
+#pragma unroll
+        for (int q = 0; q < NV; ++q) in.d[q] = q < n_dot ? dot[q * block + r * ld + c] : 0.0;
+        return in;
+    }
+    __device__ void use(const In& in, int64_t r, int64_t c, double (&v)[NV]) const {
+        if (n_sub) w[r * ld + c] = in.x;
+        if (n_dot == 0) v[0] += in.x * in.x;
+        else
+#pragma unroll
+            for (int q = 0; q < NV; ++q) v[q] += in.x * in.d[q];
     }
 };
+// w = V v_j - beta_{j-1} v_{j-1}; w . v_j  (V v_j from the product's parts)
+struct LanczosFirst {
+    Covariance cov;
+    double* w;
+    const double *prev, *coef;
+    struct In {
+        Covariance::In cov;
+        double prev;
+    };
+    __device__ In load(int64_t r, int64_t c) const {
+        return {cov.load(r, c), prev ? prev[r * cov.ldv + c] : 0.0};
+    }
+    __device__ void use(const In& in, int64_t r, int64_t c, double (&v)[1]) const {
+        double x = cov.value(in.cov);
+        if (prev) x -= coef[c] * in.prev;
+        w[r * cov.ldv + c] = x;
+        v[0] += x * in.cov.v;
+    }
+};
+enum class LanczosMode { kAlpha, kBeta };
 struct LanczosFinish {
     LanczosState st;
     LanczosMode mode;
@@ -243,6 +338,15 @@ struct LanczosFinish {
             }
         }
         st.coef[c] = coef;
+    }
+};
+struct LanczosGroup {
+    LanczosState st;
+    int64_t k;
+    __device__ void operator()(int64_t c, const double (&t)[kLanczosGroup]) const {
+        const bool done = st.done[c] != 0;
+#pragma unroll
+        for (int q = 0; q < kLanczosGroup; ++q) st.coef[q * k + c] = done ? 0.0 : t[q];
     }
 };
 
@@ -401,13 +505,17 @@ const double* VOperator::kinship(const double* in, int64_t ldi, int64_t k, int64
     return U;
 }
 
+Covariance VOperator::covariance(const double* in, int64_t ldi, const double* U, int64_t ldu, int64_t k) const {
+    return Covariance{in, ku.get(), U, ldi, k, ldu, rm->identity ? nullptr : rm->d_rec_to_row.get(),
+                      vg, fac, vpe, ve, with_pe ? 1 : 0};
+}
+
 void VOperator::apply(const double* in, int64_t ldi, int64_t k, double* out, int64_t ldo,
                       cudaStream_t s) {
     if (k <= 0) return;
     int64_t ldu = 0;
     const double* U = kinship(in, ldi, k, ldu, s);
-    const Covariance cov{in, ku.get(), U, ldi, k, ldu, rm->identity ? nullptr : rm->d_rec_to_row.get(),
-                         vg, fac, vpe, ve, with_pe ? 1 : 0};
+    const Covariance cov = covariance(in, ldi, U, ldu, k);
     prof::Scope ps("covariance_combine", s, 0.0, 8.0 * 3.0 * (double)rm->n_rec * k);
     k_combine<<<grid_for(rm->n_rec * k), 256, 0, s>>>(out, ldo, cov, rm->n_rec, k);
     CS_LAUNCH("covariance_combine");
@@ -417,8 +525,7 @@ void VOperator::apply_alpha(const double* p, int64_t k, double* out, const doubl
                             PcgWorkspace& ws, cudaStream_t s) {
     int64_t ldu = 0;
     const double* U = kinship(p, k, k, ldu, s);
-    const Covariance cov{p, ku.get(), U, k, k, ldu, rm->identity ? nullptr : rm->d_rec_to_row.get(),
-                         vg, fac, vpe, ve, with_pe ? 1 : 0};
+    const Covariance cov = covariance(p, k, U, ldu, k);
     prof::Scope ps("covariance_combine", s, 2.0 * (double)rm->n_rec * k, 8.0 * 3.0 * (double)rm->n_rec * k);
     column_reduce<1>(rm->n_rec, k, CgProduct{cov, out, k}, CgAlpha{rsold, alpha}, ws, s);
 }
@@ -458,8 +565,8 @@ void VOperator::genetic_rows(const double* in, int64_t ldi, int64_t k, double* r
 }
 
 // ---------------------------------------------------------------- dots
-void PcgWorkspace::reserve_reduction(int64_t n, int64_t k, cudaStream_t s) {
-    partial.resize(2 * chunk_count(n) * std::max<int64_t>(1, k));
+void PcgWorkspace::reserve_reduction(int64_t n, int64_t k, int sums, cudaStream_t s) {
+    partial.resize(std::max(2, sums) * chunk_count(n) * std::max<int64_t>(1, k));
     host.resize(2 * std::max<int64_t>(1, k));
     if (counter.count < (size_t)k) {
         counter.resize(k);
@@ -472,7 +579,7 @@ void destroy_pcg(PcgWorkspace* w) { delete w; }
 void column_dots(const double* A, int64_t lda, const double* B, int64_t ldb, int64_t n, int64_t k,
                  double* out_host, PcgWorkspace& ws, cudaStream_t s) {
     if (k <= 0) return;
-    ws.reserve_reduction(n, k, s);
+    ws.reserve_reduction(n, k, 2, s);
     {
         prof::Scope ps("column_dots", s, 2.0 * n * k, 16.0 * n * k);
         column_reduce<1>(n, k, Dot{A, lda, B, ldb}, StoreSum{ws.host.ptr}, ws, s);
@@ -481,10 +588,29 @@ void column_dots(const double* A, int64_t lda, const double* B, int64_t ldb, int
     std::copy(ws.host.ptr, ws.host.ptr + k, out_host);
 }
 
-void lanczos_step(double* w, const double* sub, const double* dot, int64_t n, int64_t k,
-                  const LanczosState& st, LanczosMode mode, int step, PcgWorkspace& ws, cudaStream_t s) {
-    prof::Scope ps("lanczos_step", s, 4.0 * n * k, 8.0 * (sub ? 4.0 : 2.0) * n * k);
-    column_reduce<1>(n, k, LanczosElem{w, sub, dot, st.coef, k}, LanczosFinish{st, mode, step}, ws, s);
+void lanczos_step(VOperator& V, const double* basis, int64_t k, double* w, const LanczosState& st, int step,
+                  PcgWorkspace& ws, cudaStream_t s) {
+    const int64_t n = V.rm->n_rec, block = n * k;
+    const double* const vj = basis + step * block;
+    int64_t ldu = 0;
+    const double* U = V.kinship(vj, k, k, ldu, s);
+    prof::Scope ps("lanczos_step", s, 4.0 * (step + 2) * block, 8.0 * (2 * step + 10) * block);
+    column_reduce<1>(n, k, LanczosFirst{V.covariance(vj, k, U, ldu, k), w, step ? vj - block : nullptr, st.coef},
+                     LanczosFinish{st, LanczosMode::kAlpha, step}, ws, s);
+    // full reorthogonalisation against v_0 .. v_j, sixteen at a time; each kernel subtracts what the
+    // one before it measured (first alpha v_j)
+    const double* sub = vj;
+    int n_sub = 1;
+    for (int q = 0; q <= step; q += kLanczosGroup) {
+        const int here = std::min(kLanczosGroup, step + 1 - q);
+        column_reduce<kLanczosGroup, 2>(
+            n, k, LanczosElem<kLanczosGroup>{w, sub, basis + q * block, st.coef, n_sub, here, k, block},
+            LanczosGroup{st, k}, ws, s);
+        sub = basis + q * block;
+        n_sub = here;
+    }
+    column_reduce<1, 4>(n, k, LanczosElem<1>{w, sub, nullptr, st.coef, n_sub, 0, k, block},
+                        LanczosFinish{st, LanczosMode::kBeta, step}, ws, s);
 }
 
 // ---------------------------------------------------------------- low-rank preconditioner
@@ -533,7 +659,7 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
     ws.P.resize(n * k);
     ws.AP.resize(n * k);
     ws.T.resize(n * k);
-    ws.reserve_reduction(n, k, s);
+    ws.reserve_reduction(n, k, 2, s);
     for (auto* b : {&ws.alpha, &ws.beta, &ws.rsold}) b->resize(k);
     ws.map.resize(k);
     ws.idx.resize(k);

@@ -203,7 +203,7 @@ static double slq_logdet(cs_vce* v, int probes, int steps, uint64_t seed, cudaSt
     v->slq_rng.draw(n, k, v->lw.get(), k, s);
     std::vector<double> inv(k, 1.0 / std::sqrt((double)n));
     DeviceBuffer<double> dcoef;
-    dcoef.resize(k);
+    dcoef.resize(kLanczosCoef * k);
     CS_CUDA(cudaMemcpyAsync(dcoef.get(), inv.data(), 8 * k, cudaMemcpyHostToDevice, s));
     k_scale_cols<<<grid_1d(n * k), 256, 0, s>>>(Vj(0), v->lw.get(), k, n, k, dcoef.get(), 0);
     CS_LAUNCH("scale_cols");
@@ -222,13 +222,7 @@ static double slq_logdet(cs_vce* v, int probes, int steps, uint64_t seed, cudaSt
         const LanczosState st{dcoef.get(), d_ab.get() + (int64_t)j * k, d_ab.get() + (int64_t)(m + j) * k,
                               d_done.get(), d_done.get() + k};
         double* w = v->lw.get();
-        v->V.apply(Vj(j), k, k, w, k, s);
-        // w -= beta_{j-1} v_{j-1}; alpha_j = w . v_j; w -= alpha_j v_j; full reorthogonalisation
-        // against v_0 .. v_j; beta_j = |w|: each kernel subtracts what the one before it measured
-        lanczos_step(w, j > 0 ? Vj(j - 1) : nullptr, Vj(j), n, k, st, LanczosMode::kAlpha, j, v->pw, s);
-        for (int q = 0; q <= j; ++q)
-            lanczos_step(w, q == 0 ? Vj(j) : Vj(q - 1), Vj(q), n, k, st, LanczosMode::kReorth, j, v->pw, s);
-        lanczos_step(w, Vj(j), nullptr, n, k, st, LanczosMode::kBeta, j, v->pw, s);
+        lanczos_step(v->V, v->lz.get(), k, w, st, j, v->pw, s);
         k_scale_cols<<<grid_1d(n * k), 256, 0, s>>>(Vj(j + 1), w, k, n, k, dcoef.get(), 1);
         CS_LAUNCH("scale_cols");
     }

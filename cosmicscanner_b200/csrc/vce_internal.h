@@ -44,6 +44,7 @@ struct RecordMap {
 
 // V = vg * Zr K Zr^T + vpe * Zr Zr^T + ve * I on record-level blocks, with
 // K = Z Z^T / divisor (stcg_vce.cpp:80-115).
+struct Covariance;  // pcg.cu
 struct VOperator {
     cs_kinship* op = nullptr;
     const RecordMap* rm = nullptr;
@@ -57,6 +58,10 @@ struct VOperator {
 
     // out (n_rec x ldo) = V * in (n_rec x ldi), k columns.
     void apply(const double* in, int64_t ldi, int64_t k, double* out, int64_t ldo, cudaStream_t s);
+    // ku = K Zr^T in (n_rows x k), the genetic part of V in; returns Zr^T in (n_rows x ldu).
+    const double* kinship(const double* in, int64_t ldi, int64_t k, int64_t& ldu, cudaStream_t s);
+    // V in, element by element, from what kinship(in) made.
+    Covariance covariance(const double* in, int64_t ldi, const double* U, int64_t ldu, int64_t k) const;
     // The same for CG (out = V p), with alpha[c] = rsold[c] / (p . V p)[c].
     void apply_alpha(const double* p, int64_t k, double* out, const double* rsold, double* alpha,
                      PcgWorkspace& ws, cudaStream_t s);
@@ -68,7 +73,6 @@ struct VOperator {
                       double* zt_out, int64_t ldz, cudaStream_t s);
 
    private:
-    const double* kinship(const double* in, int64_t ldi, int64_t k, int64_t& ldu, cudaStream_t s);
     const double* gather(const double* in, int64_t ldi, int64_t k, cudaStream_t s);
 };
 
@@ -122,8 +126,8 @@ struct PcgWorkspace {
     DeviceBuffer<unsigned> counter;  // column_reduce's, zero between kernels
     HostMapped host;                 // reductions read by the host: two values a column
     DeviceBuffer<double> b, x;       // a public solve's row-major blocks
-    // room for reductions over n rows of k columns
-    void reserve_reduction(int64_t n, int64_t k, cudaStream_t s);
+    // room for reductions of up to `sums` values a column over n rows of k columns
+    void reserve_reduction(int64_t n, int64_t k, int sums, cudaStream_t s);
     size_t bytes() const {
         return 8 * (R.count + P.count + AP.count + T.count + Zp.count + partial.count + b.count + x.count);
     }
@@ -161,19 +165,18 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
 void column_dots(const double* A, int64_t lda, const double* B, int64_t ldb, int64_t n, int64_t k,
                  double* out_host, PcgWorkspace& ws, cudaStream_t s);
 
-// One step of the Lanczos recurrences' vector work on row-major n x k blocks: w -= coef o sub (sub
-// null: nothing), then the column sums of w * dot (dot null: of w * w), from which `mode` leaves
-//   kAlpha   alpha[c] = the sum, coef[c] = the sum     kReorth  coef[c] = the sum
-//   kBeta    beta[c] = coef[c] = its square root, or, where that is below 1e-12, steps[c] = step + 1
-//            and the column done
-// (a done column keeps its alpha and beta, and its coef is zero).
+// Step j of k Lanczos recurrences on V (row-major n x k blocks, basis[i] = v_i at i * n * k):
+// w = V v_j - beta_{j-1} v_{j-1} (coef holds beta), alpha[c] = w . v_j, w -= alpha v_j, w
+// reorthogonalised against v_0 .. v_j, beta[c] = coef[c] = |w|, or, where that is below 1e-12,
+// steps[c] = j + 1, the column done and coef zero (a done column keeps its alpha and beta).
+// coef: kLanczosCoef * k values.
+constexpr int kLanczosCoef = 16;
 struct LanczosState {
     double *coef, *alpha, *beta;
     int32_t *done, *steps;
 };
-enum class LanczosMode { kAlpha, kReorth, kBeta };
-void lanczos_step(double* w, const double* sub, const double* dot, int64_t n, int64_t k,
-                  const LanczosState& st, LanczosMode mode, int step, PcgWorkspace& ws, cudaStream_t s);
+void lanczos_step(VOperator& V, const double* basis, int64_t k, double* w, const LanczosState& st, int step,
+                  PcgWorkspace& ws, cudaStream_t s);
 
 // The mt19937_64 stream on the device (omega.cu).
 void mt64_seed_device(uint64_t seed, uint64_t* d_state, cudaStream_t s);
