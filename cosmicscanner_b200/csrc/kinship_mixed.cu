@@ -59,6 +59,7 @@
 #include <tuple>
 #include <vector>
 
+#include "chain.cuh"
 #include "cs_internal.h"
 #include "mixed_internal.h"
 #include "sm100.cuh"
@@ -304,6 +305,7 @@ k_mixed_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         else
             tmem_alloc(tmem_slot, kTmemCols);
     }
+    chain_wait();
     tc_fence_before();
     if (PAIR)
         cluster_sync_all();
@@ -409,6 +411,7 @@ k_mixed_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
             // leave no copy in flight
             for (uint32_t q = (j >= (uint32_t)ST ? j - ST : 0); q < j; ++q)
                 mbar_wait(&full_t[q % ST], (q / ST) & 1, P.status, kTimeoutTma, 1u << 20);
+            chain_next();
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (pair: leader)
@@ -830,6 +833,7 @@ template <class T>
 __global__ void __launch_bounds__(256)
 k_col_stats(const Strided<const T> X, int64_t n, int64_t k, int kc, int64_t nb,
             double* __restrict__ part, const MixedColumns C) {
+    chain_enter();
     __shared__ double red[10][32 * 9];  // eight tiles' sums, minima, maxima; 8 lanes and a pad per (column, chunk)
     // threads in the order of memory: columns fastest in row-major input, lanes in column-major
     const int per = 256 / kc;  // 8 lanes x chunks
@@ -947,6 +951,7 @@ template <class T, int COLS, int ROWS>
 __global__ void __launch_bounds__(ROWS / 16 * COLS, 1024 / (ROWS / 16 * COLS))
 k_split_rows_operand(const Strided<const T> X, int64_t n, int64_t k, int64_t kp, int64_t n_pad,
                      const MixedColumns C, int8_t* __restrict__ B, double* __restrict__ part) {
+    chain_enter();
     constexpr int TH = ROWS / 16 * COLS;
     constexpr int kPitch = ROWS + ROWS / 16 + 1;  // one pad every 16 rows and one per column
     static_assert(COLS * kPitch >= 32 * 33, "sum_tiles's scratch");
@@ -1023,6 +1028,7 @@ __global__ void __launch_bounds__(256)
 k_reduce_rows(const double* __restrict__ part, int splits, int64_t kp, int64_t ld, int64_t R,
               const double* __restrict__ s_row, const double* __restrict__ exc_row,
               const double* __restrict__ mu, const MixedColumns C, double* __restrict__ out) {
+    chain_enter();
     __shared__ double red[2][8];
     const int64_t c = blockIdx.y;
     const RowsColumn col(C, c);
@@ -1073,6 +1079,7 @@ k_reduce_rows_out(const double* __restrict__ part, int splits, int64_t kp, int64
                   int64_t k, const double* __restrict__ s_row, const double* __restrict__ exc_row,
                   const double* __restrict__ mu, const int32_t* __restrict__ pos, const MixedColumns C,
                   StridedOut out) {
+    chain_enter();
     __shared__ double tile[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t t0 = (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
@@ -1111,6 +1118,7 @@ k_split_samples_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int
                         const double* __restrict__ resid, const MixedColumns C,
                         int8_t* __restrict__ B, double* __restrict__ inv_f,
                         double* __restrict__ cpart, double* __restrict__ c0) {
+    chain_enter();
     __shared__ double red[8];
     // W and the second operand of 2048 SNPs, one pad every 16, read in the order of memory
     __shared__ double sw[128 * 17], sb[128 * 17];
@@ -1245,6 +1253,7 @@ __global__ void __launch_bounds__(256)
 k_gather_operand(const StridedIn V, int64_t R, const int32_t* __restrict__ pos,
                  const double* __restrict__ s_row, const double* __restrict__ mu, const MixedColumns C,
                  double* __restrict__ Wt) {
+    chain_enter();
     const int64_t c = blockIdx.y;
     double mw = 0.0, mm = 0.0;
     const int64_t t0 = (int64_t)blockIdx.x * 1024;
@@ -1270,6 +1279,7 @@ template <class T>
 __global__ void __launch_bounds__(256)
 k_reduce_samples(const double* __restrict__ part, int splits, int64_t kp, int64_t ld, int64_t n,
                  int64_t k, const double* __restrict__ c0v, double inv_m, const Strided<T> Y) {
+    chain_enter();
     __shared__ double tile[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t i0 = (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
@@ -1547,18 +1557,17 @@ void launch_pass(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
         cfg.blockDim = dim3(kThreads);
         cfg.dynamicSmemBytes = Layout<ROWS, true, false, TMEMA>::kSmem;
         cfg.stream = s;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
         cfg.numAttrs = 1;
+        chain(cfg, attr);
         CS_CUDA(cudaLaunchKernelEx(&cfg, k_mixed_pass<ROWS, true, false, TMEMA>, ta, tb, tbt, P));
     } else {
-        k_mixed_pass<ROWS, false, NARROW, TMEMA>
-            <<<num_sms(), kThreads, Layout<ROWS, false, NARROW, TMEMA>::kSmem, s>>>(
-            ta, tb, tbt, P);
+        launch_chained(k_mixed_pass<ROWS, false, NARROW, TMEMA>, num_sms(), kThreads,
+                       Layout<ROWS, false, NARROW, TMEMA>::kSmem, s, ta, tb, tbt, P);
     }
 }
 
@@ -1911,14 +1920,16 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, Stri
         int kc = 1;
         while (X.rs != 1 && kc < k && kc < 32) kc *= 2;
         const int64_t per = 32 / kc;  // chunks per block
-        k_col_stats<T><<<dim3((unsigned)((nst + per - 1) / per), (unsigned)((k + kc - 1) / kc)), 256, 0, s>>>(
-            X, n, k, kc, nst, ws.colpart.get(), C);
+        launch_chained(k_col_stats<T>, dim3((unsigned)((nst + per - 1) / per), (unsigned)((k + kc - 1) / kc)),
+                       256, 0, s, X, n, k, kc, nst, ws.colpart.get(), C);
         if (kp <= 16)
-            k_split_rows_operand<T, 4, 512><<<dim3((unsigned)((n_pad + 511) / 512), (unsigned)((kp + 3) / 4)),
-                                              128, 0, s>>>(X, n, k, kp, n_pad, C, ws.b1.get(), ws.colpart.get());
+            launch_chained(k_split_rows_operand<T, 4, 512>,
+                           dim3((unsigned)((n_pad + 511) / 512), (unsigned)((kp + 3) / 4)), 128, 0, s, X, n, k,
+                           kp, n_pad, C, ws.b1.get(), ws.colpart.get());
         else
-            k_split_rows_operand<T, 16, 256><<<dim3((unsigned)(n_pad / 256), (unsigned)((kp + 15) / 16)), 256,
-                                               0, s>>>(X, n, k, kp, n_pad, C, ws.b1.get(), ws.colpart.get());
+            launch_chained(k_split_rows_operand<T, 16, 256>,
+                           dim3((unsigned)(n_pad / 256), (unsigned)((kp + 15) / 16)), 256, 0, s, X, n, k, kp,
+                           n_pad, C, ws.b1.get(), ws.colpart.get());
         CS_LAUNCH("mixed rows operand");
     }
     PassArgs P{};
@@ -1959,11 +1970,12 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, Stri
     {
         prof::Scope ps("mixed_reduce_rows", s, 0.0, 8.0 * splits * kp * R + 8.0 * R * k);
         if (Wt)
-            k_reduce_rows<<<dim3((unsigned)((R + 1023) / 1024), (unsigned)k), 256, 0, s>>>(
-                ws.part.get(), splits, kp, r_pad, R, r.s.get(), r.exc.get(), r.mu.get(), C, Wt);
+            launch_chained(k_reduce_rows, dim3((unsigned)((R + 1023) / 1024), (unsigned)k), 256, 0, s,
+                           ws.part.get(), splits, kp, r_pad, R, r.s.get(), r.exc.get(), r.mu.get(), C, Wt);
         else
-            k_reduce_rows_out<<<dim3((unsigned)((R + 31) / 32), (unsigned)((k + 31) / 32)), 256, 0, s>>>(
-                ws.part.get(), splits, kp, r_pad, R, k, r.s.get(), r.exc.get(), r.mu.get(), pos, C, out);
+            launch_chained(k_reduce_rows_out, dim3((unsigned)((R + 31) / 32), (unsigned)((k + 31) / 32)), 256,
+                           0, s, ws.part.get(), splits, kp, r_pad, R, k, r.s.get(), r.exc.get(), r.mu.get(),
+                           pos, C, out);
         CS_LAUNCH("reduce_rows");
     }
 }
@@ -2007,8 +2019,8 @@ void samples_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, c
         const dim3 g((unsigned)nrb, (unsigned)kp);
         const MixedColumns C = ws.columns(k, s);
         auto split = [&](auto kern) {
-            kern<<<g, 128, 0, s>>>(Wt, R, k, kp, r_pad, r.mu.get(), r.resid.get(), C, ws.b2.get(),
-                                   ws.inv_f.get(), ws.colpart.get(), ws.c0.get());
+            launch_chained(kern, g, 128, 0, s, Wt, R, k, kp, r_pad, r.mu.get(), r.resid.get(), C, ws.b2.get(),
+                           ws.inv_f.get(), ws.colpart.get(), ws.c0.get());
         };
         if (six) split(k_split_samples_operand<true, true>);
         else if (tmem_a) split(k_split_samples_operand<false, true>);
@@ -2054,8 +2066,8 @@ void samples_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, c
     }
     {
         prof::Scope ps("mixed_reduce_samples", s, 0.0, 8.0 * splits * kp * n + 8.0 * n * k);
-        k_reduce_samples<T><<<dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)), 256, 0, s>>>(
-            ws.part.get(), splits, kp, n_pad, n, k, ws.c0.get(), inv_m, Y);
+        launch_chained(k_reduce_samples<T>, dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)), 256, 0,
+                       s, ws.part.get(), splits, kp, n_pad, n, k, ws.c0.get(), inv_m, Y);
         CS_LAUNCH("reduce_samples");
     }
 }
@@ -2165,8 +2177,8 @@ void mixed_multiply_z(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cuda
     CS_CUDA(cudaMemsetAsync(C.max_wmu, 0, 8 * k, s));
     {
         prof::Scope ps("mixed_gather_operand", s, 0.0, 16.0 * R * k);
-        k_gather_operand<<<dim3((unsigned)((R + 1023) / 1024), (unsigned)k), 256, 0, s>>>(
-            V, R, op->d_view_pos.get(), m->rows.s.get(), m->rows.mu.get(), C, ws.W.get());
+        launch_chained(k_gather_operand, dim3((unsigned)((R + 1023) / 1024), (unsigned)k), 256, 0, s, V, R,
+                       op->d_view_pos.get(), m->rows.s.get(), m->rows.mu.get(), C, ws.W.get());
         CS_LAUNCH("gather_operand");
     }
     samples_pass(m->rows, ws, ws.W.get(), k, 1.0, Y, s, op->autotune, op->sample_major_copy);

@@ -47,6 +47,7 @@
 #include <cmath>
 #include <string>
 
+#include "chain.cuh"
 #include "cs_internal.h"
 #include "mixed_internal.h"
 #include "slices_internal.h"
@@ -164,6 +165,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         else
             tmem_alloc(tmem_slot, kTmemCols);
     }
+    chain_wait();
     tc_fence_before();
     if (PAIR)
         cluster_sync_all();
@@ -234,6 +236,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                 if (--d < 0) { d = SD - 1; ph ^= 1; }
                 mbar_wait_look(&full[d], ph, P.status, kTimeoutTma, 1u << 20);
             }
+            chain_next();
         }
     } else if (warp == 2) {
         // ------------------------------------------------------------ TMA producer (packed)
@@ -567,6 +570,7 @@ __device__ __forceinline__ void add_range(ColumnRange* out, unsigned long long m
 __global__ void __launch_bounds__(256)
 k_slice_ranges(const StridedIn X, int64_t n, int64_t k, int kc, int64_t rows_per_block,
                ColumnRange* __restrict__ out) {
+    chain_enter();
     __shared__ unsigned long long s_mx[256];
     __shared__ long long s_es[256];
     __shared__ unsigned s_n[256];
@@ -686,6 +690,7 @@ template <int COLS, int ROWS>
 __global__ void __launch_bounds__(ROWS / 16 * COLS)
 k_slice_rows_operand(const StridedIn X, int64_t n, int64_t k, int64_t k_pad, int64_t n_pad,
                      int slice_rows, const SliceSums S, BLayout B, int8_t* __restrict__ out) {
+    chain_enter();
     constexpr int T = ROWS / 16 * COLS;
     static_assert(ROWS % 256 == 0 && (ROWS / 16) % 16 == 0, "a half warp covers 256 rows of a column");
     // one pad every 16 rows and one per column: conflict-free both ways
@@ -727,6 +732,7 @@ constexpr int64_t kWholeRows = 8192;
 __global__ void __launch_bounds__(kWholeRows / 16)
 k_slice_rows_operand_whole(const StridedIn X, int64_t n, int64_t k, int64_t n_pad, int slice_rows,
                            const SliceSums S, BLayout B, int8_t* __restrict__ out) {
+    chain_enter();
     __shared__ unsigned long long s_mx[16], s_sum[64][2];
     __shared__ long long s_es[16];
     __shared__ unsigned s_n[16];
@@ -795,6 +801,7 @@ __global__ void __launch_bounds__(128)
 k_slice_samples_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int64_t r_pad,
                         int slice_rows, const double* __restrict__ mu, const SliceSums S, BLayout B,
                         int8_t* __restrict__ out) {
+    chain_enter();
     // w and mu o w of 2048 SNPs, one pad every 16, read in the order of memory
     __shared__ double sw[128 * 17], sb[128 * 17];
     const int64_t c = blockIdx.y, base = (int64_t)blockIdx.x * 2048;
@@ -874,6 +881,7 @@ k_slice_reduce_rows(const double* __restrict__ part, int64_t ld, int64_t R, int6
                     const double* __restrict__ s_row, const double* __restrict__ mu,
                     const PackedRows G, const StridedIn X, int64_t n, const SliceSums S,
                     double* __restrict__ Wt, const int32_t* __restrict__ pos, StridedOut out) {
+    chain_enter();
     const int64_t c = blockIdx.y;
     const ColumnRange rg = S.range[c];
     const double f = pow2(-slice_exponent(rg.max_bits)) / (double)kTcQ;
@@ -918,6 +926,7 @@ __global__ void __launch_bounds__(256)
 k_slice_gather(const StridedIn V, int64_t R, const int32_t* __restrict__ pos,
                const double* __restrict__ s_row, const double* __restrict__ mu, const SliceSums S,
                double* __restrict__ Wt) {
+    chain_enter();
     const int64_t c = blockIdx.y;
     unsigned long long mx = 0;
     long long es = 0;
@@ -941,6 +950,7 @@ __global__ void __launch_bounds__(256)
 k_slice_reduce_samples(const double* __restrict__ part, int64_t ld, int64_t n, int64_t k,
                        const double* __restrict__ Wt, int64_t R, const double* __restrict__ mu,
                        const PackedRows G, const SliceSums S, double scale, StridedOut Y) {
+    chain_enter();
     __shared__ double tile[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t i0 = (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
@@ -1098,7 +1108,7 @@ void launch_slice_pass(const SlicePlan& p, const CUtensorMap& ta, const CUtensor
     cfg.blockDim = dim3(threads_for(groups_of<PAIR>()));
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     if constexpr (PAIR) {
         cfg.gridDim = dim3((unsigned)(num_sms() & ~1));
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1124,6 +1134,7 @@ void launch_slice_pass(const SlicePlan& p, const CUtensorMap& ta, const CUtensor
         cfg.gridDim = dim3((unsigned)std::min<int64_t>(
             num_sms(), std::max<int64_t>(1, (int64_t)A.n_tiles * A.n_ctiles * A.n_splits)));
     }
+    chain(cfg, attr);
     CS_CUDA(cudaLaunchKernelEx(&cfg, k_slice_pass<ROWS, PAIR, groups_of<PAIR>()>, ta, tb, A));
 }
 
@@ -1222,8 +1233,8 @@ void run_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSu
     if (n <= kWholeRows && p.splits <= 64) {
         prof::Scope ps("slice_prep_rows_operand", s, 0.0, 16.0 * n * k + 7.0 * k_pad * r.n_pad);
         const unsigned threads = (unsigned)round_up(r.n_pad / 16, 32);
-        k_slice_rows_operand_whole<<<(unsigned)k_pad, threads, 0, s>>>(X, n, k, r.n_pad, slice_rows, S, B,
-                                                                   so.b.get());
+        launch_chained(k_slice_rows_operand_whole, (unsigned)k_pad, threads, 0, s, X, n, k, r.n_pad,
+                       slice_rows, S, B, so.b.get());
         CS_LAUNCH("slice rows operand");
     } else {
         CS_CUDA(cudaMemsetAsync(so.words.get(), 0, 8 * c.words, s));
@@ -1231,18 +1242,18 @@ void run_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSu
         int kc = 1;
         while (X.rs != 1 && kc < k && kc < 32) kc *= 2;
         const int64_t rpb = std::max<int64_t>(256, 4096 / kc);
-        k_slice_ranges<<<dim3((unsigned)((n + rpb - 1) / rpb), (unsigned)((k + kc - 1) / kc)), 256, 0, s>>>(
-            X, n, k, kc, rpb, S.range);
+        launch_chained(k_slice_ranges, dim3((unsigned)((n + rpb - 1) / rpb), (unsigned)((k + kc - 1) / kc)),
+                       256, 0, s, X, n, k, kc, rpb, S.range);
         if (k_pad <= 1)
-            k_slice_rows_operand<1, 1024><<<dim3((unsigned)((r.n_pad + 1023) / 1024), 1), 64, 0, s>>>(
-                X, n, k, k_pad, r.n_pad, slice_rows, S, B, so.b.get());
+            launch_chained(k_slice_rows_operand<1, 1024>, dim3((unsigned)((r.n_pad + 1023) / 1024), 1), 64, 0,
+                           s, X, n, k, k_pad, r.n_pad, slice_rows, S, B, so.b.get());
         else if (k_pad <= 4)
-            k_slice_rows_operand<4, 512><<<dim3((unsigned)((r.n_pad + 511) / 512), 1), 128, 0, s>>>(
-                X, n, k, k_pad, r.n_pad, slice_rows, S, B, so.b.get());
+            launch_chained(k_slice_rows_operand<4, 512>, dim3((unsigned)((r.n_pad + 511) / 512), 1), 128, 0, s,
+                           X, n, k, k_pad, r.n_pad, slice_rows, S, B, so.b.get());
         else
-            k_slice_rows_operand<16, 256><<<dim3((unsigned)(r.n_pad / 256), (unsigned)((k_pad + 15) / 16)),
-                                            256, 0, s>>>(X, n, k, k_pad, r.n_pad, slice_rows, S, B,
-                                                         so.b.get());
+            launch_chained(k_slice_rows_operand<16, 256>,
+                           dim3((unsigned)(r.n_pad / 256), (unsigned)((k_pad + 15) / 16)), 256, 0, s, X, n, k,
+                           k_pad, r.n_pad, slice_rows, S, B, so.b.get());
         CS_LAUNCH("slice rows operand");
     }
     const CUtensorMap tb = make_map_u8(so.b.get(), (uint64_t)r.n_pad, (uint64_t)p.b_rows(true),
@@ -1271,8 +1282,9 @@ void run_samples(SliceOperator& so, MixedRows& r, const SliceCall& c, const Slic
     const int64_t k_pad = (int64_t)p.n_ctiles * p.w;
     {
         prof::Scope ps("slice_prep_samples_operand", s, 0.0, 8.0 * R * k + 14.0 * k_pad * r.r_pad);
-        k_slice_samples_operand<<<dim3((unsigned)((r.r_pad + 2047) / 2048), (unsigned)k_pad), 128, 0, s>>>(
-            so.W.get(), R, k, r.r_pad, p.kbs * kKBlock, r.mu.get(), S, p.blayout(false), so.b.get());
+        launch_chained(k_slice_samples_operand, dim3((unsigned)((r.r_pad + 2047) / 2048), (unsigned)k_pad),
+                       128, 0, s, so.W.get(), R, k, r.r_pad, p.kbs * kKBlock, r.mu.get(), S, p.blayout(false),
+                       so.b.get());
         CS_LAUNCH("slice samples operand");
     }
     const CUtensorMap tb = make_map_u8(so.b.get(), (uint64_t)r.r_pad, (uint64_t)p.b_rows(false),
@@ -1292,8 +1304,9 @@ void run_samples(SliceOperator& so, MixedRows& r, const SliceCall& c, const Slic
         CS_LAUNCH("kinship_samples_slices");
     }
     prof::Scope ps("slice_reduce_samples", s, 0.0, 8.0 * (p.splits + 1) * (double)k * n);
-    k_slice_reduce_samples<<<dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)), 256, 0, s>>>(
-        so.part.get(), r.n_pad, n, k, so.W.get(), R, r.mu.get(), PackedRows{r.rows, r.stride}, S, scale, Y);
+    launch_chained(k_slice_reduce_samples, dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)), 256, 0,
+                   s, so.part.get(), r.n_pad, n, k, so.W.get(), R, r.mu.get(), PackedRows{r.rows, r.stride}, S,
+                   scale, Y);
     CS_LAUNCH("slice_reduce_samples");
 }
 
@@ -1301,9 +1314,9 @@ void run_samples(SliceOperator& so, MixedRows& r, const SliceCall& c, const Slic
 void finish_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSums& S, StridedIn X,
                  double* Wt, const int32_t* pos, StridedOut out, cudaStream_t s) {
     prof::Scope ps("slice_reduce_rows", s, 0.0, 8.0 * (c.rows.splits + 1) * (double)c.k * r.R);
-    k_slice_reduce_rows<<<dim3((unsigned)((r.R + 1023) / 1024), (unsigned)c.k), 256, 0, s>>>(
-        so.part.get(), r.r_pad, r.R, c.k, r.s.get(), r.mu.get(), PackedRows{r.rows, r.stride}, X, r.n, S,
-        Wt, pos, out);
+    launch_chained(k_slice_reduce_rows, dim3((unsigned)((r.R + 1023) / 1024), (unsigned)c.k), 256, 0, s,
+                   so.part.get(), r.r_pad, r.R, c.k, r.s.get(), r.mu.get(), PackedRows{r.rows, r.stride}, X,
+                   r.n, S, Wt, pos, out);
     CS_LAUNCH("slice_reduce_rows");
 }
 
@@ -1388,8 +1401,8 @@ bool multiply_z_slices(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cud
         CS_CUDA(cudaMemsetAsync(so->words.get(), 0, 8 * c.words, s));
         {
             prof::Scope ps("slice_gather", s, 0.0, 16.0 * r.R * c.k);
-            k_slice_gather<<<dim3((unsigned)((r.R + 1023) / 1024), (unsigned)c.k), 256, 0, s>>>(
-                from_column(V, c0), r.R, op->d_view_pos.get(), r.s.get(), r.mu.get(), S, so->W.get());
+            launch_chained(k_slice_gather, dim3((unsigned)((r.R + 1023) / 1024), (unsigned)c.k), 256, 0, s,
+                           from_column(V, c0), r.R, op->d_view_pos.get(), r.s.get(), r.mu.get(), S, so->W.get());
             CS_LAUNCH("slice_gather");
         }
         run_samples(*so, r, c, S, 1.0, from_column(Y, c0), s);

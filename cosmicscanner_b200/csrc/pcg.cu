@@ -14,6 +14,7 @@
 #include <cmath>
 #include <utility>
 
+#include "chain.cuh"
 #include "vce_internal.h"
 
 namespace cs {
@@ -67,6 +68,7 @@ template <int NV, int Batch, class Elem, class Finish>
 __global__ void __launch_bounds__(256)
 k_column_reduce(int64_t n, int64_t k, int64_t chunk, int64_t nb, int kc, double* __restrict__ part,
                 unsigned* __restrict__ counter, const Elem elem, const Finish finish) {
+    chain_enter();
     constexpr int kScratch = NV <= 2 ? NV * 32 * 33 : NV * 256;
     __shared__ double sh[kScratch];  // lanes' sums [NV][256], then the finish
     __shared__ int last;
@@ -156,9 +158,9 @@ void column_reduce(int64_t n, int64_t k, const Elem& elem, const Finish& finish,
     int kc = 1;
     while (kc < k && kc < 32) kc *= 2;
     const int64_t nb = chunk_count(n), chunks = 32 / kc;
-    k_column_reduce<NV, Batch, Elem, Finish>
-        <<<dim3((unsigned)((nb + chunks - 1) / chunks), (unsigned)((k + kc - 1) / kc)), 256, 0, s>>>(
-            n, k, chunk_rows(n), nb, kc, ws.partial.get(), ws.counter.get(), elem, finish);
+    launch_chained(k_column_reduce<NV, Batch, Elem, Finish>,
+                   dim3((unsigned)((nb + chunks - 1) / chunks), (unsigned)((k + kc - 1) / kc)), 256, 0, s, n,
+                   k, chunk_rows(n), nb, kc, ws.partial.get(), ws.counter.get(), elem, finish);
     CS_LAUNCH("column_reduce");
 }
 
@@ -353,6 +355,7 @@ struct LanczosGroup {
 // p = z + beta p
 __global__ void k_direction_z(double* __restrict__ P, const double* __restrict__ Z, int64_t ld,
                               int64_t n, int64_t k, const double* __restrict__ beta) {
+    chain_enter();
     const int64_t total = n * k;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {
@@ -364,6 +367,7 @@ __global__ void k_direction_z(double* __restrict__ P, const double* __restrict__
 // p = r / diag + beta p
 __global__ void k_direction(double* __restrict__ P, const double* __restrict__ R, int64_t ld,
                             int64_t n, int64_t k, double diag, const double* __restrict__ beta) {
+    chain_enter();
     const int64_t total = n * k;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {
@@ -400,6 +404,7 @@ __global__ void k_records_to_rows(const double* __restrict__ V, int64_t ldv, int
 
 __global__ void k_combine(double* __restrict__ out, int64_t ldo, const Covariance cov, int64_t n_rec,
                           int64_t k) {
+    chain_enter();
     const int64_t total = n_rec * k;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {
@@ -517,7 +522,7 @@ void VOperator::apply(const double* in, int64_t ldi, int64_t k, double* out, int
     const double* U = kinship(in, ldi, k, ldu, s);
     const Covariance cov = covariance(in, ldi, U, ldu, k);
     prof::Scope ps("covariance_combine", s, 0.0, 8.0 * 3.0 * (double)rm->n_rec * k);
-    k_combine<<<grid_for(rm->n_rec * k), 256, 0, s>>>(out, ldo, cov, rm->n_rec, k);
+    launch_chained(k_combine, grid_for(rm->n_rec * k), 256, 0, s, out, ldo, cov, rm->n_rec, k);
     CS_LAUNCH("covariance_combine");
 }
 
@@ -733,11 +738,11 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
         {
             prof::Scope ps("cg_direction", s, 2.0 * n * ka, 24.0 * n * ka);
             if (M)
-                k_direction_z<<<grid_for(n * ka), 256, 0, s>>>(ws.P.get(), ws.Zp.get(), ka, n, ka,
-                                                               ws.beta.get());
+                launch_chained(k_direction_z, grid_for(n * ka), 256, 0, s, ws.P.get(), ws.Zp.get(), ka, n, ka,
+                               ws.beta.get());
             else
-                k_direction<<<grid_for(n * ka), 256, 0, s>>>(ws.P.get(), ws.R.get(), ka, n, ka,
-                                                             diag, ws.beta.get());
+                launch_chained(k_direction, grid_for(n * ka), 256, 0, s, ws.P.get(), ws.R.get(), ka, n, ka,
+                               diag, ws.beta.get());
             CS_LAUNCH("cg_direction");
         }
         CS_CUDA(cudaStreamSynchronize(s));

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "linalg_host.h"
+#include "chain.cuh"
 #include "vce_internal.h"
 
 struct cs_vce {
@@ -59,6 +60,7 @@ __global__ void k_copy_cols(const double* __restrict__ src, int64_t lds, int64_t
 // Vn[:, c] = W[:, c] * inv[c]
 __global__ void k_scale_cols(double* __restrict__ Vn, const double* __restrict__ Wm, int64_t ld,
                              int64_t n, int64_t k, const double* __restrict__ inv, int divide) {
+    chain_enter();
     const int64_t total = n * k;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {
@@ -205,7 +207,7 @@ static double slq_logdet(cs_vce* v, int probes, int steps, uint64_t seed, cudaSt
     DeviceBuffer<double> dcoef;
     dcoef.resize(kLanczosCoef * k);
     CS_CUDA(cudaMemcpyAsync(dcoef.get(), inv.data(), 8 * k, cudaMemcpyHostToDevice, s));
-    k_scale_cols<<<grid_1d(n * k), 256, 0, s>>>(Vj(0), v->lw.get(), k, n, k, dcoef.get(), 0);
+    launch_chained(k_scale_cols, grid_1d(n * k), 256, 0, s, Vj(0), v->lw.get(), k, n, k, dcoef.get(), 0);
     CS_LAUNCH("scale_cols");
     // the recurrences stay on the device: alpha and beta by step (m x k), the coefficients of the
     // axpy that follows, and which columns have broken down after how many steps
@@ -223,7 +225,7 @@ static double slq_logdet(cs_vce* v, int probes, int steps, uint64_t seed, cudaSt
                               d_done.get(), d_done.get() + k};
         double* w = v->lw.get();
         lanczos_step(v->V, v->lz.get(), k, w, st, j, v->pw, s);
-        k_scale_cols<<<grid_1d(n * k), 256, 0, s>>>(Vj(j + 1), w, k, n, k, dcoef.get(), 1);
+        launch_chained(k_scale_cols, grid_1d(n * k), 256, 0, s, Vj(j + 1), w, k, n, k, dcoef.get(), 1);
         CS_LAUNCH("scale_cols");
     }
     std::vector<double> ab(2 * (int64_t)m * k);
