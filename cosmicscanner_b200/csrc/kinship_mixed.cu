@@ -824,17 +824,19 @@ __device__ __forceinline__ void sum_tiles(const double* __restrict__ part, int64
 }
 
 // Per-column sums over tiles of 64 rows (8 interleaved lanes each, added in lane order) and minima
-// and maxima over chunks of 512, then, in the last block of a column tile, mean[c] = (sum over
+// and maxima over chunks of two tiles, then, in the last block of a column tile, mean[c] = (sum over
 // tiles) / n and max1[c] = the bits of max |x - mean| = max(max x - mean, mean - min x) (rounding is
 // monotonic, so this equals the maximum of the rounded differences); the column's maxima of W are
 // cleared.  A block covers kc columns (a power of two up to 32) x 32 / kc chunks.
-constexpr int kStatTile = 64, kStatRows = 8 * kStatTile;
+constexpr int kStatTile = 64, kStatTiles = 2, kStatRows = kStatTiles * kStatTile;
 template <class T>
 __global__ void __launch_bounds__(256)
 k_col_stats(const Strided<const T> X, int64_t n, int64_t k, int kc, int64_t nb,
             double* __restrict__ part, const MixedColumns C) {
     chain_enter();
-    __shared__ double red[10][32 * 9];  // eight tiles' sums, minima, maxima; 8 lanes and a pad per (column, chunk)
+    // the tiles' sums, minima, maxima; 8 lanes and a pad per (column, chunk); then the last block's sums
+    __shared__ double red[6][32 * 9];
+    static_assert(kStatTiles + 2 <= 6 && 6 * 32 * 9 >= 32 * 33 + 2 * 256);
     // threads in the order of memory: columns fastest in row-major input, lanes in column-major
     const int per = 256 / kc;  // 8 lanes x chunks
     const int tc = X.rs == 1 ? threadIdx.x / per : threadIdx.x % kc;
@@ -845,8 +847,8 @@ k_col_stats(const Strided<const T> X, int64_t n, int64_t k, int kc, int64_t nb,
     const int64_t nt = (n + kStatTile - 1) / kStatTile;
     const int slot = (tc * (per >> 3) + ch) * 9 + lane;
     double mn = INFINITY, mx = -INFINITY;
-#pragma unroll 4
-    for (int j = 0; j < 8; ++j) {
+#pragma unroll
+    for (int j = 0; j < kStatTiles; ++j) {
         double sm = 0.0;
         if (c < k && b < nb) {
             const int64_t r0 = b * kStatRows + j * kStatTile + lane;
@@ -861,23 +863,23 @@ k_col_stats(const Strided<const T> X, int64_t n, int64_t k, int kc, int64_t nb,
         }
         red[j][slot] = sm;
     }
-    red[8][slot] = mn;
-    red[9][slot] = mx;
+    red[kStatTiles][slot] = mn;
+    red[kStatTiles + 1][slot] = mx;
     __syncthreads();
-    {   // one thread per (column, chunk) and tile
+    if (threadIdx.x < 32 * kStatTiles) {  // one thread per (column, chunk) and tile
         const int pair = threadIdx.x & 31, j = threadIdx.x >> 5;
         const int oc = pair / (per >> 3), och = pair % (per >> 3);
         const int64_t cc = (int64_t)blockIdx.y * kc + oc, bb = (int64_t)blockIdx.x * (per >> 3) + och;
         if (cc < k && bb < nb) {
             double sm = red[j][9 * pair];
             for (int q = 1; q < 8; ++q) sm += red[j][9 * pair + q];
-            if (8 * bb + j < nt) part[(8 * bb + j) * k + cc] = sm;
+            if (kStatTiles * bb + j < nt) part[(kStatTiles * bb + j) * k + cc] = sm;
             if (j == 0) {
                 mn = INFINITY;
                 mx = -INFINITY;
                 for (int q = 0; q < 8; ++q) {
-                    mn = fmin(mn, red[8][9 * pair + q]);
-                    mx = fmax(mx, red[9][9 * pair + q]);
+                    mn = fmin(mn, red[kStatTiles][9 * pair + q]);
+                    mx = fmax(mx, red[kStatTiles + 1][9 * pair + q]);
                 }
                 part[(nt + bb) * k + cc] = mn;
                 part[(nt + nb + bb) * k + cc] = mx;
@@ -940,6 +942,133 @@ __device__ __forceinline__ void put_byte(uint32_t (&w)[4], int p, int q) {
     w[p >> 2] = __byte_perm(w[p >> 2], (uint32_t)q, 0x3210 ^ (((p & 3) ^ 4) << (4 * (p & 3))));
 }
 
+// Rows 16 g .. 16 g + 15 of a tile of 64 (`rows` of them live, g = grp % 4 the thread's place among
+// the tile's four, which are neighbours in a warp): the pieces' bytes at their K positions, and the
+// sum over the tile of the represented values in the order rows i and i + 32, then + 16, + 8, + 4,
+// + 2, + 1; each thread keeps a quarter of the pairs (j = 4 m + 2 lo + hi) as the values come.
+__device__ __forceinline__ double split16(const double* x, int rows, double mean, double f, int grp,
+                                          uint32_t (&w1)[4], uint32_t (&w2)[4], uint32_t (&w3)[4]) {
+    const bool hi = grp & 2, lo = grp & 1;
+    double val[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        double v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int j = 4 * m + q;
+            double a, b, d;
+            int q1, q2, q3;
+            quantise3(j < rows ? __dmul_rn(x[j] - mean, f) : 0.0, a, b, d, q1, q2, q3);
+            put_byte(w1, position_of(j), q1);
+            put_byte(w2, position_of(j), q2);
+            put_byte(w3, position_of(j), q3);
+            v[q] = a + small_quotient<254>(b) + small_quotient<64516>(d);
+        }
+        const double x0 = (hi ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[1], 2);
+        const double x1 = (hi ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, hi ? v[2] : v[3], 2);
+        val[m] = (lo ? x1 : x0) + __shfl_xor_sync(0xffffffffu, lo ? x0 : x1, 1);
+    }
+    double sum = (val[0] + val[2]) + (val[1] + val[3]);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    return sum;
+}
+
+// Both of the above for n <= kWholeRows: a block per column holds it in shared memory, and a thread
+// quantises 16 rows.  The same sums in the same order as k_col_stats and k_split_rows_operand, without
+// a second kernel, the counters and the reading of the partial sums, which is what those two spend 22 us
+// on at n=2000 and 34 columns: an AI-REML of 453 such products takes 45.5 ms with it and 48.8 without
+// (of which the shorter chains of k_col_stats, k_reduce_samples and the solver's sums are a part).
+constexpr int kWholeRows = 8192;
+template <class T>
+__global__ void __launch_bounds__(kWholeRows / 16)
+k_rows_operand_whole(const Strided<const T> X, int64_t n, int64_t k, int64_t kp, int64_t n_pad,
+                     const MixedColumns C, int8_t* __restrict__ B) {
+    chain_enter();
+    extern __shared__ double col[];  // [n_pad], one pad every 16
+    __shared__ double sums[kWholeRows / 64], lo[16], hi[16], stat[2];
+    const int64_t c = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int rows = (int)n, nt = (rows + 63) / 64;
+    const bool live = c < k;
+    double mn = INFINITY, mx = -INFINITY;
+#pragma unroll 4
+    for (int r = threadIdx.x; r < (int)n_pad; r += blockDim.x) {
+        double v = 0.0;
+        if (live && r < rows) {
+            v = (double)X.p[r * X.rs + c * X.cs];
+            mn = fmin(mn, v);
+            mx = fmax(mx, v);
+        }
+        col[r + (r >> 4)] = v;
+    }
+    for (int off = 16; off; off >>= 1) {
+        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    }
+    if (lane == 0) {
+        lo[warp] = mn;
+        hi[warp] = mx;
+    }
+    __syncthreads();
+    // tiles of 64 rows, eight interleaved lanes added in lane order
+    for (int t = threadIdx.x >> 3; t < (int)n_pad / 64; t += blockDim.x >> 3) {
+        double sm = 0.0;
+#pragma unroll
+        for (int q = 0; q < 64; q += 8) {
+            const int r = 64 * t + q + (threadIdx.x & 7);
+            if (r < rows) sm += col[r + (r >> 4)];
+        }
+        double tot = __shfl_sync(0xffffffffu, sm, lane & 24);
+#pragma unroll
+        for (int j = 1; j < 8; ++j) tot += __shfl_sync(0xffffffffu, sm, (lane & 24) + j);
+        if ((threadIdx.x & 7) == 0) sums[t] = tot;
+    }
+    __syncthreads();
+    auto column_sum = [&]() {  // by one warp, as sum_tiles adds
+        double sm = 0.0;
+        for (int t = lane; t < nt; t += 32) sm += sums[t];
+        for (int off = 16; off; off >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, off);
+        return sm;
+    };
+    if (warp == 0) {
+        const double m = column_sum() / (double)n;
+        double a = lane < warps ? lo[lane & 15] : INFINITY, b = lane < warps ? hi[lane & 15] : -INFINITY;
+        for (int off = 16; off; off >>= 1) {
+            a = fmin(a, __shfl_xor_sync(0xffffffffu, a, off));
+            b = fmax(b, __shfl_xor_sync(0xffffffffu, b, off));
+        }
+        if (lane == 0) {
+            stat[0] = m;
+            stat[1] = fmax(fmax(b - m, m - a), 0.0);
+        }
+    }
+    __syncthreads();
+    const double mean = stat[0];
+    const unsigned long long max1 = (unsigned long long)__double_as_longlong(stat[1]);
+    const int i0 = 16 * threadIdx.x;  // blockDim.x * 16 == n_pad rounded up to 512
+    uint32_t w1[4] = {}, w2[4] = {}, w3[4] = {};
+    const double sum = split16(col + 17 * threadIdx.x, live && i0 < rows ? min(16, rows - i0) : 0, mean,
+                               live ? quant_factor(max1) : 0.0, threadIdx.x, w1, w2, w3);
+    if (i0 < (int)n_pad) {
+        *reinterpret_cast<uint4*>(B + c * n_pad + i0) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+        *reinterpret_cast<uint4*>(B + (kp + c) * n_pad + i0) = make_uint4(w2[0], w2[1], w2[2], w2[3]);
+        *reinterpret_cast<uint4*>(B + (2 * kp + c) * n_pad + i0) = make_uint4(w3[0], w3[1], w3[2], w3[3]);
+        if ((threadIdx.x & 3) == 0) sums[threadIdx.x >> 2] = sum;
+    }
+    __syncthreads();
+    if (warp == 0 && live) {
+        const double q = column_sum();
+        if (lane == 0) {
+            C.mean[c] = mean;
+            C.max1[c] = max1;
+            C.qsum[c] = q;
+            C.max_w[c] = 0;
+            C.max_wmu[c] = 0;
+        }
+    }
+}
+
 // Rows-pass operand: B1[q*kp + c][pos(i)] (int8 pieces of (x_ic - mean_c) 127 / max_c, i < n_pad;
 // pos interleaves each group of 16 samples as the decoded tiles do) and the sums Q_c of the
 // represented values: in tiles of 64 rows (rows i and i + 32, then the 32 pairs in a tree), the
@@ -965,41 +1094,16 @@ k_split_rows_operand(const Strided<const T> X, int64_t n, int64_t k, int64_t kp,
     __syncthreads();
     const int grp = threadIdx.x % (ROWS / 16), cc = threadIdx.x / (ROWS / 16);
     const int64_t c = c0 + cc, i0 = r0 + 16 * grp;
-    // rows 16 g + j of a tile, g = the thread's place among its four: + 32 and + 16 as the values come,
-    // each thread keeping a quarter (j = 4 m + 2 lo + hi), then + 8, + 4, + 2, + 1
-    const bool hi = grp & 2, lo = grp & 1;
     const double f = c < k ? quant_factor(C.max1[c]) : 0.0;
     const double mc = c < k ? C.mean[c] : 0.0;
-    const double* const mine = tile + cc * kPitch + 17 * grp;
-    const int rows = c < k ? (int)min((int64_t)16, n - i0) : 0;  // may be negative
-    uint32_t w1[4] = {}, w2[4] = {}, w3[4] = {};  // the 16 bytes of each piece at their K positions
-    double val[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        double v[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = 4 * m + q;
-            double a, b, d;
-            int q1, q2, q3;
-            quantise3(j < rows ? __dmul_rn(mine[j] - mc, f) : 0.0, a, b, d, q1, q2, q3);
-            put_byte(w1, position_of(j), q1);
-            put_byte(w2, position_of(j), q2);
-            put_byte(w3, position_of(j), q3);
-            v[q] = a + small_quotient<254>(b) + small_quotient<64516>(d);
-        }
-        const double x0 = (hi ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[1], 2);
-        const double x1 = (hi ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, hi ? v[2] : v[3], 2);
-        val[m] = (lo ? x1 : x0) + __shfl_xor_sync(0xffffffffu, lo ? x0 : x1, 1);
-    }
+    uint32_t w1[4] = {}, w2[4] = {}, w3[4] = {};
+    const double sum = split16(tile + cc * kPitch + 17 * grp, c < k ? (int)min((int64_t)16, n - i0) : 0, mc, f, grp,
+                               w1, w2, w3);
     if (c < kp && i0 < n_pad) {
         *reinterpret_cast<uint4*>(B + c * n_pad + i0) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
         *reinterpret_cast<uint4*>(B + (kp + c) * n_pad + i0) = make_uint4(w2[0], w2[1], w2[2], w2[3]);
         *reinterpret_cast<uint4*>(B + (2 * kp + c) * n_pad + i0) = make_uint4(w3[0], w3[1], w3[2], w3[3]);
     }
-    double sum = (val[0] + val[2]) + (val[1] + val[3]);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     const int64_t nt = (n + 63) / 64;
     if ((grp & 3) == 0 && c < k && i0 < n) part[(i0 >> 6) * k + c] = sum;
     if (c0 >= k || !last_block(C.counter + blockIdx.y, gridDim.x)) return;
@@ -1035,6 +1139,7 @@ k_reduce_rows(const double* __restrict__ part, int splits, int64_t kp, int64_t l
     double mw = 0.0, mm = 0.0;
     const int64_t t0 = (int64_t)blockIdx.x * 1024 + threadIdx.x;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
     for (int z = 0; z < splits; ++z) {
         const double* p = part + ((int64_t)z * kp + c) * ld + t0;  // ld >= R rounded up to 256
 #pragma unroll
@@ -1284,15 +1389,22 @@ k_reduce_samples(const double* __restrict__ part, int splits, int64_t kp, int64_
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t i0 = (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
     const int64_t i = i0 + tx;
+    // four columns a thread, slices in order, four slices' loads at a time
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    const double* p = part + (c0 + ty) * ld + i;  // i < n <= ld
+#pragma unroll 4
+    for (int z = 0; z < splits; ++z, p += kp * ld) {
 #pragma unroll
-    for (int cc = ty; cc < 32; cc += 8) {
-        const int64_t c = c0 + cc;
+        for (int j = 0; j < 4; ++j)
+            if (c0 + ty + 8 * j < k && i < n) acc[j] += p[8 * j * ld];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int64_t c = c0 + ty + 8 * j;
         if (c >= k || i >= n) continue;
-        double acc = 0.0;
-        for (int z = 0; z < splits; ++z) acc += part[((int64_t)z * kp + c) * ld + i];
-        const double v = (acc - c0v[c]) * inv_m;
+        const double v = (acc[j] - c0v[c]) * inv_m;
         if (Y.rs == 1) Y.p[i + c * Y.cs] = (T)v;
-        else tile[cc][tx] = v;
+        else tile[ty + 8 * j][tx] = v;
     }
     if (Y.rs == 1) return;
     __syncthreads();
@@ -1503,6 +1615,11 @@ void configure_kernels() {
     static PerDeviceOnce configured;
     once_per_device(configured, [] {
         cudaError_t err = allow_smem<true, false>();
+        constexpr int kWholeBytes = 8 * (kWholeRows + kWholeRows / 16 + 16);
+        if (err == cudaSuccess)
+            err = cudaFuncSetAttribute(k_rows_operand_whole<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeBytes);
+        if (err == cudaSuccess)
+            err = cudaFuncSetAttribute(k_rows_operand_whole<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeBytes);
         if (err == cudaSuccess) err = allow_smem<false, false>();
         if (err == cudaSuccess) err = allow_smem<true, true>();
         if (err == cudaSuccess) err = allow_smem<false, true>();
@@ -1917,19 +2034,25 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, Stri
     }
     {
         prof::Scope ps("mixed_prep_rows_operand", s, 0.0, 24.0 * n * k + 3.0 * kp * n_pad);
-        int kc = 1;
-        while (X.rs != 1 && kc < k && kc < 32) kc *= 2;
-        const int64_t per = 32 / kc;  // chunks per block
-        launch_chained(k_col_stats<T>, dim3((unsigned)((nst + per - 1) / per), (unsigned)((k + kc - 1) / kc)),
-                       256, 0, s, X, n, k, kc, nst, ws.colpart.get(), C);
-        if (kp <= 16)
-            launch_chained(k_split_rows_operand<T, 4, 512>,
-                           dim3((unsigned)((n_pad + 511) / 512), (unsigned)((kp + 3) / 4)), 128, 0, s, X, n, k,
-                           kp, n_pad, C, ws.b1.get(), ws.colpart.get());
-        else
-            launch_chained(k_split_rows_operand<T, 16, 256>,
-                           dim3((unsigned)(n_pad / 256), (unsigned)((kp + 15) / 16)), 256, 0, s, X, n, k, kp,
-                           n_pad, C, ws.b1.get(), ws.colpart.get());
+        if (n <= kWholeRows) {
+            const unsigned threads = (unsigned)round_up(n_pad / 16, 32);
+            launch_chained(k_rows_operand_whole<T>, (unsigned)kp, threads, 8 * (n_pad + n_pad / 16 + 16), s, X, n,
+                           k, kp, n_pad, C, ws.b1.get());
+        } else {
+            int kc = 1;
+            while (X.rs != 1 && kc < k && kc < 32) kc *= 2;
+            const int64_t per = 32 / kc;  // chunks per block
+            launch_chained(k_col_stats<T>, dim3((unsigned)((nst + per - 1) / per), (unsigned)((k + kc - 1) / kc)),
+                           256, 0, s, X, n, k, kc, nst, ws.colpart.get(), C);
+            if (kp <= 16)
+                launch_chained(k_split_rows_operand<T, 4, 512>,
+                               dim3((unsigned)((n_pad + 511) / 512), (unsigned)((kp + 3) / 4)), 128, 0, s, X, n, k,
+                               kp, n_pad, C, ws.b1.get(), ws.colpart.get());
+            else
+                launch_chained(k_split_rows_operand<T, 16, 256>,
+                               dim3((unsigned)(n_pad / 256), (unsigned)((kp + 15) / 16)), 256, 0, s, X, n, k, kp,
+                               n_pad, C, ws.b1.get(), ws.colpart.get());
+        }
         CS_LAUNCH("mixed rows operand");
     }
     PassArgs P{};

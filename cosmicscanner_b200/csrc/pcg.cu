@@ -55,7 +55,7 @@ namespace {
 // before it uses them, and the last block reads the partials in the order of memory, several at
 // once.  CG's update (n=20000, 34 columns) takes 23 us, 31 with one row at a time and a warp to a
 // column; n=2000 9.3 us against 12.5.
-constexpr int kChunkRows = 64, kMaxChunks = 512;
+constexpr int kChunkRows = 16, kMaxChunks = 512;
 int64_t chunk_rows(int64_t n) {
     return kChunkRows * std::max<int64_t>(1, (n + (int64_t)kChunkRows * kMaxChunks - 1) /
                                                  ((int64_t)kChunkRows * kMaxChunks));
