@@ -1804,8 +1804,8 @@ void check_status(MixedWorkspace& ws, cudaStream_t s) {
 // ---------------------------------------------------------------- pass plans and the autotuner
 // A pass runs with a plan: CTA pairs or single CTAs, the layout (A in shared memory or in TMEM),
 // the column-tile width cap and the number of K slices.  The default plan is the heuristic: up
-// to 32 right-hand sides the narrow single-CTA layout with A in TMEM, 33 to 64 its 64-wide
-// form, above that CTA pairs with A in TMEM (tiles of at most 64); slices so that about 8
+// to 32 right-hand sides the four-K-block kernel (mixed_narrow_pass) or, in short slices, the narrow
+// single-CTA layout with A in TMEM, 33 to 64 its 64-wide form, above that CTA pairs with A in TMEM (tiles of at most 64); slices so that about 8
 // units per CTA cover the GPU.  The autotuner times the layout x width candidates of a shape
 // once (shapes bucketed: rows and samples by factors of 1.25, columns to multiples of 16) and
 // keeps the fastest.  It never changes the slice count (the order of the slice sums) nor, in
@@ -1815,7 +1815,8 @@ struct PassPlan {
     bool pairs = false;
     bool narrow = false;  // single-CTA layout for column tiles of at most 32
     int tmem_a = 0;       // A operand in TMEM: 1 / 2 single CTA (tiles <= 32 / 64), 3 / 4 CTA
-                          // pairs (rows / samples, tiles <= 64), 5 the five-set samples pairs
+                          // pairs (rows / samples, tiles <= 64), 5 the five-set samples pairs,
+                          // 6 mixed_narrow_pass
     int max_w = 0;
     int splits = 1;
     bool same_kernel(const PassPlan& o) const {
@@ -1824,8 +1825,28 @@ struct PassPlan {
 };
 
 // the samples-pass form of a plan: six operand sets over the sample-major copy with the fixed
-// dosage table (TMEMA 1, 2, 4), five otherwise
-bool six_set_samples(const PassPlan& p) { return p.tmem_a == 1 || p.tmem_a == 2 || p.tmem_a == 4; }
+// dosage table (TMEMA 1, 2, 4, and 6), five otherwise
+bool six_set_samples(const PassPlan& p) {
+    return p.tmem_a == 1 || p.tmem_a == 2 || p.tmem_a == 4 || p.tmem_a == 6;
+}
+
+Tiling plan_tiling(const PassPlan& p, int64_t k) {
+    if (p.tmem_a != 6) return tiling_for(k, p.max_w);
+    const int w = (int)round_up(k, 8);
+    return Tiling{1, w, w, w};
+}
+
+// Whether mixed_narrow_pass takes k columns in slices of kbs K-blocks.  Up to 24 columns it is the
+// faster one at every slice length measured (us a pass, rows / samples, with it and with the 32-wide
+// form: 2,000 x 10,000, k = 1 12.7 / 12.8 and 14.7 / 14.8; 10,000 x 20,000, k = 24 41.4 / 41.8 and
+// 49.6 / 53.5; 40,000 x 40,000, k = 1 169 / 170 and 239 / 248, k = 24 187 / 190 and 278 / 300); with 25 to 32
+// there is room for one accumulator only, which short slices (10 K-blocks: no difference) wait for,
+// long ones do not (40,000 x 40,000, k = 30 212 / 205 and 279 / 300).  33 to 48 are left to the tuner (34 at
+// N=50k, M=100k: a product of 1.60 ms against 1.71).
+bool narrow_pass(bool rows, int64_t k, int kb, int splits) {
+    const int kbs = (kb + splits - 1) / splits;
+    return mixed_narrow_fits(rows, round_up(k, 8)) && kbs >= (k <= 24 ? 2 : 16);
+}
 
 PassPlan default_plan(bool rows, int64_t tiles, int kb, int64_t k) {
     PassPlan p;
@@ -1847,6 +1868,7 @@ PassPlan default_plan(bool rows, int64_t tiles, int kb, int64_t k) {
     const Tiling tl = tiling_for(k, p.max_w);
     p.splits = p.pairs ? choose_splits(tiles / 2 * tl.n_ctiles, kb, 4LL * num_sms())
                        : choose_splits(tiles * tl.n_ctiles, kb, 8LL * num_sms());
+    if (p.tmem_a == 1 && narrow_pass(rows, k, kb, p.splits)) p.tmem_a = 6;
     return p;
 }
 
@@ -1917,6 +1939,14 @@ PassPlan choose_plan(bool rows, bool allow, int64_t R, int64_t n, int64_t k, int
             p.splits = def.splits;
             cands.push_back(p);
         }
+    if (mode != 2 && narrow_layouts() && tmem_a_default() && narrow_pass(rows, k, kb, def.splits)) {
+        PassPlan p;
+        p.narrow = true;
+        p.tmem_a = 6;
+        p.max_w = k <= kNarrowRowsW ? kNarrowRowsW : kTmemA64W;
+        p.splits = def.splits;
+        cands.push_back(p);
+    }
     if (mode != 2 && narrow_layouts() && tmem_a_default() && k > kNarrowRowsW)
         for (int w = 48; w <= kTmemA64W; w += 16) {
             PassPlan p;
@@ -2007,7 +2037,7 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, Stri
                     int64_t k, double* Wt, const int32_t* pos, StridedOut out, cudaStream_t s) {
     const int64_t tiles = r.r_pad / kTile;
     const bool pairs = plan.pairs;
-    const Tiling tl = tiling_for(k, plan.max_w);
+    const Tiling tl = plan_tiling(plan, k);
     const int64_t n = r.n, R = r.R, n_pad = r.n_pad, r_pad = r.r_pad, kp = tl.kp;
     const int kb = (int)(n_pad / kKBlock);
     const int kbs = (kb + plan.splits - 1) / plan.splits;
@@ -2076,7 +2106,10 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, Stri
         // algorithmic work: 2 n R k flops, one pass over the packed rows
         prof::Scope ps("kinship_rows_tc", s, 2.0 * (double)n * (double)R * (double)k,
                        (double)R * (double)((n + 3) / 4));
-        if (pairs && plan.tmem_a == 3)
+        if (plan.tmem_a == 6)
+            mixed_narrow_pass(true, r, ws.b1.get(), kp, splits, kbs, nullptr, ws.part.get(), ws.status.get(),
+                              poll_sleep_ns(), s);
+        else if (pairs && plan.tmem_a == 3)
             launch_pass<true, true, false, 3>(r.tm, ws.tm_b1, ws.tm_b1t, P, s);
         else if (pairs)
             launch_pass<true, true>(r.tm, ws.tm_b1, ws.tm_b1t, P, s);
@@ -2110,7 +2143,7 @@ void samples_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, c
                        int64_t k, double inv_m, Strided<T> Y, cudaStream_t s) {
     const int64_t tiles = r.n_pad / kTile;
     const bool pairs = plan.pairs;
-    const Tiling tl = tiling_for(k, plan.max_w);
+    const Tiling tl = plan_tiling(plan, k);
     const int64_t n = r.n, R = r.R, n_pad = r.n_pad, r_pad = r.r_pad, kp = tl.kp;
     const int kb = (int)(r_pad / kKBlock);
     const int kbs = (kb + plan.splits - 1) / plan.splits;
@@ -2171,7 +2204,10 @@ void samples_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, c
     {
         prof::Scope ps("kinship_samples_tc", s, 2.0 * (double)n * (double)R * (double)k,
                        (double)R * (double)((n + 3) / 4));
-        if (pairs && plan.tmem_a == 5)
+        if (plan.tmem_a == 6)
+            mixed_narrow_pass(false, r, ws.b2.get(), kp, splits, kbs, ws.inv_f.get(), ws.part.get(),
+                              ws.status.get(), poll_sleep_ns(), s);
+        else if (pairs && plan.tmem_a == 5)
             launch_pass<false, true, false, 5>(r.tm_t, ws.tm_b2, ws.tm_b2t, P, s);
         else if (pairs && tmem_a)
             launch_pass<false, true, false, 4>(r.tm_t, ws.tm_b2, ws.tm_b2t, P, s);
@@ -2323,7 +2359,8 @@ std::string autotune_json() {
                       first ? "" : ", ", kv.first.rows ? "rows" : "samples", (long long)e.R,
                       (long long)e.n, (long long)e.k, e.plan.pairs ? "true" : "false",
                       e.plan.narrow ? "true" : "false",
-                      e.plan.tmem_a == 5 ? "\"pair64_five\"" : e.plan.tmem_a >= 3 ? "\"pair64\""
+                      e.plan.tmem_a == 6   ? "\"48\""
+                      : e.plan.tmem_a == 5 ? "\"pair64_five\"" : e.plan.tmem_a >= 3 ? "\"pair64\""
                       : e.plan.tmem_a == 2 ? "64" : e.plan.tmem_a ? "32" : "false",
                       e.plan.max_w,
                       e.plan.splits, e.candidates,

@@ -40,6 +40,11 @@
 // wider tiles are digit-major in widths of 8 per CTA.  TMEM (512 columns) holds the
 // accumulators (rows: main and missing-call sums apart, 13 per column; samples: 7) and the
 // A stages (64 columns each).
+//
+// The mixed form's passes of up to 48 columns run on the same kernel with three digits (mixed_narrow_pass):
+// it decodes a packed tile of four K-blocks at a time where kinship_mixed.cu's kernels take one, which
+// is what bounds few columns.  At N=40k, M=40k, 24 columns a pass takes 187 us (rows) and 190 (samples)
+// instead of 278 and 300.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -87,6 +92,9 @@ struct SliceArgs {
     const uint32_t* lut;    // rows pass: imputed code of each 2-bit code, per SNP row
     const double* mu;       // rows pass: per SNP row
     const longlong2* ksum;  // [n_splits][k]: sum of the fixed-point values (hi, lo) per slice
+    const double* resid;    // mixed rows pass: mu - q / 63 per SNP row
+    const double* inv_f;    // mixed samples pass: per column
+    int set_step;           // global B rows from one set to the next
     double* part;           // [n_splits][k][ld]
     int64_t ld;
     int* status;
@@ -116,7 +124,10 @@ __device__ __forceinline__ double rows_value(const RowCentre& c, int64_t mh, int
     return d + (((m0 - c.ah * sl) - pe) + fma(c.b, x, c.al * (x - (sh + sl))));
 }
 
-template <bool ROWS, bool PAIR, int G>
+// DIGITS = 7: the FP64 form.  DIGITS = 3: the mixed form of kinship_mixed.cu (pieces of base 254,
+// one column tile on single CTAs), with that file's operands, K slices (any number of K-blocks)
+// and epilogue arithmetic, so that the bits are those of its own kernels.
+template <bool ROWS, bool PAIR, int G, int DIGITS>
 __global__ void __launch_bounds__(threads_for(G), 1)
 k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
              const SliceArgs P) {
@@ -225,7 +236,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
 #pragma unroll
                         for (int q = 0; q < kSets; ++q)
                             tma_load_2d(smem_b + d * b_bytes + q * P.set_rows * 128, &tm_b, kb * kKBlock,
-                                        row0 + q * P.set_rows, &full[d]);
+                                        row0 + q * P.set_step, &full[d]);
                         ++loaded;
                         if (++d == SD) { d = 0; ph ^= 1; }
                     }
@@ -350,8 +361,11 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         // Stage of this group's next K-block.  Every unit holds a multiple of four K-blocks and the
         // ring has at least four stages, so that a group is never more than a lap ahead of the
         // MMAs on the stage that it waits for (a parity tells one lap from the next, no more).
+        // (Units of any length, DIGITS = 3: groups take K-blocks in turn across units, j0 counts them,
+        // so that a group's K-blocks are four apart all the same.)
+        static_assert(DIGITS == kDigits || (!PAIR && kOwn == 1));
         int sp = 0, d = grp;
-        uint32_t ph_p = 0, ph_d = 0;
+        uint32_t ph_p = 0, ph_d = 0, j0 = 0;
         bool ok = true;
         for (int u = u0; u < units && ok; u += ustep) {
             int tile, ct, split, kb0, kb1;
@@ -362,10 +376,21 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                 ok = __all_sync(0xffffffffu, mbar_wait_look(&full_p[sp], ph_p, P.status, kTimeoutDecode));
                 if (!ok) break;
                 const unsigned char* src = smem_p + sp * kPackedBytes + r * 128;
+                int mine = grp;
+                if constexpr (DIGITS != kDigits) {
+                    const int here = min(kPackedKb, kb1 - kb);
+                    mine = (int)((uint32_t)grp - j0) & (kPackedKb - 1);
+                    j0 += (uint32_t)here;
+                    if (mine >= here) {  // none of this tile's
+                        if (lane == 0) mbar_arrive(&empty_p[sp]);
+                        if (++sp == SP) { sp = 0; ph_p ^= 1; }
+                        continue;
+                    }
+                }
                 uint32_t words[kOwn][8];
 #pragma unroll
                 for (int o = 0; o < kOwn; ++o) {
-                    const int c = 2 * (grp + o * G);  // 16-byte chunk of the row, 128-byte swizzle
+                    const int c = 2 * (mine + o * G);  // 16-byte chunk of the row, 128-byte swizzle
                     const uint4 p0 = *reinterpret_cast<const uint4*>(src + ((c ^ (r & 7)) << 4));
                     const uint4 p1 = *reinterpret_cast<const uint4*>(src + (((c + 1) ^ (r & 7)) << 4));
                     words[o][0] = p0.x; words[o][1] = p0.y; words[o][2] = p0.z; words[o][3] = p0.w;
@@ -423,7 +448,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
             unit_coords(u, tile, ct, split, kb0, kb1);
             const int64_t row = (int64_t)tile * kTile + 32 * q + lane;
             RowCentre rc{0.0, 0.0, 0.0};
-            if (ROWS) {
+            if (ROWS && DIGITS == kDigits) {
                 const double m = P.mu[row];
                 rc.ah = (double)kTcQ * m;
                 rc.al = fma((double)kTcQ, m, -rc.ah);
@@ -436,6 +461,29 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
             const int c_base = ct * P.w;
             const int cols = min(P.w, P.k - c_base);
             double* dst = P.part + ((int64_t)split * P.k + c_base) * P.ld + row;
+            if constexpr (DIGITS == 3) {
+                const double ib = 1.0 / 254.0, ib2 = 1.0 / (254.0 * 254.0), inv_q = 1.0 / (double)kTcQ;
+                const double rt = ROWS ? P.resid[row] : 0.0;
+                for (int c0 = 0; c0 < P.w; c0 += 8) {
+                    int32_t m1[8], m2[8], m3[8];
+                    double v[8];
+                    tmem_ld8i(tb + c0, m1);
+                    tmem_ld8i(tb + P.w + c0, m2);
+                    tmem_ld8i(tb + 2 * P.w + c0, m3);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        v[i] = fma((double)m3[i], ib2, fma((double)m2[i], ib, (double)m1[i]));
+                    if (ROWS) {
+                        tmem_ld8i(tb + P.nm + c0, m1);
+                        tmem_ld8i(tb + P.nm + P.w + c0, m2);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        dst[(int64_t)(c0 + i) * P.ld] =
+                            ROWS ? fma(v[i], inv_q, __dmul_rn(rt, fma((double)m2[i], ib, (double)m1[i])))
+                                 : __dmul_rn(v[i], P.inv_f[c0 + i]);
+                }
+            }
             const longlong2* ks = P.ksum + (int64_t)split * P.k + c_base;
             auto emit = [&](int c, int64_t mh, int64_t ml, int64_t xh, int64_t xl) {
                 const longlong2 sum = ks[c];
@@ -446,7 +494,9 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                     v = fma((double)(mh - sum.x), 4294967296.0, (double)(ml - sum.y));
                 dst[(int64_t)c * P.ld] = v;
             };
-            if (P.cmajor) {
+            if (DIGITS == 3) {
+                // written above
+            } else if (P.cmajor) {
                 for (int c = 0; c < cols; ++c) {
                     int32_t m[8];
                     int64_t mh, ml, xh = 0, xl = 0;
@@ -1000,23 +1050,24 @@ struct SlicePlan {
     }
 };
 
-// Layout of column tiles of w columns; false when it does not fit.
-bool lay_out(bool rows, bool pair, int w, int64_t k, SlicePlan& p) {
+// Layout of column tiles of w columns, with two accumulators where they leave room for `stages2`
+// stages; false when it does not fit.
+bool lay_out(bool rows, bool pair, int w, int64_t k, SlicePlan& p, int digits = kDigits, int stages2 = 4) {
     const int halves = pair ? 2 : 1;
     p.pair = pair;
     p.w = w;
     p.hw = w / halves;
-    p.cmajor = w <= 4 ? 1 : 0;
+    p.cmajor = w <= 4 && digits == kDigits ? 1 : 0;
     p.n_ctiles = (int)((k + w - 1) / w);
     auto up16 = [](int x) { return (x + 15) / 16 * 16; };
-    const int half_m = p.cmajor ? up16(8 * w) : up16(kDigits * p.hw);
-    const int half_x = p.cmajor ? half_m : up16((kDigits - 1) * p.hw);
+    const int half_m = p.cmajor ? up16(8 * w) : up16(digits * p.hw);
+    const int half_x = p.cmajor ? half_m : up16((digits - 1) * p.hw);
     p.nm = halves * half_m;
     p.nx = halves * half_x;
     p.set_rows = half_m;
     if (p.nm > 256) return false;
     p.acc_stride = (uint32_t)(rows ? p.nm + p.nx : p.nm);
-    p.nb = 2 * p.acc_stride + 4 * kAStage <= kTmemCols ? 2 : 1;
+    p.nb = 2 * p.acc_stride + stages2 * kAStage <= kTmemCols ? 2 : 1;
     p.a0 = (p.nb * p.acc_stride + 31) / 32 * 32;
     p.sp = 4;
     const int b_bytes = (rows ? 1 : 2) * p.set_rows * 128;
@@ -1084,9 +1135,9 @@ constexpr int kSingleGroups = 4, kPairGroups = 2;
 template <bool PAIR>
 constexpr int groups_of() { return PAIR ? kPairGroups : kSingleGroups; }
 
-template <bool ROWS, bool PAIR>
+template <bool ROWS, bool PAIR, int DIGITS = kDigits>
 cudaError_t allow_smem() {
-    return cudaFuncSetAttribute(k_slice_pass<ROWS, PAIR, groups_of<PAIR>()>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_slice_pass<ROWS, PAIR, groups_of<PAIR>(), DIGITS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSmemMax);
 }
 
@@ -1097,11 +1148,13 @@ void configure_slices() {
         if (e == cudaSuccess) e = allow_smem<false, false>();
         if (e == cudaSuccess) e = allow_smem<true, true>();
         if (e == cudaSuccess) e = allow_smem<false, true>();
+        if (e == cudaSuccess) e = allow_smem<true, false, 3>();
+        if (e == cudaSuccess) e = allow_smem<false, false, 3>();
         return e;
     }, "configure slice kernels");
 }
 
-template <bool ROWS, bool PAIR>
+template <bool ROWS, bool PAIR, int DIGITS = kDigits>
 void launch_slice_pass(const SlicePlan& p, const CUtensorMap& ta, const CUtensorMap& tb,
                        const SliceArgs& A, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
@@ -1126,7 +1179,7 @@ void launch_slice_pass(const SlicePlan& p, const CUtensorMap& ta, const CUtensor
             cudaLaunchConfig_t probe = cfg;
             probe.dynamicSmemBytes = kSmemMax;
             int c = 0;
-            CS_CUDA(cudaOccupancyMaxActiveClusters(&c, k_slice_pass<ROWS, true, kPairGroups>, &probe));
+            CS_CUDA(cudaOccupancyMaxActiveClusters(&c, k_slice_pass<ROWS, true, kPairGroups, DIGITS>, &probe));
             pairs = std::max(1, std::min(c, num_sms() / 2));
         }
         cfg.gridDim = dim3((unsigned)(2 * pairs));
@@ -1135,7 +1188,7 @@ void launch_slice_pass(const SlicePlan& p, const CUtensorMap& ta, const CUtensor
             num_sms(), std::max<int64_t>(1, (int64_t)A.n_tiles * A.n_ctiles * A.n_splits)));
     }
     chain(cfg, attr);
-    CS_CUDA(cudaLaunchKernelEx(&cfg, k_slice_pass<ROWS, PAIR, groups_of<PAIR>()>, ta, tb, A));
+    CS_CUDA(cudaLaunchKernelEx(&cfg, k_slice_pass<ROWS, PAIR, groups_of<PAIR>(), DIGITS>, ta, tb, A));
 }
 
 }  // namespace
@@ -1211,7 +1264,7 @@ SliceArgs slice_args(const SlicePlan& p, bool rows, int64_t tiles, int kb, int64
     A.cmajor = p.cmajor;
     A.nm = p.nm;
     A.nx = rows ? p.nx : p.nm;
-    A.set_rows = p.set_rows;
+    A.set_rows = A.set_step = p.set_rows;
     A.sp = p.sp;
     A.sd = p.sd;
     A.nb = p.nb;
@@ -1417,6 +1470,42 @@ void check_slices(cs_kinship* op, cudaStream_t s) {
     CS_CUDA(cudaStreamSynchronize(s));
     if (status != kPassStatusOk)
         fail(CS_ERR_CUDA, "tensor-core kinship kernel gave up waiting (status " + std::to_string(status) + ")");
+}
+
+// ---------------------------------------------------------------- the mixed form's narrow passes
+bool mixed_narrow_fits(bool rows, int64_t kp) {
+    SlicePlan p;
+    return kp > 0 && kp <= 256 && lay_out(rows, false, (int)kp, kp, p, 3);
+}
+
+void mixed_narrow_pass(bool rows, MixedRows& r, const int8_t* b, int64_t kp, int splits, int kbs,
+                       const double* inv_f, double* part, int* status, uint32_t poll_ns, cudaStream_t s) {
+    configure_slices();
+    SlicePlan p;
+    // long slices: two more stages are worth more than an epilogue beside the next unit's MMAs
+    // (N=50k, M=100k, a product of 20 columns 1.22 ms against 1.38)
+    if (!lay_out(rows, false, (int)kp, kp, p, 3, kbs >= 64 ? 6 : 4)) fail(CS_ERR_UNSUPPORTED, "narrow pass: too many columns");
+    p.splits = splits;
+    p.kbs = kbs;
+    const int64_t m = rows ? r.r_pad : r.n_pad, kk = rows ? r.n_pad : r.r_pad;
+    const int kb = (int)(kk / kKBlock);
+    SliceArgs A = slice_args(p, rows, m / kTile, kb, kp);
+    A.kb_total = kb;
+    A.set_step = (int)(3 * kp);
+    A.lut = r.lut.get();
+    A.resid = r.resid.get();
+    A.inv_f = inv_f;
+    A.part = part;
+    A.ld = m;
+    A.status = status;
+    A.poll_ns = poll_ns;
+    const int64_t stride = rows ? r.stride : r.r_pad / 4, packed_rows = rows ? std::max<int64_t>(r.R, 1) : r.n_pad;
+    const CUtensorMap ta = make_map_u8(rows ? r.rows : r.packed_t.get(), stride, packed_rows, stride, 128, kTile, true);
+    const CUtensorMap tb = make_map_u8(b, kk, (rows ? 3 : 6) * kp, kk, kKBlock, p.set_rows, true);
+    if (rows)
+        launch_slice_pass<true, false, 3>(p, ta, tb, A, s);
+    else
+        launch_slice_pass<false, false, 3>(p, ta, tb, A, s);
 }
 
 }  // namespace cs

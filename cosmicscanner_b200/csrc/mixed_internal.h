@@ -32,6 +32,13 @@ void ensure_transposed(MixedRows& r, cudaStream_t s);
 // The operator's tables (made on first use).
 MixedRows& mixed_rows_for(cs_kinship* op);
 
+// The mixed passes of at most 48 columns on the kernel of the FP64 form (kinship_slices.cu), which
+// decodes four K-blocks at a time: kp columns (a multiple of 8) in one tile, operands and partial sums
+// as the passes here lay them out, the six-set form in the samples pass.
+bool mixed_narrow_fits(bool rows, int64_t kp);
+void mixed_narrow_pass(bool rows, MixedRows& r, const int8_t* b, int64_t kp, int splits, int kbs,
+                       const double* inv_f, double* part, int* status, uint32_t poll_ns, cudaStream_t s);
+
 // 2D uint8 tensor map: inner extent `inner` bytes, `outer` rows of `row_bytes`.
 CUtensorMap make_map_u8(const void* base, uint64_t inner, uint64_t outer, uint64_t row_bytes,
                         uint32_t box_inner, uint32_t box_outer, bool swizzle);
