@@ -50,6 +50,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <string>
 
 #include "chain.cuh"
@@ -80,6 +81,9 @@ constexpr int kBarBytes = (4 * kMaxStages + 2 * 2 + 1) * 8 + 8;
 constexpr int kSmemMax = 227 * 1024;
 constexpr int kPassStatusOk = kOk;
 
+// The mixed form uses hw for the global B rows from one set to the next, and mu for mu - q / 63 (rows
+// pass, per SNP row) or 1 / f (samples pass, per column): three fields more, at the end, made the passes
+// of one column 7 and 12 % longer (482 and 502 us for 449 at N=50k, M=100k) with the same kernel code.
 struct SliceArgs {
     int n_tiles, n_ctiles, n_splits;
     int kb_total, kb_per_split;
@@ -92,9 +96,6 @@ struct SliceArgs {
     const uint32_t* lut;    // rows pass: imputed code of each 2-bit code, per SNP row
     const double* mu;       // rows pass: per SNP row
     const longlong2* ksum;  // [n_splits][k]: sum of the fixed-point values (hi, lo) per slice
-    const double* resid;    // mixed rows pass: mu - q / 63 per SNP row
-    const double* inv_f;    // mixed samples pass: per column
-    int set_step;           // global B rows from one set to the next
     double* part;           // [n_splits][k][ld]
     int64_t ld;
     int* status;
@@ -236,7 +237,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
 #pragma unroll
                         for (int q = 0; q < kSets; ++q)
                             tma_load_2d(smem_b + d * b_bytes + q * P.set_rows * 128, &tm_b, kb * kKBlock,
-                                        row0 + q * P.set_step, &full[d]);
+                                        row0 + q * (DIGITS == kDigits ? P.set_rows : P.hw), &full[d]);
                         ++loaded;
                         if (++d == SD) { d = 0; ph ^= 1; }
                     }
@@ -376,7 +377,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                 ok = __all_sync(0xffffffffu, mbar_wait_look(&full_p[sp], ph_p, P.status, kTimeoutDecode));
                 if (!ok) break;
                 const unsigned char* src = smem_p + sp * kPackedBytes + r * 128;
-                int mine = grp;
+                int mine = 0;
                 if constexpr (DIGITS != kDigits) {
                     const int here = min(kPackedKb, kb1 - kb);
                     mine = (int)((uint32_t)grp - j0) & (kPackedKb - 1);
@@ -390,7 +391,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                 uint32_t words[kOwn][8];
 #pragma unroll
                 for (int o = 0; o < kOwn; ++o) {
-                    const int c = 2 * (mine + o * G);  // 16-byte chunk of the row, 128-byte swizzle
+                    const int c = 2 * ((DIGITS == kDigits ? grp : mine) + o * G);  // 16-byte chunk of the row, 128-byte swizzle
                     const uint4 p0 = *reinterpret_cast<const uint4*>(src + ((c ^ (r & 7)) << 4));
                     const uint4 p1 = *reinterpret_cast<const uint4*>(src + (((c + 1) ^ (r & 7)) << 4));
                     words[o][0] = p0.x; words[o][1] = p0.y; words[o][2] = p0.z; words[o][3] = p0.w;
@@ -463,7 +464,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
             double* dst = P.part + ((int64_t)split * P.k + c_base) * P.ld + row;
             if constexpr (DIGITS == 3) {
                 const double ib = 1.0 / 254.0, ib2 = 1.0 / (254.0 * 254.0), inv_q = 1.0 / (double)kTcQ;
-                const double rt = ROWS ? P.resid[row] : 0.0;
+                const double rt = ROWS ? P.mu[row] : 0.0;
                 for (int c0 = 0; c0 < P.w; c0 += 8) {
                     int32_t m1[8], m2[8], m3[8];
                     double v[8];
@@ -481,7 +482,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                     for (int i = 0; i < 8; ++i)
                         dst[(int64_t)(c0 + i) * P.ld] =
                             ROWS ? fma(v[i], inv_q, __dmul_rn(rt, fma((double)m2[i], ib, (double)m1[i])))
-                                 : __dmul_rn(v[i], P.inv_f[c0 + i]);
+                                 : __dmul_rn(v[i], P.mu[c0 + i]);
                 }
             }
             const longlong2* ks = P.ksum + (int64_t)split * P.k + c_base;
@@ -1264,7 +1265,7 @@ SliceArgs slice_args(const SlicePlan& p, bool rows, int64_t tiles, int kb, int64
     A.cmajor = p.cmajor;
     A.nm = p.nm;
     A.nx = rows ? p.nx : p.nm;
-    A.set_rows = A.set_step = p.set_rows;
+    A.set_rows = p.set_rows;
     A.sp = p.sp;
     A.sd = p.sd;
     A.nb = p.nb;
@@ -1373,14 +1374,21 @@ void finish_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const Slic
     CS_LAUNCH("slice_reduce_rows");
 }
 
+// CS_B200_FP64_DMMA or CS_B200_FP64_NARROW, which choose among the FP64-pipe kernels, keep these.
+bool pipe_kernels_chosen() {
+    static const bool on = std::getenv("CS_B200_FP64_DMMA") || std::getenv("CS_B200_FP64_NARROW");
+    return on;
+}
+
 // The operator's slice state with room for k columns, or null (no sample-major copy allowed, or no
 // device memory for it or for the operands).  The slices are taken at every shape: against the
-// FP64-pipe kernels an apply took (us) 36 / 99 at n=40, M=1000 and one column, 52 / 152 at n=2000,
-// M=10000, 950 / 7210 at n=50000, M=100000; 56 / 187, 110 / 470 and 212 / 954 at n=2000, M=10000 and
-// 8, 80 and 200 columns; 2570 / 23480 at n=18009, M=27006 and 266.
+// FP64-pipe kernels an apply took (us) 27 / 99 at n=40, M=1000 and one column, 31 / 152 at n=2000,
+// M=10000, 930 / 7210 at n=50000, M=100000; 35 / 187, 86 / 470 and 168 / 954 at n=2000, M=10000 and
+// 8, 80 and 200 columns; 2750 / 23480 at n=18009, M=27006 and 266.
 SliceOperator* slices_for(cs_kinship* op, int64_t k, bool samples, cudaStream_t s) {
     const int64_t R = op->n_active;
-    if (!op->sample_major_copy || op->slices_unavailable || R == 0 || k <= 0) return nullptr;
+    if (!op->sample_major_copy || op->slices_unavailable || R == 0 || k <= 0 || pipe_kernels_chosen())
+        return nullptr;
     try {
         MixedRows& r = mixed_rows_for(op);
         configure_slices();
@@ -1491,10 +1499,9 @@ void mixed_narrow_pass(bool rows, MixedRows& r, const int8_t* b, int64_t kp, int
     const int kb = (int)(kk / kKBlock);
     SliceArgs A = slice_args(p, rows, m / kTile, kb, kp);
     A.kb_total = kb;
-    A.set_step = (int)(3 * kp);
+    A.hw = (int)(3 * kp);
     A.lut = r.lut.get();
-    A.resid = r.resid.get();
-    A.inv_f = inv_f;
+    A.mu = rows ? r.resid.get() : inv_f;
     A.part = part;
     A.ld = m;
     A.status = status;
