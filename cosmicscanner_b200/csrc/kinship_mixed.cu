@@ -225,7 +225,6 @@ struct PassArgs {
     int* status;
     uint32_t poll_ns;            // pairs: pause between polls of the long, off-critical-path waits
     uint32_t poll_dec_ns;        // pairs: pause between the decoders' polls for a free stage
-    int decode_alt;              // TMEMA: two groups of four decoder warps take alternate K-blocks
 };
 
 // decode_word_interleaved for 16 codes of 16 different SNPs (a word of the sample-major copy): the observed
@@ -245,7 +244,9 @@ __device__ __forceinline__ void decode_word_imputed(uint32_t w, const uint4& q, 
     dos.z = __byte_perm(kObservedCodes, 0u, so) | (mis.z & q.z);
     dos.w = __byte_perm(kObservedCodes, 0u, so >> 16) | (mis.w & q.w);
 }
-template <bool ROWS, bool PAIR, bool NARROW, int TMEMA>
+// ALT (A in TMEM): the decoder warps in two groups that take alternate K-blocks whole.  Known at
+// compile time: as an argument it cost the rows pass of 96 columns at 31,001 x 52,003 4 % (517 us for 495).
+template <bool ROWS, bool PAIR, bool NARROW, int TMEMA, bool ALT>
 __global__ void __launch_bounds__(kThreads, 1)
 k_mixed_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
              const __grid_constant__ CUtensorMap tm_bt, PassArgs P) {
@@ -277,7 +278,7 @@ k_mixed_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     // TMEMA: the decoder warps either share every K-block (each its lane quarter and one half of
     // K) or split into two groups of four that take alternate K-blocks whole, so that two
     // K-blocks are in decode at once
-    const bool alt = TMEMA != 0 && P.decode_alt != 0;
+    constexpr bool alt = TMEMA != 0 && ALT;
     const uint32_t dec_arrivals = alt ? 4u : (uint32_t)kDecodeWarps;
     if (threadIdx.x == 0) {
         for (int s = 0; s < ST; ++s) {
@@ -1606,9 +1607,14 @@ namespace {
 
 template <bool ROWS, bool PAIR, bool NARROW = false, int TMEMA = 0>
 cudaError_t allow_smem() {
-    return cudaFuncSetAttribute(k_mixed_pass<ROWS, PAIR, NARROW, TMEMA>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                Layout<ROWS, PAIR, NARROW, TMEMA>::kSmem);
+    constexpr int bytes = Layout<ROWS, PAIR, NARROW, TMEMA>::kSmem;
+    cudaError_t e = cudaFuncSetAttribute(k_mixed_pass<ROWS, PAIR, NARROW, TMEMA, false>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if constexpr (TMEMA != 0)
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_mixed_pass<ROWS, PAIR, NARROW, TMEMA, true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return e;
 }
 
 void configure_kernels() {
@@ -1658,15 +1664,15 @@ int resident_pairs() {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        CS_CUDA(cudaOccupancyMaxActiveClusters(&clusters, k_mixed_pass<ROWS, true, false, 0>, &cfg));
+        CS_CUDA(cudaOccupancyMaxActiveClusters(&clusters, k_mixed_pass<ROWS, true, false, 0, false>, &cfg));
         n = std::max(1, std::min(clusters, num_sms() / 2));
     }
     return n;
 }
 
 // One CTA per SM, or (PAIR) as many clusters of two CTAs as are resident together.
-template <bool ROWS, bool PAIR, bool NARROW = false, int TMEMA = 0>
-void launch_pass(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tbt,
+template <bool ROWS, bool PAIR, bool NARROW, int TMEMA, bool ALT>
+void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tbt,
                  const PassArgs& P, cudaStream_t s) {
     if constexpr (PAIR) {
         cudaLaunchConfig_t cfg = {};
@@ -1681,11 +1687,22 @@ void launch_pass(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
         attr[0].val.clusterDim.z = 1;
         cfg.numAttrs = 1;
         chain(cfg, attr);
-        CS_CUDA(cudaLaunchKernelEx(&cfg, k_mixed_pass<ROWS, true, false, TMEMA>, ta, tb, tbt, P));
+        CS_CUDA(cudaLaunchKernelEx(&cfg, k_mixed_pass<ROWS, true, false, TMEMA, ALT>, ta, tb, tbt, P));
     } else {
-        launch_chained(k_mixed_pass<ROWS, false, NARROW, TMEMA>, num_sms(), kThreads,
+        launch_chained(k_mixed_pass<ROWS, false, NARROW, TMEMA, ALT>, num_sms(), kThreads,
                        Layout<ROWS, false, NARROW, TMEMA>::kSmem, s, ta, tb, tbt, P);
     }
+}
+
+template <bool ROWS, bool PAIR, bool NARROW = false, int TMEMA = 0>
+void launch_pass(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tbt,
+                 const PassArgs& P, cudaStream_t s) {
+    if constexpr (TMEMA == 0)
+        launch_form<ROWS, PAIR, NARROW, 0, false>(ta, tb, tbt, P, s);
+    else if (decode_alt_mode())
+        launch_form<ROWS, PAIR, NARROW, TMEMA, true>(ta, tb, tbt, P, s);
+    else
+        launch_form<ROWS, PAIR, NARROW, TMEMA, false>(ta, tb, tbt, P, s);
 }
 
 // Per-row statistics: mu_t, exc_t = S_t - mu_t n_t (from code counts c00, c01, c10, c11),
@@ -2101,7 +2118,6 @@ void rows_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, Stri
     P.status = ws.status.get();
     P.poll_ns = poll_sleep_ns();
     P.poll_dec_ns = poll_dec_sleep_ns();
-    P.decode_alt = decode_alt_mode();
     {
         // algorithmic work: 2 n R k flops, one pass over the packed rows
         prof::Scope ps("kinship_rows_tc", s, 2.0 * (double)n * (double)R * (double)k,
@@ -2200,7 +2216,6 @@ void samples_pass_plan(const PassPlan& plan, MixedRows& r, MixedWorkspace& ws, c
     P.status = ws.status.get();
     P.poll_ns = poll_sleep_ns();
     P.poll_dec_ns = poll_dec_sleep_ns();
-    P.decode_alt = decode_alt_mode();
     {
         prof::Scope ps("kinship_samples_tc", s, 2.0 * (double)n * (double)R * (double)k,
                        (double)R * (double)((n + 3) / 4));
