@@ -329,14 +329,26 @@ static bool upload_staged(const uint8_t* src, int64_t M, int64_t bps, int spare,
     return true;
 }
 
+static bool pageable(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
 // .bed rows (bps bytes each) to device rows of `stride` bytes; padding bytes and the last byte's
-// spare codes become the missing code.  Matrices below 2 MiB, where a piece or two leave threads
-// nothing to share (at 2.1 MB staged 0.40 ms against 1.31), and rows too long for the pieces go in
-// one copy from where they are.
+// spare codes become the missing code.  One copy takes matrices below 2 MiB, where a piece or two leave
+// threads nothing to share (at 2.1 MB staged 0.40 ms against 1.31), rows too long for the pieces, and
+// sources that are page-locked already, which the link reads where they are (50,000 samples, 1.25 GB
+// 24.9 ms, staged 30 to 37), unless their rows are short (a strided copy pays 40 to 130 ns a row: 203
+// samples x 300,000 variants 12.7 ms, staged 3.5).
 static void upload_rows(const uint8_t* src, int64_t M, int64_t bps, int64_t n_samples, uint8_t* dst,
                         int64_t stride, cudaStream_t s) {
     const int spare = (int)(n_samples % 4);  // codes in use in the last byte, 0: all four
     if (M * stride >= (2 << 20) && stride <= (1 << 18) &&
+        (bps < 4096 || (pageable(src) && pageable(src + M * bps - 1))) &&
         upload_staged(src, M, bps, spare, dst, stride, s))
         return;
     CS_CUDA(cudaMemsetAsync(dst, kMissingByte, M * stride, s));

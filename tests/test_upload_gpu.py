@@ -13,14 +13,20 @@ synth = pytest.importorskip("cosmicscanner_b200.synth")
 import oracle  # noqa: E402
 
 
-def check(n, m, seed):
+def check(n, m, seed, pinned=False):
     d = synth.cohort(n, m, seed, missing=0.03, n_causal=2, maf_lo=0.05)
     rows = d["bed"][3:].reshape(m, -1)
     ref = oracle.Bed(rows.copy(), n)
     if n % 4:
         rows[:, -1] |= (0xFF << (2 * (n % 4))) & 0xFF  # spare codes of the last byte: not samples
     d["bed"][3:] = rows.ravel()
-    g = cs.Genotypes.from_bed_bytes(d["bed"], n, m)
+    bed = d["bed"]
+    if pinned:
+        torch = pytest.importorskip("torch")
+        hold = torch.empty(bed.size, dtype=torch.uint8, pin_memory=True)
+        hold.numpy()[:] = bed
+        bed = hold.numpy()
+    g = cs.Genotypes.from_bed_bytes(bed, n, m)
     s = g.stats()
     assert np.array_equal(s["mean"], ref.mean) and np.array_equal(s["inv_std"], ref.inv_std)
     op = cs.createKinshipOperator(g)
@@ -35,6 +41,11 @@ def check(n, m, seed):
 @pytest.mark.parametrize("n,m", [(253, 32767), (256, 32768), (1001, 8193), (1002, 40000), (1003, 9000), (70001, 130)])
 def test_staged_upload(n, m):
     check(n, m, n)
+
+
+@pytest.mark.parametrize("n,m", [(253, 32768), (1002, 9000), (16383, 600), (16385, 600)])
+def test_page_locked_source(n, m):
+    check(n, m, n, pinned=True)
 
 
 def test_uploads_from_several_threads():
