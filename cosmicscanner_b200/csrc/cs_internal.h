@@ -286,6 +286,9 @@ MixedScan* mixed_scan_create(const cs_packed_view& v, const double* row_mean, co
 void mixed_scan_destroy(MixedScan* m);
 void mixed_scan_project(MixedScan* m, const double* B, int64_t ldb, int64_t k, double* T,
                         int64_t ldt, cudaStream_t s);
+// The same in the FP64 form (int8 digits); false where it cannot run (decode_gemm_rows_fp64 then).
+bool scan_project_fp64(MixedScan* m, const double* B, int64_t ldb, int64_t k, double* T, int64_t ldt,
+                       cudaStream_t s);
 
 // Per-row genotype code counts over a view's samples: c[4*t + code].
 void row_code_counts(const cs_packed_view& v, int32_t* d_counts, cudaStream_t s);

@@ -2398,6 +2398,8 @@ const double* mixed_rows_output(const cs_kinship* op, int64_t* R, int64_t* k) {
 struct MixedScan {
     MixedRows rows;
     MixedWorkspace ws;
+    SliceOperator* slices = nullptr;  // scan_project_fp64's
+    ~MixedScan() { destroy_slices(slices); }
 };
 
 MixedScan* mixed_scan_create(const cs_packed_view& v, const double* row_mean, const int32_t* counts) {
@@ -2423,6 +2425,11 @@ void mixed_scan_project(MixedScan* m, const double* B, int64_t ldb, int64_t k, d
                         int64_t ldt, cudaStream_t s) {
     rows_pass(m->rows, m->ws, StridedIn{B, ldb, 1}, k, nullptr, nullptr, StridedOut{T, ldt, 1}, s, true);
     check_status(m->ws, s);
+}
+
+bool scan_project_fp64(MixedScan* m, const double* B, int64_t ldb, int64_t k, double* T, int64_t ldt,
+                       cudaStream_t s) {
+    return scan_project_slices(m->slices, m->rows, StridedIn{B, ldb, 1}, k, StridedOut{T, ldt, 1}, s);
 }
 
 }  // namespace cs

@@ -948,7 +948,7 @@ k_slice_reduce_rows(const double* __restrict__ part, int64_t ld, int64_t R, int6
             Wt[c * R + t] = w;
             range_of(mu[t] > 1.0 ? mu[t] * w : w, mx, es, cnt);
         } else {
-            out.p[(int64_t)pos[t] * out.rs + c * out.cs] = v * s;
+            out.p[(pos ? (int64_t)pos[t] : t) * out.rs + c * out.cs] = v * s;
         }
     };
     if (direct) {
@@ -1471,13 +1471,49 @@ bool multiply_z_slices(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cud
     return true;
 }
 
-void check_slices(cs_kinship* op, cudaStream_t s) {
-    if (!op->slices || !op->slices->words.get()) return;
+static void check_slices(SliceOperator* so, cudaStream_t s) {
+    if (!so || !so->words.get()) return;
     int status = 0;
-    CS_CUDA(cudaMemcpyAsync(&status, op->slices->words.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    CS_CUDA(cudaMemcpyAsync(&status, so->words.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
     CS_CUDA(cudaStreamSynchronize(s));
     if (status != kPassStatusOk)
         fail(CS_ERR_CUDA, "tensor-core kinship kernel gave up waiting (status " + std::to_string(status) + ")");
+}
+
+void check_slices(cs_kinship* op, cudaStream_t s) { check_slices(op->slices, s); }
+
+bool scan_project_slices(SliceOperator*& state, MixedRows& r, StridedIn X, int64_t k, StridedOut T,
+                         cudaStream_t s) {
+    if (r.R == 0 || k <= 0 || pipe_kernels_chosen()) return false;
+    try {
+        configure_slices();
+        if (!state) state = new SliceOperator();
+        SliceOperator& so = *state;
+        if (!so.map_rows) {
+            so.tm_packed = make_map_u8(r.rows, r.stride, r.R, r.stride, 128, kTile, true);
+            so.map_rows = true;
+        }
+        auto reserve_rows = [&](const SliceCall& c) {
+            so.b.resize(c.rows.b_rows(true) * r.n_pad);
+            so.part.resize(c.k * c.rows.splits * r.r_pad);
+            so.words.resize(c.words);
+        };
+        if (k >= kChunkColumns) reserve_rows(plan_call(r, kChunkColumns));
+        if (k % kChunkColumns) reserve_rows(plan_call(r, k % kChunkColumns));
+    } catch (const Error&) {  // no device memory for the operands
+        destroy_slices(state);
+        state = nullptr;
+        return false;
+    }
+    SliceOperator& so = *state;
+    for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
+        const SliceSums S = sums_of(so, c);
+        const StridedIn x = from_column(X, c0);
+        run_rows(so, r, c, S, x, s);
+        finish_rows(so, r, c, S, x, nullptr, nullptr, from_column(T, c0), s);
+    });
+    check_slices(&so, s);
+    return true;
 }
 
 // ---------------------------------------------------------------- the mixed form's narrow passes

@@ -1142,6 +1142,25 @@ static void scan_finish(cs_lmm* l, int64_t M, const std::vector<double>& fr, dou
     }
 }
 
+// The scan's context over its view, made when the view is new.
+static MixedScan* scan_context(cs_lmm* l, bool cached, const cs_packed_view& v, const std::vector<double>& row_mean) {
+    if (!cached || !l->scan_mixed) {
+        mixed_scan_destroy(l->scan_mixed);
+        l->scan_mixed = nullptr;
+        l->scan_mixed = mixed_scan_create(v, row_mean.data(), l->scan_counts.data());
+    }
+    return l->scan_mixed;
+}
+
+// T = Z_c^T B over the scan's view: on the int8 digits (N=50k, M=100k, 260 columns 17 ms), or on the
+// FP64 pipe (112) where their operands do not fit.
+static void project_fp64(cs_lmm* l, bool cached, const cs_packed_view& v, const std::vector<double>& row_mean,
+                         const double* B, int64_t ldb, int64_t k, double* T, int64_t ldt, cudaStream_t s) {
+    if (scan_project_fp64(scan_context(l, cached, v, row_mean), B, ldb, k, T, ldt, s)) return;
+    Workspace ws;
+    decode_gemm_rows_fp64(v, l->d_lut.get(), B, ldb, k, T, ldt, ws, s);
+}
+
 // LmmEngine::scan's exact branch (src/lmm_engine.cpp:1363-1474) over SNPs [snp_begin,
 // snp_end): the null quantities in the eigenbasis on the host (O(n p^2)), then per chunk of
 // W_proj's columns the projection T = W_proj[:, chunk]^T G_c of every SNP (tensor cores in the
@@ -1206,26 +1225,20 @@ static void lmm_scan_exact(cs_lmm* l, const cs_genotypes* g, const int32_t* keep
         CS_CUDA(cudaMemcpyAsync(l->d_inv.get(), xvx_inv.data(), 8 * p * p, cudaMemcpyHostToDevice, s));
     }
     CS_CUDA(cudaMemsetAsync(l->d_acc.get(), 0, 8 * M * (2 + p), s));
-    if (precision == CS_PRECISION_MIXED && (!enc.cached || !l->scan_mixed)) {
-        mixed_scan_destroy(l->scan_mixed);
-        l->scan_mixed = nullptr;
-        l->scan_mixed = mixed_scan_create(l->scan_view, enc.row_mean.data(), l->scan_counts.data());
-    }
+    scan_context(l, enc.cached, l->scan_view, enc.row_mean);
     // chunk width: 1024 columns, fewer when the window is long (T stays within 4 GiB)
     int64_t kc = std::min<int64_t>(1024, std::max<int64_t>(64, ((int64_t)1 << 29) / M));
     kc = std::max<int64_t>(16, kc / 16 * 16);
     kc = std::min<int64_t>(kc, round_up(ne, 16));
     l->d_chunk.resize(n * kc);
     l->d_T.resize(M * kc);
-    Workspace ws;
     for (int64_t c0 = 0; c0 < ne; c0 += kc) {
         const int64_t k = std::min<int64_t>(kc, ne - c0);
         colmajor_to_rowmajor(d.W.get() + c0 * n, n, n, k, l->d_chunk.get(), kc, s);
         if (precision == CS_PRECISION_MIXED)
             mixed_scan_project(l->scan_mixed, l->d_chunk.get(), kc, k, l->d_T.get(), kc, s);
         else
-            decode_gemm_rows_fp64(l->scan_view, l->d_lut.get(), l->d_chunk.get(), kc, k,
-                                  l->d_T.get(), kc, ws, s);
+            project_fp64(l, true, l->scan_view, enc.row_mean, l->d_chunk.get(), kc, k, l->d_T.get(), kc, s);
         prof::Scope ps("exact_scan_accumulate", s, (4.0 + 2.0 * p) * M * k, 8.0 * M * k);
         const int blocks = (int)std::min<int64_t>((M * 32 + 255) / 256, 64LL * num_sms());
         k_exact_accumulate<<<std::max(blocks, 1), 256, 0, s>>>(
@@ -1364,7 +1377,6 @@ void lmm_scan_window(cs_lmm* l, const cs_genotypes* g, const int32_t* keep, int6
     ScanEncoding enc = scan_encoding(l, g, keep, n_keep, snp_begin, snp_end, min_maf, s);
     const bool cached = enc.cached;
     const cs_packed_view& v = l->scan_view;
-    const std::vector<int32_t>& counts = l->scan_counts;
     std::vector<double>&lut = enc.lut, &gn2 = enc.gn2, &fr = enc.fr, &row_mean = enc.row_mean;
     std::vector<uint8_t>& pass = enc.pass;
     l->d_lut.resize(std::max<int64_t>(1, 4 * M));
@@ -1431,16 +1443,10 @@ void lmm_scan_window(cs_lmm* l, const cs_genotypes* g, const int32_t* keep, int6
             CS_CUDA(cudaMemcpy2DAsync(l->d_bt.get() + bw, 8 * ldc, hy.data(), 8 * tc, 8 * tc, n,
                                       cudaMemcpyHostToDevice, s));
             if (precision == CS_PRECISION_MIXED) {
-                if (!cached || !l->scan_mixed) {
-                    mixed_scan_destroy(l->scan_mixed);
-                    l->scan_mixed = nullptr;
-                    l->scan_mixed = mixed_scan_create(v, row_mean.data(), counts.data());
-                }
+                scan_context(l, cached, v, row_mean);
                 mixed_scan_project(l->scan_mixed, l->d_bt.get(), ldc, ldc, l->d_tc.get(), ldc, s);
             } else {
-                Workspace ws;
-                decode_gemm_rows_fp64(v, l->d_lut.get(), l->d_bt.get(), ldc, ldc, l->d_tc.get(),
-                                      ldc, ws, s);
+                project_fp64(l, cached, v, row_mean, l->d_bt.get(), ldc, ldc, l->d_tc.get(), ldc, s);
             }
             CS_CUDA(cudaStreamSynchronize(s));  // hy is a host temporary
             l->tcache_valid = true;
@@ -1467,11 +1473,7 @@ void lmm_scan_window(cs_lmm* l, const cs_genotypes* g, const int32_t* keep, int6
         Tptr = l->d_tc.get();
         ldt = ldc;
     } else if (precision == CS_PRECISION_MIXED) {
-        if (!cached || !l->scan_mixed) {
-            mixed_scan_destroy(l->scan_mixed);
-            l->scan_mixed = nullptr;
-            l->scan_mixed = mixed_scan_create(v, row_mean.data(), counts.data());
-        }
+        scan_context(l, cached, v, row_mean);
         // The U block from the kept sketch apply when every analysed sample is in the
         // operator (then the scan's centring means are the operator's) and every SNP that can
         // be tested has an operator row.  X and py come from the same apply when it carried
@@ -1535,8 +1537,7 @@ void lmm_scan_window(cs_lmm* l, const cs_genotypes* g, const int32_t* keep, int6
             mixed_scan_project(l->scan_mixed, Bm, bw, bw, l->d_T.get(), bw, s);
         }
     } else {
-        Workspace ws;
-        decode_gemm_rows_fp64(v, l->d_lut.get(), Bm, bw, bw, l->d_T.get(), bw, ws, s);
+        project_fp64(l, cached, v, row_mean, Bm, bw, bw, l->d_T.get(), bw, s);
     }
     ScanParams P;
     P.n_snps = M; P.rank = r; P.p = p; P.ldt = ldt; P.base = base;

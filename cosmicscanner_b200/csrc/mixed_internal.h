@@ -39,6 +39,11 @@ bool mixed_narrow_fits(bool rows, int64_t kp);
 void mixed_narrow_pass(bool rows, MixedRows& r, const int8_t* b, int64_t kp, int splits, int kbs,
                        const double* inv_f, double* part, int* status, uint32_t poll_ns, cudaStream_t s);
 
+// T = Z_c^T X (rows of r, k columns) in the FP64 form on the int8 digits, with the state's buffers (made
+// on first use); false, and nothing done, without device memory for them.
+bool scan_project_slices(SliceOperator*& state, MixedRows& r, StridedIn X, int64_t k, StridedOut T,
+                         cudaStream_t s);
+
 // 2D uint8 tensor map: inner extent `inner` bytes, `outer` rows of `row_bytes`.
 CUtensorMap make_map_u8(const void* base, uint64_t inner, uint64_t outer, uint64_t row_bytes,
                         uint32_t box_inner, uint32_t box_outer, bool swizzle);
