@@ -1,5 +1,9 @@
 // FP64 decode-GEMM passes on the FP64 tensor datapath (DMMA, mma.sync m8n8k4 f64).
 //
+// The operator's products run on the int8 digits (kinship_slices.cu); these kernels take those that
+// cannot: no device memory for the digits, operators that keep no sample-major copy, the multi-trait
+// scan.
+//
 // The plain (all-FP64) form of the kinship operator computes the same two products as the
 // SIMT kernels of kinship_fp64.cu,
 //   rows pass    out[t, c] = sum_i lut_t[code(t,i)] B[i, c]   (Z^T V: SNP-major output)

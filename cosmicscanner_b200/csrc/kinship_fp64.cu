@@ -1,5 +1,5 @@
 // FP64 decode-GEMM kernels: the plain (all-FP64) form of the kinship operator and of the
-// scan's basis projection.
+// scan's basis projection, where the digit form (kinship_slices.cu) cannot run.
 //
 // The packed 2-bit genotypes are expanded inside the kernel through a per-row lookup
 // table lut_t[code] (e.g. {(2-mu)s, 0, (1-mu)s, -mu s} for Z, exactly the values

@@ -1,5 +1,9 @@
 // FP64 decode-GEMV passes for one to four right-hand sides.
 //
+// The operator's products run on the int8 digits (kinship_slices.cu); these kernels take those that
+// cannot: no device memory for the digits, operators that keep no sample-major copy, the multi-trait
+// scan.
+//
 // A kinship apply with a single vector is what the reference's MatrixFreePCG issues on every
 // CG step (STCG_VCE::apply_G through GenotypeMatrix::multiply_Zt_v / multiply_Z_v,
 // libCosmicCore/src/plink_reader.cpp:241-438).  With so few columns the tile GEMMs idle: the
