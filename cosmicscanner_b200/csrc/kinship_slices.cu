@@ -926,7 +926,7 @@ __device__ double direct_row(const PackedRows& G, int64_t t, double mu, const St
 
 // Rows-pass result u / s = 2^-e / 63 sum_z part (or the direct sum).  1024 SNPs per block, one column
 // per blockIdx.y.  With Wt: W^T (column-major, R per column) = s^2 (u / s) and the ranges of
-// max(|W|, |mu W|) for the samples operand; with out: s (u / s) at row pos[t].
+// max(|W|, |mu W|) for the samples operand; with out: s (u / s) at row pos[t] (or t).
 __global__ void __launch_bounds__(256)
 k_slice_reduce_rows(const double* __restrict__ part, int64_t ld, int64_t R, int64_t k,
                     const double* __restrict__ s_row, const double* __restrict__ mu,
