@@ -240,7 +240,7 @@ int cs_kinship_apply_host(cs_kinship* op, const double* X, int64_t ldx, int64_t 
         CS_CUDA(cudaMemcpy2D(dx.get(), n * 8, X, ldx * 8, n * 8, k, cudaMemcpyHostToDevice));
         cs::kinship_apply_colmajor(op, dx.get(), n, k, dx.get(), n, precision, 0);
         CS_CUDA(cudaMemcpy2D(Y, ldy * 8, dx.get(), n * 8, n * 8, k, cudaMemcpyDeviceToHost));
-        cs::check_slices(op, 0);
+        if (precision == CS_PRECISION_FP64) cs::check_slices(op, 0);
     });
 }
 
@@ -283,7 +283,7 @@ int cs_genotype_multiply_zt_host(cs_kinship* op, const double* X, int64_t ldx, i
         CS_CUDA(cudaMemcpy2D(dx.get(), n * 8, X, ldx * 8, n * 8, k, cudaMemcpyHostToDevice));
         cs::genotype_multiply_zt(op, dx.get(), n, k, du.get(), nv, precision, 0);
         CS_CUDA(cudaMemcpy2D(U, ldu * 8, du.get(), nv * 8, nv * 8, k, cudaMemcpyDeviceToHost));
-        cs::check_slices(op, 0);
+        if (precision == CS_PRECISION_FP64) cs::check_slices(op, 0);
     });
 }
 
@@ -302,7 +302,7 @@ int cs_genotype_multiply_z_host(cs_kinship* op, const double* V, int64_t ldv, in
         CS_CUDA(cudaMemcpy2D(dv.get(), nv * 8, V, ldv * 8, nv * 8, k, cudaMemcpyHostToDevice));
         cs::genotype_multiply_z(op, dv.get(), nv, k, dy.get(), n, precision, 0);
         CS_CUDA(cudaMemcpy2D(Y, ldy * 8, dy.get(), n * 8, n * 8, k, cudaMemcpyDeviceToHost));
-        cs::check_slices(op, 0);
+        if (precision == CS_PRECISION_FP64) cs::check_slices(op, 0);
     });
 }
 

@@ -193,7 +193,7 @@ struct cs_kinship {
     cs::MixedOperator* mixed = nullptr;
     cs::SliceOperator* slices = nullptr;
     bool slices_unavailable = false;  // no device memory for them: FP64-pipe kernels only
-    bool defer_checks = false;        // a solver's loop checks its passes itself (kinship_check)
+    bool defer_checks = false;        // a solver's loop checks its passes itself (DeferChecks)
     cs::PcgWorkspace* pcg = nullptr;  // kept from one solve on this operator to the next (pcg.cu)
     bool autotune = true;  // the tensor-core passes may tune their plan on new shapes
     // the samples pass may keep a sample-major copy of the packed view (one more packed matrix
@@ -236,13 +236,24 @@ const double* mixed_rows_output(const cs_kinship* op, int64_t* R, int64_t* k);
 void mixed_multiply_zt(cs_kinship* op, StridedIn X, int64_t k, StridedOut U, cudaStream_t s);
 void mixed_multiply_z(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cudaStream_t s);
 
-// Waits for the stream and fails if the operator's last FP64 tensor-core pass gave up waiting (its
-// results are NaN; kinship_slices.cu), or a mixed one has (kinship_mixed.cu), or either.
+// Waits for the stream and fails if an FP64 tensor-core pass gave up waiting (its results are NaN;
+// kinship_slices.cu) since the operator's last call began, or a mixed one has (kinship_mixed.cu), or
+// either; what is reported is cleared.  With defer_checks calls do not begin afresh: clear_* does.
 void check_slices(cs_kinship* op, cudaStream_t s);
 void check_mixed(cs_kinship* op, cudaStream_t s);
+void clear_slices(cs_kinship* op, cudaStream_t s);
+void clear_mixed(cs_kinship* op, cudaStream_t s);
 inline void kinship_check(cs_kinship* op, cudaStream_t s) {
     check_mixed(op, s);
     check_slices(op, s);
+}
+// kinship_apply_rowmajor for callers in the library, which go on with the result: fails if a pass gave
+// up, unless the caller has deferred that.  (The mixed form looks by itself, public FP64 calls
+// on device buffers do not wait for the stream.)
+inline void kinship_apply_checked(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* Y,
+                                  int64_t ldy, int precision, cudaStream_t s) {
+    kinship_apply_rowmajor(op, X, ldx, k, Y, ldy, precision, s);
+    if (precision == CS_PRECISION_FP64 && !op->defer_checks) check_slices(op, s);
 }
 
 // The reference's Gaussian test matrix (std::normal_distribution over std::mt19937_64) on the

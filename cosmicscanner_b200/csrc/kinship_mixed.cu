@@ -2319,6 +2319,10 @@ void kinship_apply_mixed(cs_kinship* op, Strided<const T> X, int64_t k, Strided<
 void check_mixed(cs_kinship* op, cudaStream_t s) {
     if (op->mixed && op->mixed->ws.status.get()) check_status(op->mixed->ws, s);
 }
+void clear_mixed(cs_kinship* op, cudaStream_t s) {
+    if (op->mixed && op->mixed->ws.status.get())
+        CS_CUDA(cudaMemsetAsync(op->mixed->ws.status.get(), 0, sizeof(int), s));
+}
 
 template void kinship_apply_mixed<double>(cs_kinship*, Strided<const double>, int64_t, Strided<double>,
                                           cudaStream_t);

@@ -49,6 +49,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <string>
@@ -616,12 +617,30 @@ __device__ __forceinline__ void add_range(ColumnRange* out, unsigned long long m
     atomicAdd(&out->count, n);
 }
 
+// The words a chunk clears before its kernels add to them (see SliceCall), and the status that its
+// passes report to: they only ever set it, and the first kernel of a call clears it (`clear`), not of
+// a chunk, nor of a call whose caller looks at it after several (DeferChecks).
+struct SliceSums {
+    int* status;
+    int clear;
+    ColumnRange* range;        // of X, per column
+    ColumnRange* range_w;      // of the samples operand
+    unsigned long long* sum;   // [slices][k][2]: (hi, lo) sums of the fixed-point values, rows pass
+    unsigned long long* sum_w; // the same of mu o w, samples pass
+    int splits, splits_w;
+};
+
+__device__ __forceinline__ void clear_status(const SliceSums& S, bool first_block) {
+    if (first_block && S.clear && threadIdx.x == 0) *S.status = kPassStatusOk;
+}
+
 // Ranges of X's columns: a block covers kc columns x rows_per_block rows, kc a power of two: one for
 // column-major input, otherwise up to 32, so that a warp reads adjacent elements either way.
 __global__ void __launch_bounds__(256)
 k_slice_ranges(const StridedIn X, int64_t n, int64_t k, int kc, int64_t rows_per_block,
-               ColumnRange* __restrict__ out) {
+               const SliceSums S) {
     chain_enter();
+    clear_status(S, blockIdx.x == 0 && blockIdx.y == 0);
     __shared__ unsigned long long s_mx[256];
     __shared__ long long s_es[256];
     __shared__ unsigned s_n[256];
@@ -649,7 +668,7 @@ k_slice_ranges(const StridedIn X, int64_t n, int64_t k, int kc, int64_t rows_per
         }
         __syncthreads();
     }
-    if (tr == 0 && c < k) add_range(&out[c], s_mx[threadIdx.x], s_es[threadIdx.x], s_n[threadIdx.x]);
+    if (tr == 0 && c < k) add_range(&S.range[c], s_mx[threadIdx.x], s_es[threadIdx.x], s_n[threadIdx.x]);
 }
 
 // Transposes 4 x 4 bytes: out[j] = byte j of in[0..3].
@@ -706,16 +725,6 @@ struct BLayout {
         const int in = cmajor ? 8 * cl + p : p * hw + cl;
         return ((ct * halves + h) * sets + q) * set_rows + in;
     }
-};
-
-// The words a call clears before its kernels add to them (see SliceCall).
-struct SliceSums {
-    int* status;
-    ColumnRange* range;        // of X, per column
-    ColumnRange* range_w;      // of the samples operand
-    unsigned long long* sum;   // [slices][k][2]: (hi, lo) sums of the fixed-point values, rows pass
-    unsigned long long* sum_w; // the same of mu o w, samples pass
-    int splits, splits_w;
 };
 
 __device__ __forceinline__ void add_sums(unsigned long long* dst, int64_t hi, int64_t lo) {
@@ -806,7 +815,7 @@ k_slice_rows_operand_whole(const StridedIn X, int64_t n, int64_t k, int64_t n_pa
         s_n[warp] = cnt;
     }
     for (int z = threadIdx.x; z < 2 * S.splits; z += blockDim.x) s_sum[z >> 1][z & 1] = 0;
-    if (c == 0 && threadIdx.x == 0) *S.status = kPassStatusOk;
+    clear_status(S, c == 0);
     if (c < k) {
         if (threadIdx.x == 0) S.range_w[c] = ColumnRange{0, 0, 0, 0};
         for (int z = threadIdx.x; z < 2 * S.splits_w; z += blockDim.x)
@@ -978,6 +987,7 @@ k_slice_gather(const StridedIn V, int64_t R, const int32_t* __restrict__ pos,
                const double* __restrict__ s_row, const double* __restrict__ mu, const SliceSums S,
                double* __restrict__ Wt) {
     chain_enter();
+    clear_status(S, blockIdx.x == 0 && blockIdx.y == 0);
     const int64_t c = blockIdx.y;
     unsigned long long mx = 0;
     long long es = 0;
@@ -1155,6 +1165,18 @@ void configure_slices() {
     }, "configure slice kernels");
 }
 
+// CS_B200_GIVE_UP=i: the process's FP64 pass number i (from 0) is reported as one that gave up waiting
+// (the word is set behind it on the stream), so that tests can see what each caller makes of that.
+void report_as_given_up(int* status, cudaStream_t s) {
+    static const long long which = [] {
+        const char* v = std::getenv("CS_B200_GIVE_UP");
+        return v ? std::atoll(v) : -1LL;
+    }();
+    if (which < 0) return;
+    static std::atomic<long long> passes{0};
+    if (passes.fetch_add(1) == which) CS_CUDA(cudaMemsetAsync(status, 1, sizeof(int), s));
+}
+
 template <bool ROWS, bool PAIR, int DIGITS = kDigits>
 void launch_slice_pass(const SlicePlan& p, const CUtensorMap& ta, const CUtensorMap& tb,
                        const SliceArgs& A, cudaStream_t s) {
@@ -1190,6 +1212,7 @@ void launch_slice_pass(const SlicePlan& p, const CUtensorMap& ta, const CUtensor
     }
     chain(cfg, attr);
     CS_CUDA(cudaLaunchKernelEx(&cfg, k_slice_pass<ROWS, PAIR, groups_of<PAIR>(), DIGITS>, ta, tb, A));
+    if (DIGITS == kDigits) report_as_given_up(A.status, s);
 }
 
 }  // namespace
@@ -1198,6 +1221,7 @@ struct SliceOperator {
     DeviceBuffer<int8_t> b;
     DeviceBuffer<double> part, W;
     DeviceBuffer<unsigned long long> words;  // SliceCall's
+    DeviceBuffer<int> status;                // a word of its own: the chunks of a call share it
     // packed rows and their sample-major copy, 128 rows x 128 bytes at a time (both belong to the
     // operator and keep their place for its lifetime)
     CUtensorMap tm_packed{}, tm_packed_t{};
@@ -1212,8 +1236,8 @@ namespace {
 // keeps a K slice's digits in L2.
 constexpr int64_t kChunkColumns = 288;
 
-// One chunk of columns: the plans of the passes it runs and its cleared words (status: 8 words;
-// ranges of X and W: 4 a column; slice sums of both passes: 2 a column and slice).
+// One chunk of columns: the plans of the passes it runs and its cleared words (ranges of X and W: 4 a
+// column; slice sums of both passes: 2 a column and slice).
 struct SliceCall {
     SlicePlan rows, samples;
     int64_t k = 0, range = 0, range_w = 0, sum = 0, sum_w = 0, words = 0;
@@ -1224,7 +1248,7 @@ SliceCall plan_call(const MixedRows& r, int64_t k) {
     c.k = k;
     c.rows = choose_slice_plan(true, r.r_pad / kTile, (int)(r.n_pad / kKBlock), k);
     c.samples = choose_slice_plan(false, r.n_pad / kTile, (int)(r.r_pad / kKBlock), k);
-    c.range = 8;
+    c.range = 0;
     c.range_w = c.range + 4 * k;
     c.sum = c.range_w + 4 * k;
     c.sum_w = c.sum + 2 * k * c.rows.splits;
@@ -1232,10 +1256,11 @@ SliceCall plan_call(const MixedRows& r, int64_t k) {
     return c;
 }
 
-SliceSums sums_of(SliceOperator& so, const SliceCall& c) {
+SliceSums sums_of(SliceOperator& so, const SliceCall& c, bool clear) {
     unsigned long long* z = so.words.get();
     SliceSums S;
-    S.status = reinterpret_cast<int*>(z);
+    S.status = so.status.get();
+    S.clear = clear ? 1 : 0;
     S.range = reinterpret_cast<ColumnRange*>(z + c.range);
     S.range_w = reinterpret_cast<ColumnRange*>(z + c.range_w);
     S.sum = z + c.sum;
@@ -1250,6 +1275,13 @@ void reserve(SliceOperator& so, const MixedRows& r, const SliceCall& c) {
     so.part.resize(c.k * std::max(c.rows.splits * r.r_pad, c.samples.splits * r.n_pad));
     so.W.resize(r.R * c.k);
     so.words.resize(c.words);
+}
+
+// The status word, clear when it is new.
+void make_status(SliceOperator& so, cudaStream_t s) {
+    if (so.status.get()) return;
+    so.status.resize(1);
+    CS_CUDA(cudaMemsetAsync(so.status.get(), 0, sizeof(int), s));
 }
 
 SliceArgs slice_args(const SlicePlan& p, bool rows, int64_t tiles, int kb, int64_t k) {
@@ -1297,7 +1329,7 @@ void run_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSu
         while (X.rs != 1 && kc < k && kc < 32) kc *= 2;
         const int64_t rpb = std::max<int64_t>(256, 4096 / kc);
         launch_chained(k_slice_ranges, dim3((unsigned)((n + rpb - 1) / rpb), (unsigned)((k + kc - 1) / kc)),
-                       256, 0, s, X, n, k, kc, rpb, S.range);
+                       256, 0, s, X, n, k, kc, rpb, S);
         if (k_pad <= 1)
             launch_chained(k_slice_rows_operand<1, 1024>, dim3((unsigned)((r.n_pad + 1023) / 1024), 1), 64, 0,
                            s, X, n, k, k_pad, r.n_pad, slice_rows, S, B, so.b.get());
@@ -1394,6 +1426,7 @@ SliceOperator* slices_for(cs_kinship* op, int64_t k, bool samples, cudaStream_t 
         configure_slices();
         if (!op->slices) op->slices = new SliceOperator();
         SliceOperator& so = *op->slices;
+        make_status(so, s);
         if (!so.map_rows) {
             so.tm_packed = make_map_u8(r.rows, r.stride, R, r.stride, 128, kTile, true);
             so.map_rows = true;
@@ -1431,7 +1464,7 @@ bool kinship_apply_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut Y, 
     if (!so) return false;
     MixedRows& r = mixed_rows_for(op);
     for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
-        const SliceSums S = sums_of(*so, c);
+        const SliceSums S = sums_of(*so, c, c0 == 0 && !op->defer_checks);
         const StridedIn x = from_column(X, c0);
         run_rows(*so, r, c, S, x, s);
         finish_rows(*so, r, c, S, x, so->W.get(), nullptr, StridedOut{}, s);
@@ -1445,7 +1478,7 @@ bool multiply_zt_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut U, cu
     if (!so) return false;
     MixedRows& r = mixed_rows_for(op);
     for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
-        const SliceSums S = sums_of(*so, c);
+        const SliceSums S = sums_of(*so, c, c0 == 0 && !op->defer_checks);
         const StridedIn x = from_column(X, c0);
         run_rows(*so, r, c, S, x, s);
         finish_rows(*so, r, c, S, x, nullptr, op->d_view_pos.get(), from_column(U, c0), s);
@@ -1458,7 +1491,7 @@ bool multiply_z_slices(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cud
     if (!so) return false;
     MixedRows& r = mixed_rows_for(op);
     for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
-        const SliceSums S = sums_of(*so, c);
+        const SliceSums S = sums_of(*so, c, c0 == 0 && !op->defer_checks);
         CS_CUDA(cudaMemsetAsync(so->words.get(), 0, 8 * c.words, s));
         {
             prof::Scope ps("slice_gather", s, 0.0, 16.0 * r.R * c.k);
@@ -1472,15 +1505,23 @@ bool multiply_z_slices(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cud
 }
 
 static void check_slices(SliceOperator* so, cudaStream_t s) {
-    if (!so || !so->words.get()) return;
+    if (!so || !so->status.get()) return;
     int status = 0;
-    CS_CUDA(cudaMemcpyAsync(&status, so->words.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    CS_CUDA(cudaMemcpyAsync(&status, so->status.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
     CS_CUDA(cudaStreamSynchronize(s));
-    if (status != kPassStatusOk)
+    if (status != kPassStatusOk) {
+        cudaMemsetAsync(so->status.get(), 0, sizeof(int), s);
+        cudaStreamSynchronize(s);
         fail(CS_ERR_CUDA, "tensor-core kinship kernel gave up waiting (status " + std::to_string(status) + ")");
+    }
 }
 
 void check_slices(cs_kinship* op, cudaStream_t s) { check_slices(op->slices, s); }
+
+void clear_slices(cs_kinship* op, cudaStream_t s) {
+    if (op->slices && op->slices->status.get())
+        CS_CUDA(cudaMemsetAsync(op->slices->status.get(), 0, sizeof(int), s));
+}
 
 bool scan_project_slices(SliceOperator*& state, MixedRows& r, StridedIn X, int64_t k, StridedOut T,
                          cudaStream_t s) {
@@ -1489,6 +1530,7 @@ bool scan_project_slices(SliceOperator*& state, MixedRows& r, StridedIn X, int64
         configure_slices();
         if (!state) state = new SliceOperator();
         SliceOperator& so = *state;
+        make_status(so, s);
         if (!so.map_rows) {
             so.tm_packed = make_map_u8(r.rows, r.stride, r.R, r.stride, 128, kTile, true);
             so.map_rows = true;
@@ -1507,7 +1549,7 @@ bool scan_project_slices(SliceOperator*& state, MixedRows& r, StridedIn X, int64
     }
     SliceOperator& so = *state;
     for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
-        const SliceSums S = sums_of(so, c);
+        const SliceSums S = sums_of(so, c, c0 == 0);
         const StridedIn x = from_column(X, c0);
         run_rows(so, r, c, S, x, s);
         finish_rows(so, r, c, S, x, nullptr, nullptr, from_column(T, c0), s);

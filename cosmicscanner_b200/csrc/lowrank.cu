@@ -736,7 +736,7 @@ void lmm_prepare_lowrank(cs_lmm* l, cs_kinship* op, const double* y, const doubl
     t.trace = op->trace;
     t.apply = [op, precision](const double* X_, int64_t ldx, int64_t k, double* Y_, int64_t ldy,
                               cudaStream_t st) {
-        kinship_apply_rowmajor(op, X_, ldx, k, Y_, ldy, precision, st);
+        kinship_apply_checked(op, X_, ldx, k, Y_, ldy, precision, st);
     };
     t.fuse_scan_columns = precision == CS_PRECISION_MIXED && op->keep_identity;
     lmm_prepare_lowrank_target(l, t, y, X, p, rank, oversample, seed, trace_threshold, min_rank,

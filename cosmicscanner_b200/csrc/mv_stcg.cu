@@ -124,7 +124,7 @@ struct MvState {
     // Out = Q (Vg (x) K + Ve (x) I) W over the first k columns (whole groups)
     void apply(const double* W, int64_t k, double* Out, cudaStream_t s) {
         KW.resize(n * C);
-        kinship_apply_rowmajor(op, W, C, k, KW.get(), C, precision, s);
+        kinship_apply_checked(op, W, C, k, KW.get(), C, precision, s);
         ++applies;
         apply_cols += k;
         prof::Scope ps("mv_kron_combine", s, 4.0 * (double)n * k * d, 24.0 * (double)n * k);
@@ -150,6 +150,7 @@ int64_t solve_groups(MvState& st, const double* B, double* Xs, int64_t k, double
     const int64_t n = st.n, C = st.C;
     const int d = st.d;
     const int64_t g = k / d;
+    const DeferChecks defer(st.op, s);
     ws.R.resize(n * C);
     ws.P.resize(n * C);
     ws.AP.resize(n * C);
@@ -207,6 +208,7 @@ int64_t solve_groups(MvState& st, const double* B, double* Xs, int64_t k, double
         k_cg_dir<<<grid_1d(n * k), 256, 0, s>>>(ws.P.get(), ws.Zp.get(), C, n, k, ws.beta.get());
         CS_LAUNCH("mv_cg_dir");
     }
+    kinship_check(st.op, s);
     CS_CUDA(cudaStreamSynchronize(s));
     return iters;
 }
@@ -332,7 +334,7 @@ void mv_stcg_solve(cs_kinship* op, double divisor, const double* Y, int32_t d, c
         CS_CUDA(cudaMemcpy2DAsync(KP.get() + d, 8 * k, Bk.get() + d, 8 * k, 8 * S * d, n,
                                   cudaMemcpyDeviceToDevice, s));
         st.KW.resize(n * k);
-        kinship_apply_rowmajor(op, KP.get(), k, k, st.KW.get(), k, opt.precision, s);
+        kinship_apply_checked(op, KP.get(), k, k, st.KW.get(), k, opt.precision, s);
         ++st.applies;
         st.apply_cols += k;
         // cross products: [P Y | P Z]^T [fac K PY | fac K Z] and [P Y | P Z]^T [PY | Z]

@@ -504,7 +504,7 @@ const double* VOperator::kinship(const double* in, int64_t ldi, int64_t k, int64
     const double* U = gather(in, ldi, k, s);
     ldu = rm->identity ? ldi : k;
     ku.resize(std::max<int64_t>(1, rm->n_rows * k));
-    kinship_apply_rowmajor(op, U, ldu, k, ku.get(), k, precision, s);
+    kinship_apply_checked(op, U, ldu, k, ku.get(), k, precision, s);
     ++applies;
     apply_cols += k;
     return U;
@@ -541,7 +541,7 @@ void VOperator::derivatives(const double* in, int64_t ldi, int64_t k, double* g_
     const double* U = gather(in, ldi, k, s);
     const int64_t ldu = rm->identity ? ldi : k;
     ku.resize(std::max<int64_t>(1, rm->n_rows * k));
-    kinship_apply_rowmajor(op, U, ldu, k, ku.get(), k, precision, s);
+    kinship_apply_checked(op, U, ldu, k, ku.get(), k, precision, s);
     ++applies;
     apply_cols += k;
     prof::Scope ps("records_scatter", s, 0.0, 8.0 * 2.0 * (double)rm->n_rec * k);
@@ -557,7 +557,7 @@ void VOperator::genetic_rows(const double* in, int64_t ldi, int64_t k, double* r
     const double* U = gather(in, ldi, k, s);
     const int64_t ldu = rm->identity ? ldi : k;
     ku.resize(std::max<int64_t>(1, rm->n_rows * k));
-    kinship_apply_rowmajor(op, U, ldu, k, ku.get(), k, precision, s);
+    kinship_apply_checked(op, U, ldu, k, ku.get(), k, precision, s);
     ++applies;
     apply_cols += k;
     k_scale_copy<<<grid_for(rm->n_rows * k), 256, 0, s>>>(ku.get(), k, rm->n_rows, k, fac,
@@ -658,7 +658,7 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
     st.column_iterations = 0;
     if (k <= 0) return;
     const int64_t n = A.rm->n_rec;
-    const DeferChecks defer(A.op);
+    const DeferChecks defer(A.op, s);
     CS_CUDA(cudaMemset2DAsync(X, ldx * 8, 0, k * 8, n, s));
     ws.R.resize(n * k);
     ws.P.resize(n * k);
@@ -747,7 +747,7 @@ void pcg_solve_block(VOperator& A, double diag, const double* B, int64_t ldb, in
         }
         CS_CUDA(cudaStreamSynchronize(s));
         for (int64_t c = 0; c < ka; ++c)
-            if (std::isnan(rr_h[c])) {  // an apply that gave up leaves NaN
+            if (std::isnan(rr_h[c])) {  // an FP64 apply that gave up leaves NaN (a mixed one may not)
                 kinship_check(A.op, s);
                 break;
             }

@@ -219,7 +219,7 @@ static double slq_logdet(cs_vce* v, int probes, int steps, uint64_t seed, cudaSt
     std::fill(actual.begin() + k, actual.end(), m);
     CS_CUDA(cudaMemsetAsync(d_ab.get(), 0, 16 * (int64_t)m * k, s));
     CS_CUDA(cudaMemcpyAsync(d_done.get(), actual.data(), 8 * k, cudaMemcpyHostToDevice, s));
-    const DeferChecks defer(v->V.op);
+    const DeferChecks defer(v->V.op, s);
     for (int j = 0; j < m; ++j) {
         const LanczosState st{dcoef.get(), d_ab.get() + (int64_t)j * k, d_ab.get() + (int64_t)(m + j) * k,
                               d_done.get(), d_done.get() + k};
@@ -347,7 +347,7 @@ void vce_solve_stcg(cs_vce* v, cs_kinship* op, double divisor, const int32_t* re
             const int prec = opt.precision;
             t.apply = [op, prec](const double* X_, int64_t ldx, int64_t k, double* Y_, int64_t ldy,
                                  cudaStream_t st2) {
-                kinship_apply_rowmajor(op, X_, ldx, k, Y_, ldy, prec, st2);
+                kinship_apply_checked(op, X_, ldx, k, Y_, ldy, prec, st2);
             };
             std::vector<double> Xc(std::max<int64_t>(1, n * p));
             std::copy(X, X + n * p, Xc.begin());

@@ -134,11 +134,18 @@ struct PcgWorkspace {
 };
 
 // Applies inside a solver's loop leave the check for a pass that gave up waiting to the loop's own
-// synchronisations (kinship_check), instead of waiting for the stream after each apply.
+// synchronisations (kinship_check), instead of waiting for the stream after each apply.  The outermost
+// one begins with a clear status; the applies below it only add to that.
 struct DeferChecks {
     cs_kinship* op;
     bool before;
-    explicit DeferChecks(cs_kinship* o) : op(o), before(o->defer_checks) { op->defer_checks = true; }
+    DeferChecks(cs_kinship* o, cudaStream_t s) : op(o), before(o->defer_checks) {
+        if (!before) {
+            clear_slices(op, s);
+            clear_mixed(op, s);
+        }
+        op->defer_checks = true;
+    }
     ~DeferChecks() { op->defer_checks = before; }
     DeferChecks(const DeferChecks&) = delete;
     DeferChecks& operator=(const DeferChecks&) = delete;
