@@ -931,9 +931,9 @@ def main():
         f_ms = ftop["ms"] / ftop["launches"]
         f_ach = ftop["flops"] / ftop["launches"] / (f_ms * 1e-3) / 1e12
         if "_slices" in ftop["name"]:
-            # seven int8 digits a column: 13 (rows) or 14 (samples) int8 products for each of the
+            # eight int8 digits a column: 15 (rows) or 16 (samples) int8 products for each of the
             # algorithmic ones
-            f_sets = 13 if "rows" in ftop["name"] else 14
+            f_sets = 15 if "rows" in ftop["name"] else 16
             fpeaks, fkind = measured_peaks()
             f_peak = fpeaks["bf16_tflops"]
             f_roof = {"bound": "tensor", "peak_kind": f"bf16_tflops ({fkind})",

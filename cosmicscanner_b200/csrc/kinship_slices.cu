@@ -1,24 +1,30 @@
 // The FP64 form of the kinship products on the int8 tensor cores.
 //
-// Arithmetic.  Each right-hand side column becomes a 55-bit fixed-point column (one power of two
-// per column, the largest element just below 2^55), split into seven int8 digits of base 256
-// (balanced, -128..127): x = 2^-e sum_p d_p 256^(6-p) with an error of at most 2^-55 of the
+// Arithmetic.  Each right-hand side column becomes a 63-bit fixed-point column (one power of two
+// per column, the largest element just below 2^63), split into eight int8 digits of base 256
+// (balanced, -128..127): x = 2^-e sum_p d_p 256^(7-p) with an error of at most 2^-63 of the
 // column's maximum.  Genotype codes are small integers, so every product and every sum of the
-// int8 MMAs is exact in int32, the seven sums of an output are put together in 64-bit
-// integers, and the centring by the SNP means is done on those before the single conversion
-// to FP64.  (Splitting a floating-point operand into slices whose products accumulate exactly:
-// Ozaki, Ogita, Oishi, Rump 2012; on integer matrix units: Ootomo, Ozaki, Yokota 2024.)  An
-// FP64 sum of K products carries a rounding error of the order of 2^-53 sqrt(K) of the result
-// at best; here only the operand's own rounding remains.
+// int8 MMAs is exact in int32, the eight sums of an output are put together in two 64-bit
+// integers (three digits and five), and the centring by the SNP means is done on those before the
+// single conversion to FP64.  (Splitting a floating-point operand into slices whose products
+// accumulate exactly: Ozaki, Ogita, Oishi, Rump 2012; on integer matrix units: Ootomo, Ozaki,
+// Yokota 2024.)  An FP64 sum of K products carries a rounding error of the order of 2^-53 sqrt(K)
+// of the result at best; here only the operand's own rounding remains.
+//   Eight digits and not seven: an element 2^-b of its column's maximum keeps 63 - b bits, and b
+// is large where a column is uneven.  W = s^2 o Z^T x of the samples pass is: a variant that one
+// sample carries has s^2 = n.  With 5 % of such variants among 3,000 at 6,000 samples K x was off by
+// 1.5e-15 to 2.9e-15 with seven digits, 1.1e-15 as FP64 sums, 8e-17 with eight.  The eighth digit costs wide
+// blocks MMAs (18,009 x 27,006 and 266 columns: 3.23 ms instead of 2.74) and narrow ones nothing (up to four
+// columns a column has eight B rows either way; 50,000 x 100,000 and one column 0.93 ms).
 //
 //   rows pass     63 u_t / s_t = sum_obs 63 G x + sum_miss q_t x + (63 mu_t - q_t) sum_miss x
 //                                - 63 mu_t sum x
 //     with the imputed-code tile (63 G, or q_t = rint(63 mu_t) for a missing call) against the
-//     seven digits and the missing-indicator tile against the first six (|63 mu_t - q_t| <= 1/2
+//     eight digits and the missing-indicator tile against the first seven (|63 mu_t - q_t| <= 1/2
 //     takes the place of the last); 63 mu_t and the sums are carried in two doubles each, so the
 //     difference of the large terms does not round.
 //   samples pass  M y_i = sum_t G w + sum_miss (mu w) - sum_t (mu w),  w = s o U
-//     with w and mu o w split at one scale (seven digits each) into the same accumulators; the
+//     with w and mu o w split at one scale (eight digits each) into the same accumulators; the
 //     last sum is taken over the same digits, so that a missing call cancels exactly.
 //
 // Kernel.  The passes keep the genotype tiles in tensor memory (A, K-major: the packed rows in
@@ -31,14 +37,14 @@
 // and a packed tile spans four K-blocks.  What bounds them now is the decode: 13 integer
 // operations per 16 genotypes at half rate are 208 of the 400 clocks a K-block takes, the ring and
 // wait instructions of all warps about 120 more (ncu: ALU pipe 70 % busy, tensor pipe 14 %, DRAM a
-// third of its rate).  Wide blocks are bound by the MMAs: 448 clocks a K-block of a 16-column
-// rows tile, 896 of a 32-column samples tile.  Wide blocks run on CTA pairs (cta_group::2):
+// third of its rate).  Wide blocks are bound by the MMAs: 512 clocks a K-block of a 16-column
+// rows tile, 1024 of a 32-column samples tile (N / 2 an instruction).  Wide blocks run on CTA pairs (cta_group::2):
 // each CTA holds half of the B rows, which halves the L2 reads of B that would otherwise bound
 // a wide block (64 bytes per clock and SM at the full MMA rate).
 //
 // Column tiles.  Up to 4 columns a column's digits sit in eight adjacent B rows (N = 8 w);
 // wider tiles are digit-major in widths of 8 per CTA.  TMEM (512 columns) holds the
-// accumulators (rows: main and missing-call sums apart, 13 per column; samples: 7) and the
+// accumulators (rows: main and missing-call sums apart, 15 per column; samples: 8) and the
 // A stages (64 columns each).
 //
 // The mixed form's passes of up to 48 columns run on the same kernel with three digits (mixed_narrow_pass):
@@ -68,7 +74,7 @@ using namespace sm100;
 
 constexpr int kTile = kTcTile;
 constexpr int kKBlock = 128;
-constexpr int kDigits = 7;
+constexpr int kDigits = 8;
 constexpr int kEpiWarp0 = 4, kDecWarp0 = 8;
 // decoder groups of four warps: G, by kernel
 constexpr int threads_for(int groups) { return (kDecWarp0 + 4 * groups) * 32; }
@@ -103,10 +109,17 @@ struct SliceArgs {
     uint32_t poll_ns, poll_dec_ns;
 };
 
-// hi 2^32 + lo of the seven digit sums of one output
+// hi 2^40 + lo of the eight digit sums of one output: hi of three digits, below 2^47, so that its
+// conversion is exact and a difference of large terms does not round; lo of five, at most
+// 126 * 2^17 (K) * 2^39.006 < 2^63.
+constexpr double kLowDigits = 1099511627776.0;  // 2^40
 __device__ __forceinline__ void join_digits(const int32_t (&m)[8], int64_t& hi, int64_t& lo) {
-    hi = ((int64_t)m[0] << 16) + ((int64_t)m[1] << 8) + (int64_t)m[2];
-    lo = ((int64_t)m[3] << 24) + ((int64_t)m[4] << 16) + ((int64_t)m[5] << 8) + (int64_t)m[6];
+    hi = lo = 0;
+#pragma unroll
+    for (int p = 0; p < kDigits; ++p) {
+        if (p < 3) hi = hi * 256 + m[p];
+        else lo = lo * 256 + m[p];
+    }
 }
 
 // Per SNP row: 63 mu in two doubles and 63 mu - q.
@@ -118,15 +131,14 @@ struct RowCentre {
 // of the slice's fixed-point values.
 __device__ __forceinline__ double rows_value(const RowCentre& c, int64_t mh, int64_t ml, int64_t xh,
                                              int64_t xl, double sh, double sl) {
-    const double two32 = 4294967296.0;
-    const double m1 = (double)mh * two32, m0 = (double)ml;
-    const double x = fma((double)xh, two32, (double)xl);
+    const double m1 = (double)mh * kLowDigits, m0 = (double)ml;
+    const double x = fma((double)xh, kLowDigits, (double)xl);
     const double p = c.ah * sh, pe = fma(c.ah, sh, -p);
     const double d = m1 - p;
     return d + (((m0 - c.ah * sl) - pe) + fma(c.b, x, c.al * (x - (sh + sl))));
 }
 
-// DIGITS = 7: the FP64 form.  DIGITS = 3: the mixed form of kinship_mixed.cu (pieces of base 254,
+// DIGITS = 8: the FP64 form.  DIGITS = 3: the mixed form of kinship_mixed.cu (pieces of base 254,
 // one column tile on single CTAs), with that file's operands, K slices (any number of K-blocks)
 // and epilogue arithmetic, so that the bits are those of its own kernels.
 template <bool ROWS, bool PAIR, int G, int DIGITS>
@@ -491,9 +503,9 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                 const longlong2 sum = ks[c];
                 double v;
                 if (ROWS)
-                    v = rows_value(rc, mh, ml, xh, xl, (double)sum.x * 4294967296.0, (double)sum.y);
+                    v = rows_value(rc, mh, ml, xh, xl, (double)sum.x * kLowDigits, (double)sum.y);
                 else
-                    v = fma((double)(mh - sum.x), 4294967296.0, (double)(ml - sum.y));
+                    v = fma((double)(mh - sum.x), kLowDigits, (double)(ml - sum.y));
                 dst[(int64_t)c * P.ld] = v;
             };
             if (DIGITS == 3) {
@@ -506,7 +518,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                     join_digits(m, mh, ml);
                     if (ROWS) {
                         tmem_ld8i(tb + P.nm + 8 * c, m);
-                        m[6] = 0;
+                        m[kDigits - 1] = 0;
                         join_digits(m, xh, xl);
                     }
                     emit(c, mh, ml, xh, xl);
@@ -576,14 +588,14 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
 
 // ---------------------------------------------------------------- operand preparation
 
-// Exponent e of the column's scale: |x| 2^e <= 127 2^48 for every element, 2^54 <= max 2^e or the
+// Exponent e of the column's scale: |x| 2^e <= 127 2^56 for every element, 2^62 <= max 2^e or the
 // half of it.
 __device__ __forceinline__ int slice_exponent(unsigned long long max_bits) {
     if (max_bits == 0) return 0;
     const int ex = (int)(max_bits >> 52) - 1023;
-    // mantissa above 127/64 would round up to 128 2^48
+    // mantissa above 127/64 would round up to 128 2^56
     const bool top = (max_bits & 0xFFFFFFFFFFFFFull) > 0xFC00000000000ull;
-    return max(-kSliceMaxExp, min(kSliceMaxExp + 60, (top ? 53 : 54) - ex));
+    return max(-kSliceMaxExp, min(kSliceMaxExp + 62, (top ? 61 : 62) - ex));
 }
 __device__ __forceinline__ double pow2(int e) {
     return __longlong_as_double((long long)(e + 1023) << 52);
@@ -681,7 +693,7 @@ __device__ __forceinline__ void transpose4(const uint32_t (&in)[4], uint32_t (&o
     out[3] = __byte_perm(c, d, 0x7632);
 }
 
-// The seven digits of 16 fixed-point values, each digit's 16 bytes in the interleaved order of
+// The eight digits of 16 fixed-point values, each digit's 16 bytes in the interleaved order of
 // the decoded tiles: dig[p] for digit p (0 the most significant).
 __device__ __forceinline__ void digits16(const int64_t (&v)[16], uint4 (&dig)[kDigits]) {
 #pragma unroll
@@ -690,29 +702,30 @@ __device__ __forceinline__ void digits16(const int64_t (&v)[16], uint4 (&dig)[kD
         uint32_t lo[4], hi[4], tl[4], th[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            // adding 128 to each of the lower six digits makes the plain bytes the balanced
+            // adding 128 to each of the lower seven digits makes the plain bytes the balanced
             // digits plus 128
-            const uint64_t u = (uint64_t)v[sample_at(4 * g + j)] + 0x0000808080808080ull;
+            const uint64_t u = (uint64_t)v[sample_at(4 * g + j)] + 0x0080808080808080ull;
             lo[j] = (uint32_t)u ^ 0x80808080u;
-            hi[j] = (uint32_t)(u >> 32) ^ 0x00008080u;
+            hi[j] = (uint32_t)(u >> 32) ^ 0x00808080u;
         }
         transpose4(lo, tl);
         transpose4(hi, th);
         uint32_t* w = reinterpret_cast<uint32_t*>(dig);
-        w[0 * 4 + g] = th[2];
-        w[1 * 4 + g] = th[1];
-        w[2 * 4 + g] = th[0];
-        w[3 * 4 + g] = tl[3];
-        w[4 * 4 + g] = tl[2];
-        w[5 * 4 + g] = tl[1];
-        w[6 * 4 + g] = tl[0];
+        w[0 * 4 + g] = th[3];
+        w[1 * 4 + g] = th[2];
+        w[2 * 4 + g] = th[1];
+        w[3 * 4 + g] = th[0];
+        w[4 * 4 + g] = tl[3];
+        w[5 * 4 + g] = tl[2];
+        w[6 * 4 + g] = tl[1];
+        w[7 * 4 + g] = tl[0];
     }
 }
 
-// (hi, lo) of v = hi 2^32 + lo with lo the value of the four lower digits
+// (hi, lo) of v = hi 2^40 + lo with lo the value of the five lower digits
 __device__ __forceinline__ void split_value(int64_t v, int64_t& hi, int64_t& lo) {
-    hi = (v + 0x80808080ll) >> 32;
-    lo = v - (hi << 32);
+    hi = (v + 0x8080808080ll) >> 40;
+    lo = v - (hi << 40);
 }
 
 struct BLayout {
@@ -944,7 +957,7 @@ k_slice_reduce_rows(const double* __restrict__ part, int64_t ld, int64_t R, int6
     chain_enter();
     const int64_t c = blockIdx.y;
     const ColumnRange rg = S.range[c];
-    const double f = pow2(-slice_exponent(rg.max_bits)) / (double)kTcQ;
+    const double f = pow2(-slice_exponent(rg.max_bits));
     const bool direct = range_excluded(rg);
     unsigned long long mx = 0;
     long long es = 0;
@@ -970,7 +983,7 @@ k_slice_reduce_rows(const double* __restrict__ part, int64_t ld, int64_t R, int6
         for (int64_t t = t0 + threadIdx.x; t < t1; t += 256) {
             double acc = 0.0;
             for (int z = 0; z < S.splits; ++z) acc += part[((int64_t)z * k + c) * ld + t];
-            finish(t, checked(acc * f, S.status));
+            finish(t, checked(acc * f * (1.0 / (double)kTcQ), S.status));
         }
     }
     if (!Wt) return;
@@ -1029,7 +1042,7 @@ k_slice_reduce_samples(const double* __restrict__ part, int64_t ld, int64_t n, i
             acc *= scale;
         } else {
             for (int z = 0; z < S.splits_w; ++z) acc += part[((int64_t)z * k + c) * ld + i];
-            acc = checked(acc * (pow2(-slice_exponent(rg.max_bits)) * scale), S.status);
+            acc = checked(acc * pow2(-slice_exponent(rg.max_bits)) * scale, S.status);
         }
         if (Y.rs == 1) Y.p[i + c * Y.cs] = acc;
         else tile[cc][tx] = acc;
@@ -1232,7 +1245,7 @@ void destroy_slices(SliceOperator* s) { delete s; }
 
 namespace {
 
-// Columns per call of the passes: bounds the operand buffers (14 bytes per row and column) and
+// Columns per call of the passes: bounds the operand buffers (16 bytes per row and column) and
 // keeps a K slice's digits in L2.
 constexpr int64_t kChunkColumns = 288;
 
@@ -1317,14 +1330,14 @@ void run_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSu
     const BLayout B = p.blayout(true);
     const int slice_rows = p.kbs * kKBlock;
     if (n <= kWholeRows && p.splits <= 64) {
-        prof::Scope ps("slice_prep_rows_operand", s, 0.0, 16.0 * n * k + 7.0 * k_pad * r.n_pad);
+        prof::Scope ps("slice_prep_rows_operand", s, 0.0, 16.0 * n * k + 8.0 * k_pad * r.n_pad);
         const unsigned threads = (unsigned)round_up(r.n_pad / 16, 32);
         launch_chained(k_slice_rows_operand_whole, (unsigned)k_pad, threads, 0, s, X, n, k, r.n_pad,
                        slice_rows, S, B, so.b.get());
         CS_LAUNCH("slice rows operand");
     } else {
         CS_CUDA(cudaMemsetAsync(so.words.get(), 0, 8 * c.words, s));
-        prof::Scope ps("slice_prep_rows_operand", s, 0.0, 16.0 * n * k + 7.0 * k_pad * r.n_pad);
+        prof::Scope ps("slice_prep_rows_operand", s, 0.0, 16.0 * n * k + 8.0 * k_pad * r.n_pad);
         int kc = 1;
         while (X.rs != 1 && kc < k && kc < 32) kc *= 2;
         const int64_t rpb = std::max<int64_t>(256, 4096 / kc);
@@ -1367,7 +1380,7 @@ void run_samples(SliceOperator& so, MixedRows& r, const SliceCall& c, const Slic
     const SlicePlan& p = c.samples;
     const int64_t k_pad = (int64_t)p.n_ctiles * p.w;
     {
-        prof::Scope ps("slice_prep_samples_operand", s, 0.0, 8.0 * R * k + 14.0 * k_pad * r.r_pad);
+        prof::Scope ps("slice_prep_samples_operand", s, 0.0, 8.0 * R * k + 16.0 * k_pad * r.r_pad);
         launch_chained(k_slice_samples_operand, dim3((unsigned)((r.r_pad + 2047) / 2048), (unsigned)k_pad),
                        128, 0, s, so.W.get(), R, k, r.r_pad, p.kbs * kKBlock, r.mu.get(), S, p.blayout(false),
                        so.b.get());

@@ -466,9 +466,9 @@ int64_t server_submit(cs_server* sv, const cs_serve_request* q) {
     r->own_view = (double)n < sv->opt.subset_fraction * (double)N;
     r->est_bytes = 8 * n * sk * 4 + W * ((n + 3) / 4 + 64 + 8 * (sk + r->p + 2)) + 64 * n;
     if (sv->opt.precision == CS_PRECISION_FP64) {
-        // the scan's seven digits a column and the partial sums of its projection
+        // the scan's eight digits a column and the partial sums of its projection
         const int64_t kp = round_up(std::min<int64_t>(sk + r->p + 1, 288), 16);
-        r->est_bytes += 7 * kp * round_up(n, 256) + 4 * 8 * kp * round_up(W, 256);
+        r->est_bytes += 8 * kp * round_up(n, 256) + 4 * 8 * kp * round_up(W, 256);
     }
     if (r->own_view) {
         // the packed copy of the cohort's columns, the right-hand-side pieces of both passes

@@ -17,15 +17,16 @@ struct ColumnRange {
     unsigned long long pad;
 };
 
-// A fixed-point column of 55 bits below its maximum holds every element to 2^-55 of that
-// maximum.  Normwise that is always finer than FP64 sums are (max <= sqrt(n) rms), but a row
-// whose large elements all meet missing calls depends on the small ones alone, so a column
-// whose elements lie on average more than 2^kSliceRange below its maximum is computed on the FP64
-// pipe, like one with a non-finite value or a maximum near the ends of the exponent range.  A
-// normal sample of 50,000 lies 2^3 below its maximum; W = s^2 o Z^T X down to a minor allele
-// frequency of 0.01 at most 2^4 more.
+// A fixed-point column holds every element to 2^-63 of its maximum.  A column whose nonzero elements
+// lie on (geometric) average more than 2^kSliceRange below that maximum is computed on the FP64 pipe:
+// up to there the average element has the 53 bits of an FP64 value, so that also what depends on the
+// small elements alone (a row whose large ones all meet missing calls) is as good as FP64 sums.  So is
+// a column with a non-finite value or a maximum near the ends of the exponent range (the scales and
+// the scaled results stay normal numbers).  A normal sample of 50,000 lies 2^3 below its maximum;
+// W = s^2 o Z^T X 2^4 more with minor allele frequencies down to 0.01, and 2^7 with 1 % of the variants at
+// allele counts of 1 to 20 among 200,000 samples.
 constexpr int kSliceRange = 10;
-constexpr int kSliceMaxExp = 960;
+constexpr int kSliceMaxExp = 940;
 
 __device__ __forceinline__ bool range_excluded(const ColumnRange& r) {
     const int ex = (int)(r.max_bits >> 52) - 1023;
