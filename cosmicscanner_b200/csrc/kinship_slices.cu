@@ -13,15 +13,15 @@
 //   Eight digits and not seven: an element 2^-b of its column's maximum keeps 63 - b bits, and b
 // is large where a column is uneven.  W = s^2 o Z^T x of the samples pass is: a variant that one
 // sample carries has s^2 = n.  With 5 % of such variants among 3,000 at 6,000 samples K x was off by
-// 1.5e-15 to 2.9e-15 with seven digits, 1.1e-15 as FP64 sums, 8e-17 with eight.  The eighth digit costs wide
-// blocks MMAs (18,009 x 27,006 and 266 columns: 3.23 ms instead of 2.74) and narrow ones nothing (up to four
-// columns a column has eight B rows either way; 50,000 x 100,000 and one column 0.93 ms).
+// 1.5e-15 to 2.9e-15 with seven digits, 1.1e-15 as FP64 sums, 8e-17 with eight.  An even column (range_uneven)
+// needs no more than seven; its last digit is zero, whatever its neighbours are, and its results are those of
+// seven digits.  A product of 266 columns at 18,009 x 27,006 takes 2.90 ms, 2.73 with seven digits for all.
 //
 //   rows pass     63 u_t / s_t = sum_obs 63 G x + sum_miss q_t x + (63 mu_t - q_t) sum_miss x
 //                                - 63 mu_t sum x
 //     with the imputed-code tile (63 G, or q_t = rint(63 mu_t) for a missing call) against the
-//     eight digits and the missing-indicator tile against the first seven (|63 mu_t - q_t| <= 1/2
-//     takes the place of the last); 63 mu_t and the sums are carried in two doubles each, so the
+//     digits and the missing-indicator tile against all but the column's last (|63 mu_t - q_t| <= 1/2
+//     takes its place); 63 mu_t and the sums are carried in two doubles each, so the
 //     difference of the large terms does not round.
 //   samples pass  M y_i = sum_t G w + sum_miss (mu w) - sum_t (mu w),  w = s o U
 //     with w and mu o w split at one scale (eight digits each) into the same accumulators; the
@@ -37,10 +37,10 @@
 // and a packed tile spans four K-blocks.  What bounds them now is the decode: 13 integer
 // operations per 16 genotypes at half rate are 208 of the 400 clocks a K-block takes, the ring and
 // wait instructions of all warps about 120 more (ncu: ALU pipe 70 % busy, tensor pipe 14 %, DRAM a
-// third of its rate).  Wide blocks are bound by the MMAs: 512 clocks a K-block of a 16-column
-// rows tile, 1024 of a 32-column samples tile (N / 2 an instruction).  Wide blocks run on CTA pairs (cta_group::2):
-// each CTA holds half of the B rows, which halves the L2 reads of B that would otherwise bound
-// a wide block (64 bytes per clock and SM at the full MMA rate).
+// third of its rate).  Wide blocks come nearer to the MMAs (N / 2 clocks each): 512 of the 660 clocks that
+// a K-block of a 16-column rows tile takes, and a 32-column samples tile is at theirs, 1024.  Wide blocks run
+// on CTA pairs (cta_group::2): each CTA holds half of the B rows, which halves the L2 reads of B that would
+// otherwise bound a wide block (64 bytes per clock and SM at the full MMA rate).
 //
 // Column tiles.  Up to 4 columns a column's digits sit in eight adjacent B rows (N = 8 w);
 // wider tiles are digit-major in widths of 8 per CTA.  TMEM (512 columns) holds the
@@ -499,6 +499,11 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                 }
             }
             const longlong2* ks = P.ksum + (int64_t)split * P.k + c_base;
+            // the missing-call sums leave out a column's last digit (the ranges stand in front of the sums:
+            // SliceCall)
+            const ColumnRange* const range = reinterpret_cast<const ColumnRange*>(P.ksum) - P.k + c_base;
+            const unsigned uneven = ROWS && DIGITS == kDigits
+                ? __ballot_sync(0xffffffffu, lane < cols && range_uneven(range[lane])) : 0u;
             auto emit = [&](int c, int64_t mh, int64_t ml, int64_t xh, int64_t xl) {
                 const longlong2 sum = ks[c];
                 double v;
@@ -519,6 +524,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                     if (ROWS) {
                         tmem_ld8i(tb + P.nm + 8 * c, m);
                         m[kDigits - 1] = 0;
+                        if (!(uneven >> c & 1u)) m[kDigits - 2] = 0;
                         join_digits(m, xh, xl);
                     }
                     emit(c, mh, ml, xh, xl);
@@ -550,6 +556,7 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                             tmem_ld8i(cx + p * P.hw, m);
 #pragma unroll
                             for (int i = 0; i < 8; ++i) {
+                                if (p == kDigits - 2 && !(uneven >> (c0 + i) & 1u)) m[i] = 0;
                                 if (p < 3) xh[i] = xh[i] * 256 + m[i];
                                 else xl[i] = xl[i] * 256 + m[i];
                             }
@@ -683,6 +690,17 @@ k_slice_ranges(const StridedIn X, int64_t n, int64_t k, int kc, int64_t rows_per
     if (tr == 0 && c < k) add_range(&S.range[c], s_mx[threadIdx.x], s_es[threadIdx.x], s_n[threadIdx.x]);
 }
 
+// The scale of a column: its fixed-point values are rint(x f) << shift, the low digit zero in an even one.
+struct SliceScale {
+    double f;
+    int shift;
+    __device__ __forceinline__ explicit SliceScale(const ColumnRange& r)
+        : f(pow2(slice_exponent(r.max_bits) - (range_uneven(r) ? 0 : 8))), shift(range_uneven(r) ? 0 : 8) {}
+    __device__ __forceinline__ int64_t value(double x) const {
+        return (int64_t)((uint64_t)__double2ll_rn(x * f) << shift);
+    }
+};
+
 // Transposes 4 x 4 bytes: out[j] = byte j of in[0..3].
 __device__ __forceinline__ void transpose4(const uint32_t (&in)[4], uint32_t (&out)[4]) {
     const uint32_t a = __byte_perm(in[0], in[1], 0x5140), b = __byte_perm(in[2], in[3], 0x5140);
@@ -780,11 +798,11 @@ k_slice_rows_operand(const StridedIn X, int64_t n, int64_t k, int64_t k_pad, int
     const bool live = c < k_pad && i0 < n_pad;
     int64_t sh = 0, sl = 0;
     if (live) {
-        const double f = c < k ? pow2(slice_exponent(S.range[c].max_bits)) : 0.0;
+        const SliceScale sc(c < k ? S.range[c] : ColumnRange{0, 0, 0, 0});
         int64_t v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            v[j] = __double2ll_rn(tile[cc][17 * grp + j] * f);
+            v[j] = sc.value(tile[cc][17 * grp + j]);
             int64_t h, l;
             split_value(v[j], h, l);
             sh += h;
@@ -843,12 +861,13 @@ k_slice_rows_operand_whole(const StridedIn X, int64_t n, int64_t k, int64_t n_pa
         es += s_es[w];
         n_all += s_n[w];
     }
-    if (threadIdx.x == 0 && c < k) S.range[c] = ColumnRange{mx, es, n_all, 0};
-    const double f = pow2(slice_exponent(mx));
+    const ColumnRange rg{mx, es, n_all, 0};
+    if (threadIdx.x == 0 && c < k) S.range[c] = rg;
+    const SliceScale sc(rg);
     int64_t v[16], sh = 0, sl = 0;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-        v[j] = __double2ll_rn(x[j] * f);
+        v[j] = sc.value(x[j]);
         int64_t h, l;
         split_value(v[j], h, l);
         sh += h;
@@ -890,14 +909,14 @@ k_slice_samples_operand(const double* __restrict__ Wt, int64_t R, int64_t k, int
     const bool live = t0 < r_pad;
     int64_t sh = 0, sl = 0;
     if (live) {
-        const double f = c < k ? pow2(slice_exponent(S.range_w[c].max_bits)) : 0.0;
+        const SliceScale sc(c < k ? S.range_w[c] : ColumnRange{0, 0, 0, 0});
         int64_t v[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = __double2ll_rn(sw[17 * threadIdx.x + j] * f);
+        for (int j = 0; j < 16; ++j) v[j] = sc.value(sw[17 * threadIdx.x + j]);
         emit_digits(v, B, c, 0, t0, r_pad, out);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            v[j] = __double2ll_rn(sb[17 * threadIdx.x + j] * f);
+            v[j] = sc.value(sb[17 * threadIdx.x + j]);
             int64_t h, l;
             split_value(v[j], h, l);
             sh += h;
@@ -1129,18 +1148,21 @@ void choose_slices(SlicePlan& p, int64_t units, int kb, int ctas) {
 }
 
 // The plan with the least estimated time.  A K-block costs its MMAs (N / 2 clocks for each of
-// 4 + 4 instructions on a CTA) or its decode, whichever is longer.
+// 4 + 4 instructions on a CTA) or its decode, whichever is longer.  The costs are those of seven
+// digits: with them the plans were measured, the eighth digit's MMAs do not show (1.28 and 1.30 ms a rows pass,
+// 1.04 and 1.04 a samples pass of 266 columns at 18,009 x 27,006), and the K slices, whose sums are added in
+// FP64, stay where they were.
 SlicePlan choose_slice_plan(bool rows, int64_t tiles, int kb, int64_t k) {
     SlicePlan best;
     best.cost = 1e300;
     auto consider = [&](bool pair, int w) {
-        SlicePlan p;
-        if (!lay_out(rows, pair, w, k, p)) return;
+        SlicePlan p, seven;
+        if (!lay_out(rows, pair, w, k, p) || !lay_out(rows, pair, w, k, seven, kDigits - 1)) return;
         const int ctas = pair ? num_sms() / 2 : num_sms();
         choose_slices(p, (pair ? tiles / 2 : tiles) * p.n_ctiles, kb, ctas);
-        const double mma = 2.0 * (rows ? p.nm + p.nx : 2 * p.nm);
+        const double mma = 2.0 * (rows ? seven.nm + seven.nx : 2 * seven.nm);
         // a single CTA streams all B rows from L2 itself
-        const double l2 = (pair ? 0.5 : 1.0) * (rows ? 1 : 2) * p.nm * 128.0 / 28.0;
+        const double l2 = (pair ? 0.5 : 1.0) * (rows ? 1 : 2) * seven.nm * 128.0 / 28.0;
         p.cost *= std::max(std::max(mma, l2), pair ? 420.0 : 380.0);
         if (p.cost < best.cost) best = p;
     };
@@ -1249,8 +1271,8 @@ namespace {
 // keeps a K slice's digits in L2.
 constexpr int64_t kChunkColumns = 288;
 
-// One chunk of columns: the plans of the passes it runs and its cleared words (ranges of X and W: 4 a
-// column; slice sums of both passes: 2 a column and slice).
+// One chunk of columns: the plans of the passes it runs and its cleared words: the ranges of X (4 a column)
+// and behind them the slice sums of the rows pass (2 a column and slice), then the same of W.
 struct SliceCall {
     SlicePlan rows, samples;
     int64_t k = 0, range = 0, range_w = 0, sum = 0, sum_w = 0, words = 0;
@@ -1262,9 +1284,9 @@ SliceCall plan_call(const MixedRows& r, int64_t k) {
     c.rows = choose_slice_plan(true, r.r_pad / kTile, (int)(r.n_pad / kKBlock), k);
     c.samples = choose_slice_plan(false, r.n_pad / kTile, (int)(r.r_pad / kKBlock), k);
     c.range = 0;
-    c.range_w = c.range + 4 * k;
-    c.sum = c.range_w + 4 * k;
-    c.sum_w = c.sum + 2 * k * c.rows.splits;
+    c.sum = c.range + 4 * k;
+    c.range_w = c.sum + 2 * k * c.rows.splits;
+    c.sum_w = c.range_w + 4 * k;
     c.words = c.sum_w + 2 * k * c.samples.splits;
     return c;
 }
