@@ -192,17 +192,22 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     }
     chain_wait();
     tc_fence_before();
-    if (PAIR)
-        cluster_sync_all();
-    else
-        __syncthreads();
+    if (PAIR) cluster_sync_all();
+    // nothing to do where no column is inside the fixed-point range (the ranges stand in front of the
+    // sums: SliceCall)
+    int live = DIGITS != kDigits;
+    if (DIGITS == kDigits) {
+        const ColumnRange* range = reinterpret_cast<const ColumnRange*>(P.ksum) - P.k;
+        for (int c = threadIdx.x; c < P.k; c += (int)blockDim.x) live |= !range_excluded(range[c]);
+    }
+    live = __syncthreads_or(live);
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
     // A unit is one M tile (pair: two) x one column tile x one K slice, column tiles fastest so
     // that the CTAs running at one time share packed tiles through L2.
     const int groups = PAIR ? P.n_tiles / 2 : P.n_tiles;
-    const int units = groups * P.n_ctiles * P.n_splits;
+    const int units = live ? groups * P.n_ctiles * P.n_splits : 0;
     const int u0 = PAIR ? (int)cluster_id_x() : (int)blockIdx.x;
     const int ustep = PAIR ? (int)cluster_count_x() : (int)gridDim.x;
     auto unit_coords = [&](int u, int& tile, int& ct, int& split, int& kb0, int& kb1) {
@@ -945,71 +950,276 @@ struct PackedRows {
     int64_t stride;
 };
 
-// u_t / s_t of a column outside the fixed-point range: the plain FP64 sum over a packed row by one
-// warp, 64 samples per lane at a time.  Missing calls multiply by zero, so a non-finite value
-// reaches every row, as it does in the FP64-pipe kernels.
-__device__ double direct_row(const PackedRows& G, int64_t t, double mu, const StridedIn& X, int64_t c,
-                             int64_t n, int lane) {
-    double acc = 0.0;
-    for (int64_t i0 = 64 * lane; i0 < n; i0 += 64 * 32) {
-        const uint4 w = *reinterpret_cast<const uint4*>(G.rows + t * G.stride + (i0 >> 2));
-        const uint32_t words[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            for (int j = 0; j < 16; ++j) {
-                const int64_t i = i0 + 16 * q + j;
-                if (i < n) acc = fma(centred((words[q] >> (2 * j)) & 3u, mu), X.p[i * X.rs + c * X.cs], acc);
-            }
+// ---------------------------------------------------------------- columns outside the fixed-point range
+// Plain FP64 sums of (G - mu) times the operand for up to kDirectCols columns at a time, by the blocks that
+// reduce the other columns: which columns these are is known on the device only, and a kernel of
+// their own would cost every small product its launch.  A decode value comes from a table in
+// shared memory laid out so that no mix of codes conflicts (two wavefronts a value) and serves four
+// columns; a block whose outputs are too few for its threads splits the sum over them.  Missing calls
+// multiply by zero, so a non-finite value reaches every output, as it does in the FP64-pipe kernels.
+// FP64 K x where every column of x is outside, ms (a value of -9999 left among normals), with the FP64-pipe kernels
+// that took such columns before, with a warp to a SNP row and a thread to a sample, and so: 50,000 x 100,000, one
+// column 7.2, 42.4, 3.3, 34 columns 58.7, 634, 30.2; 18,009 x 27,006, 34 columns 5.6, 76, 3.3, 266 columns 23.5, 462,
+// 21.4; 2,000 x 10,000, one column 0.163, 1.59, 0.053.  One of 34 columns at 50,000 x 100,000: 58.7, 59.5, 11.8.
+// What bounds them is the shared-memory pipe (twelve wavefronts for 16 multiply-adds a lane).
+constexpr int kDirectCols = 4;
+constexpr int kDirectRows = 1024;  // rows of a table at most, four values each; SNPs of one
+constexpr int kDirectSnps = 512;
+
+// The columns that a block of column c takes: c and the next excluded ones where c is the first, fifth, ..
+// excluded column, none otherwise.  Every thread of the block calls it.
+__device__ __forceinline__ int direct_group(const ColumnRange* range, int64_t k, int64_t c, int* cols, int* count) {
+    if (threadIdx.x < 32) {
+        int before = 0, here = 0;
+        for (int64_t j0 = 0; j0 < k && here < kDirectCols; j0 += 32) {
+            const int64_t j = j0 + threadIdx.x;
+            unsigned m = __ballot_sync(0xffffffffu, j < k && range_excluded(range[j]));
+            const unsigned low = c >= j0 + 32 ? 0xffffffffu : c > j0 ? (1u << (int)(c - j0)) - 1u : 0u;
+            before += __popc(m & low);
+            for (m &= ~low; m && here < kDirectCols; m &= m - 1u, ++here)
+                if (threadIdx.x == 0) cols[here] = (int)(j0 + __ffs(m) - 1);
+        }
+        if (threadIdx.x == 0) *count = before % kDirectCols == 0 ? here : 0;
     }
-    for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    return acc;
+    __syncthreads();
+    return *count;
 }
 
-// Rows-pass result u / s = 2^-e / 63 sum_z part (or the direct sum).  1024 SNPs per block, one column
+// Whether a thread's sums have all become NaN, which nothing that follows changes.
+template <int NG>
+__device__ __forceinline__ int all_nan(const double (&acc)[4][NG], int ng) {
+    bool lost = true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int g = 0; g < NG; ++g) lost = lost && (g >= ng || acc[i][g] != acc[i][g]);
+    return lost;
+}
+
+template <int NG>
+__device__ __forceinline__ void load_values(const double* p, double (&v)[NG]) {
+    if constexpr (NG == 4) {
+        const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+        v[0] = a.x;
+        v[1] = a.y;
+        v[2] = b.x;
+        v[3] = b.y;
+    } else {
+        v[0] = *p;
+    }
+}
+
+// buf[g * rpb + row] = sum_i (G - mu) x_i,cols[g] of `rows` SNPs from t0 on and NG columns; rpb (64, 256 or
+// 1024) rows a block, four of them a thread, 1024 / rpb threads to a row.
+template <int NG>
+__device__ __forceinline__ void direct_rows(const PackedRows& G, int64_t t0, int rows, int rpb,
+                                            const double* __restrict__ mu, const StridedIn& X, const int* cols,
+                                            int ng, int64_t n, double* buf) {
+    const int groups = rpb / 4, parts = 256 / groups, grp = threadIdx.x % groups, part = threadIdx.x / groups;
+    // [code][row]: a warp's lanes read neighbouring rows, whatever their codes
+    for (int e = threadIdx.x; e < 4 * rpb; e += 256)
+        buf[e] = e % rpb < rows ? centred((uint32_t)(e / rpb), mu[t0 + e % rpb]) : 0.0;
+    __syncthreads();
+    const uint8_t* const src = G.rows + t0 * G.stride;
+    uint32_t row_at[4];  // at most 1024 rows further
+#pragma unroll
+    for (int i = 0; i < 4; ++i) row_at[i] = (uint32_t)min(grp + groups * i, rows - 1) * (uint32_t)G.stride;
+    // 256 samples at a time, `here` of them to a part: x read by one thread a sample while the ones before
+    // are used (past the last it is zero)
+    const int here = 256 / parts, pitch = here * NG + 4;
+    double* const xs = buf + 4 * rpb;
+    double* const mine = xs + (threadIdx.x / here) * pitch + (threadIdx.x % here) * NG;
+    double next[NG];
+    auto fetch = [&](int64_t i) {
+#pragma unroll
+        for (int g = 0; g < NG; ++g) next[g] = i < n && g < ng ? X.p[i * X.rs + cols[g] * X.cs] : 0.0;
+    };
+    fetch(threadIdx.x);
+    const double* const lut = buf + grp;
+    double acc[4][NG] = {};
+    int lost = 0;
+    for (int64_t base = 0; base < n; base += 256) {
+        if (__syncthreads_and(lost)) break;
+#pragma unroll
+        for (int g = 0; g < NG; ++g) mine[g] = next[g];
+        __syncthreads();
+        fetch(base + 256 + threadIdx.x);
+        const int64_t i0 = base + part * here;
+        const double* x = xs + part * pitch;
+#pragma unroll 1
+        for (int64_t at = i0; at < min(n, i0 + here); at += 16) {
+            uint32_t word[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) word[i] = *reinterpret_cast<const uint32_t*>(src + row_at[i] + (at >> 2));
+#pragma unroll 4
+            for (int j = 0; j < 16; ++j, x += NG) {
+                double xv[NG];
+                load_values<NG>(x, xv);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const double z = lut[(int)((word[i] >> (2 * j)) & 3u) * rpb + groups * i];
+#pragma unroll
+                    for (int g = 0; g < NG; ++g) acc[i][g] = fma(z, xv[g], acc[i][g]);
+                }
+            }
+        }
+        lost = all_nan(acc, ng);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int g = 0; g < NG; ++g) buf[(part * NG + g) * rpb + grp + groups * i] = acc[i][g];
+    __syncthreads();
+    for (int e = threadIdx.x; e < NG * rpb; e += 256) {
+        double v = buf[e];
+        for (int p = 1; p < parts; ++p) v += buf[p * NG * rpb + e];
+        buf[e] = v;
+    }
+    __syncthreads();
+}
+
+// sum_t (G - mu) W_t,cols[g] of samples i0 .. i0 + 31: thread g * 32 + sample (< 32 NG) returns its own.
+// Four samples of a SNP a thread, 32 SNPs at a time, tables of 512 SNPs.
+template <int NG>
+__device__ __forceinline__ double direct_samples(const PackedRows& G, int64_t i0, const double* __restrict__ mu,
+                                                 const double* __restrict__ Wt, int64_t R,
+                                                 const int64_t (&cols)[kDirectCols], int ng, double* buf) {
+    const int bc = threadIdx.x & 7, part = threadIdx.x >> 3;
+    const uint8_t* src = G.rows + (i0 >> 2) + bc;
+    double* const wv = buf + 4 * kDirectSnps;
+    double acc[4][NG] = {};
+    int lost = 0;
+    for (int64_t base = 0; base < R; base += kDirectSnps) {
+        const int here = (int)min((int64_t)kDirectSnps, R - base);
+        if (__syncthreads_and(lost)) break;
+        for (int e = threadIdx.x; e < here; e += 256) {
+            const double m = mu[base + e];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) buf[4 * e + q] = centred((uint32_t)q, m);
+#pragma unroll
+            for (int g = 0; g < NG; ++g) wv[NG * e + g] = g < ng ? Wt[cols[g] * R + base + e] : 0.0;
+        }
+        __syncthreads();
+        for (int r0 = part; r0 < here; r0 += 8 * 32) {
+            uint32_t codes[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) codes[j] = r0 + 32 * j < here ? src[(base + r0 + 32 * j) * G.stride] : 0u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int row = r0 + 32 * j;
+                if (row >= here) break;
+                double w[NG];
+                load_values<NG>(wv + NG * row, w);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const double z = buf[4 * row + (int)((codes[j] >> (2 * i)) & 3u)];
+#pragma unroll
+                    for (int g = 0; g < NG; ++g) acc[i][g] = fma(z, w[g], acc[i][g]);
+                }
+            }
+        }
+        lost = all_nan(acc, ng);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            double v = acc[i][g];
+            v += __shfl_xor_sync(0xffffffffu, v, 8);
+            v += __shfl_xor_sync(0xffffffffu, v, 16);
+            if ((threadIdx.x & 31) < 8) buf[((threadIdx.x >> 5) * NG + g) * 32 + 4 * bc + i] = v;
+        }
+    __syncthreads();
+    double v = 0.0;
+    if (threadIdx.x < 32 * NG)
+        for (int p = 0; p < 8; ++p) v += buf[p * 32 * NG + threadIdx.x];
+    __syncthreads();
+    return v;
+}
+
+// Rows-pass result u / s = 2^-e / 63 sum_z part (or the direct sum).  rpb SNPs per block, one column
 // per blockIdx.y.  With Wt: W^T (column-major, R per column) = s^2 (u / s) and the ranges of
 // max(|W|, |mu W|) for the samples operand; with out: s (u / s) at row pos[t] (or t).
-__global__ void __launch_bounds__(256)
-k_slice_reduce_rows(const double* __restrict__ part, int64_t ld, int64_t R, int64_t k,
+__global__ void __launch_bounds__(256, 3)
+k_slice_reduce_rows(const double* __restrict__ part, int64_t ld, int64_t R, int64_t k, int rpb,
                     const double* __restrict__ s_row, const double* __restrict__ mu,
                     const PackedRows G, const StridedIn X, int64_t n, const SliceSums S,
                     double* __restrict__ Wt, const int32_t* __restrict__ pos, StridedOut out) {
     chain_enter();
+    __shared__ __align__(16) double buf[4 * kDirectRows + 256 * kDirectCols + 64];
+    __shared__ unsigned long long s_mx[8];
+    __shared__ long long s_es[8];
+    __shared__ unsigned s_n[8];
+    __shared__ int s_cols[kDirectCols], s_count;
     const int64_t c = blockIdx.y;
     const ColumnRange rg = S.range[c];
-    const double f = pow2(-slice_exponent(rg.max_bits));
-    const bool direct = range_excluded(rg);
     unsigned long long mx = 0;
     long long es = 0;
     unsigned cnt = 0;
-    const int64_t t0 = (int64_t)blockIdx.x * 1024, t1 = min(R, t0 + 1024);
-    auto finish = [&](int64_t t, double v) {
+    const int64_t t0 = (int64_t)blockIdx.x * rpb;
+    const int rows = (int)min((int64_t)rpb, R - t0);
+    auto finish = [&](int64_t col, int64_t t, double v) {
         const double s = s_row[t];
         if (Wt) {
             const double w = v * s * s;
-            Wt[c * R + t] = w;
+            Wt[col * R + t] = w;
             range_of(mu[t] > 1.0 ? mu[t] * w : w, mx, es, cnt);
         } else {
-            out.p[(pos ? (int64_t)pos[t] : t) * out.rs + c * out.cs] = v * s;
+            out.p[(pos ? (int64_t)pos[t] : t) * out.rs + col * out.cs] = v * s;
         }
     };
-    if (direct) {
-        const int lane = threadIdx.x & 31;
-        for (int64_t t = t0 + (threadIdx.x >> 5); t < t1; t += 8) {
-            const double v = direct_row(G, t, mu[t], X, c, n, lane);
-            if (lane == 0) finish(t, v);
+    auto close = [&](int64_t col) {  // the block's range, one atomic each
+        if (!Wt) return;
+        mx = shfl_max(mx, 32);
+        es = shfl_sum(es, 32);
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if ((threadIdx.x & 31) == 0) {
+            s_mx[threadIdx.x >> 5] = mx;
+            s_es[threadIdx.x >> 5] = es;
+            s_n[threadIdx.x >> 5] = cnt;
         }
-    } else {
-        for (int64_t t = t0 + threadIdx.x; t < t1; t += 256) {
-            double acc = 0.0;
-            for (int z = 0; z < S.splits; ++z) acc += part[((int64_t)z * k + c) * ld + t];
-            finish(t, checked(acc * f * (1.0 / (double)kTcQ), S.status));
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < 8; ++w) {
+                mx = max(mx, s_mx[w]);
+                es += s_es[w];
+                cnt += s_n[w];
+            }
+            add_range(&S.range_w[col], mx, es, cnt);
         }
+        __syncthreads();
+    };
+    if (!range_excluded(rg)) {
+        const double f = pow2(-slice_exponent(rg.max_bits));
+        // four rows a thread at a time: few blocks are resident beside the direct sums' registers
+        double acc[4] = {};
+        const double* p = part + c * ld + t0 + threadIdx.x;
+        for (int z = 0; z < S.splits; ++z, p += k * ld) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if ((int)threadIdx.x + 256 * j < rows) acc[j] += p[256 * j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int e = threadIdx.x + 256 * j;
+            if (e < rows) finish(c, t0 + e, checked(acc[j] * f * (1.0 / (double)kTcQ), S.status));
+        }
+        close(c);
+        return;
     }
-    if (!Wt) return;
-    mx = shfl_max(mx, 32);
-    es = shfl_sum(es, 32);
-    cnt = __reduce_add_sync(0xffffffffu, cnt);
-    if ((threadIdx.x & 31) == 0) add_range(&S.range_w[c], mx, es, cnt);
+    const int ng = direct_group(S.range, k, c, s_cols, &s_count);
+    if (ng == 0) return;
+    if (ng == 1) direct_rows<1>(G, t0, rows, rpb, mu, X, s_cols, ng, n, buf);
+    else direct_rows<kDirectCols>(G, t0, rows, rpb, mu, X, s_cols, ng, n, buf);
+    for (int g = 0; g < ng; ++g) {
+        mx = 0;
+        es = 0;
+        cnt = 0;
+        for (int e = threadIdx.x; e < rows; e += 256) finish(s_cols[g], t0 + e, buf[g * rpb + e]);
+        close(s_cols[g]);
+    }
 }
 
 // The samples operand of a half-pass: W^T[c][t] = s_t V[pos[t]][c] and its ranges (1024 SNPs per
@@ -1039,32 +1249,50 @@ k_slice_gather(const StridedIn V, int64_t R, const int32_t* __restrict__ pos,
 // Samples-pass result: Y[i][c] = scale 2^-e sum_z part[z][c][i] (or the direct sum over the column's
 // W).  Column-major output: a warp's lanes are samples; row-major: tiles of 32 samples x 32 columns
 // through shared memory, so that both sides are coalesced.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 k_slice_reduce_samples(const double* __restrict__ part, int64_t ld, int64_t n, int64_t k,
                        const double* __restrict__ Wt, int64_t R, const double* __restrict__ mu,
                        const PackedRows G, const SliceSums S, double scale, StridedOut Y) {
     chain_enter();
     __shared__ double tile[32][33];
+    __shared__ __align__(16) double buf[(4 + kDirectCols) * kDirectSnps];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t i0 = (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
     const int64_t i = i0 + tx;
-    for (int cc = ty; cc < 32; cc += 8) {
-        const int64_t c = c0 + cc;
-        if (c >= k || i >= n) continue;
-        const ColumnRange rg = S.range_w[c];
-        double acc = 0.0;
-        if (range_excluded(rg)) {
-            const uint8_t* g = G.rows + (i >> 2);
-            const int sh = 2 * (int)(i & 3);
-            for (int64_t t = 0; t < R; ++t)
-                acc = fma(centred((g[t * G.stride] >> sh) & 3u, mu[t]), Wt[c * R + t], acc);
-            acc *= scale;
-        } else {
-            for (int z = 0; z < S.splits_w; ++z) acc += part[((int64_t)z * k + c) * ld + i];
-            acc = checked(acc * pow2(-slice_exponent(rg.max_bits)) * scale, S.status);
-        }
-        if (Y.rs == 1) Y.p[i + c * Y.cs] = acc;
-        else tile[cc][tx] = acc;
+    const unsigned direct = __ballot_sync(0xffffffffu, c0 + tx < k && range_excluded(S.range_w[c0 + tx]));
+    auto store = [&](int cc, double v) {
+        if (Y.rs == 1) Y.p[i + (c0 + cc) * Y.cs] = v;
+        else tile[cc][tx] = v;
+    };
+    // four columns a thread at a time, as above
+    double acc[4] = {};
+    const double* p = part + (c0 + ty) * ld + i;
+    for (int z = 0; z < S.splits_w; ++z, p += k * ld) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (c0 + ty + 8 * j < k && i < n) acc[j] += p[8 * j * ld];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int cc = ty + 8 * j;
+        if (c0 + cc >= k || i >= n || (direct >> cc & 1u)) continue;
+        store(cc, checked(acc[j] * pow2(-slice_exponent(S.range_w[c0 + cc].max_bits)) * scale, S.status));
+    }
+    for (unsigned m = direct; m;) {
+        int64_t cols[kDirectCols] = {};
+        int ng = 0, mine = 0;
+#pragma unroll
+        for (int g = 0; g < kDirectCols; ++g)
+            if (m) {
+                const int cc = __ffs(m) - 1;
+                cols[g] = c0 + cc;
+                if (ty == g) mine = cc;
+                m &= m - 1u;
+                ++ng;
+            }
+        const double v = ng == 1 ? direct_samples<1>(G, i0, mu, Wt, R, cols, ng, buf)
+                                 : direct_samples<kDirectCols>(G, i0, mu, Wt, R, cols, ng, buf);
+        if (ty < ng && i < n) store(mine, v * scale);
     }
     if (Y.rs == 1) return;
     __syncthreads();
@@ -1435,8 +1663,12 @@ void run_samples(SliceOperator& so, MixedRows& r, const SliceCall& c, const Slic
 void finish_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSums& S, StridedIn X,
                  double* Wt, const int32_t* pos, StridedOut out, cudaStream_t s) {
     prof::Scope ps("slice_reduce_rows", s, 0.0, 8.0 * (c.rows.splits + 1) * (double)c.k * r.R);
-    launch_chained(k_slice_reduce_rows, dim3((unsigned)((r.R + 1023) / 1024), (unsigned)c.k), 256, 0, s,
-                   so.part.get(), r.r_pad, r.R, c.k, r.s.get(), r.mu.get(), PackedRows{r.rows, r.stride}, X,
+    // as many rows a block as leave two blocks for every SM if all columns are summed directly
+    const int64_t groups = (c.k + kDirectCols - 1) / kDirectCols;
+    int rpb = kDirectRows;
+    while (rpb > 64 && (r.R + rpb - 1) / rpb * groups < 2 * num_sms()) rpb /= 4;
+    launch_chained(k_slice_reduce_rows, dim3((unsigned)((r.R + rpb - 1) / rpb), (unsigned)c.k), 256, 0, s,
+                   so.part.get(), r.r_pad, r.R, c.k, rpb, r.s.get(), r.mu.get(), PackedRows{r.rows, r.stride}, X,
                    r.n, S, Wt, pos, out);
     CS_LAUNCH("slice_reduce_rows");
 }

@@ -18,7 +18,7 @@ struct ColumnRange {
 };
 
 // A fixed-point column holds every element to 2^-63 of its maximum.  A column whose nonzero elements
-// lie on (geometric) average more than 2^kSliceRange below that maximum is computed on the FP64 pipe:
+// lie on (geometric) average more than 2^kSliceRange below that maximum is summed in FP64 (direct_rows):
 // up to there the average element has the 53 bits of an FP64 value, so that also what depends on the
 // small elements alone (a row whose large ones all meet missing calls) is as good as FP64 sums.  So is
 // a column with a non-finite value or a maximum near the ends of the exponent range (the scales and
@@ -51,8 +51,8 @@ __device__ __forceinline__ bool range_uneven(const ColumnRange& r) {
 struct SliceOperator;
 void destroy_slices(SliceOperator* s);
 
-// FP64 products through the slices where the operator has (or may have) a sample-major copy and
-// the shape is large enough; false when the FP64-pipe kernels are to be used.  Results may
+// FP64 products through the slices where the operator has (or may have) a sample-major copy and there
+// is device memory for it and the operands; false when the FP64-pipe kernels are to be used.  Results may
 // overwrite the input.
 // Y (rows x k) = K X.
 bool kinship_apply_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut Y, cudaStream_t s);
