@@ -20,6 +20,11 @@ struct Error : std::runtime_error {
     Error(int c, const std::string& msg) : std::runtime_error(msg), code(c) {}
 };
 
+// A device allocation that found no room: callers that can do with less catch this alone.
+struct OutOfMemory : Error {
+    using Error::Error;
+};
+
 [[noreturn]] inline void fail(int code, const std::string& msg) { throw Error(code, msg); }
 
 // The calling thread's message for cs_last_error() (abi.cpp).
@@ -77,6 +82,8 @@ constexpr int64_t kRowAlign = 64;
 // block (the same guarantee cudaFree gives).
 void* device_alloc(size_t bytes);
 void device_free(void* p) noexcept;
+// What the current device has left for this process: its free memory and the pool's free blocks.
+size_t device_room();
 // For a thread whose device work all runs on one stream of its own (a request worker of the
 // serving loop): the thread's frees are ordered on that stream (cudaFreeAsync there) instead of
 // waiting for the whole device, so a buffer is only reused after the work queued before its
@@ -192,7 +199,7 @@ struct cs_kinship {
     cs::DeviceBuffer<double> buf_x, buf_u, buf_y;
     cs::MixedOperator* mixed = nullptr;
     cs::SliceOperator* slices = nullptr;
-    bool slices_unavailable = false;  // no device memory for them: FP64-pipe kernels only
+    size_t slices_need = 0;  // bytes that were not there for them: FP64-pipe kernels until they are
     bool defer_checks = false;        // a solver's loop checks its passes itself (DeferChecks)
     cs::PcgWorkspace* pcg = nullptr;  // kept from one solve on this operator to the next (pcg.cu)
     bool autotune = true;  // the tensor-core passes may tune their plan on new shapes

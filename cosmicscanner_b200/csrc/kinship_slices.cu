@@ -1489,6 +1489,12 @@ struct SliceOperator {
     // operator and keep their place for its lifetime)
     CUtensorMap tm_packed{}, tm_packed_t{};
     bool map_rows = false, map_samples = false;
+    void release_operands() {
+        b.release();
+        part.release();
+        W.release();
+        words.release();
+    }
 };
 
 void destroy_slices(SliceOperator* s) { delete s; }
@@ -1533,9 +1539,18 @@ SliceSums sums_of(SliceOperator& so, const SliceCall& c, bool clear) {
     return S;
 }
 
+int64_t digit_bytes(const MixedRows& r, const SliceCall& c) {
+    return std::max(c.rows.b_rows(true) * r.n_pad, c.samples.b_rows(false) * r.r_pad);
+}
+int64_t part_values(const MixedRows& r, const SliceCall& c) {
+    return c.k * std::max(c.rows.splits * r.r_pad, c.samples.splits * r.n_pad);
+}
+size_t operand_bytes(const MixedRows& r, const SliceCall& c) {
+    return (size_t)(digit_bytes(r, c) + 8 * (part_values(r, c) + r.R * c.k + c.words));
+}
 void reserve(SliceOperator& so, const MixedRows& r, const SliceCall& c) {
-    so.b.resize(std::max(c.rows.b_rows(true) * r.n_pad, c.samples.b_rows(false) * r.r_pad));
-    so.part.resize(c.k * std::max(c.rows.splits * r.r_pad, c.samples.splits * r.n_pad));
+    so.b.resize(digit_bytes(r, c));
+    so.part.resize(part_values(r, c));
     so.W.resize(r.R * c.k);
     so.words.resize(c.words);
 }
@@ -1679,46 +1694,79 @@ bool pipe_kernels_chosen() {
     return on;
 }
 
-// The operator's slice state with room for k columns, or null (no sample-major copy allowed, or no
-// device memory for it or for the operands).  The slices are taken at every shape: against the
+// Columns per call of the passes, at most kChunkColumns, whose operands `reserve(columns)` finds device memory
+// for: half as many after each failure (`release` gives back what was had), until it throws for eight.
+template <class Reserve, class Release>
+int64_t widest_chunk(int64_t k, Reserve&& reserve, Release&& release) {
+    for (int64_t w = kChunkColumns;; w = std::min(w, k) / 2) {
+        try {
+            if (k >= w) reserve(w);
+            if (k % w) reserve(k % w);
+            return w;
+        } catch (const OutOfMemory&) {
+            release();
+            if (std::min(w, k) / 2 < 8) throw;
+        }
+    }
+}
+
+// The operator's slice state with room for chunks of `columns` of the k columns; null without a
+// sample-major copy where that is needed and not allowed, or without device memory for it or for the
+// operands.  In that case it gives back what it had taken and is tried again by the first call that
+// finds the memory.  The slices are taken at every shape: against the
 // FP64-pipe kernels an apply took (us) 27 / 99 at n=40, M=1000 and one column, 31 / 152 at n=2000,
 // M=10000, 930 / 7210 at n=50000, M=100000; 35 / 187, 86 / 470 and 168 / 954 at n=2000, M=10000 and
-// 8, 80 and 200 columns; 2750 / 23480 at n=18009, M=27006 and 266.
-SliceOperator* slices_for(cs_kinship* op, int64_t k, bool samples, cudaStream_t s) {
+// 8, 80 and 200 columns; 2900 / 23480 at n=18009, M=27006 and 266.
+struct SliceRoom {
+    SliceOperator* so = nullptr;
+    int64_t columns = 0;
+    explicit operator bool() const { return so != nullptr; }
+};
+
+SliceRoom slices_for(cs_kinship* op, int64_t k, bool samples, cudaStream_t s) {
     const int64_t R = op->n_active;
-    if (!op->sample_major_copy || op->slices_unavailable || R == 0 || k <= 0 || pipe_kernels_chosen())
-        return nullptr;
+    if (!op->sample_major_copy || R == 0 || k <= 0 || pipe_kernels_chosen()) return {};
+    if (op->slices_need && device_room() < op->slices_need) return {};
+    MixedRows* r = nullptr;
+    bool new_copy = false;
     try {
-        MixedRows& r = mixed_rows_for(op);
+        r = &mixed_rows_for(op);
         configure_slices();
+        new_copy = samples && !r->packed_t.get();
         if (!op->slices) op->slices = new SliceOperator();
         SliceOperator& so = *op->slices;
         make_status(so, s);
         if (!so.map_rows) {
-            so.tm_packed = make_map_u8(r.rows, r.stride, R, r.stride, 128, kTile, true);
+            so.tm_packed = make_map_u8(r->rows, r->stride, R, r->stride, 128, kTile, true);
             so.map_rows = true;
         }
-        if (samples) ensure_transposed(r, s);
+        if (samples) ensure_transposed(*r, s);
         if (samples && !so.map_samples) {
-            so.tm_packed_t = make_map_u8(r.packed_t.get(), r.r_pad / 4, r.n_pad, r.r_pad / 4, 128, kTile, true);
+            so.tm_packed_t = make_map_u8(r->packed_t.get(), r->r_pad / 4, r->n_pad, r->r_pad / 4, 128, kTile, true);
             so.map_samples = true;
         }
-        if (k >= kChunkColumns) reserve(so, r, plan_call(r, kChunkColumns));
-        if (k % kChunkColumns) reserve(so, r, plan_call(r, k % kChunkColumns));
-        return &so;
-    } catch (const Error&) {
+        const int64_t columns = widest_chunk(
+            k, [&](int64_t w) { reserve(so, *r, plan_call(*r, w)); }, [&] { so.release_operands(); });
+        op->slices_need = 0;
+        return {&so, columns};
+    } catch (const OutOfMemory&) {
         // the FP64-pipe kernels need neither the copy nor the operands
         destroy_slices(op->slices);
         op->slices = nullptr;
-        op->slices_unavailable = true;
-        return nullptr;
+        op->slices_need = 1;
+        if (r) op->slices_need += operand_bytes(*r, plan_call(*r, std::min<int64_t>(k, 8)));
+        if (new_copy) {
+            r->packed_t.release();
+            op->slices_need += (size_t)(r->n_pad * r->r_pad / 4);
+        }
+        return {};
     }
 }
 
 template <class Chunk>
-void for_chunks(const MixedRows& r, int64_t k, Chunk&& chunk) {
-    for (int64_t c0 = 0; c0 < k; c0 += kChunkColumns)
-        chunk(c0, plan_call(r, std::min(kChunkColumns, k - c0)));
+void for_chunks(const MixedRows& r, int64_t k, int64_t columns, Chunk&& chunk) {
+    for (int64_t c0 = 0; c0 < k; c0 += columns)
+        chunk(c0, plan_call(r, std::min(columns, k - c0)));
 }
 
 StridedIn from_column(StridedIn m, int64_t c) { return StridedIn{m.p + c * m.cs, m.rs, m.cs}; }
@@ -1727,10 +1775,11 @@ StridedOut from_column(StridedOut m, int64_t c) { return StridedOut{m.p + c * m.
 }  // namespace
 
 bool kinship_apply_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut Y, cudaStream_t s) {
-    SliceOperator* so = slices_for(op, k, true, s);
-    if (!so) return false;
+    const SliceRoom room = slices_for(op, k, true, s);
+    if (!room) return false;
+    SliceOperator* const so = room.so;
     MixedRows& r = mixed_rows_for(op);
-    for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
+    for_chunks(r, k, room.columns, [&](int64_t c0, const SliceCall& c) {
         const SliceSums S = sums_of(*so, c, c0 == 0 && !op->defer_checks);
         const StridedIn x = from_column(X, c0);
         run_rows(*so, r, c, S, x, s);
@@ -1741,10 +1790,11 @@ bool kinship_apply_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut Y, 
 }
 
 bool multiply_zt_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut U, cudaStream_t s) {
-    SliceOperator* so = slices_for(op, k, false, s);
-    if (!so) return false;
+    const SliceRoom room = slices_for(op, k, false, s);
+    if (!room) return false;
+    SliceOperator* const so = room.so;
     MixedRows& r = mixed_rows_for(op);
-    for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
+    for_chunks(r, k, room.columns, [&](int64_t c0, const SliceCall& c) {
         const SliceSums S = sums_of(*so, c, c0 == 0 && !op->defer_checks);
         const StridedIn x = from_column(X, c0);
         run_rows(*so, r, c, S, x, s);
@@ -1754,10 +1804,11 @@ bool multiply_zt_slices(cs_kinship* op, StridedIn X, int64_t k, StridedOut U, cu
 }
 
 bool multiply_z_slices(cs_kinship* op, StridedIn V, int64_t k, StridedOut Y, cudaStream_t s) {
-    SliceOperator* so = slices_for(op, k, true, s);
-    if (!so) return false;
+    const SliceRoom room = slices_for(op, k, true, s);
+    if (!room) return false;
+    SliceOperator* const so = room.so;
     MixedRows& r = mixed_rows_for(op);
-    for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
+    for_chunks(r, k, room.columns, [&](int64_t c0, const SliceCall& c) {
         const SliceSums S = sums_of(*so, c, c0 == 0 && !op->defer_checks);
         CS_CUDA(cudaMemsetAsync(so->words.get(), 0, 8 * c.words, s));
         {
@@ -1793,6 +1844,7 @@ void clear_slices(cs_kinship* op, cudaStream_t s) {
 bool scan_project_slices(SliceOperator*& state, MixedRows& r, StridedIn X, int64_t k, StridedOut T,
                          cudaStream_t s) {
     if (r.R == 0 || k <= 0 || pipe_kernels_chosen()) return false;
+    int64_t columns = 0;
     try {
         configure_slices();
         if (!state) state = new SliceOperator();
@@ -1807,15 +1859,15 @@ bool scan_project_slices(SliceOperator*& state, MixedRows& r, StridedIn X, int64
             so.part.resize(c.k * c.rows.splits * r.r_pad);
             so.words.resize(c.words);
         };
-        if (k >= kChunkColumns) reserve_rows(plan_call(r, kChunkColumns));
-        if (k % kChunkColumns) reserve_rows(plan_call(r, k % kChunkColumns));
-    } catch (const Error&) {  // no device memory for the operands
+        columns = widest_chunk(
+            k, [&](int64_t w) { reserve_rows(plan_call(r, w)); }, [&] { so.release_operands(); });
+    } catch (const OutOfMemory&) {
         destroy_slices(state);
         state = nullptr;
         return false;
     }
     SliceOperator& so = *state;
-    for_chunks(r, k, [&](int64_t c0, const SliceCall& c) {
+    for_chunks(r, k, columns, [&](int64_t c0, const SliceCall& c) {
         const SliceSums S = sums_of(so, c, c0 == 0);
         const StridedIn x = from_column(X, c0);
         run_rows(so, r, c, S, x, s);

@@ -39,6 +39,13 @@ bool poison_allocations() {
     return on;
 }
 
+// CS_B200_ALLOC_LIMIT=bytes refuses larger blocks as a full device would; read at each allocation, so
+// that a test can take it back.
+size_t alloc_limit() {
+    const char* v = std::getenv("CS_B200_ALLOC_LIMIT");
+    return v && *v ? (size_t)std::strtoull(v, nullptr, 10) : SIZE_MAX;
+}
+
 thread_local cublasHandle_t t_blas[kMaxDevices] = {};
 thread_local cusolverDnHandle_t t_solver[kMaxDevices] = {};
 // Handles given back by threads that ended (release_thread_handles), reused by new threads:
@@ -83,8 +90,9 @@ void* device_alloc(size_t bytes) {
     CS_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < kMaxDevices) prepare_pool(dev);
     void* p = nullptr;
-    cudaError_t e = cudaMallocAsync(&p, bytes, 0);
-    if (e == cudaErrorMemoryAllocation) {
+    const bool refused = bytes > alloc_limit();
+    cudaError_t e = refused ? cudaErrorMemoryAllocation : cudaMallocAsync(&p, bytes, 0);
+    if (e == cudaErrorMemoryAllocation && !refused) {
         // The pool keeps freed blocks reserved; when the device has no room left for a new
         // block, hand the reserved free blocks back and try once more.
         cudaGetLastError();
@@ -93,13 +101,29 @@ void* device_alloc(size_t bytes) {
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
-        fail(CS_ERR_CUDA, std::string("device allocation of ") + std::to_string(bytes) +
-                              " bytes failed: " + cudaGetErrorString(e));
+        const std::string msg = std::string("device allocation of ") + std::to_string(bytes) +
+                                " bytes failed: " + cudaGetErrorString(e);
+        if (e == cudaErrorMemoryAllocation) throw OutOfMemory(CS_ERR_CUDA, msg);
+        fail(CS_ERR_CUDA, msg);
     }
     if (poison_allocations()) CS_CUDA(cudaMemsetAsync(p, 0xFF, bytes, 0));
     // usable from every stream once the allocation is ordered on the legacy stream
     CS_CUDA(cudaStreamSynchronize(0));
     return p;
+}
+
+size_t device_room() {
+    size_t room = 0, total = 0;
+    CS_CUDA(cudaMemGetInfo(&room, &total));
+    int dev = 0;
+    cudaMemPool_t pool;
+    uint64_t reserved = 0, used = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
+        room += reserved - used;
+    cudaGetLastError();
+    return room;
 }
 
 void* pinned_alloc(size_t bytes) {
