@@ -359,7 +359,7 @@ void genotype_multiply_zt(cs_kinship* op, const double* X, int64_t ldx, int64_t 
         return;
     }
     if (multiply_zt_slices(op, x, k, StridedOut{U, 1, ldu}, s)) return;
-    if (x.rs == 1) {
+    if (x.p == X) {
         op->buf_x.resize(n * k);
         colmajor_to_rowmajor(X, ldx, n, k, op->buf_x.get(), k, s);
     }
@@ -395,7 +395,7 @@ void genotype_multiply_z(cs_kinship* op, const double* V, int64_t ldv, int64_t k
         return;
     }
     if (multiply_z_slices(op, v, k, StridedOut{Y, 1, ldy}, s)) return;
-    if (v.rs == 1) {
+    if (v.p == V) {
         op->buf_x.resize(nv * k);
         colmajor_to_rowmajor(V, ldv, nv, k, op->buf_x.get(), k, s);
     }
