@@ -605,17 +605,21 @@ void vce_history(const cs_vce* v, double* out, int64_t* n_iter) {
 }
 
 // The operator's workspace for public solves: kept between them (sixteen allocations and as many
-// waits of the allocator a solve otherwise), unless it has grown past a gigabyte.
-static PcgWorkspace& solve_workspace(cs_kinship* op) {
-    if (!op->pcg) op->pcg = new PcgWorkspace();
-    return *op->pcg;
-}
-static void trim_workspace(cs_kinship* op) {
-    if (op->pcg && op->pcg->bytes() > (size_t(1) << 30)) {
+// waits of the allocator a solve otherwise), unless it has grown past a gigabyte or the solve failed.
+struct SolveWorkspace {
+    cs_kinship* op;
+    bool solved = false;
+    explicit SolveWorkspace(cs_kinship* o) : op(o) {
+        if (!op->pcg) op->pcg = new PcgWorkspace();
+    }
+    ~SolveWorkspace() {
+        if (solved && op->pcg->bytes() <= (size_t(1) << 30)) return;
         destroy_pcg(op->pcg);
         op->pcg = nullptr;
     }
-}
+    SolveWorkspace(const SolveWorkspace&) = delete;
+    SolveWorkspace& operator=(const SolveWorkspace&) = delete;
+};
 
 // Public multi-RHS solve of (sg2 K + se2 I) X = B on device column-major blocks.
 void pcg_solve_public(cs_kinship* op, double divisor, double sg2, double se2, const double* B,
@@ -635,7 +639,8 @@ void pcg_solve_public(cs_kinship* op, double divisor, double sg2, double se2, co
     V.vg = sg2;
     V.ve = se2;
     V.precision = precision;
-    PcgWorkspace& ws = solve_workspace(op);
+    SolveWorkspace kept(op);
+    PcgWorkspace& ws = *op->pcg;
     PcgStats st;
     ws.b.resize(n * k);
     ws.x.resize(n * k);
@@ -644,7 +649,7 @@ void pcg_solve_public(cs_kinship* op, double divisor, double sg2, double se2, co
     pcg_solve_block(V, diag, ws.b.get(), k, k, ws.x.get(), k, tol, relative != 0, max_iter, ws, st, s);
     rowmajor_to_colmajor(ws.x.get(), k, n, k, X, ldx, s);
     CS_CUDA(cudaStreamSynchronize(s));
-    trim_workspace(op);
+    kept.solved = true;
     if (iterations) std::copy(st.iterations.begin(), st.iterations.end(), iterations);
 }
 
@@ -670,7 +675,8 @@ void pcg_solve_records_public(cs_kinship* op, double divisor, const int32_t* rec
     V.ve = se2;
     V.with_pe = with_pe;
     V.precision = precision;
-    PcgWorkspace& ws = solve_workspace(op);
+    SolveWorkspace kept(op);
+    PcgWorkspace& ws = *op->pcg;
     PcgStats st;
     ws.b.resize(n_rec * k);
     ws.x.resize(n_rec * k);
@@ -680,7 +686,7 @@ void pcg_solve_records_public(cs_kinship* op, double divisor, const int32_t* rec
     pcg_solve_block(V, diag, ws.b.get(), k, k, ws.x.get(), k, tol, relative != 0, max_iter, ws, st, s);
     rowmajor_to_colmajor(ws.x.get(), k, n_rec, k, X, ldx, s);
     CS_CUDA(cudaStreamSynchronize(s));
-    trim_workspace(op);
+    kept.solved = true;
     if (iterations) std::copy(st.iterations.begin(), st.iterations.end(), iterations);
 }
 

@@ -88,3 +88,34 @@ def test_wide_call_that_fails_leaves_narrow_ones_alone(genotypes, limit):
     limit(None)
     got, on_digits = routed(lambda: op.apply(X[:, :1]))
     assert on_digits and np.array_equal(got, want)
+
+
+def pool_used():
+    """Bytes in use in the device's default memory pool."""
+    import ctypes as C
+
+    cuda = C.CDLL("libcuda.so.1")
+    dev, pool, used = C.c_int(), C.c_void_p(), C.c_uint64()
+    assert cuda.cuDeviceGet(C.byref(dev), 0) == 0
+    assert cuda.cuDeviceGetDefaultMemPool(C.byref(pool), dev) == 0
+    assert cuda.cuMemPoolGetAttribute(pool, 7, C.byref(used)) == 0  # CU_MEMPOOL_ATTR_USED_MEM_CURRENT
+    return used.value
+
+
+def test_failed_solve_keeps_no_workspace(genotypes, limit):
+    """64 columns' blocks take 3 MB each; the product's buffers do not fit, so the solve fails with the
+    blocks made.  What a failed product leaves with its operator is there before."""
+    pytest.importorskip("torch")
+    op = cs.createKinshipOperator(genotypes)
+    B = np.random.default_rng(3).standard_normal((N, 64))
+    pcg = cs.MatrixFreePCG(op, 0.5, 0.5, precision="fp64")
+    limit(4 << 20)
+    with pytest.raises(cs.CosmicError, match="allocation"):
+        op.apply(B)
+    before = pool_used()
+    with pytest.raises(cs.CosmicError, match="allocation"):
+        pcg.solve(B)
+    assert pool_used() - before < 1 << 20
+    limit(None)
+    x = pcg.solve(B)
+    assert np.isfinite(x).all()
