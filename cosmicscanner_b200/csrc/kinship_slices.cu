@@ -15,7 +15,8 @@
 // sample carries has s^2 = n.  With 5 % of such variants among 3,000 at 6,000 samples K x was off by
 // 1.5e-15 to 2.9e-15 with seven digits, 1.1e-15 as FP64 sums, 8e-17 with eight.  An even column (range_uneven)
 // needs no more than seven; its last digit is zero, whatever its neighbours are, and its results are those of
-// seven digits.  A product of 266 columns at 18,009 x 27,006 takes 2.90 ms, 2.73 with seven digits for all.
+// seven digits.  A product of 266 columns at 18,009 x 27,006 takes 2.76 ms where all are even, 2.90 otherwise, and took
+// 2.73 with seven digits.
 //
 //   rows pass     63 u_t / s_t = sum_obs 63 G x + sum_miss q_t x + (63 mu_t - q_t) sum_miss x
 //                                - 63 mu_t sum x
@@ -38,7 +39,7 @@
 // operations per 16 genotypes at half rate are 208 of the 400 clocks a K-block takes, the ring and
 // wait instructions of all warps about 120 more (ncu: ALU pipe 70 % busy, tensor pipe 14 %, DRAM a
 // third of its rate).  Wide blocks come nearer to the MMAs (N / 2 clocks each): 512 of the 660 clocks that
-// a K-block of a 16-column rows tile takes, and a 32-column samples tile is at theirs, 1024.  Wide blocks run
+// a K-block of a 16-column rows tile takes, and a 32-column samples tile is at theirs, 896 or 1024.  Wide blocks run
 // on CTA pairs (cta_group::2): each CTA holds half of the B rows, which halves the L2 reads of B that would
 // otherwise bound a wide block (64 bytes per clock and SM at the full MMA rate).
 //
@@ -192,15 +193,25 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     }
     chain_wait();
     tc_fence_before();
-    if (PAIR) cluster_sync_all();
-    // nothing to do where no column is inside the fixed-point range (the ranges stand in front of the
-    // sums: SliceCall)
-    int live = DIGITS != kDigits;
-    if (DIGITS == kDigits) {
-        const ColumnRange* range = reinterpret_cast<const ColumnRange*>(P.ksum) - P.k;
-        for (int c = threadIdx.x; c < P.k; c += (int)blockDim.x) live |= !range_excluded(range[c]);
+    // Pairs, whose time is the MMAs': nothing to do where no column is inside the fixed-point range, no MMAs for
+    // an eighth digit that no column has (the ranges stand in front of the sums: SliceCall).  A product of 266
+    // even columns at 18,009 x 27,006 takes 2.76 ms with that and 2.90 without.  In the single-CTA kernels, at
+    // their limit of 80 registers, the same cost a pass of one column 2 % (459 us for 450).
+    int live = 1, eighth = 1;
+    if constexpr (PAIR) {
+        const ColumnRange* const range = reinterpret_cast<const ColumnRange*>(P.ksum) - P.k;
+        int in = 0, uneven = 0;
+        for (int c = threadIdx.x; c < P.k; c += (int)blockDim.x) {
+            in |= !range_excluded(range[c]);
+            uneven |= range_uneven(range[c]);
+        }
+        cluster_sync_all();
+        live = __syncthreads_or(in);
+        eighth = __syncthreads_or(uneven);
+    } else {
+        __syncthreads();
     }
-    live = __syncthreads_or(live);
+    const int nm = eighth ? P.nm : 2 * (((kDigits - 1) * P.hw + 15) / 16 * 16);
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -300,8 +311,8 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
             // s8 x s8 -> s32, both operands K-major, M = 128 (pair: 256)
             const uint32_t idesc0 = (2u << 4) | (1u << 7) | (1u << 10) |
                                     ((uint32_t)((PAIR ? 2 : 1) * kTile >> 4) << 24);
-            const uint32_t idesc = idesc0 | ((uint32_t)(P.nm >> 3) << 17);
-            const uint32_t idesc_x = idesc0 | ((uint32_t)((ROWS ? P.nx : P.nm) >> 3) << 17);
+            const uint32_t idesc = idesc0 | ((uint32_t)(nm >> 3) << 17);
+            const uint32_t idesc_x = idesc0 | ((uint32_t)((ROWS ? P.nx : nm) >> 3) << 17);
             int d = 0, buf = 0;
             uint32_t ph = 0, ph_a = 0;
             bool ok = true;
@@ -540,17 +551,19 @@ k_slice_pass(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
                 for (int c0 = 0; c0 < cols; c0 += 8) {
                     const int h = c0 >= P.hw ? 1 : 0;  // single CTA: hw = w
                     const int cl = c0 - h * P.hw;
-                    const uint32_t cm = tb + h * (P.nm / 2) + cl;
+                    const uint32_t cm = tb + h * (nm / 2) + cl;
                     int64_t mh[8], ml[8], xh[8], xl[8];
                     int32_t m[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) mh[i] = ml[i] = xh[i] = xl[i] = 0;
 #pragma unroll
                     for (int p = 0; p < kDigits; ++p) {
-                        tmem_ld8i(cm + p * P.hw, m);
+                        const bool none = PAIR && p == kDigits - 1 && !eighth;
+                        if (!none) tmem_ld8i(cm + p * P.hw, m);
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            if (p < 3) mh[i] = mh[i] * 256 + m[i];
+                            if (none) ml[i] *= 256;
+                            else if (p < 3) mh[i] = mh[i] * 256 + m[i];
                             else ml[i] = ml[i] * 256 + m[i];
                         }
                     }
@@ -959,8 +972,8 @@ struct PackedRows {
 // multiply by zero, so a non-finite value reaches every output, as it does in the FP64-pipe kernels.
 // FP64 K x where every column of x is outside, ms (a value of -9999 left among normals), with the FP64-pipe kernels
 // that took such columns before, with a warp to a SNP row and a thread to a sample, and so: 50,000 x 100,000, one
-// column 7.2, 42.4, 3.3, 34 columns 58.7, 634, 30.2; 18,009 x 27,006, 34 columns 5.6, 76, 3.3, 266 columns 23.5, 462,
-// 21.4; 2,000 x 10,000, one column 0.163, 1.59, 0.053.  One of 34 columns at 50,000 x 100,000: 58.7, 59.5, 11.8.
+// column 7.2, 42.4, 3.7, 34 columns 58.7, 634, 30.4; 18,009 x 27,006, 34 columns 5.6, 76, 3.3, 266 columns 23.5, 462,
+// 21.4; 2,000 x 10,000, one column 0.163, 1.59, 0.065.  One of 34 columns at 50,000 x 100,000: 58.7, 59.5, 11.8.
 // What bounds them is the shared-memory pipe (twelve wavefronts for 16 multiply-adds a lane).
 constexpr int kDirectCols = 4;
 constexpr int kDirectRows = 1024;  // rows of a table at most, four values each; SNPs of one
