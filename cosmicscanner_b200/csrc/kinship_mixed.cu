@@ -760,8 +760,9 @@ __device__ __forceinline__ void quantise2(double v, int& q1, int& q2) {
     round_to(__dmul_rn(__dsub_rn(v, a), kBase), q2);
 }
 
-// x / d for an integer |x| <= 128 and d = 254 or 254^2: one correction of x (1 / d) gives the
-// correctly rounded quotient (true for all of these x, checked one by one).
+// x / d for an integer |x| <= 128 and d = 254 or 254^2: one correction of x (1 / d) by its remainder
+// (Markstein 1990) gives the correctly rounded quotient, as tests/test_small_quotient.py checks for each of
+// these x.
 template <int D>
 __device__ __forceinline__ double small_quotient(double x) {
     constexpr double r = 1.0 / D;
@@ -1552,10 +1553,6 @@ bool narrow_layouts() {
 bool use_cta_pairs(int64_t k) {
     const int mode = pair_mode();
     return mode != 0 && (mode == 2 || k >= kPairMinColumns) && num_sms() >= 2;
-}
-
-int blocks_for(int64_t work) {
-    return (int)std::max<int64_t>(1, std::min<int64_t>((work + 255) / 256, 16LL * num_sms()));
 }
 
 // Number of K slices so that about `target` work units cover the GPU, and at least enough that

@@ -40,7 +40,6 @@ struct Covariance {
         if (with_pe) o += vpe * in.pe;
         return o + ve * in.v;
     }
-    __device__ double operator()(int64_t r, int64_t c) const { return value(load(r, c)); }
 };
 
 namespace {
@@ -402,17 +401,6 @@ __global__ void k_records_to_rows(const double* __restrict__ V, int64_t ldv, int
     }
 }
 
-__global__ void k_combine(double* __restrict__ out, int64_t ldo, const Covariance cov, int64_t n_rec,
-                          int64_t k) {
-    chain_enter();
-    const int64_t total = n_rec * k;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = e / k, c = e - r * k;
-        out[r * ldo + c] = cov(r, c);
-    }
-}
-
 // g_out = fac * KU[row(r)], pe_out = U[row(r)]   (stcg_vce.cpp:89-101)
 __global__ void k_scatter_rows(double* __restrict__ g_out, int64_t ldg, double* __restrict__ pe_out,
                                int64_t ldp, const double* __restrict__ KU, int64_t ldk,
@@ -513,17 +501,6 @@ const double* VOperator::kinship(const double* in, int64_t ldi, int64_t k, int64
 Covariance VOperator::covariance(const double* in, int64_t ldi, const double* U, int64_t ldu, int64_t k) const {
     return Covariance{in, ku.get(), U, ldi, k, ldu, rm->identity ? nullptr : rm->d_rec_to_row.get(),
                       vg, fac, vpe, ve, with_pe ? 1 : 0};
-}
-
-void VOperator::apply(const double* in, int64_t ldi, int64_t k, double* out, int64_t ldo,
-                      cudaStream_t s) {
-    if (k <= 0) return;
-    int64_t ldu = 0;
-    const double* U = kinship(in, ldi, k, ldu, s);
-    const Covariance cov = covariance(in, ldi, U, ldu, k);
-    prof::Scope ps("covariance_combine", s, 0.0, 8.0 * 3.0 * (double)rm->n_rec * k);
-    launch_chained(k_combine, grid_for(rm->n_rec * k), 256, 0, s, out, ldo, cov, rm->n_rec, k);
-    CS_LAUNCH("covariance_combine");
 }
 
 void VOperator::apply_alpha(const double* p, int64_t k, double* out, const double* rsold, double* alpha,

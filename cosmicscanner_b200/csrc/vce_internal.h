@@ -30,10 +30,11 @@ inline void check_solver_status(cusolverStatus_t st, const char* what) {
 cublasHandle_t shared_blas();
 cusolverDnHandle_t shared_solver();
 
+struct PcgWorkspace;
+struct Covariance;  // pcg.cu
+
 // Records -> genotype rows (libCosmicCore/src/stcg_vce.cpp:17-38, 64-78).  Identity when
 // every record is its own genotype row, in order.
-struct PcgWorkspace;
-
 struct RecordMap {
     int64_t n_rec = 0, n_rows = 0;
     bool identity = true;
@@ -44,7 +45,6 @@ struct RecordMap {
 
 // V = vg * Zr K Zr^T + vpe * Zr Zr^T + ve * I on record-level blocks, with
 // K = Z Z^T / divisor (stcg_vce.cpp:80-115).
-struct Covariance;  // pcg.cu
 struct VOperator {
     cs_kinship* op = nullptr;
     const RecordMap* rm = nullptr;
@@ -56,13 +56,11 @@ struct VOperator {
     int64_t applies = 0;     // kinship applies issued
     int64_t apply_cols = 0;  // right-hand sides they carried
 
-    // out (n_rec x ldo) = V * in (n_rec x ldi), k columns.
-    void apply(const double* in, int64_t ldi, int64_t k, double* out, int64_t ldo, cudaStream_t s);
     // ku = K Zr^T in (n_rows x k), the genetic part of V in; returns Zr^T in (n_rows x ldu).
     const double* kinship(const double* in, int64_t ldi, int64_t k, int64_t& ldu, cudaStream_t s);
     // V in, element by element, from what kinship(in) made.
     Covariance covariance(const double* in, int64_t ldi, const double* U, int64_t ldu, int64_t k) const;
-    // The same for CG (out = V p), with alpha[c] = rsold[c] / (p . V p)[c].
+    // out = V p (n_rec x k, row-major) for CG, with alpha[c] = rsold[c] / (p . V p)[c].
     void apply_alpha(const double* p, int64_t k, double* out, const double* rsold, double* alpha,
                      PcgWorkspace& ws, cudaStream_t s);
     // g_out = Zr K Zr^T in (dV/d sigma2_g); pe_out (optional) = Zr Zr^T in.
