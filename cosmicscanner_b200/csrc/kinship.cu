@@ -175,8 +175,8 @@ cs_kinship* kinship_create(const cs_genotypes* g, const int32_t* keep, int64_t n
     return op;
 }
 
-// FP64 form: U = Z^T X (pass over rows), Y = Z U / M (pass over samples).
-static void kinship_apply_fp64(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* Y,
+// FP64 form on the FP64 pipe: U = Z^T X (pass over rows), Y = Z U / M (pass over samples).
+static void kinship_apply_pipe(cs_kinship* op, const double* X, int64_t ldx, int64_t k, double* Y,
                                int64_t ldy, cudaStream_t s) {
     const int64_t R = op->n_active;
     const double scale = 1.0 / (double)op->num_variants;
@@ -185,7 +185,6 @@ static void kinship_apply_fp64(cs_kinship* op, const double* X, int64_t ldx, int
         CS_CUDA(cudaMemset2DAsync(Y, ldy * 8, 0, k * 8, op->rows, s));
         return;
     }
-    if (kinship_apply_slices(op, StridedIn{X, ldx, 1}, k, StridedOut{Y, ldy, 1}, s)) return;
     op->buf_u.resize(R * k);
     decode_gemm_rows_fp64(op->view, op->d_lut.get(), X, ldx, k, op->buf_u.get(), k, op->ws, s);
     decode_gemm_samples_fp64(op->view, op->d_lut.get(), op->buf_u.get(), k, k, Y, ldy, scale,
@@ -197,10 +196,10 @@ void kinship_apply_rowmajor(cs_kinship* op, const double* X, int64_t ldx, int64_
     if (k <= 0) return;
     if (precision == CS_PRECISION_MIXED)
         kinship_apply_mixed(op, StridedIn{X, ldx, 1}, k, StridedOut{Y, ldy, 1}, s);
-    else if (precision == CS_PRECISION_FP64)
-        kinship_apply_fp64(op, X, ldx, k, Y, ldy, s);
-    else
+    else if (precision != CS_PRECISION_FP64)
         fail(CS_ERR_INVALID_ARGUMENT, "unknown precision mode");
+    else if (!kinship_apply_slices(op, StridedIn{X, ldx, 1}, k, StridedOut{Y, ldy, 1}, s))
+        kinship_apply_pipe(op, X, ldx, k, Y, ldy, s);
 }
 
 // FP32 column-major (ld) <-> FP64 row-major (n x k) around the FP32 entry point.
@@ -282,18 +281,18 @@ void kinship_apply_colmajor(cs_kinship* op, const double* X, int64_t ldx, int64_
     if (ldx < op->rows || ldy < op->rows)
         fail(CS_ERR_INVALID_ARGUMENT, "PlinkKinshipOperator::apply: dimension mismatch");
     const int64_t n = op->rows;
-    if (precision == CS_PRECISION_MIXED || precision == CS_PRECISION_FP64) {
-        const StridedIn x = apart(op, X, ldx, n, Y, ldy, n, k, true, s);
-        if (precision == CS_PRECISION_MIXED) {
-            kinship_apply_mixed(op, x, k, StridedOut{Y, 1, ldy}, s);
-            return;
-        }
-        if (kinship_apply_slices(op, x, k, StridedOut{Y, 1, ldy}, s)) return;
+    if (precision != CS_PRECISION_MIXED && precision != CS_PRECISION_FP64)
+        fail(CS_ERR_INVALID_ARGUMENT, "unknown precision mode");
+    const StridedIn x = apart(op, X, ldx, n, Y, ldy, n, k, true, s);
+    if (precision == CS_PRECISION_MIXED) {
+        kinship_apply_mixed(op, x, k, StridedOut{Y, 1, ldy}, s);
+        return;
     }
+    if (kinship_apply_slices(op, x, k, StridedOut{Y, 1, ldy}, s)) return;
     op->buf_x.resize(n * k);
     op->buf_y.resize(n * k);
     colmajor_to_rowmajor(X, ldx, n, k, op->buf_x.get(), k, s);
-    kinship_apply_rowmajor(op, op->buf_x.get(), k, k, op->buf_y.get(), k, precision, s);
+    kinship_apply_pipe(op, op->buf_x.get(), k, k, op->buf_y.get(), k, s);
     rowmajor_to_colmajor(op->buf_y.get(), k, n, k, Y, ldy, s);
 }
 

@@ -3,8 +3,10 @@
 #include <cuda_runtime.h>
 #include <cusolverDn.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
+#include <cstring>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -39,11 +41,20 @@ bool poison_allocations() {
     return on;
 }
 
-// CS_B200_ALLOC_LIMIT=bytes refuses larger blocks as a full device would; read at each allocation, so
-// that a test can take it back.
-size_t alloc_limit() {
-    const char* v = std::getenv("CS_B200_ALLOC_LIMIT");
-    return v && *v ? (size_t)std::strtoull(v, nullptr, 10) : SIZE_MAX;
+// CS_B200_ALLOC_LIMIT=bytes:count refuses the process's first `count` blocks above a size as a full device
+// would, for tests of what callers do then and when there is room again.
+bool refuse_allocation(size_t bytes) {
+    static size_t limit = SIZE_MAX;
+    static std::atomic<long long> left{0};
+    static const bool set = [] {
+        const char* v = std::getenv("CS_B200_ALLOC_LIMIT");
+        const char* c = v ? std::strchr(v, ':') : nullptr;
+        if (!c) return false;
+        limit = (size_t)std::strtoull(v, nullptr, 10);
+        left = std::atoll(c + 1);
+        return true;
+    }();
+    return set && bytes > limit && left.fetch_sub(1) > 0;
 }
 
 thread_local cublasHandle_t t_blas[kMaxDevices] = {};
@@ -90,7 +101,7 @@ void* device_alloc(size_t bytes) {
     CS_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < kMaxDevices) prepare_pool(dev);
     void* p = nullptr;
-    const bool refused = bytes > alloc_limit();
+    const bool refused = refuse_allocation(bytes);
     cudaError_t e = refused ? cudaErrorMemoryAllocation : cudaMallocAsync(&p, bytes, 0);
     if (e == cudaErrorMemoryAllocation && !refused) {
         // The pool keeps freed blocks reserved; when the device has no room left for a new
