@@ -931,9 +931,9 @@ def main():
         f_ms = ftop["ms"] / ftop["launches"]
         f_ach = ftop["flops"] / ftop["launches"] / (f_ms * 1e-3) / 1e12
         if "_slices" in ftop["name"]:
-            # eight int8 digits a column: 15 (rows) or 16 (samples) int8 products for each of the
-            # algorithmic ones
-            f_sets = 15 if "rows" in ftop["name"] else 16
+            # seven int8 digits of an even column on CTA pairs (the eighth has no MMAs): 7 + 7 int8
+            # products for each of the algorithmic ones in either pass
+            f_sets = 14
             fpeaks, fkind = measured_peaks()
             f_peak = fpeaks["bf16_tflops"]
             f_roof = {"bound": "tensor", "peak_kind": f"bf16_tflops ({fkind})",
