@@ -976,7 +976,7 @@ struct PackedRows {
 // 21.4; 2,000 x 10,000, one column 0.163, 1.59, 0.065.  One of 34 columns at 50,000 x 100,000: 58.7, 59.5, 11.8.
 // What bounds them is the shared-memory pipe (twelve wavefronts for 16 multiply-adds a lane).
 constexpr int kDirectCols = 4;
-constexpr int kDirectRows = 1024;  // rows of a table at most, four values each; SNPs of one
+constexpr int kDirectRows = 1024;  // SNPs of a table: of direct_rows at most, of direct_samples
 constexpr int kDirectSnps = 512;
 
 // The columns that a block of column c takes: c and the next excluded ones where c is the first, fifth, ..
@@ -1034,7 +1034,7 @@ __device__ __forceinline__ void direct_rows(const PackedRows& G, int64_t t0, int
         buf[e] = e % rpb < rows ? centred((uint32_t)(e / rpb), mu[t0 + e % rpb]) : 0.0;
     __syncthreads();
     const uint8_t* const src = G.rows + t0 * G.stride;
-    uint32_t row_at[4];  // at most 1024 rows further
+    uint32_t row_at[4];  // below 2^32: finish_rows
 #pragma unroll
     for (int i = 0; i < 4; ++i) row_at[i] = (uint32_t)min(grp + groups * i, rows - 1) * (uint32_t)G.stride;
     // 256 samples at a time, `here` of them to a part: x read by one thread a sample while the ones before
@@ -1691,10 +1691,11 @@ void run_samples(SliceOperator& so, MixedRows& r, const SliceCall& c, const Slic
 void finish_rows(SliceOperator& so, MixedRows& r, const SliceCall& c, const SliceSums& S, StridedIn X,
                  double* Wt, const int32_t* pos, StridedOut out, cudaStream_t s) {
     prof::Scope ps("slice_reduce_rows", s, 0.0, 8.0 * (c.rows.splits + 1) * (double)c.k * r.R);
-    // as many rows a block as leave two blocks for every SM if all columns are summed directly
+    // as many rows a block as leave two blocks for every SM if all columns are summed directly, and within
+    // 32-bit offsets (four million bytes a row, sixteen million samples, before that binds)
     const int64_t groups = (c.k + kDirectCols - 1) / kDirectCols;
     int rpb = kDirectRows;
-    while (rpb > 64 && (r.R + rpb - 1) / rpb * groups < 2 * num_sms()) rpb /= 4;
+    while (rpb > 64 && ((r.R + rpb - 1) / rpb * groups < 2 * num_sms() || rpb * r.stride >> 32)) rpb /= 4;
     launch_chained(k_slice_reduce_rows, dim3((unsigned)((r.R + rpb - 1) / rpb), (unsigned)c.k), 256, 0, s,
                    so.part.get(), r.r_pad, r.R, c.k, rpb, r.s.get(), r.mu.get(), PackedRows{r.rows, r.stride}, X,
                    r.n, S, Wt, pos, out);
